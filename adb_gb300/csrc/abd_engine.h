@@ -254,10 +254,12 @@ struct NewtonBufs {
   DBuf<int> grp_body, grp_n, grp_scene, sc_gbeg, sc_gend;  // PCG body groups (pcg_groups)
   std::vector<int> h_sc_beg, h_sc_end;  // body range of each scene (host)
   DBuf<double> dense_A, dense_y;         // dense solve: one scene's matrix and right-hand side
-  // block-tridiagonal direct solve: per-scene flags and counts, per-body link to the next
-  // body, the factor's inverse diagonal blocks, coupling blocks and forward solution
-  DBuf<int> tri_bad, tri_on, pcg_on, tri_cnt, tri_link;
+  // block-tridiagonal direct solve: per-scene flags and counts, the bodies by elimination
+  // level (tri_levels), per-body coupling flags, the factor's inverse diagonal blocks,
+  // coupling blocks and forward solution
+  DBuf<int> tri_bad, tri_on, pcg_on, tri_cnt, tri_lv_body, tri_lv_off, tri_fl;
   DBuf<double> tri_Li, tri_W, tri_y;
+  int tri_nlev = 0, tri_width = 0;       // levels, bodies of the first (largest) one
   // adjoint: friction-frame Jacobians and contributions per pair, the exact system's
   // blocks, GMRES bases
   DBuf<double> fj_pt, fj_ee, fc_pt, fc_ee, D_ex, ovr_ex, adj_V, adj_Z, adj_w, adj_t, adj_x;
@@ -299,9 +301,10 @@ int pcg_solve(const Geo& g, PairSet& S, NewtonBufs& nb, const SolveOpts& o, cons
               const std::vector<char>& on, double* dq, cudaStream_t s, int* status, int* scene_iters);
 // Block-tridiagonal scenes (tri.cu; after the row-block copy of pcg_solve): tri_classify
 // marks the scenes whose blocks only join consecutive bodies (tri_on, when enable) and the
-// others solved (pcg_on), returning both counts; tri_solve factorizes and solves every run
-// of linked bodies of the tri_on scenes (x, dq = -x) and writes x = 0, dq = -0 for the
-// scenes with sc_on == 0.
+// others solved (pcg_on), returning both counts; tri_solve factorizes and solves the tri_on
+// scenes (x, dq = -x) and writes x = 0, dq = -0 for the scenes with sc_on == 0. tri_levels
+// (once per handle) lists the bodies by elimination level.
+void tri_levels(const std::vector<int>& sc_beg, const std::vector<int>& sc_end, NewtonBufs& nb, cudaStream_t s);
 void tri_classify(const Geo& g, PairSet& S, NewtonBufs& B, int enable, const int* sc_on, cudaStream_t s,
                   int* n_pcg, int* n_tri);
 void tri_solve(const Geo& g, PairSet& S, NewtonBufs& B, const int* sc_on, double* dq, cudaStream_t s);

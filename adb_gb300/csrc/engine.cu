@@ -165,6 +165,9 @@ struct Engine {
     nbufs.e_out.release(); nbufs.red.release(); nbufs.status.release();
     nbufs.xr.release(); nbufs.rt.release(); nbufs.dqc.release(); nbufs.it_ref.release();
     nbufs.dense_A.release(); nbufs.dense_y.release();
+    nbufs.tri_bad.release(); nbufs.tri_on.release(); nbufs.pcg_on.release(); nbufs.tri_cnt.release();
+    nbufs.tri_lv_body.release(); nbufs.tri_lv_off.release(); nbufs.tri_fl.release();
+    nbufs.tri_Li.release(); nbufs.tri_W.release(); nbufs.tri_y.release();
     nbufs.fj_pt.release(); nbufs.fj_ee.release(); nbufs.fc_pt.release(); nbufs.fc_ee.release();
     nbufs.D_ex.release(); nbufs.ovr_ex.release(); nbufs.has_ex.release(); nbufs.adj_V.release();
     nbufs.adj_Z.release(); nbufs.adj_w.release(); nbufs.adj_t.release(); nbufs.adj_x.release();
@@ -309,6 +312,7 @@ struct Engine {
     upload(sc_beg, h_sc_beg.data(), ns);
     upload(sc_end, h_sc_end.data(), ns);
     abd::pcg_groups(h_sc_beg, h_sc_end, nbufs, s);
+    abd::tri_levels(h_sc_beg, h_sc_end, nbufs, s);
     sc_on.ensure(ns);
     sc_alpha.ensure(ns);
     sc_factor.ensure(ns);

@@ -1,44 +1,53 @@
 // Direct solve of block-tridiagonal scenes (chains, stacks): the Newton matrix of a scene
 // whose contacts only join consecutive bodies is block-tridiagonal in body order. The
 // reference solves every Newton system with a sparse direct factorization (Pardiso LLT,
-// model/abd.cpp:233-264), which on such a matrix is a block Cholesky along the bodies;
-// here each run of linked bodies (a maximal sequence i, i+1, ... with a contact block
-// between each neighbour pair) is factorized and solved by one CTA:
+// model/abd.cpp:233-264); here it is a block Cholesky in odd-even (cyclic reduction) order.
+// With i the body's place in its scene, counted from 1, the bodies whose i has l trailing
+// zero bits are eliminated at level l, all of them at once: their neighbours still present
+// are i - 2^l and i + 2^l. With the couplings U_- and U_+ to those,
 //
-//   S_0 = D_0,  S_k = D_k - W_{k-1}^T W_{k-1},  S_k = L_k L_k^T,  W_k = L_k^-1 U_k
-//   (U_k = H[k][k+1]);  y_k = L_k^-1 (b_k - W_{k-1}^T y_{k-1});
-//   x_last = L_last^-T y_last,  x_k = L_k^-T (y_k - W_k x_{k+1}).
+//   S = D - sum over the neighbours eliminated at levels m < l of W^T W,   S = L L^T,
+//   W_- = L^-1 U_-,  W_+ = L^-1 U_+,  y = L^-1 (b - sum of W^T y),
 //
-// Runs are independent, so a chain broken into segments by missing contacts solves in
-// parallel; a body without neighbours is a run of one. The preconditioned CG keeps the
-// other scenes. Every sum runs in a fixed order, and a run's arithmetic depends only on
-// its own blocks, so a scene gets the same solution in a batch as alone.
+// a level l > 0 coupling being -W_-^T W_+ of the body half-way, and from the last level back
+//   x = L^-T (y - W_- x_- - W_+ x_+).
+//
+// What bounds it: the dependent FP64 chain of one 12 x 12 factorization and the chain of
+// loads before it. In body order a chain of n links is n of them, one after the other on one
+// SM; by levels it is log2 n, at about twice the operations. Measured per solve, in body
+// order and by levels: 200 links in contact 2.49 -> 0.26 ms, 256 columns (8212 bodies in all)
+// 1.83 -> 0.62 ms, a stack of ten 0.117 -> 0.091 ms.
+// Couplings that are absent (runs broken by missing contacts) are flagged and cost nothing.
+// Every sum runs in a fixed order, and a body's arithmetic depends only on its own scene and
+// its place there, so a scene gets the same solution in a batch as alone.
+#include <cooperative_groups.h>
+
+#include <vector>
+
 #include "abd_engine.h"
+
+namespace cg = cooperative_groups;
 
 namespace abd {
 namespace {
 
-constexpr int TNT = 160;  // threads per run: 144 for the 12 x 12 entries, lanes for the rest
+constexpr int TNT = 160;  // threads per body: 144 for the 12 x 12 entries, 12 for the right-hand side
+constexpr int TWARPS = TNT / 32;
 
 inline int nblk_t(long long n, int t) { return (int)((n + t - 1) / t); }
 
-// Flags of the block structure from the row-block copy of the system (k_pcg_rows: per body
-// its diagonal block, then the neighbour blocks that hold a contribution): link[i] = 1 when
-// body i has a block with body i + 1; a scene with any block between bodies further apart
-// is marked in bad[scene].
-__global__ void k_tri_mark(int nb, const int* row_ptr, const int* rcol, const int* rn, const int* bscene, int* link,
-                           int* bad) {
+// Marks in bad[scene] the scenes with a block between bodies that are not consecutive, from
+// the row-block copy of the system (k_pcg_rows: per body its diagonal block, then the
+// neighbour blocks that hold a contribution).
+__global__ void k_tri_mark(int nb, const int* row_ptr, const int* rcol, const int* rn, const int* bscene, int* bad) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nb) return;
   const int base = i + row_ptr[i], n = rn[i];
-  int l = 0;
   bool far = false;
   for (int j = 1; j < n; ++j) {
     const int c = rcol[base + j];
-    if (c == i + 1) l = 1;
-    else if (c != i - 1) far = true;
+    far |= c != i + 1 && c != i - 1;
   }
-  link[i] = l;
   if (far) atomicOr(&bad[bscene[i]], 1);
 }
 
@@ -57,10 +66,14 @@ __global__ void k_tri_masks(int ns, int enable, const int* sc_on, const int* bad
 struct TriArgs {
   const int *row_ptr, *rcol, *rn;
   const double* Hrow;
-  const int *bscene, *sc_on, *tri_on, *link;
+  const int *bscene, *sc_end, *sc_on, *tri_on;
   const double* b;
-  double *Li, *W, *y;  // per body: inverse of the factor's diagonal block, coupling block, forward solution
+  double *Li, *W, *y;  // per body: inverse of the factor's diagonal block, the two coupling blocks
+                       // (towards lower and higher bodies), forward solution
   double *x, *dq;
+  int* fl;             // per body: bit 0 / 1 = coupled to a lower / higher body when eliminated
+  const int *lv_body, *lv_off;  // bodies by level (lv_off: nlev + 1)
+  int nlev;
   int* status;
 };
 
@@ -76,142 +89,184 @@ __device__ __forceinline__ void tri_pivot(double a, double* r, double* lkk, int*
   *lkk = a * q;
 }
 
-// One CTA per body; the CTA of the first body of each run in a directly solved scene
-// factorizes and solves the run. Bodies of scenes that take no step get x = 0, dq = -0
-// (what the CG writes for them).
+// acc += sum over r of P[r][i] Q[r], Q read with stride qs (a column of a 12 x 12 block: 12,
+// a vector: 1).
+__device__ __forceinline__ double tri_dot_t(const double* P, int i, const double* Q, int qs, double acc) {
+#pragma unroll
+  for (int r = 0; r < 12; ++r) acc += P[12 * r + i] * Q[qs * r];
+  return acc;
+}
+
+// One cooperative launch: the levels of the elimination in order with a grid barrier after
+// each, then the back substitution from the last level to the first. A CTA eliminates one
+// body at a time.
 //
-// A link's 12 x 12 work is spread over 144 threads (thread (i, j) = (t / 12, t % 12)),
-// because on this part a dependent FP64 instruction of one warp waits ~64 cycles: the
-// Cholesky factor is right-looking, one barrier per column (the column scaled and the
-// trailing triangle updated in the same phase; the thread that updates the next pivot takes
-// its reciprocal square root), and row c of L^-1, which needs L's column c, is formed one
-// phase later by the threads of columns <= c, which the factorization no longer uses. The
-// next link's diagonal block and right-hand side are loaded while this one factorizes.
+// The 12 x 12 work of a body is spread over 156 threads (thread t < 144: entry (t / 12,
+// t % 12); 144..155: the right-hand side as a 13th column), because on this part a dependent
+// FP64 instruction of one warp waits ~64 cycles: the Cholesky factor is right-looking, one
+// barrier per column (the column scaled and the trailing triangle updated in the same
+// phase; the thread that updates the next pivot takes its reciprocal square root), and row
+// c of L^-1, which needs L's column c, is formed one phase later by the threads of columns
+// <= c, which the factorization no longer uses.
 __global__ void __launch_bounds__(TNT) k_tri_solve(TriArgs a) {
-  __shared__ double sA[12][13], sL[12][13], sT[12][13], sLi[12][13], sW[12][13], sU[12][13];
-  __shared__ double sy[12], st[12], sx[12], sv[12], sR[12];
-  __shared__ int s_u;
-  const int b0 = blockIdx.x, t = threadIdx.x;
-  const int sc = a.bscene[b0];
-  if (!a.sc_on[sc]) {
-    if (t < 12) {
-      a.x[12 * b0 + t] = 0.0;
-      a.dq[12 * b0 + t] = -0.0;
-    }
-    return;
-  }
-  if (!a.tri_on[sc]) return;
-  if (b0 > 0 && a.bscene[b0 - 1] == sc && a.link[b0 - 1]) return;  // not the first body of its run
-  const bool act = t < 144;
-  const int ei = t / 12, ej = t - 12 * (t / 12);
-  int k = b0;
-  int base = k + a.row_ptr[k];
-  // this link's diagonal entries (i, j), (j, i) and right-hand side entry
-  double d_ij = act ? a.Hrow[(size_t)base * 144 + 12 * ei + ej] : 0.0;
-  double d_ji = act ? a.Hrow[(size_t)base * 144 + 12 * ej + ei] : 0.0;
-  double b_t = t < 12 ? a.b[12 * k + t] : 0.0;
-  for (;;) {
-    if (t == 0) {
-      // the coupling block to body k + 1 in k's row list (rows of k, columns of k + 1)
-      int u = -1;
-      if (a.link[k]) {
+  cg::grid_group grid = cg::this_grid();
+  __shared__ double sA[12][13], sL[12][13], sT[12][13], sLi[12][13], sU[2][12][13];
+  __shared__ double st[12], sR[12];
+  const int t = threadIdx.x;
+  const bool ent = t < 144, act = t < 156;
+  const int ei = ent ? t / 12 : (act ? t - 144 : 0), ej = ent ? t - 12 * (t / 12) : 12;
+  for (int l = 0; l < a.nlev; ++l) {
+    const int h = 1 << l, hh = h >> 1;
+    for (int it = a.lv_off[l] + blockIdx.x; it < a.lv_off[l + 1]; it += gridDim.x) {
+      const int k = a.lv_body[it];
+      const int sc = a.bscene[k];
+      if (!a.sc_on[sc] || !a.tri_on[sc]) continue;
+      const int end = a.sc_end[sc];
+      const int base = k + a.row_ptr[k];
+      // the two couplings: blocks of the matrix at level 0, else minus the product of the
+      // two coupling blocks of the body half-way (eliminated one level earlier)
+      int cl = 0, cr = 0;  // coupled; at level 0 the slot of the block in k's row list
+      if (l == 0) {
         const int n = a.rn[k];
-        for (int j = 1; j < n; ++j)
-          if (a.rcol[base + j] == k + 1) u = base + j;
-      }
-      s_u = u;
-    }
-    // S_k = sym(D_k) - W_{k-1}^T W_{k-1}; right-hand side b_k - W_{k-1}^T y_{k-1}
-    if (act) {
-      double v = 0.5 * (d_ij + d_ji);
-      if (k > b0) {
-#pragma unroll
-        for (int m = 0; m < 12; ++m) v -= sW[m][ei] * sW[m][ej];
-      }
-      sA[ei][ej] = v;
-      sT[ei][ej] = ei == ej ? 1.0 : 0.0;
-      if (t == 0) tri_pivot(v, &sR[0], &sL[0][0], a.status);
-    }
-    if (t < 12) {
-      double v = b_t;
-      if (k > b0) {
-#pragma unroll
-        for (int m = 0; m < 12; ++m) v -= sW[m][t] * sy[m];
-      }
-      st[t] = v;
-    }
-    __syncthreads();
-    const int u = s_u;
-    if (act && u >= 0) {
-      sU[ei][ej] = a.Hrow[(size_t)u * 144 + t];
-      // the next link's block and right-hand side, in flight during the factorization
-      base = (k + 1) + a.row_ptr[k + 1];
-      d_ij = a.Hrow[(size_t)base * 144 + 12 * ei + ej];
-      d_ji = a.Hrow[(size_t)base * 144 + 12 * ej + ei];
-      if (t < 12) b_t = a.b[12 * (k + 1) + t];
-    }
-    // S = L L^T column by column (threads of columns >= c); row c - 1 of L^-1 beside it
-    // (threads of columns <= c - 1). T holds I minus the finished rows' contributions.
-    for (int c = 0; c <= 12; ++c) {
-      if (act && c < 12 && ej >= c && ei >= ej) {
-        const double r = sR[c];
-        if (ej == c) {
-          if (ei > c) sL[ei][c] = sA[ei][c] * r;
-        } else {
-          const double v = sA[ei][ej] - (sA[ei][c] * r) * (sA[ej][c] * r);
-          sA[ei][ej] = v;
-          if (ei == ej && ej == c + 1) tri_pivot(v, &sR[c + 1], &sL[c + 1][c + 1], a.status);
+        for (int j = 1; j < n; ++j) {
+          const int c = a.rcol[base + j];
+          if (c == k - 1) cl = base + j;
+          if (c == k + 1) cr = base + j;
         }
+      } else {
+        cl = a.fl[k - hh] == 3;
+        cr = k + hh < end && a.fl[k + hh] == 3;
       }
-      if (act && c >= 1 && ej <= c - 1 && ei >= c - 1) {
-        const int rw = c - 1;
-        const double l = sT[rw][ej] * sR[rw];
-        if (ei == rw) sLi[rw][ej] = l;
-        else sT[ei][ej] -= sL[ei][rw] * l;
+      double v = 0.0, ul = 0.0, ur = 0.0;
+      if (ent) {
+        const double* Hd = a.Hrow + (size_t)base * 144;
+        v = 0.5 * (Hd[t] + Hd[12 * ej + ei]);
+        if (l == 0) {
+          if (cl) ul = a.Hrow[(size_t)cl * 144 + t];
+          if (cr) ur = a.Hrow[(size_t)cr * 144 + t];
+        } else {
+          if (cl) {
+            const double* Wm = a.W + (size_t)288 * (k - hh);
+            ul = -tri_dot_t(Wm + 144, ei, Wm + ej, 12, 0.0);
+          }
+          if (cr) {
+            const double* Wm = a.W + (size_t)288 * (k + hh);
+            ur = -tri_dot_t(Wm, ei, Wm + 144 + ej, 12, 0.0);
+          }
+        }
+      } else if (act) {
+        v = a.b[12 * k + ei];
+      }
+      // the Schur complement: the bodies eliminated next to this one at the earlier levels
+      if (act) {
+        double accl = 0.0, accr = 0.0;
+        for (int m = 0; m < l; ++m) {
+          const int kl = k - (1 << m), kr = k + (1 << m);
+          if (a.fl[kl] & 2) {
+            const double* Wr = a.W + (size_t)288 * kl + 144;
+            accl = tri_dot_t(Wr, ei, ent ? Wr + ej : a.y + 12 * kl, ent ? 12 : 1, accl);
+          }
+          if (kr < end && (a.fl[kr] & 1)) {
+            const double* Wl = a.W + (size_t)288 * kr;
+            accr = tri_dot_t(Wl, ei, ent ? Wl + ej : a.y + 12 * kr, ent ? 12 : 1, accr);
+          }
+        }
+        v -= accl + accr;
+      }
+      __syncthreads();  // the previous body's shared blocks are no longer read
+      if (ent) {
+        sA[ei][ej] = v;
+        sT[ei][ej] = ei == ej ? 1.0 : 0.0;
+        sU[0][ei][ej] = ul;
+        sU[1][ei][ej] = ur;
+        if (t == 0) tri_pivot(v, &sR[0], &sL[0][0], a.status);
+      } else if (act) {
+        st[ei] = v;
       }
       __syncthreads();
-    }
-    // y_k = L^-1 rhs, W_k = L^-1 U_k (L^-1 lower triangular)
-    if (t < 12) {
-      double v = 0.0;
-      for (int m = 0; m <= t; ++m) v += sLi[t][m] * st[m];
-      sy[t] = v;
-      a.y[12 * k + t] = v;
-    }
-    if (act) {
-      a.Li[(size_t)144 * k + t] = ej <= ei ? sLi[ei][ej] : 0.0;
-      if (u >= 0) {
-        double v = 0.0;
-        for (int m = 0; m <= ei; ++m) v += sLi[ei][m] * sU[m][ej];
-        sW[ei][ej] = v;
-        a.W[(size_t)144 * k + t] = v;
+      // S = L L^T column by column (threads of columns >= c); row c - 1 of L^-1 beside it
+      // (threads of columns <= c - 1). T holds I minus the finished rows' contributions.
+      for (int c = 0; c <= 12; ++c) {
+        if (ent && c < 12 && ej >= c && ei >= ej) {
+          const double r = sR[c];
+          if (ej == c) {
+            if (ei > c) sL[ei][c] = sA[ei][c] * r;
+          } else {
+            const double w = sA[ei][ej] - (sA[ei][c] * r) * (sA[ej][c] * r);
+            sA[ei][ej] = w;
+            if (ei == ej && ej == c + 1) tri_pivot(w, &sR[c + 1], &sL[c + 1][c + 1], a.status);
+          }
+        }
+        if (ent && c >= 1 && ej <= c - 1 && ei >= c - 1) {
+          const int rw = c - 1;
+          const double li = sT[rw][ej] * sR[rw];
+          if (ei == rw) sLi[rw][ej] = li;
+          else sT[ei][ej] -= sL[ei][rw] * li;
+        }
+        __syncthreads();
+      }
+      // y = L^-1 rhs, W = L^-1 U for both couplings (L^-1 lower triangular)
+      if (ent) {
+        a.Li[(size_t)144 * k + t] = ej <= ei ? sLi[ei][ej] : 0.0;
+        double wl = 0.0, wr = 0.0;
+        if (cl || cr)
+          for (int m = 0; m <= ei; ++m) {
+            const double li = sLi[ei][m];
+            wl += li * sU[0][m][ej];
+            wr += li * sU[1][m][ej];
+          }
+        if (cl) a.W[(size_t)288 * k + t] = wl;
+        if (cr) a.W[(size_t)288 * k + 144 + t] = wr;
+        if (t == 0) a.fl[k] = (cl ? 1 : 0) | (cr ? 2 : 0);
+      } else if (act) {
+        double w = 0.0;
+        for (int m = 0; m <= ei; ++m) w += sLi[ei][m] * st[m];
+        a.y[12 * k + ei] = w;
       }
     }
-    __syncthreads();
-    if (u < 0) break;
-    ++k;
+    grid.sync();
   }
-  // back substitution from the last body of the run
-  for (int kk = k; kk >= b0; --kk) {
-    if (t < 12) {
-      double v = a.y[12 * kk + t];
-      if (kk < k) {
-        const double* W = a.W + (size_t)144 * kk;
-#pragma unroll
-        for (int m = 0; m < 12; ++m) v -= W[12 * t + m] * sx[m];
+  // back substitution, one warp per body: lanes 0..11 the rows' lower coupling, lanes
+  // 16..27 the upper one, then x = L^-T v with the even terms on the low half, the odd ones
+  // on the high half. Bodies of scenes that take no step get x = 0, dq = -0.
+  const int w = t >> 5, lane = t & 31, row = lane & 15, side = lane >> 4;
+  const bool rl = row < 12;
+  for (int l = a.nlev - 1; l >= 0; --l) {
+    const int h = 1 << l;
+    for (int it = a.lv_off[l] + blockIdx.x * TWARPS + w; it < a.lv_off[l + 1]; it += gridDim.x * TWARPS) {
+      const int k = a.lv_body[it];
+      const int sc = a.bscene[k];
+      if (!a.sc_on[sc]) {
+        if (lane < 12) {
+          a.x[12 * k + lane] = 0.0;
+          a.dq[12 * k + lane] = -0.0;
+        }
+        continue;
       }
-      sv[t] = v;
+      if (!a.tri_on[sc]) continue;
+      double v = rl && side == 0 ? a.y[12 * k + row] : 0.0;
+      const int f = a.fl[k];
+      if (rl && (f & (1 << side))) {
+        const double* W = a.W + (size_t)288 * k + 144 * side + 12 * row;
+        const double* xn = a.x + 12 * (side ? k + h : k - h);
+#pragma unroll
+        for (int m = 0; m < 12; ++m) v -= W[m] * xn[m];
+      }
+      v += __shfl_xor_sync(0xffffffffu, v, 16);
+      const double* Li = a.Li + (size_t)144 * k;
+      double xv = 0.0;
+#pragma unroll
+      for (int m = 0; m < 12; m += 2) {
+        const double vm = __shfl_sync(0xffffffffu, v, m + side);
+        if (rl) xv += Li[12 * (m + side) + row] * vm;
+      }
+      xv += __shfl_xor_sync(0xffffffffu, xv, 16);
+      if (lane < 12) {
+        a.x[12 * k + lane] = xv;
+        a.dq[12 * k + lane] = -xv;
+      }
     }
-    __syncthreads();
-    if (t < 12) {
-      const double* Li = a.Li + (size_t)144 * kk;
-      double v = 0.0;
-      for (int m = t; m < 12; ++m) v += Li[12 * m + t] * sv[m];
-      a.x[12 * kk + t] = v;
-      a.dq[12 * kk + t] = -v;
-      sx[t] = v;
-    }
-    __syncthreads();
+    if (l > 0) grid.sync();
   }
 }
 
@@ -224,11 +279,10 @@ void tri_classify(const Geo& g, PairSet& S, NewtonBufs& B, int enable, const int
   B.tri_on.ensure(ns);
   B.pcg_on.ensure(ns);
   B.tri_cnt.ensure(2);
-  B.tri_link.ensure(nb);
   CK(cudaMemsetAsync(B.tri_bad.p, 0, ns * sizeof(int), s));
   CK(cudaMemsetAsync(B.tri_cnt.p, 0, 2 * sizeof(int), s));
   KLAUNCH(K_BLOCK_INVERSE, s, k_tri_mark<<<nblk_t(nb, 256), 256, 0, s>>>(nb, S.row_ptr.p, B.rcol.p, B.rn.p, g.bscene,
-                                                                       B.tri_link.p, B.tri_bad.p));
+                                                                       B.tri_bad.p));
   KLAUNCH(K_BLOCK_INVERSE, s, k_tri_masks<<<nblk_t(ns, 256), 256, 0, s>>>(ns, enable, sc_on, B.tri_bad.p, B.tri_on.p,
                                                                         B.pcg_on.p, B.tri_cnt.p));
   CK(cudaMemcpyAsync(B.h_int + 8, B.tri_cnt.p, 2 * sizeof(int), cudaMemcpyDeviceToHost, s));
@@ -237,17 +291,53 @@ void tri_classify(const Geo& g, PairSet& S, NewtonBufs& B, int enable, const int
   *n_tri = B.h_int[9];
 }
 
+void tri_levels(const std::vector<int>& sc_beg, const std::vector<int>& sc_end, NewtonBufs& B, cudaStream_t s) {
+  std::vector<std::vector<int>> lv;
+  for (size_t k = 0; k < sc_beg.size(); ++k)
+    for (int b = sc_beg[k]; b < sc_end[k]; ++b) {
+      size_t l = 0;
+      for (unsigned i = (unsigned)(b - sc_beg[k]) + 1u; !(i & 1u); i >>= 1) ++l;
+      if (lv.size() <= l) lv.resize(l + 1);
+      lv[l].push_back(b);
+    }
+  std::vector<int> body, off{0};
+  for (auto& v : lv) {
+    body.insert(body.end(), v.begin(), v.end());
+    off.push_back((int)body.size());
+  }
+  B.tri_nlev = (int)lv.size();
+  B.tri_width = lv.empty() ? 0 : (int)lv[0].size();
+  B.tri_lv_body.ensure(body.size() + 1);
+  B.tri_lv_off.ensure(off.size());
+  if (!body.empty())
+    CK(cudaMemcpyAsync(B.tri_lv_body.p, body.data(), body.size() * sizeof(int), cudaMemcpyHostToDevice, s));
+  CK(cudaMemcpyAsync(B.tri_lv_off.p, off.data(), off.size() * sizeof(int), cudaMemcpyHostToDevice, s));
+  CK(cudaStreamSynchronize(s));
+}
+
 void tri_solve(const Geo& g, PairSet& S, NewtonBufs& B, const int* sc_on, double* dq, cudaStream_t s) {
   const int nb = g.nb;
   B.tri_Li.ensure(144 * (size_t)nb);
-  B.tri_W.ensure(144 * (size_t)nb);
+  B.tri_W.ensure(288 * (size_t)nb);
   B.tri_y.ensure(12 * (size_t)nb);
-  TriArgs a{S.row_ptr.p, B.rcol.p, B.rn.p, B.Hrow.p, g.bscene, sc_on, B.tri_on.p, B.tri_link.p, B.grad.p,
-            B.tri_Li.p, B.tri_W.p, B.tri_y.p, B.x.p, dq, B.status.p};
-  KLAUNCH(K_PCG, s, k_tri_solve<<<nb, TNT, 0, s>>>(a));
+  B.tri_fl.ensure(nb);
+  static int max_blocks = 0;
+  if (!max_blocks) {
+    int dev, sms, per;
+    CK(cudaGetDevice(&dev));
+    CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_tri_solve, TNT, 0));
+    max_blocks = sms * (per > 0 ? per : 1);
+  }
+  TriArgs a{S.row_ptr.p, B.rcol.p,   B.rn.p,  B.Hrow.p,        g.bscene,       g.sc_end,
+            sc_on,       B.tri_on.p, B.grad.p, B.tri_Li.p,     B.tri_W.p,      B.tri_y.p,  B.x.p,
+            dq,          B.tri_fl.p, B.tri_lv_body.p, B.tri_lv_off.p, B.tri_nlev, B.status.p};
+  void* args[] = {&a};
+  const int grid = B.tri_width < max_blocks ? B.tri_width : max_blocks;
+  KLAUNCH(K_PCG, s, CK(cudaLaunchCooperativeKernel((void*)k_tri_solve, dim3(grid), dim3(TNT), args, 0, s)));
   // per body: its diagonal and coupling blocks read, the factor's blocks written and read
-  // back (4 x 1152 B), the right-hand side, y and x
-  prof_work(K_PCG, 1, 6.0 * 1152.0 * nb);
+  // back (6 x 1152 B), the right-hand side, y and x
+  prof_work(K_PCG, 1, 8.0 * 1152.0 * nb);
 }
 
 }  // namespace abd
