@@ -106,6 +106,7 @@ struct CullScratch {
   DBuf<double> ovcull;
   DBuf<float> ovcull_f;
   DBuf<float> vbox, ebox, fbox;
+  DBuf<float> vend;                     // float positions of each vertex at q and at the target
   DBuf<int> order, order_cnt;           // narrow-phase processing order of the overlaps
   DBuf<int> bin_cnt, bin_off, lst;
   DBuf<long long> cand_cnt, cand_off;
@@ -187,6 +188,11 @@ void launch_project(const Geo& g, int which, double alpha, cudaStream_t s);
 void cull(const Geo& g, const Params& P, int vtn, double alpha, CullScratch& cs, PairSet& out, double* toi_p,
           double* toi_g, cudaStream_t s);
 
+// Float boxes of the vertices, edges and faces, rounded outward, of X or of the trajectory from
+// Xq to X (cs.vbox / ebox / fbox), and the float positions of the vertices at Xq and X (cs.vend).
+void prim_boxes(const Geo& g, bool traj, CullScratch& cs, cudaStream_t s);
+void traj_floats(const Geo& g, CullScratch& cs, cudaStream_t s);
+
 // Line-search cull at q + alpha dq (per-scene steps of g) that reuses the overlaps and the
 // refined primitive lists of the trajectory cull H of the same step (vtn 3 over q -> q + dq
 // with the step not yet scaled down): the pair set equals that of a full vtn 2 cull.
@@ -212,21 +218,29 @@ struct ShParams {
   double min_xyz, dx, safe_factor;
   int bits, fix_edge, full_ccd;
 };
+// Cells of a primitive's box per axis: the first and the last.
+struct ShCells {
+  int l[3], u[3];
+};
 struct ShTable {
-  DBuf<long long> cnt, off, scan_tmp;
-  DBuf<unsigned long long> keys;
-  DBuf<int> bstart, bend;
-  long long n = 0;
-  long long h_tot = 0;
+  DBuf<ShCells> cells;       // cell ranges of the registered primitives
+  DBuf<int> cnt, beg, cur;   // per bucket: entries (0 where unused), segment, write position
+  DBuf<int> used, ctl;       // buckets in use; [0] their number, [1] entries, [2..3] cells in all
+  DBuf<int2> ent;            // (primitive, body) by bucket
+  unsigned long long h_tot = 0;
 };
 struct ShScratch {
   ShTable tab;
-  DBuf<int> qcnt, qoff, scan_i, flag, pos;
+  DBuf<ShCells> qcells;
+  DBuf<int2> cand;           // candidates left by the FP32 tests
+  DBuf<unsigned long long> n;  // candidates, accepted pairs
+  DBuf<int> scan_i, flag, pos;
   DBuf<unsigned long long> pt_keys, ee_keys, bp_all, tkeys;
   DBuf<unsigned> bp_pt, bp_ee;
   int* h_int = nullptr;
-  unsigned long long* h_toi = nullptr;
+  unsigned long long *h_n = nullptr, *h_toi = nullptr;
   int h_toi_cap = 0;
+  void release();
 };
 // gen_collision_set: pair set of the configuration at q (vtn 1) or q + alpha dq (vtn 2).
 void sh_cull(const Geo& g, const Params& P, const ShParams& H, int vtn, double alpha, ShScratch& W, CullScratch& cs,

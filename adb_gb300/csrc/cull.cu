@@ -201,6 +201,16 @@ __global__ void k_vert_boxes(Geo g, int traj, float* vb) {
   box b = traj ? box2(p, ldX(g.Xq, g.nv, t)) : box{p, p};
   put_fbox(vb + 6 * t, b);
 }
+// Float positions (to nearest) of every vertex at q and at the target, for the FP32
+// certificates of the trajectories.
+__global__ void k_traj_floats(Geo g, float* ve) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= g.nv) return;
+  const d3 p = ldX(g.Xq, g.nv, t), q = ldX(g.X, g.nv, t);
+  float* o = ve + 6 * (size_t)t;
+  o[0] = __double2float_rn(p.x); o[1] = __double2float_rn(p.y); o[2] = __double2float_rn(p.z);
+  o[3] = __double2float_rn(q.x); o[4] = __double2float_rn(q.y); o[5] = __double2float_rn(q.z);
+}
 __device__ __forceinline__ void fbox_union(float* o, const float* a, const float* b) {
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
@@ -1243,6 +1253,22 @@ void launch_project(const Geo& g, int which, double alpha, cudaStream_t s) {
   prof_work(K_PROJECT, g.nv, 48.0 * g.nv);  // rest read + world write per vertex
 }
 
+void prim_boxes(const Geo& g, bool traj, CullScratch& cs, cudaStream_t s) {
+  cs.vbox.ensure(6 * (size_t)g.nv + 6);
+  cs.ebox.ensure(6 * (size_t)g.ne + 6);
+  cs.fbox.ensure(6 * (size_t)g.nf + 6);
+  if (g.nv > 0) KLAUNCH(K_PRIM_BOXES, s, k_vert_boxes<<<nblk(g.nv, 256), 256, 0, s>>>(g, traj ? 1 : 0, cs.vbox.p));
+  if (g.ne + g.nf > 0) {
+    KLAUNCH(K_PRIM_BOXES, s, k_prim_boxes<<<nblk((long long)g.ne + g.nf, 256), 256, 0, s>>>(g, cs.vbox.p, cs.ebox.p,
+                                                                                             cs.fbox.p));
+  }
+}
+
+void traj_floats(const Geo& g, CullScratch& cs, cudaStream_t s) {
+  cs.vend.ensure(6 * (size_t)g.nv + 6);
+  if (g.nv > 0) KLAUNCH(K_PRIM_BOXES, s, k_traj_floats<<<nblk(g.nv, 256), 256, 0, s>>>(g, cs.vend.p));
+}
+
 // Narrow phase of a pair cull over binned (and refined, ordered) lists of nov overlaps:
 // classification with staging (grown and repeated when it overflows), per-overlap counts
 // and offsets, one host read of the totals (pt, ee, vg, staged, unstaged overlaps), then
@@ -1353,14 +1379,7 @@ void cull(const Geo& g_in, const Params& P, int vtn, double alpha, CullScratch& 
     KLAUNCH(K_OV_LOWER, s, k_ov_lower<<<nblk(nnz, 256), 256, 0, s>>>(nnz, S.row_ptr.p, S.col.p, cs.rowid.p, S.upidx.p));
   }
   // 4. primitive boxes and binning
-  cs.vbox.ensure(6 * (size_t)g.nv + 6);
-  cs.ebox.ensure(6 * (size_t)g.ne + 6);
-  cs.fbox.ensure(6 * (size_t)g.nf + 6);
-  if (g.nv > 0) KLAUNCH(K_PRIM_BOXES, s, k_vert_boxes<<<nblk(g.nv, 256), 256, 0, s>>>(g, traj, cs.vbox.p));
-  if (g.ne + g.nf > 0) {
-    KLAUNCH(K_PRIM_BOXES, s, k_prim_boxes<<<nblk((long long)g.ne + g.nf, 256), 256, 0, s>>>(g, cs.vbox.p, cs.ebox.p,
-                                                                                             cs.fbox.p));
-  }
+  prim_boxes(g, traj, cs, s);
   int nlst = 0;
   if (nov > 0) {
     cs.bin_cnt.ensure(6 * (size_t)nov + 6);
@@ -1476,11 +1495,7 @@ void cull_trial(const Geo& g_in, const Params& P, double alpha, CullScratch& cs,
   }
   S.nnz = nnz;
   S.nov = nov;
-  if (g.nv > 0) KLAUNCH(K_PRIM_BOXES, s, k_vert_boxes<<<nblk(g.nv, 256), 256, 0, s>>>(g, 0, cs.vbox.p));
-  if (g.ne + g.nf > 0) {
-    KLAUNCH(K_PRIM_BOXES, s, k_prim_boxes<<<nblk((long long)g.ne + g.nf, 256), 256, 0, s>>>(g, cs.vbox.p, cs.ebox.p,
-                                                                                             cs.fbox.p));
-  }
+  prim_boxes(g, false, cs, s);
   int npt = 0, nee = 0, nvg = 0;
   if (nov > 0) {
     narrow_pairs(g, P, float_round_up(P.d_sqrt), nov, S.ovI.p, S.ovJ.p, cs, S, npt, nee, s);

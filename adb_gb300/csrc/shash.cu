@@ -5,11 +5,21 @@
 //
 // Grid: a point x lies in cell int(max(x - min_xyz, 0) / dx) per axis; a cell's bucket
 // keeps the low xyz_bits bits of each coordinate (spatial_hashing.cpp:11-21), so cells
-// that agree modulo 2^xyz_bits share a bucket. Registration writes one 64-bit key
-// (bucket << 32 | primitive) per covered cell; the keys are sorted, so every bucket is a
-// contiguous, ordered run. A query walks the buckets of its cell range in the
-// reference's loop order; a registered primitive is taken in the first query cell whose
-// bucket holds it (the reference gathers, sorts and de-duplicates per query).
+// that agree modulo 2^xyz_bits share a bucket. A registered primitive is a candidate of a
+// query when one of the query's cells has a bucket that holds it (the reference gathers,
+// sorts and de-duplicates per query).
+//
+// How the candidates are found. Registration counts each bucket's entries, gives every used
+// bucket a segment and writes (primitive, body) into it; the order inside a bucket is free,
+// because pairs are sorted by key afterwards and times of impact are min-reduced. One warp
+// per query primitive then walks the buckets of its cells, an entry per lane. With the
+// reference's default cell (0.8) a bucket holds hundreds to thousands of primitives and
+// nearly all of them are far away, so the walk runs in FP32 only: an outward-rounded box
+// test for the culls, the certificates of abd_ccd_filter.cuh for the trajectories. What
+// is left is appended to a list that a second kernel evaluates in FP64, a pair per thread.
+// (One thread per query used to walk the buckets, with six FP64 divisions per entry for
+// its cell range, count and write passes for the culls and a sort of all entries. A frame of
+// 33 icospheres, 5 culls and 2 bounds: 476 -> 6.2 ms, of which the hash takes 2.5.)
 //
 // Distance culling keeps the pairs of different bodies with squared distance below
 // dhat * safe_factor^2 (PT: vertex of any body against a triangle; EE: edges of bodies
@@ -24,6 +34,7 @@
 #include <cstring>
 #include <stdexcept>
 
+#include "abd_ccd_filter.cuh"
 #include "abd_engine.h"
 #include "abd_exact.cuh"
 
@@ -99,54 +110,106 @@ __device__ __forceinline__ void reg_box(const Geo& g, int kind, int id, int traj
   }
 }
 
-__global__ void k_reg_count(Geo g, ShGrid G, int kind, int n, int traj, int fix_edge, long long* cnt) {
-  int id = blockIdx.x * blockDim.x + threadIdx.x;
-  if (id >= n) return;
-  d3 lo, hi;
-  reg_box(g, kind, id, traj, fix_edge, lo, hi);
-  int l[3], u[3];
-  sh_cells(lo, G, l);
-  sh_cells(hi, G, u);
-  cnt[id] = (long long)(u[0] - l[0] + 1) * (u[1] - l[1] + 1) * (u[2] - l[2] + 1);
+// Cells of the registered primitives (kind 0: vertices, 1: edges) and the number of cells
+// they cover in all.
+__global__ void k_reg_cells(Geo g, ShGrid G, int kind, int n, int traj, int fix_edge, ShCells* cells,
+                            unsigned long long* total) {
+  const int id = blockIdx.x * blockDim.x + threadIdx.x;
+  unsigned long long c = 0;
+  if (id < n) {
+    d3 lo, hi;
+    reg_box(g, kind, id, traj, fix_edge, lo, hi);
+    ShCells r;
+    sh_cells(lo, G, r.l);
+    sh_cells(hi, G, r.u);
+    cells[id] = r;
+    c = (unsigned long long)(r.u[0] - r.l[0] + 1) * (r.u[1] - r.l[1] + 1) * (r.u[2] - r.l[2] + 1);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
+  if ((threadIdx.x & 31) == 0 && c) atomicAdd(total, c);
 }
 
-__global__ void k_reg_fill(Geo g, ShGrid G, int kind, int n, int traj, int fix_edge, const long long* off,
-                           unsigned long long* keys) {
-  int id = blockIdx.x * blockDim.x + threadIdx.x;
-  if (id >= n) return;
-  d3 lo, hi;
-  reg_box(g, kind, id, traj, fix_edge, lo, hi);
-  int l[3], u[3];
-  sh_cells(lo, G, l);
-  sh_cells(hi, G, u);
-  long long o = off[id];
-  for (int i = l[0]; i <= u[0]; ++i)
-    for (int j = l[1]; j <= u[1]; ++j)
-      for (int k = l[2]; k <= u[2]; ++k)
-        keys[o++] = ((unsigned long long)sh_hash(i, j, k, G.bits) << 32) | (unsigned)id;
+// The buckets of a cell range, each once (f(bucket)): cells 2^bits apart share a bucket, so
+// no axis takes more than 2^bits of them.
+template <typename F>
+__device__ __forceinline__ void for_buckets(const ShCells& r, int bits, F&& f) {
+  const int M = 1 << bits;
+  const int n0 = min(r.u[0] - r.l[0] + 1, M), n1 = min(r.u[1] - r.l[1] + 1, M), n2 = min(r.u[2] - r.l[2] + 1, M);
+  for (int i = 0; i < n0; ++i)
+    for (int j = 0; j < n1; ++j)
+      for (int k = 0; k < n2; ++k) f(sh_hash(r.l[0] + i, r.l[1] + j, r.l[2] + k, bits));
 }
 
-__global__ void k_bucket_bounds(const unsigned long long* keys, long long n, int* bstart, int* bend) {
-  long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  unsigned b = (unsigned)(keys[i] >> 32);
-  if (i == 0 || (unsigned)(keys[i - 1] >> 32) != b) bstart[b] = (int)i;
-  if (i == n - 1 || (unsigned)(keys[i + 1] >> 32) != b) bend[b] = (int)(i + 1);
+// Table build: empty the buckets used last (cnt is zero outside them), count, give each
+// used bucket its segment, fill. ctl: [0] used buckets, [1] entries.
+__global__ void k_bucket_clear(const int* ctl, const int* used, int* cnt) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < ctl[0]; i += gridDim.x * blockDim.x) cnt[used[i]] = 0;
+}
+__global__ void k_bucket_count(ShGrid G, int n, const ShCells* cells, int* cnt, int* used, int* ctl) {
+  const int id = blockIdx.x * blockDim.x + threadIdx.x;
+  if (id >= n) return;
+  for_buckets(cells[id], G.bits, [&](unsigned b) {
+    if (atomicAdd(&cnt[b], 1) == 0) used[atomicAdd(&ctl[0], 1)] = (int)b;
+  });
+}
+__global__ void k_bucket_alloc(int* ctl, const int* used, const int* cnt, int* beg, int* cur) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= ctl[0]) return;
+  const int b = used[i];
+  const int o = atomicAdd(&ctl[1], cnt[b]);
+  beg[b] = o;
+  cur[b] = o;
+}
+__global__ void k_bucket_fill(Geo g, ShGrid G, int kind, int n, const ShCells* cells, int* cur, int2* ent) {
+  const int id = blockIdx.x * blockDim.x + threadIdx.x;
+  if (id >= n) return;
+  const int body = g.vbody[kind ? g.ev[2 * id] : id];
+  for_buckets(cells[id], G.bits, [&](unsigned b) { ent[atomicAdd(&cur[b], 1)] = make_int2(id, body); });
 }
 
 struct ShQuery {
   ShGrid G;
-  const unsigned long long* keys;
-  const int *bstart, *bend;
+  const ShCells *rcells, *qcells;   // of the registered and of the query primitives
+  const int *cnt, *beg;             // buckets
+  const int2* ent;                  // (primitive, body)
   double qd;     // query box growth (d_sqrt * safe_factor); 0 for trajectories
+  float qd_f;    // the same, rounded up past every rounding of the FP64 distance
   double thr;    // squared-distance threshold (dhat * safe_factor^2)
-  double marg;   // prefilter margin: boxes farther apart than qd + marg cannot pass thr
-  int traj, fix_edge;
+  const float *vb, *eb, *fb;        // float boxes of the primitives (culls)
+  const float* vend;                // float positions of the vertices at q and at the target (trajectories)
+  int2* cand;                       // candidates: (query primitive, registered primitive)
+  unsigned long long cand_cap;
+  unsigned long long* n;            // [0] candidates, [1] accepted pairs
 };
 
-__device__ __forceinline__ bool box_apart(const d3& alo, const d3& ahi, const d3& blo, const d3& bhi, double m) {
-  return ahi.x < blo.x - m || blo.x > ahi.x + m || ahi.y < blo.y - m || blo.y > ahi.y + m || ahi.z < blo.z - m ||
-         blo.z > ahi.z + m;
+// Cells of the query primitives (kind 0: triangles, 1: edges): the box at the target, grown
+// by qd, or of the whole trajectory.
+__global__ void k_query_cells(Geo g, ShGrid G, int kind, int nq, int traj, double qd, ShCells* cells) {
+  const int id = blockIdx.x * blockDim.x + threadIdx.x;
+  if (id >= nq) return;
+  const int nvtx = kind ? 2 : 3;
+  const int* vid = kind ? g.ev + 2 * id : g.fv + 3 * id;
+  d3 lo = ldX(g.X, g.nv, vid[0]), hi = lo;
+  for (int k = 1; k < nvtx; ++k) {
+    const d3 p = ldX(g.X, g.nv, vid[k]);
+    lo = dmin3(lo, p);
+    hi = dmax3(hi, p);
+  }
+  if (traj) {
+    for (int k = 0; k < nvtx; ++k) {
+      const d3 p = ldX(g.Xq, g.nv, vid[k]);
+      lo = dmin3(lo, p);
+      hi = dmax3(hi, p);
+    }
+  } else {
+    lo = mk(XA(lo.x, -qd), XA(lo.y, -qd), XA(lo.z, -qd));
+    hi = mk(XA(hi.x, qd), XA(hi.y, qd), XA(hi.z, qd));
+  }
+  ShCells r;
+  sh_cells(lo, G, r.l);
+  sh_cells(hi, G, r.u);
+  cells[id] = r;
 }
 
 __device__ __forceinline__ unsigned long long pair_key(int A, int a, int B, int b, int sub) {
@@ -155,135 +218,138 @@ __device__ __forceinline__ unsigned long long pair_key(int A, int a, int B, int 
          (unsigned long long)b;
 }
 
-// PT query, thread per triangle. MODE 0: count, 1: write keys, 2: time of impact.
-template <int MODE>
-__global__ void k_pt_query(Geo g, ShQuery Q, const int* off, unsigned long long* out,
-                           unsigned long long* toi_key, int* cnt) {
-  int f = blockIdx.x * blockDim.x + threadIdx.x;
-  if (f >= g.nf) return;
-  int i0 = g.fv[3 * f], i1 = g.fv[3 * f + 1], i2 = g.fv[3 * f + 2];
-  int J = g.vbody[i0];
-  if (!scene_on(g, J)) {
-    if (MODE == 0) cnt[f] = 0;
-    return;
-  }
-  d3 t0 = ldX(g.X, g.nv, i0), t1 = ldX(g.X, g.nv, i1), t2 = ldX(g.X, g.nv, i2);
-  d3 lo = dmin3(dmin3(t0, t1), t2), hi = dmax3(dmax3(t0, t1), t2);
-  d3 f0[3], f1[3] = {t0, t1, t2};
-  if (MODE == 2) {
-    f0[0] = ldX(g.Xq, g.nv, i0);
-    f0[1] = ldX(g.Xq, g.nv, i1);
-    f0[2] = ldX(g.Xq, g.nv, i2);
-    lo = dmin3(lo, dmin3(dmin3(f0[0], f0[1]), f0[2]));
-    hi = dmax3(hi, dmax3(dmax3(f0[0], f0[1]), f0[2]));
+__device__ __forceinline__ f3 ldf3(const float* p) { return f3{p[0], p[1], p[2]}; }
+
+// Candidates of the query primitives [qbeg, qend), one warp each. KIND 0: triangles against vertices of
+// other bodies; 1: edges against the edges of lower bodies (of the same scene both). An entry
+// in several of the query's buckets is taken in the first cell that holds it, as by its cell
+// range (the test every entry used to pay for, here only for those the FP32 test leaves).
+template <int KIND, bool TRAJ>
+__global__ void __launch_bounds__(128) k_sh_query(Geo g, ShQuery Q, int qbeg, int qend) {
+  const int q = qbeg + (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+  if (q >= qend) return;
+  constexpr int NV = KIND ? 2 : 3;
+  const int* qv = KIND ? g.ev + 2 * q : g.fv + 3 * q;
+  const int J = g.vbody[qv[0]], sc = g.bscene[J];
+  if (!scene_on(g, J)) return;
+  f3 q0[NV], q1[NV];
+  float qb[6];
+  if (TRAJ) {
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+      const float* p = Q.vend + 6 * (size_t)qv[k];
+      q0[k] = ldf3(p);
+      q1[k] = ldf3(p + 3);
+    }
   } else {
-    lo = mk(XA(lo.x, -Q.qd), XA(lo.y, -Q.qd), XA(lo.z, -Q.qd));
-    hi = mk(XA(hi.x, Q.qd), XA(hi.y, Q.qd), XA(hi.z, Q.qd));
+    const float* p = (KIND ? Q.eb : Q.fb) + 6 * (size_t)q;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      qb[c] = __fsub_rd(p[c], Q.qd_f);
+      qb[c + 3] = __fadd_ru(p[c + 3], Q.qd_f);
+    }
   }
-  int l[3], u[3];
-  sh_cells(lo, Q.G, l);
-  sh_cells(hi, Q.G, u);
-  int c = 0;
-  long long w = MODE == 1 ? off[f] : 0;
-  double tmin = 1.0;
-  const int f_loc = f - g.f_off[J];
-  for (int i = l[0]; i <= u[0]; ++i)
-    for (int j = l[1]; j <= u[1]; ++j)
-      for (int k = l[2]; k <= u[2]; ++k) {
-        unsigned b = sh_hash(i, j, k, Q.G.bits);
-        for (int e = Q.bstart[b]; e < Q.bend[b]; ++e) {
-          if (e > Q.bstart[b] && Q.keys[e] == Q.keys[e - 1]) continue;  // registered twice in one bucket
-          int v = (int)(Q.keys[e] & 0xffffffffull);
-          int I = g.vbody[v];
-          if (I == J || g.bscene[I] != g.bscene[J]) continue;
-          d3 rlo, rhi;
-          reg_box(g, 0, v, Q.traj, 0, rlo, rhi);
-          int rl[3], ru[3];
-          sh_cells(rlo, Q.G, rl);
-          sh_cells(rhi, Q.G, ru);
-          if (i != first_hit(l[0], rl[0], ru[0], Q.G.bits) || j != first_hit(l[1], rl[1], ru[1], Q.G.bits) ||
-              k != first_hit(l[2], rl[2], ru[2], Q.G.bits))
-            continue;
-          if (MODE == 2) {
-            tmin = dmin(tmin, pt_collision_time(ldX(g.Xq, g.nv, v), f0, ldX(g.X, g.nv, v), f1));
-            continue;
+  const ShCells r = Q.qcells[q];
+  const int M = 1 << Q.G.bits;
+  const int e0 = r.l[0] + min(r.u[0] - r.l[0], M - 1), e1 = r.l[1] + min(r.u[1] - r.l[1], M - 1),
+            e2 = r.l[2] + min(r.u[2] - r.l[2], M - 1);
+  for (int i = r.l[0]; i <= e0; ++i)
+    for (int j = r.l[1]; j <= e1; ++j)
+      for (int k = r.l[2]; k <= e2; ++k) {
+        const unsigned b = sh_hash(i, j, k, Q.G.bits);
+        const int n = Q.cnt[b];
+        if (n == 0) continue;  // an unused bucket has no segment
+        const int2* ent = Q.ent + Q.beg[b];
+        for (int t0 = 0; t0 < n; t0 += 32) {
+          bool take = false;
+          int id = 0;
+          if (t0 + lane < n) {
+            const int2 e = ent[t0 + lane];
+            id = e.x;
+            if ((KIND ? e.y < J : e.y != J) && g.bscene[e.y] == sc) {
+              if (TRAJ) {
+                if (KIND) {
+                  const float *pa = Q.vend + 6 * (size_t)g.ev[2 * id], *pb = Q.vend + 6 * (size_t)g.ev[2 * id + 1];
+                  const f3 a0[2] = {ldf3(pa), ldf3(pb)}, a1[2] = {ldf3(pa + 3), ldf3(pb + 3)};
+                  take = !f_ee_miss(a0, a1, q0, q1);
+                } else {
+                  const float* p = Q.vend + 6 * (size_t)id;
+                  take = !f_pt_miss(ldf3(p), ldf3(p + 3), q0, q1);
+                }
+              } else {
+                const float* p = (KIND ? Q.eb : Q.vb) + 6 * (size_t)id;
+                take = p[0] <= qb[3] && p[3] >= qb[0] && p[1] <= qb[4] && p[4] >= qb[1] && p[2] <= qb[5] &&
+                       p[5] >= qb[2];
+              }
+              if (take) {
+                const ShCells c = Q.rcells[id];
+                take = i == first_hit(r.l[0], c.l[0], c.u[0], Q.G.bits) &&
+                       j == first_hit(r.l[1], c.l[1], c.u[1], Q.G.bits) &&
+                       k == first_hit(r.l[2], c.l[2], c.u[2], Q.G.bits);
+              }
+            }
           }
-          d3 p = rlo;
-          if (box_apart(p, p, lo, hi, Q.marg)) continue;
-          int ty = pt_type(p, t0, t1, t2);
-          if (!(pt_dist(p, t0, t1, t2, ty) < Q.thr)) continue;
-          if (MODE == 1) out[w++] = pair_key(I, v - g.v_off[I], J, f_loc, I < J ? 0 : 1);
-          ++c;
+          const unsigned m = __ballot_sync(0xffffffffu, take);
+          if (m) {
+            unsigned long long base = 0;
+            if (lane == 0) base = atomicAdd(&Q.n[0], (unsigned long long)__popc(m));
+            base = __shfl_sync(0xffffffffu, base, 0) + __popc(m & ((1u << lane) - 1u));
+            if (take && base < Q.cand_cap) Q.cand[base] = make_int2(q, id);
+          }
         }
       }
-  if (MODE == 0) cnt[f] = c;
-  if (MODE == 2 && tmin < 1.0) atomicMin(toi_key + 2 * g.bscene[J], dkey(tmin));
 }
 
-// EE query, thread per edge of body J against edges of bodies I < J.
-template <int MODE>
-__global__ void k_ee_query(Geo g, ShQuery Q, const int* off, unsigned long long* out,
-                           unsigned long long* toi_key, int* cnt) {
-  int ej = blockIdx.x * blockDim.x + threadIdx.x;
-  if (ej >= g.ne) return;
-  int jb0 = g.ev[2 * ej], jb1 = g.ev[2 * ej + 1];
-  int J = g.vbody[jb0];
-  if (!scene_on(g, J)) {
-    if (MODE == 0) cnt[ej] = 0;
-    return;
+// Candidates in FP64: the pairs with squared distance below thr, as keys.
+template <int KIND>
+__global__ void __launch_bounds__(128) k_sh_exact(Geo g, ShQuery Q, unsigned long long* keys,
+                                                  unsigned long long key_cap) {
+  const int n = (int)min(Q.n[0], Q.cand_cap);
+  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
+    const int2 c = Q.cand[t];
+    const int q = c.x, e = c.y;
+    unsigned long long key;
+    if (KIND == 0) {
+      const int i0 = g.fv[3 * q], I = g.vbody[e], J = g.vbody[i0];
+      const d3 p = ldX(g.X, g.nv, e), t0 = ldX(g.X, g.nv, i0), t1 = ldX(g.X, g.nv, g.fv[3 * q + 1]),
+               t2 = ldX(g.X, g.nv, g.fv[3 * q + 2]);
+      if (!(pt_dist(p, t0, t1, t2, pt_type(p, t0, t1, t2)) < Q.thr)) continue;
+      key = pair_key(I, e - g.v_off[I], J, q - g.f_off[J], I < J ? 0 : 1);
+    } else {
+      const int ia = g.ev[2 * e], ib = g.ev[2 * q], I = g.vbody[ia], J = g.vbody[ib];
+      const d3 a0 = ldX(g.X, g.nv, ia), a1 = ldX(g.X, g.nv, g.ev[2 * e + 1]), b0 = ldX(g.X, g.nv, ib),
+               b1 = ldX(g.X, g.nv, g.ev[2 * q + 1]);
+      if (!(ee_dist(a0, a1, b0, b1, ee_type(a0, a1, b0, b1)) < Q.thr)) continue;
+      key = pair_key(I, e - g.e_off[I], J, q - g.e_off[J], 2);
+    }
+    const unsigned long long o = atomicAdd(&Q.n[1], 1ull);
+    if (o < key_cap) keys[o] = key;
   }
-  d3 b0 = ldX(g.X, g.nv, jb0), b1 = ldX(g.X, g.nv, jb1);
-  d3 lo = dmin3(b0, b1), hi = dmax3(b0, b1);
-  d3 q0[2], q1[2] = {b0, b1};
-  if (MODE == 2) {
-    q0[0] = ldX(g.Xq, g.nv, jb0);
-    q0[1] = ldX(g.Xq, g.nv, jb1);
-    lo = dmin3(lo, dmin3(q0[0], q0[1]));
-    hi = dmax3(hi, dmax3(q0[0], q0[1]));
-  } else {
-    lo = mk(XA(lo.x, -Q.qd), XA(lo.y, -Q.qd), XA(lo.z, -Q.qd));
-    hi = mk(XA(hi.x, Q.qd), XA(hi.y, Q.qd), XA(hi.z, Q.qd));
+}
+
+// Candidates in FP64: the earliest time of impact per scene.
+template <int KIND>
+__global__ void __launch_bounds__(128) k_sh_toi(Geo g, ShQuery Q, unsigned long long* toi_key) {
+  const int n = (int)min(Q.n[0], Q.cand_cap);
+  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
+    const int q = Q.cand[t].x, e = Q.cand[t].y;
+    double tc;
+    int J;
+    if (KIND == 0) {
+      const int i0 = g.fv[3 * q], i1 = g.fv[3 * q + 1], i2 = g.fv[3 * q + 2];
+      J = g.vbody[i0];
+      const d3 f0[3] = {ldX(g.Xq, g.nv, i0), ldX(g.Xq, g.nv, i1), ldX(g.Xq, g.nv, i2)};
+      const d3 f1[3] = {ldX(g.X, g.nv, i0), ldX(g.X, g.nv, i1), ldX(g.X, g.nv, i2)};
+      tc = pt_collision_time(ldX(g.Xq, g.nv, e), f0, ldX(g.X, g.nv, e), f1);
+    } else {
+      const int ia0 = g.ev[2 * e], ia1 = g.ev[2 * e + 1], ib0 = g.ev[2 * q], ib1 = g.ev[2 * q + 1];
+      J = g.vbody[ib0];
+      const d3 a0[2] = {ldX(g.Xq, g.nv, ia0), ldX(g.Xq, g.nv, ia1)}, a1[2] = {ldX(g.X, g.nv, ia0), ldX(g.X, g.nv, ia1)};
+      const d3 b0[2] = {ldX(g.Xq, g.nv, ib0), ldX(g.Xq, g.nv, ib1)}, b1[2] = {ldX(g.X, g.nv, ib0), ldX(g.X, g.nv, ib1)};
+      tc = ee_collision_time(a0, b0, a1, b1);
+    }
+    if (tc < 1.0) atomicMin(toi_key + 2 * g.bscene[J], dkey(tc));
   }
-  int l[3], u[3];
-  sh_cells(lo, Q.G, l);
-  sh_cells(hi, Q.G, u);
-  int c = 0;
-  long long w = MODE == 1 ? off[ej] : 0;
-  double tmin = 1.0;
-  const int ej_loc = ej - g.e_off[J];
-  for (int i = l[0]; i <= u[0]; ++i)
-    for (int j = l[1]; j <= u[1]; ++j)
-      for (int k = l[2]; k <= u[2]; ++k) {
-        unsigned b = sh_hash(i, j, k, Q.G.bits);
-        for (int e = Q.bstart[b]; e < Q.bend[b]; ++e) {
-          if (e > Q.bstart[b] && Q.keys[e] == Q.keys[e - 1]) continue;  // registered twice in one bucket
-          int ei = (int)(Q.keys[e] & 0xffffffffull);
-          int ia0 = g.ev[2 * ei], ia1 = g.ev[2 * ei + 1];
-          int I = g.vbody[ia0];
-          if (I >= J || g.bscene[I] != g.bscene[J]) continue;
-          d3 rlo, rhi;
-          reg_box(g, 1, ei, Q.traj, Q.fix_edge, rlo, rhi);
-          int rl[3], ru[3];
-          sh_cells(rlo, Q.G, rl);
-          sh_cells(rhi, Q.G, ru);
-          if (i != first_hit(l[0], rl[0], ru[0], Q.G.bits) || j != first_hit(l[1], rl[1], ru[1], Q.G.bits) ||
-              k != first_hit(l[2], rl[2], ru[2], Q.G.bits))
-            continue;
-          if (MODE == 2) {
-            d3 a0[2] = {ldX(g.Xq, g.nv, ia0), ldX(g.Xq, g.nv, ia1)}, a1[2] = {ldX(g.X, g.nv, ia0), ldX(g.X, g.nv, ia1)};
-            tmin = dmin(tmin, ee_collision_time(a0, q0, a1, q1));
-            continue;
-          }
-          if (box_apart(rlo, rhi, lo, hi, Q.marg)) continue;
-          d3 a0 = ldX(g.X, g.nv, ia0), a1 = ldX(g.X, g.nv, ia1);
-          int ty = ee_type(a0, a1, b0, b1);
-          if (!(ee_dist(a0, a1, b0, b1, ty) < Q.thr)) continue;
-          if (MODE == 1) out[w++] = pair_key(I, ei - g.e_off[I], J, ej_loc, 2);
-          ++c;
-        }
-      }
-  if (MODE == 0) cnt[ej] = c;
-  if (MODE == 2 && tmin < 1.0) atomicMin(toi_key + 2 * g.bscene[J], dkey(tmin));
 }
 
 // Sorted pair keys -> tuples, distance types (recomputed, as in the query) and the
@@ -471,31 +537,126 @@ ShGrid grid_of(const ShParams& H) { return ShGrid{H.min_xyz, H.dx, H.bits}; }
 
 }  // namespace
 
+void ShScratch::release() {
+  tab.cells.release(); tab.cnt.release(); tab.beg.release(); tab.cur.release(); tab.used.release(); tab.ctl.release();
+  tab.ent.release(); qcells.release(); cand.release(); n.release(); scan_i.release(); flag.release(); pos.release();
+  pt_keys.release(); ee_keys.release(); bp_all.release(); tkeys.release(); bp_pt.release(); bp_ee.release();
+  if (h_int) cudaFreeHost(h_int);
+  if (h_n) cudaFreeHost(h_n);
+  if (h_toi) cudaFreeHost(h_toi);
+  h_int = nullptr;
+  h_n = nullptr;
+  h_toi = nullptr;
+  h_toi_cap = 0;
+}
+
 // Registers `n` primitives of `kind` and builds the bucket table in `T`.
 static void sh_register(const Geo& g, const ShParams& H, int kind, int n, int traj, ShTable& T, cudaStream_t s) {
   ShGrid G = grid_of(H);
-  T.cnt.ensure((size_t)n + 1);
-  T.off.ensure((size_t)n + 1);
-  size_t nbuckets = (size_t)1 << (3 * H.bits);
-  T.bstart.ensure(nbuckets);
-  T.bend.ensure(nbuckets);
-  CK(cudaMemsetAsync(T.bstart.p, 0, nbuckets * sizeof(int), s));
-  CK(cudaMemsetAsync(T.bend.p, 0, nbuckets * sizeof(int), s));
-  T.n = 0;
+  const size_t nbuckets = (size_t)1 << (3 * H.bits);
+  T.ctl.ensure(4);
+  if (T.cnt.cap < nbuckets) {
+    T.cnt.ensure(nbuckets);
+    T.beg.ensure(nbuckets);
+    T.cur.ensure(nbuckets);
+    CK(cudaMemsetAsync(T.cnt.p, 0, T.cnt.cap * sizeof(int), s));
+  } else {
+    KLAUNCH(K_SH, s, k_bucket_clear<<<152, 256, 0, s>>>(T.ctl.p, T.used.p, T.cnt.p));
+  }
+  CK(cudaMemsetAsync(T.ctl.p, 0, 4 * sizeof(int), s));
   if (n == 0) return;
-  KLAUNCH(K_SH, s, k_reg_count<<<nblk(n, 256), 256, 0, s>>>(g, G, kind, n, traj, H.fix_edge, T.cnt.p));
-  scan_exclusive_ll(T.cnt.p, T.off.p, n, T.off.p + n, s, T.scan_tmp);
-  long long tot = 0;
-  CK(cudaMemcpyAsync(&T.h_tot, T.off.p + n, sizeof(long long), cudaMemcpyDeviceToHost, s));
+  T.cells.ensure(n);
+  unsigned long long* d_tot = reinterpret_cast<unsigned long long*>(T.ctl.p + 2);
+  KLAUNCH(K_SH, s, k_reg_cells<<<nblk(n, 256), 256, 0, s>>>(g, G, kind, n, traj, H.fix_edge, T.cells.p, d_tot));
+  CK(cudaMemcpyAsync(&T.h_tot, d_tot, sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
   CK(cudaStreamSynchronize(s));
-  tot = T.h_tot;
-  if (tot > (1ll << 31) - 1) throw std::invalid_argument("spatial hash: too many cell registrations (dx too small)");
-  size_t cap = sort_padded_size((size_t)tot);
-  T.keys.ensure(cap);
-  KLAUNCH(K_SH, s, k_reg_fill<<<nblk(n, 256), 256, 0, s>>>(g, G, kind, n, traj, H.fix_edge, T.off.p, T.keys.p));
-  sort_u64(T.keys.p, (size_t)tot, cap, s);
-  KLAUNCH(K_SH, s, k_bucket_bounds<<<nblk(tot, 256), 256, 0, s>>>(T.keys.p, tot, T.bstart.p, T.bend.p));
-  T.n = tot;
+  const unsigned long long tot = T.h_tot;
+  if (tot > (1ull << 31) - 1) throw std::invalid_argument("spatial hash: too many cell registrations (dx too small)");
+  T.used.ensure(std::min((size_t)tot, nbuckets));
+  T.ent.ensure((size_t)tot);
+  KLAUNCH(K_SH, s, k_bucket_count<<<nblk(n, 256), 256, 0, s>>>(G, n, T.cells.p, T.cnt.p, T.used.p, T.ctl.p));
+  const long long most = (long long)std::min((size_t)tot, nbuckets);
+  KLAUNCH(K_SH, s, k_bucket_alloc<<<nblk(most, 256), 256, 0, s>>>(T.ctl.p, T.used.p, T.cnt.p, T.beg.p, T.cur.p));
+  KLAUNCH(K_SH, s, k_bucket_fill<<<nblk(n, 256), 256, 0, s>>>(g, G, kind, n, T.cells.p, T.cur.p, T.ent.p));
+}
+
+constexpr size_t kCandList = 1u << 21;  // candidates kept at a time (16 MB)
+
+// Registers the primitives that the queries of `kind` run against, computes the queries' cells
+// and fills Q (list and counters included).
+static void sh_prepare(const Geo& g, const ShParams& H, int kind, int traj, ShScratch& W, CullScratch& cs, ShQuery& Q,
+                       cudaStream_t s) {
+  sh_register(g, H, kind, kind ? g.ne : g.nv, traj, W.tab, s);
+  const int nq = kind ? g.ne : g.nf;
+  W.qcells.ensure(nq);
+  KLAUNCH(K_SH, s, k_query_cells<<<nblk(nq, 256), 256, 0, s>>>(g, Q.G, kind, nq, traj, Q.qd, W.qcells.p));
+  Q.rcells = W.tab.cells.p;
+  Q.qcells = W.qcells.p;
+  Q.cnt = W.tab.cnt.p;
+  Q.beg = W.tab.beg.p;
+  Q.ent = W.tab.ent.p;
+  Q.vb = cs.vbox.p;
+  Q.eb = cs.ebox.p;
+  Q.fb = cs.fbox.p;
+  Q.vend = cs.vend.p;
+  W.n.ensure(2);
+  Q.n = W.n.p;
+  W.cand.ensure(kCandList);
+  if (!W.h_n) CK(cudaMallocHost(&W.h_n, 2 * sizeof(unsigned long long)));
+}
+
+// Runs the query over all primitives of a kind, `eval` on each list and `done` on its two
+// counters (false: the same queries again). The queries are taken all at once unless they
+// leave more candidates than the list holds; then in runs of half as many, down to single
+// queries, for which the list grows (a query has at most as many as there are primitives).
+template <int KIND, bool TRAJ, typename Eval, typename Done>
+static void sh_run(const Geo& g, ShQuery& Q, ShScratch& W, cudaStream_t s, Eval&& eval, Done&& done) {
+  const int nq = KIND ? g.ne : g.nf;
+  int step = nq;
+  for (int q0 = 0; q0 < nq;) {
+    const int m = std::min(step, nq - q0);
+    Q.cand = W.cand.p;
+    Q.cand_cap = std::min<size_t>(W.cand.cap, (1ull << 31) - 1);
+    CK(cudaMemsetAsync(Q.n, 0, 2 * sizeof(unsigned long long), s));
+    KLAUNCH(K_SH, s, k_sh_query<KIND, TRAJ><<<nblk(32ll * m, 128), 128, 0, s>>>(g, Q, q0, q0 + m));
+    eval();
+    CK(cudaMemcpyAsync(W.h_n, Q.n, 2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
+    CK(cudaStreamSynchronize(s));
+    if (W.h_n[0] > Q.cand_cap) {
+      if (m == 1) W.cand.ensure((size_t)W.h_n[0]);
+      step = std::max(1, m / 2);
+      continue;
+    }
+    if (done()) q0 += m;
+  }
+}
+
+// The pairs of one kind into `keys`, sorted; returns how many. The keys grow to the counted
+// total when they overflow.
+template <int KIND>
+static int sh_pairs(const Geo& g, const ShParams& H, ShQuery& Q, ShScratch& W, CullScratch& cs,
+                    DBuf<unsigned long long>& keys, cudaStream_t s) {
+  sh_prepare(g, H, KIND, 0, W, cs, Q, s);
+  keys.ensure(1u << 15);
+  size_t np = 0, lim = 0;
+  sh_run<KIND, false>(
+      g, Q, W, s,
+      [&]() {
+        lim = sort_padded_size(1);  // most keys that the sort can pad inside the buffer
+        while (2 * lim <= keys.cap) lim *= 2;
+        KLAUNCH(K_SH, s, k_sh_exact<KIND><<<608, 128, 0, s>>>(g, Q, keys.p + np, lim - np));
+      },
+      [&]() {
+        const size_t all = np + (size_t)W.h_n[1];
+        if (all > lim) {
+          keys.ensure(sort_padded_size(all), true, np);
+          return false;
+        }
+        np = all;
+        return true;
+      });
+  if (np) sort_u64(keys.p, np, keys.cap, s);
+  return (int)np;
 }
 
 void sh_cull(const Geo& g, const Params& P, const ShParams& H, int vtn, double alpha, ShScratch& W, CullScratch& cs,
@@ -503,53 +664,19 @@ void sh_cull(const Geo& g, const Params& P, const ShParams& H, int vtn, double a
   const int nb = g.nb;
   launch_project(g, vtn == 1 ? 1 : 2, alpha, s);
   const double sf = H.safe_factor;
-  ShQuery Q;
+  ShQuery Q{};
   Q.G = grid_of(H);
   Q.qd = P.d_sqrt * sf;
+  // 1e-5 past qd: a box further apart than that has an FP64 squared distance above thr
+  Q.qd_f = nextafterf((float)(Q.qd * (1.0 + 1e-5)), INFINITY);
   Q.thr = P.dhat * (sf * sf);
-  Q.marg = 1e-6 * Q.qd;
-  Q.traj = 0;
-  Q.fix_edge = 0;
   if (!W.h_int) CK(cudaMallocHost(&W.h_int, 8 * sizeof(int)));
-  int npt = 0, nee = 0;
-  // PT: vertices registered, triangles query
-  if (P.pt && g.nv && g.nf) {
-    sh_register(g, H, 0, g.nv, 0, W.tab, s);
-    Q.keys = W.tab.keys.p;
-    Q.bstart = W.tab.bstart.p;
-    Q.bend = W.tab.bend.p;
-    W.qcnt.ensure((size_t)g.nf + 1);
-    W.qoff.ensure((size_t)g.nf + 1);
-    KLAUNCH(K_SH, s, k_pt_query<0><<<nblk(g.nf, 128), 128, 0, s>>>(g, Q, nullptr, nullptr, nullptr, W.qcnt.p));
-    scan_exclusive_int(W.qcnt.p, W.qoff.p, g.nf, W.qoff.p + g.nf, s, W.scan_i);
-    CK(cudaMemcpyAsync(W.h_int, W.qoff.p + g.nf, sizeof(int), cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
-    npt = W.h_int[0];
-    W.pt_keys.ensure(sort_padded_size(npt));
-    if (npt) {
-      KLAUNCH(K_SH, s, k_pt_query<1><<<nblk(g.nf, 128), 128, 0, s>>>(g, Q, W.qoff.p, W.pt_keys.p, nullptr, nullptr));
-      sort_u64(W.pt_keys.p, npt, W.pt_keys.cap, s);
-    }
-  }
-  // EE: edges registered, edges of the higher body query
-  if (P.ee && g.ne) {
-    sh_register(g, H, 1, g.ne, 0, W.tab, s);
-    Q.keys = W.tab.keys.p;
-    Q.bstart = W.tab.bstart.p;
-    Q.bend = W.tab.bend.p;
-    W.qcnt.ensure((size_t)g.ne + 1);
-    W.qoff.ensure((size_t)g.ne + 1);
-    KLAUNCH(K_SH, s, k_ee_query<0><<<nblk(g.ne, 128), 128, 0, s>>>(g, Q, nullptr, nullptr, nullptr, W.qcnt.p));
-    scan_exclusive_int(W.qcnt.p, W.qoff.p, g.ne, W.qoff.p + g.ne, s, W.scan_i);
-    CK(cudaMemcpyAsync(W.h_int, W.qoff.p + g.ne, sizeof(int), cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
-    nee = W.h_int[0];
-    W.ee_keys.ensure(sort_padded_size(nee));
-    if (nee) {
-      KLAUNCH(K_SH, s, k_ee_query<1><<<nblk(g.ne, 128), 128, 0, s>>>(g, Q, W.qoff.p, W.ee_keys.p, nullptr, nullptr));
-      sort_u64(W.ee_keys.p, nee, W.ee_keys.cap, s);
-    }
-  }
+  const bool do_pt = P.pt && g.nv && g.nf, do_ee = P.ee && g.ne;
+  if (do_pt || do_ee) prim_boxes(g, false, cs, s);
+  // PT: vertices registered, triangles query; EE: edges registered, edges of the higher body
+  // query
+  const int npt = do_pt ? sh_pairs<0>(g, H, Q, W, cs, W.pt_keys, s) : 0;
+  const int nee = do_ee ? sh_pairs<1>(g, H, Q, W, cs, W.ee_keys, s) : 0;
   // tuples, types and body-pair keys
   S.npt = npt;
   S.nee = nee;
@@ -605,6 +732,15 @@ void sh_cull(const Geo& g, const Params& P, const ShParams& H, int vtn, double a
   CK(cudaStreamSynchronize(s));
 }
 
+// Lowers the per-scene keys to the earliest time of impact of the candidates of one kind.
+template <int KIND>
+static void sh_toi(const Geo& g, const ShParams& H, ShQuery& Q, ShScratch& W, CullScratch& cs, cudaStream_t s) {
+  sh_prepare(g, H, KIND, 1, W, cs, Q, s);
+  sh_run<KIND, true>(
+      g, Q, W, s, [&]() { KLAUNCH(K_SH, s, k_sh_toi<KIND><<<1216, 128, 0, s>>>(g, Q, cs.toi_key.p)); },
+      []() { return true; });
+}
+
 void sh_bound(const Geo& g, const Params& P, const ShParams& H, const PairSet& cur, ShScratch& W, CullScratch& cs,
               double* toi, cudaStream_t s) {
   launch_project(g, 2, 1.0, s);
@@ -617,27 +753,12 @@ void sh_bound(const Geo& g, const Params& P, const ShParams& H, const PairSet& c
   KLAUNCH(K_SH, s, k_fill_key<<<nblk(nk, 256), 256, 0, s>>>(cs.toi_key.p, nk, b1 | 0x8000000000000000ull));
   if (H.full_ccd) {
     if (P.ground && g.nv) launch_vg_toi(g, P, cs.toi_key.p, s);
-    ShQuery Q;
+    ShQuery Q{};
     Q.G = grid_of(H);
-    Q.qd = 0.0;
-    Q.thr = 0.0;
-    Q.marg = 0.0;
-    Q.traj = 1;
-    Q.fix_edge = H.fix_edge;
-    if (P.pt && g.nv && g.nf) {
-      sh_register(g, H, 0, g.nv, 1, W.tab, s);
-      Q.keys = W.tab.keys.p;
-      Q.bstart = W.tab.bstart.p;
-      Q.bend = W.tab.bend.p;
-      KLAUNCH(K_SH, s, k_pt_query<2><<<nblk(g.nf, 128), 128, 0, s>>>(g, Q, nullptr, nullptr, cs.toi_key.p, nullptr));
-    }
-    if (P.ee && g.ne) {
-      sh_register(g, H, 1, g.ne, 1, W.tab, s);
-      Q.keys = W.tab.keys.p;
-      Q.bstart = W.tab.bstart.p;
-      Q.bend = W.tab.bend.p;
-      KLAUNCH(K_SH, s, k_ee_query<2><<<nblk(g.ne, 128), 128, 0, s>>>(g, Q, nullptr, nullptr, cs.toi_key.p, nullptr));
-    }
+    const bool do_pt = P.pt && g.nv && g.nf, do_ee = P.ee && g.ne;
+    if (do_pt || do_ee) traj_floats(g, cs, s);
+    if (do_pt) sh_toi<0>(g, H, Q, W, cs, s);
+    if (do_ee) sh_toi<1>(g, H, Q, W, cs, s);
   } else {
     KLAUNCH(K_SH, s, k_norm1_bound<<<g.ns, 256, 0, s>>>(g.sc_beg, g.sc_end, g.dq, P.d_sqrt / 2.0, H.safe_factor,
                                                         cs.toi_key.p));
