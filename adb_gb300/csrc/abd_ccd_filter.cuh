@@ -27,6 +27,8 @@
 #include <cuda_runtime.h>
 #include <math.h>
 
+#include "abd_exact.cuh"
+
 namespace abd {
 
 struct f3 {
@@ -135,5 +137,147 @@ CFD bool f_ee_miss(const f3* a0, const f3* a1, const f3* b0, const f3* b1) {
   const bool t = f3_dot(d0.c, d1.c) - f3m_slack(d0, d1) - 4e-6f * (v.len * v.len) * (q00.len * q10.len) > 0.f;
   return (s || t) && u.len < 1e9f && v.len < 1e9f && q00.len < 1e9f;
 }
+
+// The verification of a root in FP32: 1 passes, 0 fails, -1 not certain (the FP64 test then
+// decides). The vectors at the root's time are off by at most 2 E (their ends' error and the
+// roundings of the time and of the interpolation); the slacks are those of the certificates.
+CFD f3m f3m_at(f3 a0, f3 a1, float t, float E) {
+  f3m r;
+  r.c = f3{a0.x + t * (a1.x - a0.x), a0.y + t * (a1.y - a0.y), a0.z + t * (a1.z - a0.z)};
+  r.len = f3_len(r.c);
+  r.dev = 2.f * E;
+  return r;
+}
+CFD int f_pt_verify(f3 p0, f3 p1, const f3* t0, const f3* t1, float t) {
+  float m = fmaxf(f3_maxabs(p0), f3_maxabs(p1));
+#pragma unroll
+  for (int k = 0; k < 3; ++k) m = fmaxf(m, fmaxf(f3_maxabs(t0[k]), f3_maxabs(t1[k])));
+  const float E = 4.5e-7f * m + 1e-30f;
+  const f3m u = f3m_at(f3_sub(t0[1], t0[0]), f3_sub(t1[1], t1[0]), t, E);
+  const f3m v = f3m_at(f3_sub(t0[2], t0[0]), f3_sub(t1[2], t1[0]), t, E);
+  const f3m n = f3m_cross(u, v);
+  const float gam = (1e-6f + 1e-12f * m * m) * (n.len + n.dev);
+  bool in = u.len * v.len < 1e4f, out = false;  // larger areas round by more than a part of the tolerance
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const int b = (k + 1) % 3;
+    const f3m e = f3m_at(f3_sub(t0[b], t0[k]), f3_sub(t1[b], t1[k]), t, E);
+    const f3m r = f3m_at(f3_sub(p0, t0[k]), f3_sub(p1, t1[k]), t, E);
+    const f3m c = f3m_cross(e, r);
+    const float g = f3_dot(n.c, c.c), sl = f3m_slack(n, c) + 4e-6f * (u.len * v.len) * (e.len * r.len);
+    in &= g - sl > 0.f;
+    out |= g + sl + gam < 0.f;
+  }
+  if (!(n.len < 1e18f)) return -1;
+  return in ? 1 : (out ? 0 : -1);
+}
+CFD int f_ee_verify(const f3* a0, const f3* a1, const f3* b0, const f3* b1, float t) {
+  float m = 0.f;
+#pragma unroll
+  for (int k = 0; k < 2; ++k)
+    m = fmaxf(m, fmaxf(fmaxf(f3_maxabs(a0[k]), f3_maxabs(a1[k])), fmaxf(f3_maxabs(b0[k]), f3_maxabs(b1[k]))));
+  const float E = 4.5e-7f * m + 1e-30f;
+  const f3m u = f3m_at(f3_sub(a0[1], a0[0]), f3_sub(a1[1], a1[0]), t, E);
+  const f3m v = f3m_at(f3_sub(b0[1], b0[0]), f3_sub(b1[1], b1[0]), t, E);
+  const f3m q00 = f3m_at(f3_sub(b0[0], a0[0]), f3_sub(b1[0], a1[0]), t, E);
+  const f3m q01 = f3m_at(f3_sub(b0[1], a0[0]), f3_sub(b1[1], a1[0]), t, E);
+  const f3m q10 = f3m_at(f3_sub(b0[0], a0[1]), f3_sub(b1[0], a1[1]), t, E);
+  const f3m c0 = f3m_cross(u, q00), c1 = f3m_cross(u, q01), d0 = f3m_cross(v, q00), d1 = f3m_cross(v, q10);
+  const float c = f3_dot(c0.c, c1.c), cs = f3m_slack(c0, c1) + 4e-6f * (u.len * u.len) * (q00.len * q01.len);
+  const float d = f3_dot(d0.c, d1.c), ds = f3m_slack(d0, d1) + 4e-6f * (v.len * v.len) * (q00.len * q10.len);
+  if (!(u.len < 1e9f && v.len < 1e9f && q00.len < 1e9f)) return -1;
+  if (c - cs > 0.f || d - ds > 0.f) return 0;
+  return c + cs < 0.f && d + ds < 0.f ? 1 : -1;
+}
+
+// pt_collision_time and ee_collision_time with the roots verified in FP32 where that is
+// certain (about 220 and 100 FP64 instructions less a root). p / q: the four points at the
+// start and at the end.
+HD f3 f3_of(d3 a) { return f3{(float)a.x, (float)a.y, (float)a.z}; }
+template <int KIND>
+HD double toi_fast(const d3* p, const d3* q) {
+  double roots[3];
+  const int found = coplanar_roots(p, q, roots);
+  for (int i = 0; i < found; ++i) {
+    const double r = roots[i];
+    f3 a[4], b[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      a[k] = f3_of(p[k]);
+      b[k] = f3_of(q[k]);
+    }
+    int ok = KIND == 0 ? f_pt_verify(a[0], b[0], a + 1, b + 1, (float)r) : f_ee_verify(a, b, a + 2, b + 2, (float)r);
+    if (ok < 0) {
+      d3 x[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) x[k] = lerp(q[k], p[k], r);
+      ok = KIND == 0 ? verify_root_pt(x[0], x[1], x[2], x[3]) : verify_root_ee(x[0], x[1], x[2], x[3]);
+    }
+    if (ok) return r;
+  }
+  return 1.0;
+}
+
+#ifdef __CUDACC__
+// Times of impact of n trajectories (24 doubles each: four points at the start, four at the
+// end; KIND 0: point-triangle, 1: edge-edge) into toi, calling min_of with each time below 1.
+// A warp takes 32 trajectories at a time (grid-stride), certifies them in FP32 and queues the
+// others (64 slots of shared memory a warp); as soon as 32 wait it runs the FP64 test on
+// them, so that test always has a full warp.
+template <int KIND, typename F>
+__device__ __forceinline__ void toi_stream(int n, const double* x, double* toi, int* queue, F&& min_of) {
+  const int lane = threadIdx.x & 31;
+  const int warps = (int)((gridDim.x * blockDim.x) >> 5), warp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+  const unsigned below = (1u << lane) - 1u;
+  int waiting = 0;
+  for (int c = warp;; c += warps) {
+    const bool last = (long long)c * 32 >= n;
+    if (!last) {
+      const int i = c * 32 + lane;
+      bool keep = false;
+      if (i < n) {
+        const double* p = x + 24 * (size_t)i;
+        f3 a[4], b[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          a[k] = f3{(float)p[3 * k], (float)p[3 * k + 1], (float)p[3 * k + 2]};
+          b[k] = f3{(float)p[12 + 3 * k], (float)p[13 + 3 * k], (float)p[14 + 3 * k]};
+        }
+        keep = !(KIND == 0 ? f_pt_miss(a[0], b[0], a + 1, b + 1) : f_ee_miss(a, b, a + 2, b + 2));
+        if (!keep) toi[i] = 1.0;
+      }
+      const unsigned m = __ballot_sync(0xffffffffu, keep);
+      if (keep) queue[waiting + __popc(m & below)] = i;
+      waiting += __popc(m);
+      __syncwarp();
+    }
+    if (waiting >= 32 || (last && waiting > 0)) {
+      const int take = waiting < 32 ? waiting : 32;
+      if (lane < take) {
+        const int i = queue[waiting - take + lane];
+        const double* p = x + 24 * (size_t)i;
+        d3 a[4], b[4];
+#pragma unroll
+        for (int v = 0; v < 4; ++v) {
+          a[v] = mk(p[3 * v], p[3 * v + 1], p[3 * v + 2]);
+          b[v] = mk(p[12 + 3 * v], p[13 + 3 * v], p[14 + 3 * v]);
+        }
+        const double t = toi_fast<KIND>(a, b);
+        toi[i] = t;
+        if (t < 1.0) min_of(t);
+      }
+      waiting -= take;
+      __syncwarp();
+    }
+    if (last) break;
+  }
+}
+// Blocks of a streamed batch: a warp per 32 trajectories until every SM has the `per` CTAs
+// that its registers allow.
+inline int toi_blocks(int n, int threads, int per) {
+  const int b = (n + threads - 1) / threads;
+  return b < 152 * per ? b : 152 * per;
+}
+#endif
 
 }  // namespace abd

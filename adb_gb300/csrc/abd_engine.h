@@ -117,6 +117,8 @@ struct CullScratch {
   DBuf<unsigned long long> stage_key;   // sorted accepted pairs per overlap (sub, i, j)
   DBuf<int8_t> stage_ty;
   DBuf<unsigned long long> toi_key;     // 2 per scene: pt/ee, ground
+  DBuf<int2> toi_cand;                  // trajectory candidates left to the FP64 test, and their number
+  DBuf<unsigned> toi_n;
   DBuf<int> tmp_int;
   DBuf<long long> tmp_ll;
   // autotuned narrow-phase variants (index into the step table; -1 = not tuned yet) of the

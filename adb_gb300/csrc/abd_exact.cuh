@@ -318,79 +318,72 @@ HD void deflate3(const double* c, double r, double* o) {
   o[0] = XA(c[1], XM(r, o[1]));
 }
 
+// The interval that holds the first root is chosen first and refined at one place, so that the
+// threads of a warp refine together whatever case each is in (refined at the eight places
+// where the cases arise, a warp paid for each case in turn).
 HD int cubic_roots(double* roots, const double* c, double x0, double x1, double xe = 6e-7) {
   double y0 = poly3(c, x0), y1 = poly3(c, x1);
   double a = XM(c[3], 3.0), b2 = c[2], cc = c[1];
   double dc[3] = {cc, XM(2.0, b2), a};
   double delta = XS(XM(b2, b2), XM(a, cc));
+  bool has = false, more = false;          // a first root in [l, h]; others beyond `from`
+  double l = x0, h = x1, yl = y0, from = x1;
   if (delta > 0) {
     double d2 = XSQRT(delta);
     double q = -XA(b2, sgn_mul(d2, b2));
     double rv0 = XD(q, a), rv1 = XD(cc, q);
     double xa = mn_(rv0, rv1), xb = mx_(rv0, rv1);
-    if (diff_sign(y0, y1)) {
-      if (xa >= x1 || xb <= x0 || (xa <= x0 && xb >= x1)) {
-        roots[0] = cubic_bracketed(c, dc, x0, x1, y0, xe);
-        return 1;
-      }
-    } else {
-      if ((xa >= x1 || xb <= x0) || (xa <= x0 && xb >= x1)) return 0;
-    }
-    if (xa > x0) {
+    const bool mono = xa >= x1 || xb <= x0 || (xa <= x0 && xb >= x1);
+    if (mono) {
+      has = diff_sign(y0, y1);
+    } else if (xa > x0) {
       double ya = poly3(c, xa);
       if (diff_sign(y0, ya)) {
-        roots[0] = cubic_bracketed(c, dc, x0, xa, y0, xe);
-        if (diff_sign(ya, y1) || (xb < x1 && diff_sign(ya, poly3(c, xb)))) {
-          double dp[3];
-          deflate3(c, roots[0], dp);
-          return quadratic_roots(roots + 1, dp, xa, x1) + 1;
-        }
-        return 1;
-      }
-      if (xb < x1) {
+        has = true;
+        h = xa;
+        from = xa;
+        more = diff_sign(ya, y1) || (xb < x1 && diff_sign(ya, poly3(c, xb)));
+      } else if (xb < x1) {
         double yb = poly3(c, xb);
+        from = xb;
         if (diff_sign(ya, yb)) {
-          roots[0] = cubic_bracketed(c, dc, xa, xb, ya, xe);
-          if (diff_sign(yb, y1)) {
-            double dp[3];
-            deflate3(c, roots[0], dp);
-            return quadratic_roots(roots + 1, dp, xb, x1) + 1;
-          }
-          return 1;
-        }
-        if (diff_sign(yb, y1)) {
-          roots[0] = cubic_bracketed(c, dc, xb, x1, yb, xe);
-          return 1;
+          has = true;
+          l = xa;
+          h = xb;
+          yl = ya;
+          more = diff_sign(yb, y1);
+        } else {
+          has = diff_sign(yb, y1);
+          l = xb;
+          yl = yb;
         }
       } else {
-        if (diff_sign(ya, y1)) {
-          roots[0] = cubic_bracketed(c, dc, xa, x1, ya, xe);
-          return 1;
-        }
+        has = diff_sign(ya, y1);
+        l = xa;
+        yl = ya;
       }
     } else {
       double yb = poly3(c, xb);
+      from = xb;
       if (diff_sign(y0, yb)) {
-        roots[0] = cubic_bracketed(c, dc, x0, xb, y0, xe);
-        if (diff_sign(yb, y1)) {
-          double dp[3];
-          deflate3(c, roots[0], dp);
-          return quadratic_roots(roots + 1, dp, xb, x1) + 1;
-        }
-        return 1;
-      }
-      if (diff_sign(yb, y1)) {
-        roots[0] = cubic_bracketed(c, dc, xb, x1, yb, xe);
-        return 1;
+        has = true;
+        h = xb;
+        more = diff_sign(yb, y1);
+      } else {
+        has = diff_sign(yb, y1);
+        l = xb;
+        yl = yb;
       }
     }
-    return 0;
+  } else {
+    has = diff_sign(y0, y1);
   }
-  if (diff_sign(y0, y1)) {
-    roots[0] = cubic_bracketed(c, dc, x0, x1, y0, xe);
-    return 1;
-  }
-  return 0;
+  if (!has) return 0;
+  roots[0] = cubic_bracketed(c, dc, l, h, yl, xe);
+  if (!more) return 1;
+  double dp[3];
+  deflate3(c, roots[0], dp);
+  return quadratic_roots(roots + 1, dp, from, x1) + 1;
 }
 
 // Coplanarity cubic det[p1-p0, p2-p0, p3-p0](t) accumulated as the alternating sum of

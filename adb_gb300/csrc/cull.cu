@@ -19,6 +19,7 @@
 // tests first run on float copies of the boxes rounded outward (__double2float_rd/_ru):
 // a float miss implies an exact miss, so the float prefilter never changes the result
 // and saves the scarce FP64 pipe (GB300: 1.2 TFLOP/s FP64 vs 70 TFLOP/s FP32).
+#include "abd_ccd_filter.cuh"
 #include "abd_engine.h"
 #include "abd_exact.cuh"
 
@@ -551,20 +552,63 @@ __device__ __forceinline__ bool f_reject_v(const float* vb, int sub, int v0, int
 // Trajectory time of impact of one candidate (vtn 3), exact box test included.
 __device__ __forceinline__ double exact_toi(const Geo& g, int sub, int pa, int pb) {
   int nv = g.nv;
+  d3 p[4], q[4];  // at q and at the target
   if (sub < 2) {
-    d3 v1 = ldX(g.X, nv, pa), v0 = ldX(g.Xq, nv, pa);
-    int i0 = g.fv[3 * pb], i1 = g.fv[3 * pb + 1], i2 = g.fv[3 * pb + 2];
-    d3 f1[3] = {ldX(g.X, nv, i0), ldX(g.X, nv, i1), ldX(g.X, nv, i2)};
-    d3 f0[3] = {ldX(g.Xq, nv, i0), ldX(g.Xq, nv, i1), ldX(g.Xq, nv, i2)};
-    if (!overlaps(box2(v0, v1), merge(box3(f0[0], f0[1], f0[2]), box3(f1[0], f1[1], f1[2])))) return 1.0;
-    return pt_collision_time(v0, f0, v1, f1);
+    const int vid[4] = {pa, g.fv[3 * pb], g.fv[3 * pb + 1], g.fv[3 * pb + 2]};
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      p[k] = ldX(g.Xq, nv, vid[k]);
+      q[k] = ldX(g.X, nv, vid[k]);
+    }
+    if (!overlaps(box2(p[0], q[0]), merge(box3(p[1], p[2], p[3]), box3(q[1], q[2], q[3])))) return 1.0;
+    return toi_fast<0>(p, q);
   }
-  int a0 = g.ev[2 * pa], a1 = g.ev[2 * pa + 1], b0 = g.ev[2 * pb], b1 = g.ev[2 * pb + 1];
-  d3 A1[2] = {ldX(g.X, nv, a0), ldX(g.X, nv, a1)}, A0[2] = {ldX(g.Xq, nv, a0), ldX(g.Xq, nv, a1)};
-  d3 B1[2] = {ldX(g.X, nv, b0), ldX(g.X, nv, b1)}, B0[2] = {ldX(g.Xq, nv, b0), ldX(g.Xq, nv, b1)};
-  if (!overlaps(box4(A0[0], A0[1], A1[0], A1[1]), box4(B0[0], B0[1], B1[0], B1[1]))) return 1.0;
-  return ee_collision_time(A0, B0, A1, B1);
+  const int vid[4] = {g.ev[2 * pa], g.ev[2 * pa + 1], g.ev[2 * pb], g.ev[2 * pb + 1]};
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    p[k] = ldX(g.Xq, nv, vid[k]);
+    q[k] = ldX(g.X, nv, vid[k]);
+  }
+  if (!overlaps(box4(p[0], p[1], q[0], q[1]), box4(p[2], p[3], q[2], q[3]))) return 1.0;
+  return toi_fast<1>(p, q);
 }
+
+// Certificate that exact_toi of the candidate is 1, from the vertices' float positions at q
+// and at the target (6 floats each).
+__device__ __forceinline__ f3 ldf3(const float* p) { return f3{p[0], p[1], p[2]}; }
+__device__ __forceinline__ bool f_toi_miss(const Geo& g, const float* ve, int sub, int pa, int pb) {
+  if (sub < 2) {
+    f3 t0[3], t1[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const float* p = ve + 6 * (size_t)g.fv[3 * pb + k];
+      t0[k] = ldf3(p);
+      t1[k] = ldf3(p + 3);
+    }
+    const float* p = ve + 6 * (size_t)pa;
+    return f_pt_miss(ldf3(p), ldf3(p + 3), t0, t1);
+  }
+  f3 a0[2], a1[2], b0[2], b1[2];
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    const float *p = ve + 6 * (size_t)g.ev[2 * pa + k], *q = ve + 6 * (size_t)g.ev[2 * pb + k];
+    a0[k] = ldf3(p);
+    a1[k] = ldf3(p + 3);
+    b0[k] = ldf3(q);
+    b1[k] = ldf3(q + 3);
+  }
+  return f_ee_miss(a0, a1, b0, b1);
+}
+
+// Candidates of the trajectory narrow phase left to the FP64 test: (point, face) or (~edge,
+// edge) by their global ids.
+struct ToiCand {
+  const float* ve;   // float positions of the vertices at q and at the target
+  int2* cand;
+  unsigned* n;
+  unsigned cap;
+};
+constexpr unsigned kToiCand = 1u << 21;  // 16 MB; a candidate past it is evaluated where it is found
 
 struct NarrowOut {
   int *pt, *pt_ov, *ee, *ee_ov;
@@ -755,6 +799,20 @@ __global__ void k_order_place(int nov, const int* cnt, int* bc, int* order) {
   order[base + atomicAdd(&bc[NBUCKET + b], 1)] = u;
 }
 
+// The FP64 test of one candidate into its scene's key.
+__device__ __noinline__ void toi_one(const Geo& g, int sub, int pa, int pb, unsigned long long* toi_key) {
+  const double t = exact_toi(g, sub, pa, pb);
+  if (t < 1.0) atomicMin(toi_key + 2 * g.bscene[g.vbody[sub < 2 ? pa : g.ev[2 * pa]]], dkey(t));
+}
+__global__ void __launch_bounds__(128) k_toi_list(Geo g, ToiCand tc, unsigned long long* toi_key) {
+  const unsigned n = min(*tc.n, tc.cap);
+  for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
+    const int2 c = tc.cand[t];
+    if (c.x >= 0) toi_one(g, 0, c.x, c.y, toi_key);
+    else toi_one(g, 2, ~c.x, c.y, toi_key);
+  }
+}
+
 // 5a. Narrow phase, one CTA per overlap, count (MODE 0) or trajectory TOI (MODE 2).
 // For each sub-problem (v(I) x f(J), v(J) x f(I), e(I) x e(J)) the float boxes of both
 // lists are staged in shared memory. The work alternates between two phases so that the
@@ -764,13 +822,18 @@ __global__ void k_order_place(int nov, const int* cnt, int* bc, int* order) {
 //    float-box hits to a shared queue (warp-aggregated);
 //  - exact phase: the whole CTA takes the queued candidates round-robin for the exact
 //    FP64 test (MODE 0: box, lower bounds, type and distance; MODE 2: time of impact).
+// MODE 2 runs no FP64 here: it drops the candidates that an FP32 certificate proves to have no
+// time of impact (abd_ccd_filter.cuh; on the pile about 19 of 20) and appends the others to a
+// list that k_toi_list evaluates. An FP64 test is a chain of about 900 instructions of 64
+// cycles a warp, some 28 us, which a CTA with a handful of candidates per box phase used to
+// pay for each of its phases; the list fills whole warps on all SMs.
 template <int MODE, int STEP>
-__global__ void __launch_bounds__(NT, (MODE == 2 && STEP <= 36) ? 3 : 2) k_narrow_scan(Geo g, Params P, float ds_f, const int* ovI, const int* ovJ,
+__global__ void __launch_bounds__(NT, (MODE == 2 && STEP <= 36) ? 4 : 2) k_narrow_scan(Geo g, Params P, float ds_f, const int* ovI, const int* ovJ,
                                                     int* cnt, const int* off, int* lst, const float* vb,
                                                     const float* eb, const float* fb, int* sub_cnt,
                                                     unsigned long long* toi_key, unsigned long long* stage_key,
                                                     int8_t* stage_ty, int* stage_off, int* stage_total,
-                                                    int stage_cap, const int* order) {
+                                                    int stage_cap, const int* order, ToiCand tc) {
   extern __shared__ __align__(16) unsigned char smem_dyn[];
   unsigned long long* recK = reinterpret_cast<unsigned long long*>(smem_dyn);  // REC_CAP (MODE 0)
   float* sA = reinterpret_cast<float*>(smem_dyn + (MODE == 0 ? REC_CAP * sizeof(unsigned long long) : 0));
@@ -788,7 +851,6 @@ __global__ void __launch_bounds__(NT, (MODE == 2 && STEP <= 36) ? 3 : 2) k_narro
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const unsigned below = (1u << lane) - 1u;
   int c3s[3] = {0, 0, 0};
-  double tmin = 1.0;
   if (threadIdx.x == 0) {
     rec_n = 0;
     sq_n[0] = 0;
@@ -859,8 +921,11 @@ __global__ void __launch_bounds__(NT, (MODE == 2 && STEP <= 36) ? 3 : 2) k_narro
             int i = (int)(code >> 16), j = (int)(code & 0xffffu);
             if (i >= ca || j >= cb) continue;
             if (MODE == 2) {
-              int pa = L.offA + L.LA[a0 + i], pb = L.offB + L.LB[b0 + j];
-              tmin = dmin(tmin, exact_toi(g, sub, pa, pb));
+              const int pa = L.offA + L.LA[a0 + i], pb = L.offB + L.LB[b0 + j];
+              if (f_toi_miss(g, tc.ve, sub, pa, pb)) continue;
+              const unsigned o = atomicAdd(tc.n, 1u);
+              if (o < tc.cap) tc.cand[o] = make_int2(sub < 2 ? pa : ~pa, pb);
+              else toi_one(g, sub, pa, pb, toi_key);
             } else {
               const int w0 = sVA[2 * i];
               const int w1 = sub < 2 ? sVB[3 * j] : sVA[2 * i + 1];
@@ -945,10 +1010,6 @@ __global__ void __launch_bounds__(NT, (MODE == 2 && STEP <= 36) ? 3 : 2) k_narro
         stage_key[rec_base + k] = recK[k];
         stage_ty[rec_base + k] = recT[k];
       }
-  } else {
-#pragma unroll
-    for (int q = 16; q > 0; q >>= 1) tmin = dmin(tmin, __shfl_xor_sync(0xffffffffu, tmin, q));
-    if (lane == 0 && tmin < 1.0) atomicMin(toi_key + 2 * g.bscene[ovI[u]], dkey(tmin));
   }
 }
 
@@ -1163,6 +1224,7 @@ struct NarrowLaunch {
   int *stage_off, *stage_total;
   int stage_cap;
   const int* order;
+  ToiCand tc;
 };
 
 // k_narrow_scan<mode, kNarrowStep[mode][variant]> over nov overlaps
@@ -1171,7 +1233,7 @@ static void launch_narrow(int mode, int variant, int nov, const NarrowLaunch& a,
 #define ABD_NARROW_LAUNCH(M, ST)                                                                                   \
   KLAUNCH(tag, s, k_narrow_scan<M, ST><<<nov, NT, narrow_smem(M, ST), s>>>(                                       \
                       a.g, a.P, a.ds_f, a.ovI, a.ovJ, a.cnt, a.off, a.lst, a.vb, a.eb, a.fb, a.sub_cnt, a.toi_key, \
-                      a.stage_key, a.stage_ty, a.stage_off, a.stage_total, a.stage_cap, a.order))
+                      a.stage_key, a.stage_ty, a.stage_off, a.stage_total, a.stage_cap, a.order, a.tc))
   const int st = kNarrowStep[mode == 2 ? 1 : 0][variant];
   if (mode == 2) {
     if (st == 24) ABD_NARROW_LAUNCH(2, 24);
@@ -1194,6 +1256,7 @@ constexpr int kTuneMinOverlaps = 64;
 static void narrow_phase(int mode, int nov, const NarrowLaunch& a, CullScratch& cs, int* reset, cudaStream_t s) {
   const int m = mode == 2 ? 1 : 0;
   if (cs.narrow_variant[m] >= 0 || !cs.autotune || nov < kTuneMinOverlaps) {
+    CK(cudaMemsetAsync(reset, 0, 2 * sizeof(int), s));
     launch_narrow(mode, cs.narrow_variant[m] >= 0 ? cs.narrow_variant[m] : kNarrowDefault, nov, a, s);
     return;
   }
@@ -1201,7 +1264,7 @@ static void narrow_phase(int mode, int nov, const NarrowLaunch& a, CullScratch& 
   for (auto& e : ev) CK(cudaEventCreate(&e));
   CK(cudaEventRecord(ev[0], s));
   for (int v = 0; v < kNarrowVariants; ++v) {
-    if (reset) CK(cudaMemsetAsync(reset, 0, 2 * sizeof(int), s));
+    CK(cudaMemsetAsync(reset, 0, 2 * sizeof(int), s));
     launch_narrow(mode, v, nov, a, s);
     CK(cudaEventRecord(ev[v + 1], s));
   }
@@ -1287,11 +1350,10 @@ static void narrow_pairs(const Geo& g, const Params& P, float ds_f, int nov, con
     cs.stage_ty.ensure(1u << 16);
   }
   for (int attempt = 0; attempt < 4; ++attempt) {
-    CK(cudaMemsetAsync(d_tot + 6, 0, 2 * sizeof(int), s));
     narrow_smem_attr();
     NarrowLaunch a{g, P, ds_f, ovI, ovJ, cs.bin_cnt.p, cs.bin_off.p, cs.lst.p, cs.vbox.p, cs.ebox.p, cs.fbox.p,
                    cs.sub_cnt.p, nullptr, cs.stage_key.p, cs.stage_ty.p, cs.stage_off.p, d_tot + 6,
-                   (int)cs.stage_key.cap, cs.order.p};
+                   (int)cs.stage_key.cap, cs.order.p, ToiCand{}};
     narrow_phase(0, nov, a, cs, d_tot + 6, s);
     // per-overlap pair counts and their offsets, read together with the staged total
     KLAUNCH(K_NARROW_WRITE, s, k_sub_totals<<<nblk(nov, 256), 256, 0, s>>>(nov, cs.sub_cnt.p, cs.blk_a.p, cs.blk_b.p));
@@ -1435,9 +1497,14 @@ void cull(const Geo& g_in, const Params& P, int vtn, double alpha, CullScratch& 
                                                                                          cs.fbox.p));
       order_overlaps(nov, cs, s, K_NARROW_TOI);
       narrow_smem_attr();
+      traj_floats(g, cs, s);  // allocates cs.vend: before its address is taken
+      cs.toi_cand.ensure(kToiCand);
+      cs.toi_n.ensure(2);
       NarrowLaunch a{g, P, ds_f, S.ovI.p, S.ovJ.p, cs.bin_cnt.p, cs.bin_off.p, cs.lst.p, cs.vbox.p, cs.ebox.p,
-                     cs.fbox.p, nullptr, cs.toi_key.p, nullptr, nullptr, nullptr, nullptr, 0, cs.order.p};
-      narrow_phase(2, nov, a, cs, nullptr, s);
+                     cs.fbox.p, nullptr, cs.toi_key.p, nullptr, nullptr, nullptr, nullptr, 0, cs.order.p,
+                     ToiCand{cs.vend.p, cs.toi_cand.p, cs.toi_n.p, kToiCand}};
+      narrow_phase(2, nov, a, cs, reinterpret_cast<int*>(cs.toi_n.p), s);
+      KLAUNCH(K_NARROW_TOI, s, k_toi_list<<<1216, 128, 0, s>>>(g, a.tc, cs.toi_key.p));
     }
     if (P.ground && g.nv) {
       KLAUNCH(K_VG_TOI, s, k_vg_toi<<<nblk(g.nv, 256), 256, 0, s>>>(g, P, cs.toi_key.p + 1));

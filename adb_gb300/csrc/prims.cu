@@ -4,6 +4,7 @@
 // the FP64 throughput probe used as the roofline denominator of FP64-bound kernels.
 #include <vector>
 
+#include "abd_ccd_filter.cuh"
 #include "abd_engine.h"
 #include "abd_ipc.cuh"
 
@@ -65,18 +66,11 @@ __global__ void k_hess(int kind, int n, const double* x, const int* type, const 
   }
 }
 
-__global__ void k_toi(int kind, int n, const double* x, double* toi) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const double* p = x + 24 * i;
-  d3 a[4] = {ld12(p, 0), ld12(p, 1), ld12(p, 2), ld12(p, 3)};
-  d3 b[4] = {ld12(p, 4), ld12(p, 5), ld12(p, 6), ld12(p, 7)};
-  if (kind == 0) {
-    toi[i] = pt_collision_time(a[0], a + 1, b[0], b + 1);
-  } else {
-    d3 ei0[2] = {a[0], a[1]}, ej0[2] = {a[2], a[3]}, ei1[2] = {b[0], b[1]}, ej1[2] = {b[2], b[3]};
-    toi[i] = ee_collision_time(ei0, ej0, ei1, ej1);
-  }
+constexpr int TOI_THREADS = 128;
+template <int KIND>
+__global__ void __launch_bounds__(TOI_THREADS, 3) k_toi(int n, const double* x, double* toi) {
+  __shared__ int queue[TOI_THREADS / 32][64];
+  toi_stream<KIND>(n, x, toi, queue[threadIdx.x >> 5], [](double) {});
 }
 
 // Independent FMA chains; result stored per thread so nothing is optimised away.
@@ -139,7 +133,9 @@ int toi_batch(int kind, int n, const double* x, double* toi) {
   return guard([&]() {
     DevArr<double> dx(24 * (size_t)n), dt(n);
     CK(cudaMemcpy(dx.p, x, 24 * (size_t)n * sizeof(double), cudaMemcpyHostToDevice));
-    k_toi<<<nblk(n, 128), 128>>>(kind, n, dx.p, dt.p);
+    const int blocks = toi_blocks(n, TOI_THREADS, 3);
+    if (kind == 0) k_toi<0><<<blocks, TOI_THREADS>>>(n, dx.p, dt.p);
+    else k_toi<1><<<blocks, TOI_THREADS>>>(n, dx.p, dt.p);
     CK(cudaGetLastError());
     CK(cudaMemcpy(toi, dt.p, n * sizeof(double), cudaMemcpyDeviceToHost));
   });

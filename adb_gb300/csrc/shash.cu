@@ -333,21 +333,24 @@ __global__ void __launch_bounds__(128) k_sh_toi(Geo g, ShQuery Q, unsigned long 
   const int n = (int)min(Q.n[0], Q.cand_cap);
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
     const int q = Q.cand[t].x, e = Q.cand[t].y;
-    double tc;
-    int J;
+    int vid[4];
     if (KIND == 0) {
-      const int i0 = g.fv[3 * q], i1 = g.fv[3 * q + 1], i2 = g.fv[3 * q + 2];
-      J = g.vbody[i0];
-      const d3 f0[3] = {ldX(g.Xq, g.nv, i0), ldX(g.Xq, g.nv, i1), ldX(g.Xq, g.nv, i2)};
-      const d3 f1[3] = {ldX(g.X, g.nv, i0), ldX(g.X, g.nv, i1), ldX(g.X, g.nv, i2)};
-      tc = pt_collision_time(ldX(g.Xq, g.nv, e), f0, ldX(g.X, g.nv, e), f1);
+      vid[0] = e;
+      for (int k = 0; k < 3; ++k) vid[1 + k] = g.fv[3 * q + k];
     } else {
-      const int ia0 = g.ev[2 * e], ia1 = g.ev[2 * e + 1], ib0 = g.ev[2 * q], ib1 = g.ev[2 * q + 1];
-      J = g.vbody[ib0];
-      const d3 a0[2] = {ldX(g.Xq, g.nv, ia0), ldX(g.Xq, g.nv, ia1)}, a1[2] = {ldX(g.X, g.nv, ia0), ldX(g.X, g.nv, ia1)};
-      const d3 b0[2] = {ldX(g.Xq, g.nv, ib0), ldX(g.Xq, g.nv, ib1)}, b1[2] = {ldX(g.X, g.nv, ib0), ldX(g.X, g.nv, ib1)};
-      tc = ee_collision_time(a0, b0, a1, b1);
+      for (int k = 0; k < 2; ++k) {
+        vid[k] = g.ev[2 * e + k];
+        vid[2 + k] = g.ev[2 * q + k];
+      }
     }
+    const int J = g.vbody[vid[3]];
+    d3 p0[4], p1[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      p0[k] = ldX(g.Xq, g.nv, vid[k]);
+      p1[k] = ldX(g.X, g.nv, vid[k]);
+    }
+    const double tc = toi_fast<KIND>(p0, p1);
     if (tc < 1.0) atomicMin(toi_key + 2 * g.bscene[J], dkey(tc));
   }
 }
