@@ -453,6 +453,326 @@ DEV bool psd_project_small(double (&S)[N][N]) {
   return true;
 }
 
+// ---- 9 x 9 projection by one warp (mollified edge-edge pairs) ----
+// Cyclic Jacobi by rounds: round r of a sweep rotates the four disjoint index pairs with
+// i + j = r (mod 9), the index with 2 k = r sitting out, so a sweep is 9 rounds instead of 36
+// rotations one after the other. A rotation is a chain of about 25 dependent FP64 instructions
+// of 64 cycles; the sweeps before the last two run in FP32 on a copy scaled to unit size, where
+// an instruction takes 4, and the FP64 sweeps start from its eigenvectors, made orthonormal in
+// FP64 by two Newton-Schulz steps (off by e, they leave 3/8 e^2 each: 1e-6 -> 1e-24). The stop
+// test of the FP64 sweeps is the one of a Jacobi from the identity.
+struct Jac9 {
+  double S[9][9];              // the matrix
+  double A[2][9][9], V[2][9][9];
+  float Af[2][9][9], Vf[2][9][9];
+  double c[9], sg[9], dl[9];   // per index: cosine, signed sine, change of the diagonal entry
+  float cf[9], sgf[9], dlf[9];
+  int pr[9];                   // partner
+};
+DEV void jac9_rotation(double h, double apq, double& t, double& c, double& s) {
+  const double sa = h >= 0 ? apq : -apq;
+  const double r2 = fma(h, h, apq * apq);
+  if (r2 >= 1e-300) {  // as in psd_project_small
+    const double g = rsqrt(r2);
+    const double c2 = 0.5 * fma(r2, g, fabs(h)) * g;
+    const double ic = rsqrt(c2);
+    s = 0.5 * sa * g * ic;
+    c = c2 * ic;
+    t = s * ic;
+  } else {
+    const double den = fabs(h) + sqrt(r2);
+    t = den > 0.0 ? sa / den : 0.0;
+    c = rsqrt(1.0 + t * t);
+    s = t * c;
+  }
+}
+DEV void jac9_rotation(float h, float apq, float& t, float& c, float& s) {
+  const float den = fabsf(h) + sqrtf(h * h + apq * apq);
+  t = den > 0.f ? __fdividef(h >= 0.f ? apq : -apq, den) : 0.f;
+  c = rsqrtf(1.f + t * t);
+  s = t * c;
+}
+// Entry e of the upper triangle of a 9 x 9 matrix, row by row: (i, j).
+DEV void jac9_tri(int e, int& i, int& j) {
+  i = 0;
+  while (e >= 9 - i) {
+    e -= 9 - i;
+    ++i;
+  }
+  j = i + e;
+}
+// Sweeps of the warp over A (symmetric, both triangles kept) accumulating V, until the
+// off-diagonal mass is at most `stop` of the total or `most` sweeps are done; returns the
+// buffer (0 or 1) that holds the result.
+template <typename T>
+DEV int jac9_sweeps(T (*A)[9][9], T (*V)[9][9], T* c, T* sg, T* dl, int* pr, T stop, int most, bool skip_small) {
+  const int lane = threadIdx.x & 31;
+  int cur = 0;
+  int ti[2], tj[2];
+  jac9_tri(lane, ti[0], tj[0]);
+  jac9_tri(lane < 13 ? lane + 32 : 44, ti[1], tj[1]);
+  for (int sweep = 0; sweep < most; ++sweep) {
+    T off = 0, dg = 0;
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      if (k == 1 && lane >= 13) continue;
+      const T v = A[cur][ti[k]][tj[k]];
+      if (ti[k] == tj[k]) dg += v * v;
+      else off += v * v;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      off += __shfl_xor_sync(0xffffffffu, off, o);
+      dg += __shfl_xor_sync(0xffffffffu, dg, o);
+    }
+    if (off == T(0) || 2 * off <= stop * (dg + 2 * off)) break;
+    for (int r = 0; r < 9; ++r) {
+      if (lane < 5) {
+        const int k0 = (5 * r) % 9;
+        if (lane == 4) {  // the index that sits out
+          c[k0] = T(1);
+          sg[k0] = T(0);
+          dl[k0] = T(0);
+          pr[k0] = k0;
+        } else {
+          const int x = (k0 + lane + 1) % 9, y = (k0 + 8 - lane) % 9;
+          const int p = x < y ? x : y, q = x < y ? y : x;
+          const T apq = A[cur][p][q], app = A[cur][p][p], aqq = A[cur][q][q];
+          T t = 0, cc = 1, s = 0;
+          bool rot = apq != T(0);
+          if (skip_small && sweep > 2) {
+            const T g = T(100) * fabs(apq);
+            rot = rot && !(fabs(app) + g == fabs(app) && fabs(aqq) + g == fabs(aqq));
+          }
+          if (rot) jac9_rotation(T(0.5) * (aqq - app), apq, t, cc, s);
+          c[p] = cc;
+          c[q] = cc;
+          sg[p] = -s;
+          sg[q] = s;
+          dl[p] = -t * apq;
+          dl[q] = t * apq;
+          pr[p] = q;
+          pr[q] = p;
+        }
+      }
+      __syncwarp();
+      T(*a)[9] = A[cur];
+      T(*b)[9] = A[cur ^ 1];
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        if (k == 1 && lane >= 13) continue;
+        const int i = ti[k], j = tj[k], pi = pr[i], pj = pr[j];
+        T v;
+        if (i == j) {
+          v = a[i][i] + dl[i];
+        } else if (pi == j) {
+          v = T(0);
+        } else {
+          const T cj = c[j], sj = sg[j];
+          v = c[i] * (cj * a[i][j] + sj * a[i][pj]) + sg[i] * (cj * a[pi][j] + sj * a[pi][pj]);
+        }
+        b[i][j] = v;
+        b[j][i] = v;
+      }
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        const int e = lane + 32 * k;
+        if (e < 81) {
+          const int i = e / 9, j = e - 9 * i;
+          V[cur ^ 1][i][j] = c[j] * V[cur][i][j] + sg[j] * V[cur][i][pr[j]];
+        }
+      }
+      cur ^= 1;
+      __syncwarp();
+    }
+  }
+  return cur;
+}
+// C = X^T Y over the lanes (entries e = lane, lane + 32, lane + 64), or X Y.
+template <bool TRANS>
+DEV void jac9_mul(const double (*X)[9], const double (*Y)[9], double (*C)[9]) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const int e = lane + 32 * k;
+    if (e < 81) {
+      const int i = e / 9, j = e - 9 * i;
+      double v = 0.0;
+#pragma unroll
+      for (int m = 0; m < 9; ++m) v += (TRANS ? X[m][i] : X[i][m]) * Y[m][j];
+      C[i][j] = v;
+    }
+  }
+  __syncwarp();
+}
+// Projects w.S; returns in `neg` whether an eigenvalue was negative and the buffer with the
+// eigenvectors (columns) and eigenvalues (diagonal). Called by a whole warp after a __syncwarp.
+DEV int jac9_project(Jac9& w, bool& neg) {
+  const int lane = threadIdx.x & 31;
+  float mx = 0.f;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const int e = lane + 32 * k;
+    if (e < 81) mx = fmaxf(mx, fabsf(__double2float_rn(w.S[e / 9][e % 9])));
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  bool start = mx > 1e-30f && mx < 1e30f;  // else (or not finite): from the identity
+  if (start) {
+    const float sc = 1.f / mx;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const int e = lane + 32 * k;
+      if (e < 81) {
+        w.Af[0][e / 9][e % 9] = __double2float_rn(w.S[e / 9][e % 9]) * sc;
+        w.Vf[0][e / 9][e % 9] = e / 9 == e % 9 ? 1.f : 0.f;
+      }
+    }
+    __syncwarp();
+    const int f = jac9_sweeps<float>(w.Af, w.Vf, w.cf, w.sgf, w.dlf, w.pr, 1e-12f, 8, false);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const int e = lane + 32 * k;
+      if (e < 81) w.V[0][e / 9][e % 9] = (double)w.Vf[f][e / 9][e % 9];
+    }
+    __syncwarp();
+    for (int it = 0; it < 2; ++it) {  // V <- V (3 I - V^T V) / 2
+      jac9_mul<true>(w.V[0], w.V[0], w.A[0]);
+      bool bad = false;
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        const int e = lane + 32 * k;
+        if (e < 81) {
+          const double g = w.A[0][e / 9][e % 9], id = e / 9 == e % 9 ? 1.0 : 0.0;
+          bad |= !(fabs(g - id) <= 1e-5);
+          w.A[1][e / 9][e % 9] = 1.5 * id - 0.5 * g;
+        }
+      }
+      start = __all_sync(0xffffffffu, !bad);
+      __syncwarp();
+      if (!start) break;
+      jac9_mul<false>(w.V[0], w.A[1], w.V[1]);
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        const int e = lane + 32 * k;
+        if (e < 81) w.V[0][e / 9][e % 9] = w.V[1][e / 9][e % 9];
+      }
+      __syncwarp();
+    }
+  }
+  if (start) {
+    jac9_mul<false>(w.S, w.V[0], w.A[1]);
+    jac9_mul<true>(w.V[0], w.A[1], w.A[0]);
+    // both triangles from the upper one
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      if (k == 1 && lane >= 13) continue;
+      int i, j;
+      jac9_tri(lane + 32 * k, i, j);
+      w.A[0][j][i] = w.A[0][i][j];
+    }
+  } else {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const int e = lane + 32 * k;
+      if (e < 81) {
+        w.A[0][e / 9][e % 9] = w.S[e / 9][e % 9];
+        w.V[0][e / 9][e % 9] = e / 9 == e % 9 ? 1.0 : 0.0;
+      }
+    }
+  }
+  __syncwarp();
+  const int cur = jac9_sweeps<double>(w.A, w.V, w.c, w.sg, w.dl, w.pr, 1e-32, 30, true);
+  neg = false;
+#pragma unroll
+  for (int i = 0; i < 9; ++i) neg |= w.A[cur][i][i] < 0.0;
+  return cur;
+}
+// The same by FP64 rotations one after the other from the identity, the rows of a rotation
+// updated in parallel (jac9_project_serial; the result in buffer 0).
+DEV int jac9_project_serial(Jac9& w, bool& neg) {
+  const int lane = threadIdx.x & 31;
+  double(&A)[9][9] = w.A[0];
+  double(&V)[9][9] = w.V[0];
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+    const int e = lane + 32 * j;
+    if (e < 81) {
+      A[e / 9][e % 9] = w.S[e / 9][e % 9];
+      V[e / 9][e % 9] = e / 9 == e % 9 ? 1.0 : 0.0;
+    }
+  }
+  __syncwarp();
+  for (int sweep = 0; sweep < 30; ++sweep) {
+    double off = 0, tot = 0;
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      const int e = lane + 32 * j;
+      if (e < 81) {
+        const double v = A[e / 9][e % 9];
+        tot += v * v;
+        if (e / 9 != e % 9) off += v * v;
+      }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      off += __shfl_xor_sync(0xffffffffu, off, o);
+      tot += __shfl_xor_sync(0xffffffffu, tot, o);
+    }
+    if (off <= 1e-32 * tot || off == 0.0) break;
+    for (int pp = 0; pp < 8; ++pp)
+      for (int qq = pp + 1; qq < 9; ++qq) {
+        const double apq = A[pp][qq];
+        if (apq == 0.0) continue;
+        const double app = A[pp][pp], aqq = A[qq][qq];
+        const double gq = 100.0 * fabs(apq);
+        if (sweep > 2 && fabs(app) + gq == fabs(app) && fabs(aqq) + gq == fabs(aqq)) {
+          __syncwarp();
+          if (lane == 0) A[pp][qq] = A[qq][pp] = 0.0;
+          __syncwarp();
+          continue;
+        }
+        double tt, c, sn;
+        jac9_rotation(0.5 * (aqq - app), apq, tt, c, sn);
+        __syncwarp();
+        if (lane < 9 && lane != pp && lane != qq) {
+          const double akp = A[lane][pp], akq = A[lane][qq];
+          const double np_ = c * akp - sn * akq, nq = sn * akp + c * akq;
+          A[lane][pp] = np_;
+          A[pp][lane] = np_;
+          A[lane][qq] = nq;
+          A[qq][lane] = nq;
+        }
+        if (lane < 9) {
+          const double vkp = V[lane][pp], vkq = V[lane][qq];
+          V[lane][pp] = c * vkp - sn * vkq;
+          V[lane][qq] = sn * vkp + c * vkq;
+        }
+        if (lane == 0) {
+          A[pp][pp] = app - tt * apq;
+          A[qq][qq] = aqq + tt * apq;
+          A[pp][qq] = A[qq][pp] = 0.0;
+        }
+        __syncwarp();
+      }
+  }
+  neg = false;
+#pragma unroll
+  for (int i = 0; i < 9; ++i) neg |= A[i][i] < 0.0;
+  return 0;
+}
+// Entry (i, j) of the projection: V max(L, 0) V^T, or S itself without a negative eigenvalue.
+DEV double jac9_entry(const Jac9& w, int cur, bool neg, int i, int j) {
+  if (!neg) return w.S[i][j];
+  double v = 0.0;
+#pragma unroll
+  for (int k = 0; k < 9; ++k) {
+    const double lk = w.A[cur][k][k];
+    if (lk > 0) v += w.V[cur][i][k] * lk * w.V[cur][j][k];
+  }
+  return v;
+}
+
 // Destinations of a reduced 9x9 Hessian S (symmetric; producers give the entries with
 // p <= q): a local array (both triangles written) or the upper triangle of a per-pair
 // record in global memory (structure of arrays, entry k of pair i at base[k * stride + i]).

@@ -186,19 +186,24 @@ __global__ void __launch_bounds__(128) k_pair_hess(Geo g, Params P, int kind, in
 
 // Per-pair terms, part 1 for mollified edge-edge pairs (the first *n_moll entries of
 // perm): one warp per pair. Their 9x9 reduced Hessian has no low-rank structure, so it is
-// built entry by entry across the lanes and projected by a cyclic Jacobi in shared
-// memory whose rotations update the 9 rows in parallel (one lane each); a thread-serial
-// 9x9 Jacobi in local memory kept a few warps busy long after the rest of the launch.
-constexpr int MOLL_W = 4;  // warps (pairs) per CTA
+// built entry by entry across the lanes and projected by the warp (jac9_project; a chain of
+// rotations, so it is bound by their latency: 256 columns of cubes and spheres 1154 -> 164 us a launch,
+// 333 bodies of the pile 436 -> 146 us).
+// Beside a launch of at least MOLL_HIDE pairs that hides them, up to MOLL_WAVE mollified pairs
+// keep the rotations one by one: the 1024-body pile gains 2% from the rounds, and with any other
+// rounding its CG, which stops at a residual, takes an iteration more or less and moves the
+// frame's velocities by 1e-9 (below 512 bodies by 2e-11).
+constexpr int MOLL_HIDE = 65536, MOLL_WAVE = 256;
+constexpr int MOLL_W = 2;  // warps (pairs) per CTA
+constexpr int MOLL_GRID = 608;  // CTAs at most (pairs are taken grid-stride)
 __global__ void __launch_bounds__(32 * MOLL_W) k_pair_moll(Geo g, Params P, int n, const int* tup,
                                                            const int8_t* tys, const int* perm, const int* n_moll,
                                                            double* R, double* lag) {
-  __shared__ double sA[MOLL_W][9][9], sV[MOLL_W][9][9];
+  __shared__ Jac9 sj[MOLL_W];
   __shared__ MollData smd[MOLL_W];
   const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
   const int nm = *n_moll;
-  double(&A)[9][9] = sA[wi];
-  double(&V)[9][9] = sV[wi];
+  Jac9& w9 = sj[wi];
   for (int t = blockIdx.x * MOLL_W + wi; t < nm && t < n; t += gridDim.x * MOLL_W) {
     const int p = perm[t];
     int vid[4], na, Ab, Bb;
@@ -234,23 +239,14 @@ __global__ void __launch_bounds__(32 * MOLL_W) k_pair_moll(Geo g, Params P, int 
       const bool moll = pair_setup(1, ty, X, d, bp, P.eps_x, st, w, W, Gi, md, gu, gv);
       if (lane == 0) smd[wi] = md;
       __syncwarp();
-      // entries of S (upper triangle mirrored), lane e takes e, e + 32, e + 64
-      double orig[3];
+      // entries of S (upper triangle mirrored), lane e takes e, e + 32, e + 64 (zero when the
+      // pair is not mollified at this configuration after all: reduced form below)
 #pragma unroll
       for (int j = 0; j < 3; ++j) {
         const int e = lane + 32 * j;
-        orig[j] = 0.0;
         if (e < 81) {
           const int pp = e / 9, qq = e % 9;
-          double h;
-          if (moll) {
-            h = moll_entry(smd[wi], pp <= qq ? pp : qq, pp <= qq ? qq : pp);
-          } else {  // not mollified at this configuration after all: reduced form
-            h = 0.0;
-          }
-          A[pp][qq] = h;
-          V[pp][qq] = pp == qq ? 1.0 : 0.0;
-          orig[j] = h;
+          w9.S[pp][qq] = moll ? moll_entry(smd[wi], pp <= qq ? pp : qq, pp <= qq ? qq : pp) : 0.0;
         }
       }
       __syncwarp();
@@ -263,99 +259,14 @@ __global__ void __launch_bounds__(32 * MOLL_W) k_pair_moll(Geo g, Params P, int 
         }
       } else {
         bool neg = false;
-        if (P.psd) {
-          for (int sweep = 0; sweep < 30; ++sweep) {
-            double off = 0, tot = 0;
+        const int cur = !P.psd ? 0 : (nm <= MOLL_WAVE && n >= MOLL_HIDE ? jac9_project_serial(w9, neg)
+                                                                      : jac9_project(w9, neg));
 #pragma unroll
-            for (int j = 0; j < 3; ++j) {
-              const int e = lane + 32 * j;
-              if (e < 81) {
-                const double v = A[e / 9][e % 9];
-                tot += v * v;
-                if (e / 9 != e % 9) off += v * v;
-              }
-            }
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-              off += __shfl_xor_sync(0xffffffffu, off, o);
-              tot += __shfl_xor_sync(0xffffffffu, tot, o);
-            }
-            if (off <= 1e-32 * tot || off == 0.0) break;
-            for (int pp = 0; pp < 8; ++pp)
-              for (int qq = pp + 1; qq < 9; ++qq) {
-                const double apq = A[pp][qq];
-                if (apq == 0.0) continue;
-                const double app = A[pp][pp], aqq = A[qq][qq];
-                const double gq = 100.0 * fabs(apq);
-                if (sweep > 2 && fabs(app) + gq == fabs(app) && fabs(aqq) + gq == fabs(aqq)) {
-                  __syncwarp();
-                  if (lane == 0) A[pp][qq] = A[qq][pp] = 0.0;
-                  __syncwarp();
-                  continue;
-                }
-                // rotation parameters from two reciprocal square roots (g = 1 / r,
-                // c^2 = (|h| + r) / (2 r), t = sgn(h) a g / (2 c^2), s = sgn(h) a g / (2 c)),
-                // as in psd_project_small; by division below the normal range
-                const double h = 0.5 * (aqq - app);
-                const double sa = h >= 0 ? apq : -apq;
-                const double r2 = fma(h, h, apq * apq);
-                double tt, c, sn;
-                if (r2 >= 1e-300) {
-                  const double g = rsqrt(r2);
-                  const double c2 = 0.5 * fma(r2, g, fabs(h)) * g;
-                  const double ic = rsqrt(c2);
-                  sn = 0.5 * sa * g * ic;
-                  c = c2 * ic;
-                  tt = sn * ic;
-                } else {
-                  const double den = fabs(h) + sqrt(r2);
-                  tt = den > 0.0 ? sa / den : 0.0;
-                  c = rsqrt(1.0 + tt * tt);
-                  sn = tt * c;
-                }
-                __syncwarp();
-                if (lane < 9 && lane != pp && lane != qq) {
-                  const double akp = A[lane][pp], akq = A[lane][qq];
-                  const double np_ = c * akp - sn * akq, nq = sn * akp + c * akq;
-                  A[lane][pp] = np_;
-                  A[pp][lane] = np_;
-                  A[lane][qq] = nq;
-                  A[qq][lane] = nq;
-                }
-                if (lane < 9) {
-                  const double vkp = V[lane][pp], vkq = V[lane][qq];
-                  V[lane][pp] = c * vkp - sn * vkq;
-                  V[lane][qq] = sn * vkp + c * vkq;
-                }
-                if (lane == 0) {
-                  A[pp][pp] = app - tt * apq;
-                  A[qq][qq] = aqq + tt * apq;
-                  A[pp][qq] = A[qq][pp] = 0.0;
-                }
-                __syncwarp();
-              }
-          }
-#pragma unroll
-          for (int i = 0; i < 9; ++i) neg |= A[i][i] < 0.0;
-        }
-        // S+ = V max(lam, 0) V^T (or S itself when no eigenvalue is negative), upper triangle
-#pragma unroll
-        for (int j = 0; j < 3; ++j) {
-          const int e = lane + 32 * j;
-          if (e < 81) {
-            const int pp = e / 9, qq = e % 9;
-            if (pp <= qq) {
-              double v = orig[j];
-              if (neg) {
-                v = 0.0;
-                for (int k = 0; k < 9; ++k) {
-                  const double lk = A[k][k];
-                  if (lk > 0) v += V[pp][k] * lk * V[qq][k];
-                }
-              }
-              R[(REC_S + s9_index(pp, qq)) * N + p] = v;
-            }
-          }
+        for (int k = 0; k < 2; ++k) {
+          if (k == 1 && lane >= 13) continue;
+          int i, j;
+          jac9_tri(lane + 32 * k, i, j);
+          R[(REC_S + lane + 32 * k) * N + p] = jac9_entry(w9, cur, neg, i, j);
         }
       }
       __syncwarp();
@@ -2009,7 +1920,8 @@ void assemble(const Geo& g, const Params& P, PairSet& S, NewtonBufs& B, cudaStre
       }
       CK(cudaEventRecord(B.ev_fork, s));
       CK(cudaStreamWaitEvent(B.side, B.ev_fork, 0));
-      KLAUNCH(K_PAIR_TERMS, B.side, k_pair_moll<<<64, 32 * MOLL_W, 0, B.side>>>(g, P, n, tup, ty, B.perm.p, n_moll,
+      KLAUNCH(K_PAIR_TERMS, B.side, k_pair_moll<<<nblk(n, MOLL_W) < MOLL_GRID ? nblk(n, MOLL_W) : MOLL_GRID, 32 * MOLL_W, 0,
+                                                      B.side>>>(g, P, n, tup, ty, B.perm.p, n_moll,
                                                                               B.prec.p, S.ee_lag.p));
       CK(cudaEventRecord(B.ev_join, B.side));
     }
