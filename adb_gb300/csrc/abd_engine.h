@@ -256,10 +256,12 @@ enum { CONTRIB = 456 };  // dI(144) dJ(144) off(144) gI(12) gJ(12)
 struct NewtonBufs {
   DBuf<double> pt_c, ee_c;   // CONTRIB per pair (SoA)
   DBuf<int> pt_seg, ee_seg;  // nov + 1
-  DBuf<int> perm, cls_cnt, cls_off, cls_tmp;  // pairs in distance-type order
-  DBuf<double> prec;         // per-pair reduced Hessian records between the pair-term kernels
-  cudaStream_t side = nullptr;               // mollified pairs run beside the main pair kernel
-  cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+  // per kind (PT, EE: they run on different streams): pairs in distance-type order, reduced
+  // Hessian records between the pair-term kernels
+  DBuf<int> perm[2], cls_cnt[2], cls_off[2], cls_tmp[2];
+  DBuf<double> prec[2];
+  cudaStream_t side = nullptr, side_pt = nullptr;  // mollified pairs; point-triangle pairs
+  cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_fork_pt = nullptr, ev_join_pt = nullptr;
   DBuf<double> ovr;          // nov * CONTRIB
   DBuf<int> has;             // nov
   DBuf<double> D, Dinv, grad;

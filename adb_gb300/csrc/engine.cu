@@ -154,11 +154,14 @@ struct Engine {
     nbufs.ovr.release(); nbufs.has.release(); nbufs.D.release(); nbufs.Dinv.release(); nbufs.grad.release();
     nbufs.x.release(); nbufs.r.release(); nbufs.z.release(); nbufs.p.release(); nbufs.qv.release();
     nbufs.Hrow.release(); nbufs.rcol.release(); nbufs.rn.release();
-    nbufs.perm.release(); nbufs.cls_cnt.release(); nbufs.cls_off.release(); nbufs.cls_tmp.release();
-    nbufs.prec.release();
-    if (nbufs.side) cudaStreamDestroy(nbufs.side);
-    if (nbufs.ev_fork) cudaEventDestroy(nbufs.ev_fork);
-    if (nbufs.ev_join) cudaEventDestroy(nbufs.ev_join);
+    for (int k = 0; k < 2; ++k) {
+      nbufs.perm[k].release(); nbufs.cls_cnt[k].release(); nbufs.cls_off[k].release(); nbufs.cls_tmp[k].release();
+      nbufs.prec[k].release();
+    }
+    for (cudaStream_t st : {nbufs.side, nbufs.side_pt})
+      if (st) cudaStreamDestroy(st);
+    for (cudaEvent_t e : {nbufs.ev_fork, nbufs.ev_join, nbufs.ev_fork_pt, nbufs.ev_join_pt})
+      if (e) cudaEventDestroy(e);
     nbufs.gpA.release(); nbufs.gpB.release(); nbufs.grp_body.release(); nbufs.grp_n.release();
     nbufs.grp_scene.release(); nbufs.sc_gbeg.release(); nbufs.sc_gend.release(); nbufs.sc_rz.release(); nbufs.sc_bb.release();
     nbufs.sc_conv.release(); nbufs.sc_iters.release(); nbufs.n_active.release();

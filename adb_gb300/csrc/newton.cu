@@ -46,10 +46,23 @@ __global__ void k_class_count(Geo g, Params P, int kind, int n, const int* tup, 
   if (threadIdx.x < NCLS) cnt[threadIdx.x * gridDim.x + blockIdx.x] = sc[threadIdx.x];
 }
 
-// Stable partition of the pairs by class (offsets from the scan of k_class_count).
+// Stable partition of the pairs by class (offsets from the scan of k_class_count), each class
+// from a multiple of 32 on, so that no warp of k_pair_hess holds two classes: a warp pays for
+// every branch and projection size among its pairs, and a scene of a hundred pairs is a few
+// such warps. perm (class_slots(n) entries) holds -1 in the gaps.
+__host__ __device__ constexpr int class_slots(int n) { return n + 32 * NCLS; }
 __global__ void k_class_scatter(Geo g, Params P, int kind, int n, const int* tup, const int8_t* ty, const int* off,
                                 int* perm) {
   __shared__ int wc[NCLS][CLS_T / 32];
+  __shared__ int s_gap[NCLS];  // gaps before each class
+  if (threadIdx.x == 0) {
+    int gap = 0;
+    for (int k = 0; k < NCLS; ++k) {
+      s_gap[k] = gap;
+      const int c = (k + 1 < NCLS ? off[(k + 1) * gridDim.x] : n) - off[k * gridDim.x];
+      gap += (32 - (c & 31)) & 31;
+    }
+  }
   const int p = blockIdx.x * CLS_T + threadIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int c = p < n ? pair_class(g, P, kind, tup, ty, p) : -1;
   unsigned mine = 0;
@@ -61,7 +74,7 @@ __global__ void k_class_scatter(Geo g, Params P, int kind, int n, const int* tup
   }
   __syncthreads();
   if (c >= 0) {
-    int r = off[c * gridDim.x + blockIdx.x] + __popc(mine & ((1u << lane) - 1u));
+    int r = s_gap[c] + off[c * gridDim.x + blockIdx.x] + __popc(mine & ((1u << lane) - 1u));
     for (int i = 0; i < w; ++i) r += wc[c][i];
     perm[r] = p;
   }
@@ -117,12 +130,16 @@ __device__ __forceinline__ int pair_class(const Geo& g, const Params& P, int kin
 // Per-pair terms, part 1 (kind 0: PT, point on body A, triangle on body B; 1: EE): the
 // barrier's reduced Hessian and gradient, the lagged friction frame and the friction
 // terms, written to the pair's record. Threads take pairs in stencil-class order (perm).
-__global__ void __launch_bounds__(128) k_pair_hess(Geo g, Params P, int kind, int n, const int* tup,
+// One warp a CTA: a warp's FP64 instruction takes 64 cycles of its sub-partition (76 with all
+// four busy), so single warps spread over the SMs and end one by one.
+constexpr int HESS_T = 32;
+__global__ void __launch_bounds__(HESS_T) k_pair_hess(Geo g, Params P, int kind, int n, const int* tup,
                                                    const int8_t* tys, const int* perm, const int* n_moll, double* R,
                                                    double* lag) {
   int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= n || (n_moll && t < *n_moll)) return;  // mollified pairs: k_pair_moll
+  if (t >= class_slots(n) || (n_moll && t < *n_moll)) return;  // mollified pairs: k_pair_moll
   const int p = perm[t];
+  if (p < 0) return;
   int vid[4], na, A, B;
   pair_vertices(g, kind, tup, p, vid, na, A, B);
   if (!scene_on(g, A)) return;  // scene not iterating: its blocks are not used
@@ -330,7 +347,8 @@ __constant__ Sym12Table c_sym12 = Sym12Table();
 // Y_A's column 1 is zero for both kinds (body A holds vertex 0, and 1 for edge-edge) and
 // Y_B's column 0 is zero for edge-edge pairs: those terms are left out (KIND 0:
 // point-triangle, 1: edge-edge).
-template <int KIND>
+// SPLIT: the six (r, s) slices of a pair by a thread each (blockIdx.y); else one after the other.
+template <int KIND, bool SPLIT>
 __global__ void __launch_bounds__(128) k_pair_chain(Geo g, int n, const int* tup, const int* pov,
                                                     const int* ovI, const double* R, double* C) {
   constexpr int kind = KIND;
@@ -354,6 +372,7 @@ __global__ void __launch_bounds__(128) k_pair_chain(Geo g, int n, const int* tup
   double* gA = a_is_I ? gI : gJ;
   double* gB = a_is_I ? gJ : gI;
   if (R[REC_ACT * N + p] == 0.0) {
+    if (SPLIT && blockIdx.y) return;
     for (int e = 0; e < 78; ++e) {
       dI[e * N + p] = 0.0;
       dJ[e * N + p] = 0.0;
@@ -399,7 +418,7 @@ __global__ void __launch_bounds__(128) k_pair_chain(Geo g, int n, const int* tup
   const bool off_on = a_dyn && b_dyn;
   // one (r, s) slice at a time keeps the live state to Y, T and M
 #pragma unroll 1
-  for (int nidx = 0; nidx < 6; ++nidx) {
+  for (int nidx = SPLIT ? blockIdx.y : 0; nidx < (SPLIT ? blockIdx.y + 1 : 6); ++nidx) {
     const int r = nidx < 3 ? 0 : (nidx < 5 ? 1 : 2);
     const int s = nidx < 3 ? nidx : (nidx < 5 ? nidx - 2 : 2);
     {
@@ -472,6 +491,7 @@ __global__ void __launch_bounds__(128) k_pair_chain(Geo g, int n, const int* tup
         }
     }
   }
+  if (SPLIT && blockIdx.y) return;
   // body gradients
 #pragma unroll
   for (int k = 0; k < 4; ++k)
@@ -1876,6 +1896,21 @@ __global__ void k_copy(double* d, const double* s, int n) {
 
 }  // namespace
 
+// Chain rule of n pairs of a kind: slices by thread up to CHAIN_SPLIT pairs.
+// A pair's slices one after the other are a chain of 50-67 us; by thread 15 us (a stack's 96
+// pairs) to 43 us (12k). At 136k pairs the gain is 10% (309 -> 280 us) and the rounding of the
+// friction terms differs, which the large pile's truncated CG amplifies (see MOLL_HIDE).
+constexpr int CHAIN_SPLIT = 16384;
+template <int KIND>
+static void launch_chain(const Geo& g, int n, const int* tup, const int* pov, const int* ovI, const double* R,
+                         double* C, cudaStream_t s) {
+  const int nb = nblk(n, 128);
+  if (n <= CHAIN_SPLIT)
+    KLAUNCH(K_PAIR_TERMS, s, k_pair_chain<KIND, true><<<dim3(nb, 6), 128, 0, s>>>(g, n, tup, pov, ovI, R, C));
+  else
+    KLAUNCH(K_PAIR_TERMS, s, k_pair_chain<KIND, false><<<nb, 128, 0, s>>>(g, n, tup, pov, ovI, R, C));
+}
+
 void assemble(const Geo& g, const Params& P, PairSet& S, NewtonBufs& B, cudaStream_t s) {
   int nb = g.nb, npt = S.npt, nee = S.nee, nov = S.nov;
   B.pt_c.ensure((size_t)PAIRC * npt + 1);
@@ -1894,47 +1929,58 @@ void assemble(const Geo& g, const Params& P, PairSet& S, NewtonBufs& B, cudaStre
   prof_work(K_PAIR_TERMS, (double)npt + nee, 412.0 * ((double)npt + nee));
   prof_work(K_OV_REDUCE, nov, 2.0 * 1152 * nov);
   prof_work(K_BODY_SYSTEM, nb, 2.0 * 1152 * nb + 2 * 96.0 * nb);
+  // The two kinds share nothing before the overlap sums: point-triangle pairs run on a stream
+  // of their own beside the edge-edge ones (a kernel of either is a chain of 50 to 170 us
+  // however few its pairs: a chain's frame 4.75 -> 4.24 ms, a batch's 20.9 -> 18.4), and the few
+  // mollified pairs, one warp each, on a third. At MOLL_HIDE pairs the edge-edge kernels fill
+  // the chip and the two get in each other's way (a Newton step of the pile 7.40 -> 7.64 ms).
+  if (!B.side) {
+    CK(cudaStreamCreateWithFlags(&B.side, cudaStreamNonBlocking));
+    CK(cudaStreamCreateWithFlags(&B.side_pt, cudaStreamNonBlocking));
+    for (cudaEvent_t* e : {&B.ev_fork, &B.ev_join, &B.ev_fork_pt, &B.ev_join_pt})
+      CK(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
+  }
+  const bool both = npt > 0 && nee > 0 && nee < MOLL_HIDE;
+  if (both) {
+    CK(cudaEventRecord(B.ev_fork_pt, s));
+    CK(cudaStreamWaitEvent(B.side_pt, B.ev_fork_pt, 0));
+  }
   for (int kind = 0; kind < 2; ++kind) {
     int n = kind ? nee : npt;
     if (!n) continue;
+    cudaStream_t st = kind == 0 && both ? B.side_pt : s;
     int nb_c = nblk(n, CLS_T);
-    B.cls_cnt.ensure(NCLS * (size_t)nb_c);
-    B.cls_off.ensure(NCLS * (size_t)nb_c);
-    B.perm.ensure(n);
+    DBuf<int>&cnt = B.cls_cnt[kind], &off = B.cls_off[kind], &perm = B.perm[kind];
+    DBuf<double>& prec = B.prec[kind];
+    cnt.ensure(NCLS * (size_t)nb_c);
+    off.ensure(NCLS * (size_t)nb_c);
+    perm.ensure(class_slots(n));
+    CK(cudaMemsetAsync(perm.p, 0xff, class_slots(n) * sizeof(int), st));
     const int8_t* ty = kind ? S.ee_ty.p : S.pt_ty.p;
     const int* tup = kind ? S.ee.p : S.pt.p;
-    KLAUNCH(K_SEG, s, k_class_count<<<nb_c, CLS_T, 0, s>>>(g, P, kind, n, tup, ty, B.cls_cnt.p));
-    scan_exclusive_int(B.cls_cnt.p, B.cls_off.p, NCLS * nb_c, nullptr, s, B.cls_tmp);
-    KLAUNCH(K_SEG, s, k_class_scatter<<<nb_c, CLS_T, 0, s>>>(g, P, kind, n, tup, ty, B.cls_off.p, B.perm.p));
-    B.prec.ensure(REC * (size_t)n);
+    KLAUNCH(K_SEG, st, k_class_count<<<nb_c, CLS_T, 0, st>>>(g, P, kind, n, tup, ty, cnt.p));
+    scan_exclusive_int(cnt.p, off.p, NCLS * nb_c, nullptr, st, B.cls_tmp[kind]);
+    KLAUNCH(K_SEG, st, k_class_scatter<<<nb_c, CLS_T, 0, st>>>(g, P, kind, n, tup, ty, off.p, perm.p));
+    prec.ensure(REC * (size_t)n);
     // class 0 (mollified edge-edge pairs) comes first in perm; its size is the offset of
     // class 1
-    const int* n_moll = kind ? B.cls_off.p + nb_c : nullptr;
+    const int* n_moll = kind ? off.p + nb_c : nullptr;
     if (kind) {
-      // the few mollified pairs take one warp each for a long serial projection: run
-      // them on a side stream, overlapped with the main kernel
-      if (!B.side) {
-        CK(cudaStreamCreateWithFlags(&B.side, cudaStreamNonBlocking));
-        CK(cudaEventCreateWithFlags(&B.ev_fork, cudaEventDisableTiming));
-        CK(cudaEventCreateWithFlags(&B.ev_join, cudaEventDisableTiming));
-      }
-      CK(cudaEventRecord(B.ev_fork, s));
+      CK(cudaEventRecord(B.ev_fork, st));
       CK(cudaStreamWaitEvent(B.side, B.ev_fork, 0));
-      KLAUNCH(K_PAIR_TERMS, B.side, k_pair_moll<<<nblk(n, MOLL_W) < MOLL_GRID ? nblk(n, MOLL_W) : MOLL_GRID, 32 * MOLL_W, 0,
-                                                      B.side>>>(g, P, n, tup, ty, B.perm.p, n_moll,
-                                                                              B.prec.p, S.ee_lag.p));
+      const int blocks = nblk(n, MOLL_W) < MOLL_GRID ? nblk(n, MOLL_W) : MOLL_GRID;
+      KLAUNCH(K_PAIR_TERMS, B.side, k_pair_moll<<<blocks, 32 * MOLL_W, 0, B.side>>>(g, P, n, tup, ty, perm.p, n_moll,
+                                                                                  prec.p, S.ee_lag.p));
       CK(cudaEventRecord(B.ev_join, B.side));
     }
-    KLAUNCH(K_PAIR_TERMS, s, k_pair_hess<<<nblk(n, 128), 128, 0, s>>>(g, P, kind, n, tup, ty, B.perm.p, n_moll,
-                                                                    B.prec.p, kind ? S.ee_lag.p : S.pt_lag.p));
-    if (kind) CK(cudaStreamWaitEvent(s, B.ev_join, 0));
-    if (kind)
-      KLAUNCH(K_PAIR_TERMS, s, k_pair_chain<1><<<nblk(n, 128), 128, 0, s>>>(g, n, tup, S.ee_ov.p, S.ovI.p, B.prec.p,
-                                                                            B.ee_c.p));
-    else
-      KLAUNCH(K_PAIR_TERMS, s, k_pair_chain<0><<<nblk(n, 128), 128, 0, s>>>(g, n, tup, S.pt_ov.p, S.ovI.p, B.prec.p,
-                                                                            B.pt_c.p));
+    KLAUNCH(K_PAIR_TERMS, st, k_pair_hess<<<nblk(class_slots(n), HESS_T), HESS_T, 0, st>>>(
+                                  g, P, kind, n, tup, ty, perm.p, n_moll, prec.p, kind ? S.ee_lag.p : S.pt_lag.p));
+    if (kind) CK(cudaStreamWaitEvent(st, B.ev_join, 0));
+    if (kind) launch_chain<1>(g, n, tup, S.ee_ov.p, S.ovI.p, prec.p, B.ee_c.p, st);
+    else launch_chain<0>(g, n, tup, S.pt_ov.p, S.ovI.p, prec.p, B.pt_c.p, st);
+    if (st != s) CK(cudaEventRecord(B.ev_join_pt, st));
   }
+  if (both) CK(cudaStreamWaitEvent(s, B.ev_join_pt, 0));
   if (nov) {
     KLAUNCH(K_SEG, s, k_seg<<<nblk(nov + 1, 256), 256, 0, s>>>(nov, npt, S.pt_ov.p, B.pt_seg.p));
     KLAUNCH(K_SEG, s, k_seg<<<nblk(nov + 1, 256), 256, 0, s>>>(nov, nee, S.ee_ov.p, B.ee_seg.p));
@@ -1953,8 +1999,6 @@ int pcg_solve(const Geo& g, PairSet& S, NewtonBufs& B, const SolveOpts& o, const
   B.status.ensure(4);
   if (!B.h_int) CK(cudaMallocHost(&B.h_int, 16 * sizeof(int)));
   CK(cudaMemsetAsync(B.status.p, 0, 4 * sizeof(int), s));
-  KLAUNCH(K_BLOCK_INVERSE, s, k_block_inverse<<<nblk(nb, BINV_W), 32 * BINV_W, 0, s>>>(nb, B.D.p, B.Dinv.p,
-                                                                                        B.status.p));
   B.x.ensure(12 * (size_t)nb);
   B.r.ensure(12 * (size_t)nb);
   B.z.ensure(12 * (size_t)nb);
@@ -1979,7 +2023,12 @@ int pcg_solve(const Geo& g, PairSet& S, NewtonBufs& B, const SolveOpts& o, const
                                                                                         S.upidx.p, B.has.p, B.ovr.p,
                                                                                         B.D.p, B.Hrow.p, B.rcol.p,
                                                                                         B.rn.p, B.status.p + 2));
+  auto block_inverse = [&]() {
+    KLAUNCH(K_BLOCK_INVERSE, s, k_block_inverse<<<nblk(nb, BINV_W), 32 * BINV_W, 0, s>>>(nb, B.D.p, B.Dinv.p,
+                                                                                          B.status.p));
+  };
   if (o.dense) {
+    block_inverse();
     dense_solve(g, S, B, on, dq, s);
     CK(cudaMemcpyAsync(B.h_int, B.status.p, 3 * sizeof(int), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
@@ -1997,6 +2046,8 @@ int pcg_solve(const Geo& g, PairSet& S, NewtonBufs& B, const SolveOpts& o, const
     if (n_tri > 0) pcg_mask = B.pcg_on.p;
   }
   const bool run_pcg = n_tri == 0 || n_pcg > 0;
+  // the preconditioner; the direct solve checks its own pivots
+  if (run_pcg) block_inverse();
   static int max_blocks = 0, max_blocks1 = 0;
   if (!max_blocks) {
     int dev, sms, per, per1;
