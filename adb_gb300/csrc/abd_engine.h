@@ -269,7 +269,11 @@ struct NewtonBufs {
   DBuf<double> Hrow;         // row-block copy of the system for the PCG
   DBuf<int> rcol, rn;
   DBuf<double> gpA, gpB;     // per-group partial sums of the PCG
+  DBuf<unsigned long long> slots;  // words that cross between CTAs (one group per CTA)
+  DBuf<double> pnb;          // its directions of the row blocks past the registers
   DBuf<int> grp_body, grp_n, grp_scene, sc_gbeg, sc_gend;  // PCG body groups (pcg_groups)
+  DBuf<int> sc_box;          // per scene: where the boxes of its groups begin (one group per CTA)
+  size_t n_box = 0;          // values in all boxes
   std::vector<int> h_sc_beg, h_sc_end;  // body range of each scene (host)
   DBuf<double> dense_A, dense_y;         // dense solve: one scene's matrix and right-hand side
   // block-tridiagonal direct solve: per-scene flags and counts, the bodies by elimination

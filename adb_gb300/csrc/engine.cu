@@ -162,7 +162,7 @@ struct Engine {
       if (st) cudaStreamDestroy(st);
     for (cudaEvent_t e : {nbufs.ev_fork, nbufs.ev_join, nbufs.ev_fork_pt, nbufs.ev_join_pt})
       if (e) cudaEventDestroy(e);
-    nbufs.gpA.release(); nbufs.gpB.release(); nbufs.grp_body.release(); nbufs.grp_n.release();
+    nbufs.gpA.release(); nbufs.gpB.release(); nbufs.slots.release(); nbufs.pnb.release(); nbufs.sc_box.release(); nbufs.grp_body.release(); nbufs.grp_n.release();
     nbufs.grp_scene.release(); nbufs.sc_gbeg.release(); nbufs.sc_gend.release(); nbufs.sc_rz.release(); nbufs.sc_bb.release();
     nbufs.sc_conv.release(); nbufs.sc_iters.release(); nbufs.n_active.release();
     nbufs.e_off.release(); nbufs.e_chunk_cnt.release(); nbufs.e_chunk_off.release(); nbufs.e_scan_tmp.release();

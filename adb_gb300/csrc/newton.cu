@@ -839,7 +839,14 @@ struct PcgArgs {
   double tol2;
   int maxit;
   int* out;  // [0] status, [1] iterations (max over scenes)
+  unsigned long long* slots;            // k_pcg1: tagged words (pcg1_words), zero at its start
+  const int* sc_box;                    // k_pcg1: scene -> its boxes
+  double* pnb;                          // k_pcg1: directions of the row blocks past the registers
 };
+
+// 64-bit words that cross between the CTAs of k_pcg1: two each for every row of z and for three
+// sums of every pair of groups of a scene.
+inline size_t pcg1_words(const NewtonBufs& B, int nb) { return 24 * (size_t)nb + 2 * B.n_box; }
 
 // Assembled system as stored by the assembly (diagonal blocks D, off-diagonal blocks in
 // the per-overlap records), for products outside the PCG.
@@ -873,10 +880,13 @@ __device__ __forceinline__ double row_spmv(const SysView& a, int body, int row, 
 
 // One warp per body: the diagonal block, then the off-diagonal blocks with a
 // contribution in overlap-list order, transposed where the body is the record's J side.
-// kept[0] accumulates the blocks kept (for the algorithmic byte count).
+// kept[0] accumulates the blocks kept (for the algorithmic byte count). Also clears the
+// exchange words of k_pcg1.
 __global__ void k_pcg_rows(int nb, const int* row_ptr, const int* col, const int* upidx, const int* has,
-                           const double* ovr, const double* D, double* Hrow, int* rcol, int* rn, int* kept) {
+                           const double* ovr, const double* D, double* Hrow, int* rcol, int* rn, int* kept,
+                           unsigned long long* slots, size_t nslot) {
   int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  for (size_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nslot; i += gridDim.x * blockDim.x) slots[i] = 0;
   if (warp >= nb) return;
   const int body = warp;
   const int base = body + row_ptr[body];
@@ -1255,55 +1265,256 @@ __global__ void __launch_bounds__(PCG_NT) k_pcg(PcgArgs a) {
 }
 
 // The same solve when every CTA holds exactly one body group (grid = groups, the common
-// case up to 152 groups per cooperative launch): each thread keeps its row's x, r, z, p
-// and q, its row of the block-Jacobi inverse and its first two row blocks of the product
-// in registers for the whole solve, and z = M^-1 r takes the body's r from its 16-lane
-// half by shuffles. Only the neighbour reads of z and p and the group partials go through
-// memory. The arithmetic is that of k_pcg, operation for operation, so both give the same
-// iterates bit for bit.
-constexpr int PCG1_NC = 2;  // row blocks per part kept in registers
+// case up to 152 groups per cooperative launch): the vectors, the block-Jacobi inverse and the
+// first row blocks of the product stay in registers for the whole solve. The arithmetic is
+// that of k_pcg, operation for operation, so both give the same iterates bit for bit.
+//
+// What bounds it: a warp's FP64 instruction takes 64 cycles of its sub-partition, and an
+// iteration exchanges the CG scalars twice over all CTAs of the scene. So
+//  - what crosses between CTAs are words that carry the number of their iteration (the
+//    partial sums of every group, the entries of z): a reader loads them until the number is
+//    the one it waits for. There is no grid barrier, no fence and no load of the sums after
+//    it; scenes do not wait for one another, and a scene that has converged is done. A group
+//    writes its sums into every group's own box: words that all CTAs poll in one place take
+//    their turns in L2 (4.1 ms a solve, and 3.8 to 4.6 by where the words lie);
+//  - a neighbour's direction is followed from its z in the reader's registers;
+//  - four warps hold the rows (x, r, z, p, the scalars), twelve the product: one lane per
+//    (body, part, row) that holds a block, packed with the longest parts first (a group's 8
+//    bodies hold some 28 blocks: 10 warps instead of 16 half empty ones). The product's warps
+//    wait for z while the row warps reduce the scalars;
+//  - r.r and r.z share their reduction steps.
+// 1024 bodies of the pile, 359 iterations: 4.38 -> 3.40 ms a solve (9.5 us an iteration: two
+// exchanges of about 1.2 us, the product 1.5 us, the rest FP64 chains of the reductions).
+constexpr int PCG1_NC = 2;     // row blocks per part kept in registers
+constexpr int PCG1_G = 5;      // groups of a scene per lane of an exchange
+constexpr int PCG1_MAXGRP = 32 * PCG1_G;
+constexpr int PCG1_SPIN = 1 << 21;  // polls of a word (a second or two) before the solve gives up
+
+// A double as two 64-bit words (16-byte aligned), each with the iteration's number in its upper
+// half: a reader that finds the number in both has the value (64-bit accesses are single).
+struct Tagged {
+  unsigned long long hi, lo;
+};
+__device__ __forceinline__ void tag_put(Tagged* w, double v, unsigned tag) {
+  const unsigned long long t = (unsigned long long)tag << 32;
+  const unsigned long long hi = t | (unsigned)__double2hiint(v), lo = t | (unsigned)__double2loint(v);
+  asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(w), "l"(hi), "l"(lo) : "memory");
+}
+__device__ __forceinline__ Tagged tag_ld(const Tagged* w) {
+  Tagged r;
+  asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(r.hi), "=l"(r.lo) : "l"(w) : "memory");
+  return r;
+}
+__device__ __forceinline__ bool tag_ok(const Tagged& r, unsigned tag) {
+  return (unsigned)(r.hi >> 32) == tag && (unsigned)(r.lo >> 32) == tag;
+}
+__device__ __forceinline__ double tag_val(const Tagged& r) { return __hiloint2double((int)(unsigned)r.hi, (int)(unsigned)r.lo); }
+// A warp reads N tagged values a lane (w[i] null: none) into v. False when they did not all
+// arrive within PCG1_SPIN polls.
+template <int N>
+__device__ __forceinline__ bool tag_gather(const Tagged* (&w)[N], unsigned tag, double (&v)[N]) {
+  unsigned miss = 0;
+#pragma unroll
+  for (int i = 0; i < N; ++i)
+    if (w[i]) miss |= 1u << i;
+  for (int spin = 0; spin < PCG1_SPIN; ++spin) {
+    Tagged r[N];
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+      if (miss >> i & 1) r[i] = tag_ld(w[i]);
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+      if ((miss >> i & 1) && tag_ok(r[i], tag)) {
+        v[i] = tag_val(r[i]);
+        miss &= ~(1u << i);
+      }
+    if (__all_sync(0xffffffffu, miss == 0)) return true;
+  }
+  return false;
+}
+// The partials of a scene's n groups from this group's box: lane l groups l, l + 32, ...;
+// their sum is formed in the order of warp_scene_sum.
+__device__ __forceinline__ bool sum_gather(const Tagged* box, int n, unsigned tag, double (&v)[PCG1_G]) {
+  const Tagged* w[PCG1_G];
+#pragma unroll
+  for (int i = 0; i < PCG1_G; ++i) {
+    const int k = (int)(threadIdx.x & 31) + 32 * i;
+    w[i] = k < n ? box + k : nullptr;
+  }
+  return tag_gather<PCG1_G>(w, tag, v);
+}
+__device__ __forceinline__ double sum_form(const double (&v)[PCG1_G], int n) {
+  double s = 0.0;
+#pragma unroll
+  for (int i = 0; i < PCG1_G; ++i)
+    if ((int)(threadIdx.x & 31) + 32 * i < n) s += v[i];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  return s;
+}
+constexpr int PCG1_ROWT = 16 * GB;             // threads of the row warps
+constexpr int PCG1_PRODT = PCG_NT - PCG1_ROWT;  // threads of the product warps
+__device__ __forceinline__ void row_barrier() { asm volatile("bar.sync 1, %0;" ::"n"(PCG1_ROWT) : "memory"); }
+__device__ __forceinline__ void prod_barrier() { asm volatile("bar.sync 2, %0;" ::"n"(PCG1_PRODT) : "memory"); }
+// the product is in shared memory: its warps go on, the row warps wait for them
+__device__ __forceinline__ void done_arrive() { asm volatile("bar.arrive 3, %0;" ::"n"(PCG_NT) : "memory"); }
+__device__ __forceinline__ void done_wait() { asm volatile("bar.sync 3, %0;" ::"n"(PCG_NT) : "memory"); }
+// the row warps have published their z: the product warps start to poll for the others'
+__device__ __forceinline__ void sent_arrive() { asm volatile("bar.arrive 4, %0;" ::"n"(PCG_NT) : "memory"); }
+__device__ __forceinline__ void sent_wait() { asm volatile("bar.sync 4, %0;" ::"n"(PCG_NT) : "memory"); }
+
 __global__ void __launch_bounds__(PCG_NT) k_pcg1(PcgArgs a) {
-  cg::grid_group grid = cg::this_grid();
-  __shared__ double s_part[PCG_NT];
+  static_assert(PCG1_ROWT == 128 && GB * NPART == 32 && PCG1_PRODT == 12 * GB * NPART, "warps of k_pcg1");
+  __shared__ double s_part[GB * NPART * 12];               // partial rows by (body, part)
+  __shared__ double s_v[PCG1_NC][GB * NPART][12];          // neighbours' directions by item
   __shared__ double s_w[GB];
-  __shared__ __align__(16) double s_v[PCG_NT / 16][12];
-  __shared__ double s_sum[2];
-  __shared__ double s_val;
-  __shared__ double s_beta, s_rzp;  // beta from warp 1's r.z sum; the previous r.z
-  __shared__ int s_flag;
-  const int tid = blockIdx.x * blockDim.x + threadIdx.x;
+  __shared__ double s_beta, s_alpha;
+  __shared__ int s_item[GB * NPART];                       // (body, part) of each product item, longest first
+  __shared__ int s_nitem, s_rounds;
+  __shared__ int s_flag;     // 1: the scene stops
+  __shared__ int s_abort;    // an exchange did not complete
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int part = (threadIdx.x >> 4) & (NPART - 1), prow = threadIdx.x & 15;
-  const int plb = threadIdx.x / BODY_SLOTS;
-  const int hg = threadIdx.x >> 4;
-  const bool vthr = threadIdx.x < 16 * GB;
-  const int vlb = threadIdx.x >> 4, row = threadIdx.x & 15;
   const int g = blockIdx.x;
   const int sc = a.grp_scene[g], nbody = a.grp_n[g], b0 = a.grp_body[g];
-  const bool owner = g == a.sc_gbeg[sc];
-  // product-phase state
-  const bool pact = plb < nbody;
-  const int pbody = b0 + plb;
-  const int pbase = pact ? pbody + a.row_ptr[pbody] : 0, pn = pact ? a.rn[pbody] : 0;
-  int rc[PCG1_NC];
-  double hr[PCG1_NC][12];
+  const int gbeg = a.sc_gbeg[sc], ng = a.sc_gend[sc] - gbeg;
+  // z by row, then a box per group: p.q, r.r and r.z of the ng groups of its scene
+  Tagged* const t_z = reinterpret_cast<Tagged*>(a.slots);
+  Tagged* const boxes = t_z + 12 * (size_t)a.nb + a.sc_box[sc];  // of the scene's first group
+  const Tagged* const my_box = boxes + 3 * (size_t)ng * (g - gbeg);
+  // ---- product items ----
+  for (int i = threadIdx.x; i < GB * NPART * 12; i += PCG_NT) s_part[i] = 0.0;
+  if (warp == 0) {
+    const int lb = lane / NPART, part = lane - NPART * lb;
+    const int n = lb < nbody ? a.rn[b0 + lb] : 0;
+    const int cnt = n > part ? (n - part + NPART - 1) / NPART : 0;
+    const unsigned m3 = __ballot_sync(0xffffffffu, cnt >= 3), m2 = __ballot_sync(0xffffffffu, cnt == 2),
+                   m1 = __ballot_sync(0xffffffffu, cnt == 1), below = (1u << lane) - 1u;
+    const int n3 = __popc(m3), n2 = __popc(m2);
+    if (cnt > 0) {
+      const int pos = cnt >= 3 ? __popc(m3 & below) : (cnt == 2 ? n3 + __popc(m2 & below) : n3 + n2 + __popc(m1 & below));
+      s_item[pos] = lane;
+    }
+    int most = cnt;
 #pragma unroll
-  for (int jj = 0; jj < PCG1_NC; ++jj) {
-    const int j = part + NPART * jj;
-    rc[jj] = j < pn ? a.rcol[pbase + j] : 0;
-#pragma unroll
-    for (int c = 0; c < 12; ++c) hr[jj][c] = (j < pn && prow < 12) ? a.Hrow[(size_t)(pbase + j) * 144 + 12 * prow + c] : 0.0;
+    for (int o = 16; o > 0; o >>= 1) most = max(most, __shfl_xor_sync(0xffffffffu, most, o));
+    if (lane == 0) {
+      s_nitem = n3 + n2 + __popc(m1);
+      s_rounds = (most + PCG1_NC - 1) / PCG1_NC;
+      s_abort = 0;
+    }
   }
-  // per-row state
-  const bool mine = vthr && vlb < nbody && row < 12;
+  __syncthreads();
+  if (threadIdx.x >= PCG1_ROWT) {
+    // ======== product warps: q = H p by (body, part, row) ========
+    const int pt = threadIdx.x - PCG1_ROWT;
+    const int item = pt / 12, prow = pt - 12 * item;
+    const bool pact = item < s_nitem;
+    const int rounds = s_rounds;
+    const int what = pact ? s_item[item] : 0;
+    const int part = what & (NPART - 1), pbody = b0 + what / NPART;
+    const int pbase = pact ? pbody + a.row_ptr[pbody] : 0, pn = pact ? a.rn[pbody] : 0;
+    const Tagged* wz[PCG1_NC];
+    double hr[PCG1_NC][12], pnb[PCG1_NC], zn[PCG1_NC];
+#pragma unroll
+    for (int jj = 0; jj < PCG1_NC; ++jj) {
+      const int j = part + NPART * jj;
+      wz[jj] = j < pn ? t_z + 12 * (size_t)a.rcol[pbase + j] + prow : nullptr;
+      pnb[jj] = 0.0;
+      zn[jj] = 0.0;
+#pragma unroll
+      for (int c = 0; c < 12; ++c) hr[jj][c] = j < pn ? a.Hrow[(size_t)(pbase + j) * 144 + 12 * prow + c] : 0.0;
+    }
+    for (int j = part + NPART * PCG1_NC; j < pn; j += NPART) a.pnb[(size_t)(pbase + j) * 12 + prow] = 0.0;
+    bool late = false;  // told at the next common barrier: all threads leave at the same one
+    for (int k = 0;; ++k) {
+      sent_wait();
+      if (!tag_gather<PCG1_NC>(wz, (unsigned)k + 1u, zn) || late) s_abort = 1;
+      __syncthreads();  // beta, or the end
+      if (s_flag || s_abort) break;
+      const double beta = s_beta;
+      double acc = 0.0;
+      for (int rd = 0; rd < rounds; ++rd) {
+        if (rd) prod_barrier();  // the directions of the last round have been read
+#pragma unroll
+        for (int jj = 0; jj < PCG1_NC; ++jj) {
+          const int j = part + NPART * (PCG1_NC * rd + jj);
+          if (j < pn) {
+            double v;
+            if (rd == 0) {
+              v = dir(zn[jj], beta, pnb[jj]);
+              pnb[jj] = v;
+            } else {
+              // past the registers (a body of more than 8 blocks): z is there since the sums
+              // of this iteration are, its direction is kept in memory of this thread's own
+              const Tagged* w = t_z + 12 * (size_t)a.rcol[pbase + j] + prow;
+              Tagged r = tag_ld(w);
+              for (int spin = 0; !tag_ok(r, (unsigned)k + 1u) && spin < PCG1_SPIN; ++spin) r = tag_ld(w);
+              late |= !tag_ok(r, (unsigned)k + 1u);
+              double* pm = a.pnb + (size_t)(pbase + j) * 12 + prow;
+              v = dir(tag_val(r), beta, *pm);
+              *pm = v;
+            }
+            s_v[jj][item][prow] = v;
+          }
+        }
+        prod_barrier();
+#pragma unroll
+        for (int jj = 0; jj < PCG1_NC; ++jj) {
+          const int j = part + NPART * (PCG1_NC * rd + jj);
+          if (j < pn) {
+            const double* v = s_v[jj][item];
+            if (rd == 0) {
+#pragma unroll
+              for (int c = 0; c < 12; ++c) acc += hr[jj][c] * v[c];
+            } else {
+              const double* H = a.Hrow + (size_t)(pbase + j) * 144 + 12 * prow;
+#pragma unroll
+              for (int c = 0; c < 12; ++c) acc += H[c] * v[c];
+            }
+          }
+        }
+      }
+      if (pact) s_part[12 * what + prow] = acc;
+      done_arrive();
+    }
+    return;
+  }
+  // ======== row warps: two bodies a warp, 16 lanes each ========
+  const bool owner = g == gbeg;
+  const int vlb = threadIdx.x >> 4, row = threadIdx.x & 15;
+  const bool mine = vlb < nbody && row < 12;
   const int vbody = b0 + vlb, idx = 12 * vbody + row;
   double Dr[12];
 #pragma unroll
   for (int c = 0; c < 12; ++c) Dr[c] = mine ? a.Dinv[144 * vbody + 12 * row + c] : 0.0;
-  double x_r = 0.0, r_r = 0.0, z_r = 0.0, pold_r = 0.0, q_r = 0.0, pv_r = 0.0;
-  // thread 0: the scene's carried scalars
-  int conv_r = 0;
-  double bb_r = 0.0, rz_r = 1.0;
+  double x_r = 0.0, r_r = 0.0, z_r = 0.0, pold_r = 0.0;
+  double bb = 0.0;                 // warp 0, lane 0: |b|^2
+  double rz = 1.0, rz_prev = 1.0;  // warp 1: r.z, and of the iteration before
+
+  // partial sum t of kind (0 p.q, 1 r.r, 2 r.z) into the boxes of the scene's groups
+  // d0, d0 + step, ...
+  auto send = [&](int kind, double t, unsigned tag, int d0, int step) {
+    for (int d = d0; d < ng; d += step) tag_put(boxes + (3 * (size_t)d + kind) * ng + (g - gbeg), t, tag);
+  };
+  // r.r and r.z of the group (c0, c1 per row): both trees in one set of steps (the lower 8
+  // lanes of a body's 16 reduce c0, the upper 8 c1), the body pair, then the warps in order;
+  // warps 0 and 1 send r.r, warps 2 and 3 r.z
+  auto publish_rr_rz = [&](double c0, double c1, unsigned tag) {
+    const bool up = (lane & 8) != 0;
+    const double o = __shfl_xor_sync(0xffffffffu, up ? c0 : c1, 8);
+    double v = up ? c1 + o : c0 + o;
+#pragma unroll
+    for (int d = 4; d > 0; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
+    v += __shfl_down_sync(0xffffffffu, v, 16);
+    if (lane == 0 || lane == 8) s_w[2 * warp + (lane >> 3)] = v;
+    row_barrier();
+    const int which = warp >> 1;
+    double t = s_w[which];
+#pragma unroll
+    for (int i = 1; i < GB / 2; ++i) t += s_w[2 * i + which];
+    send(1 + which, t, tag, (warp & 1) * 32 + lane, 64);
+    sent_arrive();
+  };
 
   // ---- init ----
   {
@@ -1316,185 +1527,96 @@ __global__ void __launch_bounds__(PCG_NT) k_pcg1(PcgArgs a) {
 #pragma unroll
         for (int c = 0; c < 12; ++c) zv += Dr[c] * a.b[12 * vbody + c];
       }
+      tag_put(t_z + idx, zv, 1u);
       r_r = bv;
       z_r = zv;
-      a.z[idx] = zv;
-      a.pbuf[idx] = 0.0;
-      a.pbuf[12 * a.nb + idx] = 0.0;
       c0 = bv * bv;
       c1 = bv * zv;
     }
-    if (vthr) {
-      c0 = body_sum16(c0);
-      c1 = body_sum16(c1);
-    }
-    group_partial(c0, c1, s_w, a.gpB, g);
+    publish_rr_rz(c0, c1, 1u);
   }
-  if (tid == 0) {
-    a.n_active[0] = 0;
-    a.n_active[1] = 0;
-    a.n_active[2] = 0;
-  }
-  grid.sync();
-  int k = 0;
-  for (;; ++k) {
-    const int par = k & 1;
-    const double* p_old = a.pbuf + (par ^ 1) * 12 * a.nb;
-    double* p_new = a.pbuf + par * 12 * a.nb;
-    if (tid == 0) a.n_active[(k + 1) % 3] = 0;
-    // ---- A_k ----
-    if (warp < 2) {
-      double v = warp_scene_sum(a.gpB, warp, a.sc_gbeg[sc], a.sc_gend[sc]);
+  for (int k = 0;; ++k) {
+    // ---- A_k: r.r (warp 0) and r.z (warp 1) of the scene ----
+    double sl[PCG1_G];
+    if (warp == 0 && !s_abort) {
+      if (!sum_gather(my_box + ng, ng, (unsigned)k + 1u, sl)) s_abort = 1;
+      const double rr = sum_form(sl, ng);
       if (lane == 0) {
-        s_sum[warp] = v;
-        // beta = r.z / previous r.z, divided here beside warp 0's sum instead of after it
-        if (warp == 1 && k > 0) s_beta = v / s_rzp;
-      }
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      const double rr = s_sum[0], rz = s_sum[1];
-      int* conv_cur = a.sc_conv + par * a.ns;
-      if (k > 0 && conv_r) {
-        if (owner) conv_cur[sc] = 1;
-        s_flag = 1;
-      } else {
         bool conv;
         if (k == 0) {
           conv = !a.sc_on[sc] || rr == 0.0;
-          if (owner) a.sc_bb[sc] = rr;
-          bb_r = rr;
+          bb = rr;
         } else {
-          conv = !(rr > a.tol2 * bb_r);
+          conv = !(rr > a.tol2 * bb);
         }
-        s_val = k == 0 ? 0.0 : s_beta;
-        s_flag = conv || k == a.maxit;
-        conv_r = conv ? 1 : 0;
-        rz_r = rz;
-        s_rzp = rz;
-        if (owner) {
-          a.sc_rz[par * a.ns + sc] = rz;
-          conv_cur[sc] = conv ? 1 : 0;
-          if (conv) {
-            a.sc_iters[sc] = k;
-          } else if (k == a.maxit) {
-            a.sc_iters[sc] = k;
-            a.out[0] = ABD_ERR_PCG_NOCONV;
-          } else {
-            atomicAdd(&a.n_active[k % 3], 1);
-          }
+        const int stop = conv || k == a.maxit;
+        s_flag = stop;
+        if (owner && stop) {
+          a.sc_iters[sc] = k;
+          atomicMax(&a.out[1], k);
+          if (!conv) a.out[0] = ABD_ERR_PCG_NOCONV;
         }
       }
+    } else if (warp == 1 && !s_abort) {
+      if (!sum_gather(my_box + 2 * ng, ng, (unsigned)k + 1u, sl)) s_abort = 1;
+      rz_prev = rz;
+      rz = sum_form(sl, ng);
+      if (lane == 0) s_beta = k == 0 ? 0.0 : rz / rz_prev;
     }
     __syncthreads();
-    const bool act = !s_flag;
-    const double beta = act ? s_val : 0.0;
-    double acc = 0.0;
-    if (act && pact) {
-      const unsigned half = 0xffffu << (threadIdx.x & 16);
-      // the neighbour entries of both register blocks are loaded before either is used
-      double zn[PCG1_NC], pn_[PCG1_NC];
+    if (s_flag || s_abort) break;
+    const double beta = s_beta;
+    const double pv = mine ? dir(z_r, beta, pold_r) : 0.0;
+    pold_r = pv;
+    done_wait();
+    // ---- p.q ----
+    double qv = 0.0, c0 = 0.0;
+    if (mine) {
+      const double* sp = s_part + 12 * NPART * vlb + row;
+      qv = sp[0];
 #pragma unroll
-      for (int jj = 0; jj < PCG1_NC; ++jj) {
-        const bool ld = part + NPART * jj < pn && prow < 12;
-        zn[jj] = ld ? a.z[12 * rc[jj] + prow] : 0.0;
-        pn_[jj] = ld ? p_old[12 * rc[jj] + prow] : 0.0;
-      }
-#pragma unroll
-      for (int jj = 0; jj < PCG1_NC; ++jj) {
-        const int j = part + NPART * jj;
-        if (j < pn) {
-          if (prow < 12) s_v[hg][prow] = dir(zn[jj], beta, pn_[jj]);
-          __syncwarp(half);
-          if (prow < 12) {
-            const double2* v = reinterpret_cast<const double2*>(s_v[hg]);
-#pragma unroll
-            for (int c = 0; c < 6; ++c) {
-              double2 vv = v[c];
-              acc += hr[jj][2 * c] * vv.x;
-              acc += hr[jj][2 * c + 1] * vv.y;
-            }
-          }
-          __syncwarp(half);
-        }
-      }
-      for (int j = part + NPART * PCG1_NC; j < pn; j += NPART) {
-        const int cb = a.rcol[pbase + j];
-        if (prow < 12) s_v[hg][prow] = dir(a.z[12 * cb + prow], beta, p_old[12 * cb + prow]);
-        __syncwarp(half);
-        if (prow < 12) {
-          const double2* H = reinterpret_cast<const double2*>(a.Hrow + (size_t)(pbase + j) * 144 + 12 * prow);
-          const double2* v = reinterpret_cast<const double2*>(s_v[hg]);
-#pragma unroll
-          for (int c = 0; c < 6; ++c) {
-            double2 h = H[c], vv = v[c];
-            acc += h.x * vv.x;
-            acc += h.y * vv.y;
-          }
-        }
-        __syncwarp(half);
-      }
+      for (int pp = 1; pp < NPART; ++pp) qv += sp[12 * pp];
+      c0 = pv * qv;
     }
-    s_part[threadIdx.x] = acc;
-    __syncthreads();
-    if (act) {
-      double c0 = 0.0;
-      if (mine) {
-        const double* sp = s_part + vlb * BODY_SLOTS + row;
-        double qv = sp[0];
+    c0 = body_sum16(c0);
+    c0 += __shfl_down_sync(0xffffffffu, c0, 16);
+    if (lane == 0) s_w[2 * warp] = c0;
+    row_barrier();
+    {
+      double t = s_w[0];
 #pragma unroll
-        for (int pp = 1; pp < NPART; ++pp) qv += sp[16 * pp];
-        const double pv = dir(z_r, beta, pold_r);
-        p_new[idx] = pv;
-        pv_r = pv;
-        q_r = qv;
-        c0 = pv * qv;
-      }
-      if (vthr) c0 = body_sum16(c0);
-      group_partial(c0, 0.0, s_w, a.gpA, g);
+      for (int i = 1; i < GB / 2; ++i) t += s_w[2 * i];
+      send(0, t, (unsigned)k + 1u, threadIdx.x, PCG1_ROWT);
     }
-    __syncthreads();
-    if (k == a.maxit) break;
-    grid.sync();
-    // the count of scenes still iterating and the p.q partials are loaded together
-    const int nact = ld_volatile(&a.n_active[k % 3]);
-    double pq = 0.0;
-    if (!s_flag && warp == 0) pq = warp_scene_sum(a.gpA, 0, a.sc_gbeg[sc], a.sc_gend[sc]);
-    if (nact == 0) break;
-    // ---- B_k (s_flag still holds whether the scene stopped in A_k: its CG ends there) ----
-    if (!s_flag) {
-      if (threadIdx.x == 0) s_val = rz_r / pq;
-      __syncthreads();
-      double c0 = 0.0, c1 = 0.0;
-      if (mine) {
-        const double alpha = s_val;
-        x_r += alpha * pv_r;
-        r_r -= alpha * q_r;
-      }
-      if (vthr) {
-        double zv = 0;
+    if (warp == 1) {
+      if (!sum_gather(my_box, ng, (unsigned)k + 1u, sl)) s_abort = 1;
+      const double pq = sum_form(sl, ng);
+      if (lane == 0) s_alpha = rz / pq;
+    }
+    row_barrier();
+    // ---- B_k: x, r, z ----
+    double d0 = 0.0, d1 = 0.0;
+    if (mine) {
+      const double alpha = s_alpha;
+      r_r -= alpha * qv;
+      x_r += alpha * pv;
+    }
+    double zv = 0;
 #pragma unroll
-        for (int c = 0; c < 12; ++c) zv += Dr[c] * __shfl_sync(0xffffffffu, r_r, (lane & 16) + c);
-        if (mine) {
-          z_r = zv;
-          a.z[idx] = zv;
-          pold_r = pv_r;
-          c0 = r_r * r_r;
-          c1 = r_r * zv;
-        }
-        c0 = body_sum16(c0);
-        c1 = body_sum16(c1);
-      }
-      group_partial(c0, c1, s_w, a.gpB, g);
+    for (int c = 0; c < 12; ++c) zv += Dr[c] * __shfl_sync(0xffffffffu, r_r, (lane & 16) + c);
+    if (mine) {
+      tag_put(t_z + idx, zv, (unsigned)k + 2u);
+      z_r = zv;
+      d0 = r_r * r_r;
+      d1 = r_r * zv;
     }
-    __syncthreads();
-    grid.sync();
+    publish_rr_rz(d0, d1, (unsigned)k + 2u);
   }
+  if (threadIdx.x == 0 && s_abort) a.out[0] = ABD_ERR_CUDA;
   if (mine) {
     a.x[idx] = x_r;
     a.dq[idx] = -x_r;
   }
-  if (tid == 0) a.out[1] = k;
 }
 
 // ---------------------------------------------------------------------------------
@@ -2011,6 +2133,8 @@ int pcg_solve(const Geo& g, PairSet& S, NewtonBufs& B, const SolveOpts& o, const
     *status = ABD_ERR_INVALID;
     return 0;
   }
+  B.slots.ensure(pcg1_words(B, nb));
+  B.pnb.ensure(12 * ((size_t)nb + S.nnz));
   B.gpA.ensure(2 * (size_t)B.ngrp);
   B.gpB.ensure(2 * (size_t)B.ngrp);
   B.sc_rz.ensure(2 * (size_t)ns);
@@ -2022,7 +2146,7 @@ int pcg_solve(const Geo& g, PairSet& S, NewtonBufs& B, const SolveOpts& o, const
   KLAUNCH(K_BLOCK_INVERSE, s, k_pcg_rows<<<nblk((long long)nb * 32, 256), 256, 0, s>>>(nb, S.row_ptr.p, S.col.p,
                                                                                         S.upidx.p, B.has.p, B.ovr.p,
                                                                                         B.D.p, B.Hrow.p, B.rcol.p,
-                                                                                        B.rn.p, B.status.p + 2));
+                                                                                        B.rn.p, B.status.p + 2, B.slots.p, pcg1_words(B, nb)));
   auto block_inverse = [&]() {
     KLAUNCH(K_BLOCK_INVERSE, s, k_block_inverse<<<nblk(nb, BINV_W), 32 * BINV_W, 0, s>>>(nb, B.D.p, B.Dinv.p,
                                                                                           B.status.p));
@@ -2059,7 +2183,7 @@ int pcg_solve(const Geo& g, PairSet& S, NewtonBufs& B, const SolveOpts& o, const
     max_blocks1 = sms * per1;
   }
   // one group per CTA when the groups fit one cooperative wave, else groups in loop steps
-  const bool one = B.ngrp <= max_blocks1;
+  const bool one = B.ngrp <= max_blocks1 && B.ngrp <= PCG1_MAXGRP;
   int grid = one ? B.ngrp : (B.ngrp < max_blocks ? B.ngrp : max_blocks);
   if (grid < 1) grid = 1;
   PcgArgs a;
@@ -2094,6 +2218,9 @@ int pcg_solve(const Geo& g, PairSet& S, NewtonBufs& B, const SolveOpts& o, const
   a.tol2 = rel_tol * rel_tol;
   a.maxit = max_iter < 0 ? 0 : max_iter;
   a.out = B.status.p;
+  a.slots = B.slots.p;
+  a.pnb = B.pnb.p;
+  a.sc_box = B.sc_box.p;
   void* args[] = {&a};
   const void* kern = one ? (void*)k_pcg1 : (void*)k_pcg;
   if (run_pcg) KLAUNCH(K_PCG, s, CK(cudaLaunchCooperativeKernel(kern, dim3(grid), dim3(PCG_NT), args, 0, s)));
@@ -2121,6 +2248,8 @@ int pcg_solve(const Geo& g, PairSet& S, NewtonBufs& B, const SolveOpts& o, const
       KLAUNCH(K_PCG, s, k_true_residual<<<nblk(nrows, 256), 256, 0, s>>>(nb, S.row_ptr.p, B.rcol.p, B.rn.p,
                                                                          B.Hrow.p, g.bscene, pcg_mask, B.grad.p,
                                                                          B.xr.p, B.rt.p));
+      CK(cudaMemsetAsync(B.slots.p, 0, pcg1_words(B, nb) * sizeof(unsigned long long), s));
+      CK(cudaMemsetAsync(B.status.p + 1, 0, sizeof(int), s));
       KLAUNCH(K_PCG, s, CK(cudaLaunchCooperativeKernel(kern, dim3(grid), dim3(PCG_NT), cargs, 0, s)));
       KLAUNCH(K_VEC, s, k_refine_add<<<nblk(nrows, 256), 256, 0, s>>>(nrows, B.xr.p, B.x.p, dq));
       KLAUNCH(K_VEC, s, k_iter_add<<<1, 32, 0, s>>>(ns, B.status.p + 1, B.sc_iters.p, B.it_ref.p));
@@ -2145,6 +2274,7 @@ int pcg_solve(const Geo& g, PairSet& S, NewtonBufs& B, const SolveOpts& o, const
       for (int k = 0; k < ns; ++k) scene_iters[k] = 0;
   }
   *status = B.h_int[0];
+  if (*status == ABD_ERR_CUDA) throw CudaError{cudaErrorLaunchTimeout, "pcg: the sums of a group did not arrive"};
   // per iteration: the kept blocks once (1152 B each) and ~6 vector streams
   prof_work(K_PCG, B.h_int[1], B.h_int[1] * (1152.0 * B.h_int[2] + 6 * 96.0 * nb) + 1152.0 * nb);
   prof_work(K_BLOCK_INVERSE, 1, 2 * 1152.0 * B.h_int[2]);
@@ -2152,7 +2282,8 @@ int pcg_solve(const Geo& g, PairSet& S, NewtonBufs& B, const SolveOpts& o, const
 }
 
 void pcg_groups(const std::vector<int>& sc_beg, const std::vector<int>& sc_end, NewtonBufs& B, cudaStream_t s) {
-  std::vector<int> gb, gn, gs, sgb, sge;
+  std::vector<int> gb, gn, gs, sgb, sge, box;
+  size_t n_box = 0;
   for (size_t k = 0; k < sc_beg.size(); ++k) {
     sgb.push_back((int)gb.size());
     for (int b = sc_beg[k]; b < sc_end[k]; b += GB) {
@@ -2161,13 +2292,18 @@ void pcg_groups(const std::vector<int>& sc_beg, const std::vector<int>& sc_end, 
       gs.push_back((int)k);
     }
     sge.push_back((int)gb.size());
+    const size_t ng = (size_t)(sge.back() - sgb.back());
+    box.push_back((int)n_box);
+    n_box += 3 * ng * ng;
+    if (gb.size() > PCG1_MAXGRP) n_box = 0;  // k_pcg serves these; no boxes
   }
   B.ngrp = (int)gb.size();
+  B.n_box = n_box;
   B.h_sc_beg = sc_beg;
   B.h_sc_end = sc_end;
-  DBuf<int>* dst[] = {&B.grp_body, &B.grp_n, &B.grp_scene, &B.sc_gbeg, &B.sc_gend};
-  std::vector<int>* src[] = {&gb, &gn, &gs, &sgb, &sge};
-  for (int i = 0; i < 5; ++i) {
+  DBuf<int>* dst[] = {&B.grp_body, &B.grp_n, &B.grp_scene, &B.sc_gbeg, &B.sc_gend, &B.sc_box};
+  std::vector<int>* src[] = {&gb, &gn, &gs, &sgb, &sge, &box};
+  for (int i = 0; i < 6; ++i) {
     dst[i]->ensure(src[i]->size() + 1);
     if (!src[i]->empty())
       CK(cudaMemcpyAsync(dst[i]->p, src[i]->data(), src[i]->size() * sizeof(int), cudaMemcpyHostToDevice, s));
