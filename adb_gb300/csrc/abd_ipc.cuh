@@ -786,6 +786,20 @@ struct S9Rec {
   size_t stride;
 };
 DEV void s9_put(const S9Rec& o, int p, int q, double v) { o.base[(size_t)s9_index(p, q) * o.stride] = v; }
+struct S9Reg {  // upper triangle in registers (constant indices)
+  double v[45];
+};
+DEV void s9_put(S9Reg& o, int p, int q, double v) { o.v[s9_index(p, q)] = v; }
+DEV double s9_get(const S9Reg& o, int p, int q) { return o.v[p <= q ? s9_index(p, q) : s9_index(q, p)]; }
+// Entry of the vertex-space Hessian (Q (x) I) S (Q (x) I)^T: vertices i and j, components r and
+// s. A vertex has two of Q's columns: its edge's (0 for vertices 0 and 1, else 1) and the mean.
+template <class F>
+DEV double vertex_entry(int i, int j, int r, int s, F&& S) {
+  const int a = i < 2 ? 0 : 1, b = j < 2 ? 0 : 1;
+  const double t0 = Qe(i, a) * S(3 * a + r, 3 * b + s) + Qe(i, 2) * S(6 + r, 3 * b + s);
+  const double t2 = Qe(i, a) * S(3 * a + r, 6 + s) + Qe(i, 2) * S(6 + r, 6 + s);
+  return t0 * Qe(j, b) + t2 * Qe(j, 2);
+}
 
 // Reduced projection of a non-mollified pair: H lives in the span of
 // { c (x) e_x, c (x) e_y, c (x) e_z, a_k' (x) w } (a_k' = the parameter directions
