@@ -264,6 +264,9 @@ struct NewtonBufs {
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_fork_pt = nullptr, ev_join_pt = nullptr;
   DBuf<double> ovr;          // nov * CONTRIB
   DBuf<int> has;             // nov
+  DBuf<int> off_pos;         // off_blocks: place of each overlap's block, the blocks and their keys
+  DBuf<int2> off_keys;
+  DBuf<double> off_vals;
   DBuf<double> D, Dinv, grad;
   DBuf<double> x, r, z, p, qv;   // p: two buffers (iteration parity)
   DBuf<double> Hrow;         // row-block copy of the system for the PCG
@@ -301,6 +304,9 @@ struct NewtonBufs {
   int* h_int = nullptr;
 };
 void assemble(const Geo& g, const Params& P, PairSet& S, NewtonBufs& nb, cudaStream_t s);
+// Number of off-diagonal blocks of the system assembled last on S; with gather, their keys and
+// entries in overlap order in B.off_keys / B.off_vals. Synchronises.
+int off_blocks(const PairSet& S, NewtonBufs& B, bool gather, cudaStream_t s);
 // Solves H x = grad per scene (scenes with sc_on[s] == 0 get x = 0); dq = -x. Returns the
 // iterations of the longest scene; scene_iters (host, ns) receives each scene's count.
 // Body groups of the PCG (consecutive bodies of one scene, cut from the scene's first

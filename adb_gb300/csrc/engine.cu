@@ -1,6 +1,7 @@
 // Host side of the GB300 step: the handle, its device buffers, the per-frame Newton
 // loop (the reference's ABD::implicit_euler, model/abd.cpp:30-140, with ccd() :142-196
 // and line_search(dt) :198-227 / model/line_search.cpp:39-136) and the C ABI.
+#include <algorithm>
 #include <chrono>
 #include <cmath>
 #include <cstring>
@@ -151,7 +152,8 @@ struct Engine {
     if (cs.h_ll) cudaFreeHost(cs.h_ll);
     if (cs.h_toi) cudaFreeHost(cs.h_toi);
     nbufs.pt_c.release(); nbufs.ee_c.release(); nbufs.pt_seg.release(); nbufs.ee_seg.release();
-    nbufs.ovr.release(); nbufs.has.release(); nbufs.D.release(); nbufs.Dinv.release(); nbufs.grad.release();
+    nbufs.ovr.release(); nbufs.has.release(); nbufs.off_pos.release(); nbufs.off_keys.release();
+    nbufs.off_vals.release(); nbufs.D.release(); nbufs.Dinv.release(); nbufs.grad.release();
     nbufs.x.release(); nbufs.r.release(); nbufs.z.release(); nbufs.p.release(); nbufs.qv.release();
     nbufs.Hrow.release(); nbufs.rcol.release(); nbufs.rn.release();
     for (int k = 0; k < 2; ++k) {
@@ -863,23 +865,12 @@ int abd_newton_system(abd_handle* h, const double* q, double* grad, double* diag
     abd::PairSet& S = e.sets[e.cur];
     if (grad) CK(cudaMemcpy(grad, e.nbufs.grad.p, 12 * (size_t)e.nb * sizeof(double), cudaMemcpyDeviceToHost));
     if (diag) CK(cudaMemcpy(diag, e.nbufs.D.p, 144 * (size_t)e.nb * sizeof(double), cudaMemcpyDeviceToHost));
-    int nov = S.nov;
-    std::vector<int> has(nov + 1), oi(nov + 1), oj(nov + 1);
-    if (nov) {
-      CK(cudaMemcpy(has.data(), e.nbufs.has.p, nov * sizeof(int), cudaMemcpyDeviceToHost));
-      CK(cudaMemcpy(oi.data(), S.ovI.p, nov * sizeof(int), cudaMemcpyDeviceToHost));
-      CK(cudaMemcpy(oj.data(), S.ovJ.p, nov * sizeof(int), cudaMemcpyDeviceToHost));
-    }
-    int k = 0;
-    for (int u = 0; u < nov; ++u) {
-      if (!has[u]) continue;
-      if (off_keys && k < max_off) {
-        off_keys[2 * k] = oi[u];
-        off_keys[2 * k + 1] = oj[u];
-        CK(cudaMemcpy(off_vals + 144 * (size_t)k, e.nbufs.ovr.p + (size_t)u * abd::CONTRIB + 288,
-                      144 * sizeof(double), cudaMemcpyDeviceToHost));
-      }
-      ++k;
+    const bool want = off_keys && max_off > 0;
+    const int k = abd::off_blocks(S, e.nbufs, want, e.s);
+    const int m = std::min(k, max_off);
+    if (want && m > 0) {
+      CK(cudaMemcpy(off_keys, e.nbufs.off_keys.p, 2 * (size_t)m * sizeof(int), cudaMemcpyDeviceToHost));
+      CK(cudaMemcpy(off_vals, e.nbufs.off_vals.p, 144 * (size_t)m * sizeof(double), cudaMemcpyDeviceToHost));
     }
     if (n_off) *n_off = k;
     return (int)ABD_OK;

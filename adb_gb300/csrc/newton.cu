@@ -575,6 +575,17 @@ __global__ void __launch_bounds__(512) k_ov_reduce(int nov, const int* pt_seg, c
   }
 }
 
+// Off-diagonal blocks of the overlaps with a contribution, in overlap order: keys (I, J) and
+// the 144 entries, one CTA per overlap (pos: exclusive scan of has).
+__global__ void __launch_bounds__(160) k_off_blocks(int nov, const int* has, const int* pos, const int* ovI,
+                                                    const int* ovJ, const double* ovr, int2* keys, double* vals) {
+  const int u = blockIdx.x;
+  if (u >= nov || !has[u]) return;
+  const int k = pos[u], t = threadIdx.x;
+  if (t < 144) vals[(size_t)k * 144 + t] = ovr[(size_t)u * CONTRIB + 288 + t];
+  if (t == 144) keys[k] = make_int2(ovI[u], ovJ[u]);
+}
+
 // Per-body diagonal block and gradient: one CTA per body, threads 0..143 own the
 // Hessian entries, 144..155 the gradient entries.
 __global__ void __launch_bounds__(160) k_body_system(Geo g, Params P, const int* row_ptr, const int* col,
@@ -2111,6 +2122,24 @@ void assemble(const Geo& g, const Params& P, PairSet& S, NewtonBufs& B, cudaStre
   }
   KLAUNCH(K_BODY_SYSTEM, s, k_body_system<<<nb, 160, 0, s>>>(g, P, S.row_ptr.p, S.col.p, S.upidx.p, B.ovr.p, B.has.p, S.vg.p, S.vg_seg.p,
                                    S.vg_lam.p, B.D.p, B.grad.p));
+}
+
+int off_blocks(const PairSet& S, NewtonBufs& B, bool gather, cudaStream_t s) {
+  const int nov = S.nov;
+  if (!nov) return 0;
+  B.off_pos.ensure((size_t)nov + 1);
+  scan_exclusive_int(B.has.p, B.off_pos.p, nov, B.off_pos.p + nov, s, B.cls_tmp[1]);
+  int n = 0;
+  CK(cudaMemcpyAsync(&n, B.off_pos.p + nov, sizeof(int), cudaMemcpyDeviceToHost, s));
+  CK(cudaStreamSynchronize(s));
+  if (gather && n) {
+    B.off_keys.ensure(n);
+    B.off_vals.ensure(144 * (size_t)n);
+    KLAUNCH(K_VEC, s, k_off_blocks<<<nov, 160, 0, s>>>(nov, B.has.p, B.off_pos.p, S.ovI.p, S.ovJ.p, B.ovr.p,
+                                                       B.off_keys.p, B.off_vals.p));
+    CK(cudaStreamSynchronize(s));
+  }
+  return n;
 }
 
 int pcg_solve(const Geo& g, PairSet& S, NewtonBufs& B, const SolveOpts& o, const int* sc_on,
