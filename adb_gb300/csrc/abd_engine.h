@@ -112,9 +112,10 @@ struct CullScratch {
   DBuf<long long> cand_cnt, cand_off;
   DBuf<uint8_t> flags;
   DBuf<int> blk_a, blk_b, blk_a_off, blk_b_off;
-  DBuf<int> vflag_cnt, vflag_off, sub_cnt, stage_off;
+  DBuf<int> vflag_cnt, vflag_off, stage_ov;
+  DBuf<int4> stage_seg;
   DBuf<int> vg_cnt;  // vertex-ground pairs per block of vertices
-  DBuf<unsigned long long> stage_key;   // sorted accepted pairs per overlap (sub, i, j)
+  DBuf<unsigned long long> stage_key;   // sorted candidates per overlap (sub, i, j)
   DBuf<int8_t> stage_ty;
   DBuf<unsigned long long> toi_key;     // 2 per scene: pt/ee, ground
   DBuf<int2> toi_cand;                  // trajectory candidates left to the FP64 test, and their number

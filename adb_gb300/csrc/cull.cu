@@ -19,6 +19,7 @@
 // tests first run on float copies of the boxes rounded outward (__double2float_rd/_ru):
 // a float miss implies an exact miss, so the float prefilter never changes the result
 // and saves the scarce FP64 pipe (GB300: 1.2 TFLOP/s FP64 vs 70 TFLOP/s FP32).
+#include <algorithm>
 #include "abd_ccd_filter.cuh"
 #include "abd_engine.h"
 #include "abd_exact.cuh"
@@ -347,22 +348,22 @@ __global__ void __launch_bounds__(256, 3) k_bin(Geo g, int nov, int pass, int tr
 
 constexpr int NT = 256;     // narrow-phase threads per CTA
 constexpr int TILE = 384;   // primitives of one list staged in shared memory (2 x 9 kB)
-constexpr int REC_CAP = 2048;  // accepted pairs of one overlap kept in shared memory for sorting
-// Box-phase candidates per thread between two exact phases (STEP), and the queue of
-// float-box hits they fill (NT * STEP entries). A longer box phase runs the exact phase
+constexpr int REC_CAP = 2048;  // candidates of one overlap kept in shared memory for sorting
+// Box-phase candidates per thread between two test phases (STEP), and the queue of
+// float-box hits they fill (NT * STEP entries). A longer box phase runs the phase after it
 // less often; a shorter one leaves shared memory for more CTAs per SM. The result does not
-// depend on STEP (accepted pairs are sorted by key before they are written, TOIs are
+// depend on STEP (candidates are sorted by key before they are written, TOIs are
 // min-reduced), so the autotuner picks among these variants by time: pair cull (mode 0)
-// 32 / 64 / 96, CCD (mode 2) 24 / 36 / 64; the defaults are the middle ones (measured
-// fastest on the pile when the choice was fixed).
+// 16 / 8 / 48, CCD (mode 2) 24 / 36 / 64; the defaults are the middle ones (columns: 237 us
+// with 16 at 3 CTAs per SM, 212 us with 8 at 4; the pile 198 us with either).
 constexpr int kNarrowVariants = 3;
-constexpr int kNarrowStep[2][kNarrowVariants] = {{32, 64, 96}, {24, 36, 64}};
+constexpr int kNarrowStep[2][kNarrowVariants] = {{16, 8, 48}, {24, 36, 64}};
 constexpr int kNarrowDefault = 1;
-// dynamic shared memory of k_narrow_scan<MODE, STEP>: boxes, queue, accepted pairs (MODE 0)
+// dynamic shared memory of k_narrow_scan<MODE, STEP>: boxes, queue, candidates (MODE 0)
 // (MODE 0 also stages the vertex ids of the staged primitives: 2 per A entry, 3 per B)
 __host__ __device__ constexpr size_t narrow_smem(int mode, int step) {
   return 2 * TILE * 6 * sizeof(float) + (size_t)NT * step * sizeof(unsigned) +
-         (mode == 0 ? REC_CAP * (sizeof(unsigned long long) + 1) + 5 * TILE * sizeof(int) : 0);
+         (mode == 0 ? REC_CAP * sizeof(unsigned long long) + 5 * TILE * sizeof(int) : 0);
 }
 
 __device__ __forceinline__ void finflate(const float* s, float ds, float* o) {
@@ -610,6 +611,21 @@ struct ToiCand {
 };
 constexpr unsigned kToiCand = 1u << 21;  // 16 MB; a candidate past it is evaluated where it is found
 
+// Candidates of the pair cull left to the FP64 test, by overlap, each overlap's sorted by
+// (sub, i, j): the point-triangle ones from the front of the buffer, the edge-edge ones from its
+// end, so that a warp of k_narrow_exact runs one kind. seg: an overlap's two segments (first
+// entry, count; first entry -1: not staged); total: both kinds' candidates (more than cap
+// together: the segments are not valid and the cull is repeated with a larger buffer).
+struct StageOut {
+  unsigned long long* key;
+  int* ov;
+  int8_t* ty;  // distance type, -1: rejected (k_narrow_exact)
+  int4* seg;   // {first PT, PT count, first EE, EE count}
+  int* total;
+  int cap;
+  __device__ __forceinline__ bool valid() const { return (long long)total[0] + total[1] <= cap; }
+};
+
 struct NarrowOut {
   int *pt, *pt_ov, *ee, *ee_ov;
   int8_t *pt_ty, *ee_ty;
@@ -813,46 +829,45 @@ __global__ void __launch_bounds__(128) k_toi_list(Geo g, ToiCand tc, unsigned lo
   }
 }
 
-// 5a. Narrow phase, one CTA per overlap, count (MODE 0) or trajectory TOI (MODE 2).
+// 5a. Narrow phase, one CTA per overlap: pair cull (MODE 0) or trajectory (MODE 2).
 // For each sub-problem (v(I) x f(J), v(J) x f(I), e(I) x e(J)) the float boxes of both
 // lists are staged in shared memory. The work alternates between two phases so that the
 // FP64 work is spread evenly over the CTA:
 //  - box phase: each thread keeps one A box in registers and walks its B boxes (a
 //    shared-memory broadcast per step), STEP candidates per thread, and appends the
 //    float-box hits to a shared queue (warp-aggregated);
-//  - exact phase: the whole CTA takes the queued candidates round-robin for the exact
-//    FP64 test (MODE 0: box, lower bounds, type and distance; MODE 2: time of impact).
-// MODE 2 runs no FP64 here: it drops the candidates that an FP32 certificate proves to have no
-// time of impact (abd_ccd_filter.cuh; on the pile about 19 of 20) and appends the others to a
-// list that k_toi_list evaluates. An FP64 test is a chain of about 900 instructions of 64
-// cycles a warp, some 28 us, which a CTA with a handful of candidates per box phase used to
-// pay for each of its phases; the list fills whole warps on all SMs.
+//  - test phase: the whole CTA takes the queued candidates round-robin for the FP32 tests:
+//    lower bounds of the distance (MODE 0, f_reject), certificates that there is no time of
+//    impact (MODE 2, abd_ccd_filter.cuh).
+// No FP64 runs here. The candidates left go to lists that k_narrow_exact and k_toi_list
+// evaluate, a thread each: an FP64 test is a chain of some 300 (distance) or 900 (time of
+// impact) instructions of 64 cycles a warp, which a CTA with a handful of candidates used to
+// pay for each sub-problem and box phase. MODE 0 keeps an overlap's candidates in shared
+// memory and writes them sorted, so that the accepted ones come out in order. One cull of a
+// batch of columns (7291 overlaps, 11 candidates each) 893 -> 280 us, of the pile (9871, 19
+// each) 583 -> 310 us, the FP64 kernel included.
 template <int MODE, int STEP>
-__global__ void __launch_bounds__(NT, (MODE == 2 && STEP <= 36) ? 4 : 2) k_narrow_scan(Geo g, Params P, float ds_f, const int* ovI, const int* ovJ,
-                                                    int* cnt, const int* off, int* lst, const float* vb,
-                                                    const float* eb, const float* fb, int* sub_cnt,
-                                                    unsigned long long* toi_key, unsigned long long* stage_key,
-                                                    int8_t* stage_ty, int* stage_off, int* stage_total,
-                                                    int stage_cap, const int* order, ToiCand tc) {
+__global__ void __launch_bounds__(NT, MODE == 0 ? (STEP <= 8 ? 4 : STEP <= 16 ? 3 : 2) : (STEP <= 36 ? 4 : 2))
+    k_narrow_scan(Geo g, Params P, float ds_f, const int* ovI, const int* ovJ, int* cnt, const int* off, int* lst,
+                  const float* vb, const float* eb, const float* fb, unsigned long long* toi_key, StageOut so,
+                  const int* order, ToiCand tc) {
   extern __shared__ __align__(16) unsigned char smem_dyn[];
   unsigned long long* recK = reinterpret_cast<unsigned long long*>(smem_dyn);  // REC_CAP (MODE 0)
   float* sA = reinterpret_cast<float*>(smem_dyn + (MODE == 0 ? REC_CAP * sizeof(unsigned long long) : 0));
   float* sB = sA + TILE * 6;
   unsigned int* sq = reinterpret_cast<unsigned int*>(sB + TILE * 6);
-  int8_t* recT = reinterpret_cast<int8_t*>(sq + NT * STEP);
-  int* sVA = MODE == 0 ? reinterpret_cast<int*>(recT + REC_CAP) : nullptr;  // 2 * TILE (MODE 0)
-  int* sVB = MODE == 0 ? sVA + 2 * TILE : nullptr;                           // 3 * TILE (MODE 0)                         // REC_CAP (MODE 0)
+  int* sVA = MODE == 0 ? reinterpret_cast<int*>(sq + NT * STEP) : nullptr;  // 2 * TILE (MODE 0)
+  int* sVB = MODE == 0 ? sVA + 2 * TILE : nullptr;                          // 3 * TILE (MODE 0)
   __shared__ int sq_n[2];
-  __shared__ int rec_n, rec_base;
+  __shared__ int rec_n, rec_np, rec_base[2];
   const int u = order[blockIdx.x];
   const float lim_f = __double2float_ru(P.dhat * (1.0 + 1e-4));
   int* n = cnt + 6 * u;
   const int* o = off + 6 * u;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const unsigned below = (1u << lane) - 1u;
-  int c3s[3] = {0, 0, 0};
   if (threadIdx.x == 0) {
-    rec_n = 0;
+    rec_n = rec_np = 0;
     sq_n[0] = 0;
     sq_n[1] = 0;
   }
@@ -861,7 +876,6 @@ __global__ void __launch_bounds__(NT, (MODE == 2 && STEP <= 36) ? 4 : 2) k_narro
   for (int sub = 0; sub < 3; ++sub) {
     SubLists L = sub_lists(g, sub, ovI[u], ovJ[u], n, o, lst, vb, eb, fb);  // lists refined by k_refine
     if (L.nA == 0 || L.nB == 0) continue;
-    int cs = 0;
 #pragma unroll 1
     for (int a0 = 0; a0 < L.nA; a0 += TILE) {
       const int ca = min(TILE, L.nA - a0);
@@ -889,7 +903,7 @@ __global__ void __launch_bounds__(NT, (MODE == 2 && STEP <= 36) ? 4 : 2) k_narro
         for (int st = 0; st < steps; ++st) {
           // box phase
 #pragma unroll 1
-          for (int it = 0; it < STEP; ++it) {
+          for (int it = 0, its = min(STEP, max_items - st * STEP); it < its; ++it) {
             bool hit = false;
             unsigned code = 0;
             if (ri < nrow) {
@@ -912,7 +926,7 @@ __global__ void __launch_bounds__(NT, (MODE == 2 && STEP <= 36) ? 4 : 2) k_narro
             }
           }
           __syncthreads();
-          // exact phase
+          // test phase
           const int nq = sq_n[par];
           if (threadIdx.x == 0) sq_n[par ^ 1] = 0;
 #pragma unroll 1
@@ -931,16 +945,11 @@ __global__ void __launch_bounds__(NT, (MODE == 2 && STEP <= 36) ? 4 : 2) k_narro
               const int w1 = sub < 2 ? sVB[3 * j] : sVA[2 * i + 1];
               const int w2 = sub < 2 ? sVB[3 * j + 1] : sVB[3 * j];
               const int w3 = sub < 2 ? sVB[3 * j + 2] : sVB[3 * j + 1];
-              int f = f_reject_v(vb, sub, w0, w1, w2, w3, lim_f) ? 0 : exact_pair_v(g, P, sub, w0, w1, w2, w3);
-              if (f) {
-                ++cs;
-                int slot = atomicAdd(&rec_n, 1);
-                if (slot < REC_CAP) {
-                  recK[slot] = ((unsigned long long)sub << 60) | ((unsigned long long)(a0 + i) << 30) |
-                               (unsigned long long)(b0 + j);
-                  recT[slot] = (int8_t)(f - 1);
-                }
-              }
+              if (f_reject_v(vb, sub, w0, w1, w2, w3, lim_f)) continue;
+              const int slot = atomicAdd(&rec_n, 1);
+              if (slot < REC_CAP)
+                recK[slot] = ((unsigned long long)sub << 60) | ((unsigned long long)(a0 + i) << 30) |
+                             (unsigned long long)(b0 + j);
             }
           }
           par ^= 1;
@@ -948,170 +957,201 @@ __global__ void __launch_bounds__(NT, (MODE == 2 && STEP <= 36) ? 4 : 2) k_narro
         }
       }
     }
-    c3s[sub] = cs;
   }
   if (MODE == 0) {
-    __shared__ int sh[3][NT / 32];
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      int v = c3s[k];
-#pragma unroll
-      for (int q = 16; q > 0; q >>= 1) v += __shfl_xor_sync(0xffffffffu, v, q);
-      if (lane == 0) sh[k][w] = v;
-    }
+    // Sort the (sub, i, j) keys and stage them: up to NT by rank (keys differ; each thread
+    // counts the keys below its own), more by a bitonic sort in shared memory. Overlaps with more
+    // candidates than REC_CAP are marked and go through passes that recompute their tests.
     __syncthreads();
-    if (threadIdx.x < 3) {
-      int t = 0;
-      for (int q = 0; q < NT / 32; ++q) t += sh[threadIdx.x][q];
-      sub_cnt[3 * u + threadIdx.x] = t;
-    }
-    // Sort the collected (sub, i, j) keys (bitonic, shared memory) and stage them, so
-    // the write pass only copies. Overlaps with more pairs than REC_CAP are marked
-    // (stage_off = -1) and written by the recomputing pass instead.
-    // stage_total[1] counts the overlaps left to the recomputing pass
-    int nr = rec_n;
+    const int nr = rec_n;
     if (nr > REC_CAP || nr == 0) {
-      if (threadIdx.x == 0) {
-        stage_off[u] = (nr == 0) ? 0 : -1;
-        if (nr) atomicAdd(stage_total + 1, 1);
-      }
+      if (threadIdx.x == 0) so.seg[u] = make_int4(nr == 0 ? 0 : -1, 0, 0, 0);
       return;
     }
-    int np2 = 1;
-    while (np2 < nr) np2 <<= 1;
-    for (int k = nr + threadIdx.x; k < np2; k += NT) recK[k] = ~0ull;
-    __syncthreads();
-    for (int size = 2; size <= np2; size <<= 1)
-      for (int stride = size >> 1; stride > 0; stride >>= 1) {
-        for (int t = threadIdx.x; t < (np2 >> 1); t += NT) {
-          int lo = 2 * t - (t & (stride - 1));
-          int hi = lo + stride;
-          bool up = ((lo & size) == 0);
-          unsigned long long a = recK[lo], b = recK[hi];
-          if ((a > b) == up) {
-            recK[lo] = b;
-            recK[hi] = a;
-            int8_t ta = recT[lo];
-            recT[lo] = recT[hi];
-            recT[hi] = ta;
-          }
-        }
-        __syncthreads();
-      }
-    if (threadIdx.x == 0) {
-      int base = atomicAdd(stage_total, nr);
-      rec_base = (base + nr <= stage_cap) ? base : -2;
-      stage_off[u] = rec_base;
-      if (rec_base < 0) atomicAdd(stage_total + 1, 1);
-    }
-    __syncthreads();
-    if (rec_base >= 0)
-      for (int k = threadIdx.x; k < nr; k += NT) {
-        stage_key[rec_base + k] = recK[k];
-        stage_ty[rec_base + k] = recT[k];
-      }
-  }
-}
-
-// 5b'. Copy of the staged, sorted pairs of each overlap to their final slots.
-__global__ void k_narrow_copy(int nov, const int* ovI, const int* ovJ, const int* off, const int* lst,
-                              const int* sub_cnt, const unsigned long long* stage_key, const int8_t* stage_ty,
-                              const int* stage_off, const int* ov_pt_off, const int* ov_ee_off, NarrowOut out) {
-  int u = blockIdx.x;
-  if (u >= nov) return;
-  const int* sc = sub_cnt + 3 * u;
-  int nr = sc[0] + sc[1] + sc[2];
-  int so = stage_off[u];
-  if (nr == 0 || so < 0) return;
-  int I = ovI[u], J = ovJ[u];
-  const int* o = off + 6 * u;
-  for (int k = threadIdx.x; k < nr; k += blockDim.x) {
-    unsigned long long key = stage_key[so + k];
-    int sub = (int)(key >> 60);
-    int i = (int)((key >> 30) & 0x3fffffffull), j = (int)(key & 0x3fffffffull);
-    int la = sub == 0 ? 0 : (sub == 1 ? 3 : 1), lb = sub == 0 ? 5 : (sub == 1 ? 2 : 4);
-    int A = (sub == 1) ? J : I, B = (sub == 1) ? I : J;
-    int a_id = lst[o[la] + i], b_id = lst[o[lb] + j];
-    if (sub < 2) {
-      int idx = ov_pt_off[u] + k;
-      out.pt[4 * idx] = A; out.pt[4 * idx + 1] = a_id; out.pt[4 * idx + 2] = B; out.pt[4 * idx + 3] = b_id;
-      out.pt_ty[idx] = stage_ty[so + k];
-      out.pt_ov[idx] = u;
+    unsigned long long key = threadIdx.x < nr ? recK[threadIdx.x] : ~0ull;
+    int c = 0;
+    for (int k = threadIdx.x; k < nr; k += NT) c += (int)(recK[k] >> 60) < 2;
+    if (c) atomicAdd(&rec_np, c);
+    if (nr <= NT) {
+      int r = 0;
+      if (threadIdx.x < nr)
+        for (int k = 0; k < nr; ++k) r += recK[k] < key;
+      __syncthreads();
+      if (threadIdx.x < nr) recK[r] = key;
     } else {
-      int idx = ov_ee_off[u] + (k - sc[0] - sc[1]);
-      out.ee[4 * idx] = A; out.ee[4 * idx + 1] = a_id; out.ee[4 * idx + 2] = B; out.ee[4 * idx + 3] = b_id;
-      out.ee_ty[idx] = stage_ty[so + k];
-      out.ee_ov[idx] = u;
+      int np2 = NT;
+      while (np2 < nr) np2 <<= 1;
+      for (int k = nr + threadIdx.x; k < np2; k += NT) recK[k] = ~0ull;
+      __syncthreads();
+      for (int size = 2; size <= np2; size <<= 1)
+        for (int stride = size >> 1; stride > 0; stride >>= 1) {
+          for (int t = threadIdx.x; t < (np2 >> 1); t += NT) {
+            int lo = 2 * t - (t & (stride - 1));
+            int hi = lo + stride;
+            bool up = ((lo & size) == 0);
+            unsigned long long a = recK[lo], b = recK[hi];
+            if ((a > b) == up) {
+              recK[lo] = b;
+              recK[hi] = a;
+            }
+          }
+          __syncthreads();
+        }
     }
+    __syncthreads();
+    const int np = rec_np, ne = nr - np;
+    if (threadIdx.x == 0) {
+      const int bp = np ? atomicAdd(so.total, np) : 0, be = ne ? atomicAdd(so.total + 1, ne) : 0;
+      const bool ok = bp <= so.cap - np && be <= so.cap - ne;
+      rec_base[0] = ok ? bp : -1;
+      rec_base[1] = so.cap - be - ne;
+      so.seg[u] = make_int4(rec_base[0], np, rec_base[1], ne);
+    }
+    __syncthreads();
+    if (rec_base[0] >= 0)
+      for (int k = threadIdx.x; k < nr; k += NT) {
+        const int p = k < np ? rec_base[0] + k : rec_base[1] + (k - np);
+        so.key[p] = recK[k];
+        so.ov[p] = u;
+      }
   }
 }
 
-// 5b. Ordered write for the overlaps whose pairs did not fit the shared-memory sort. The
-// (i, j) space of each sub-problem is walked in row-major order (the order of the
-// reference's nested loops), NT candidates at a time, with a CTA-wide ordered
-// compaction, stopping once the sub-problem's count (from the count pass) is written.
-__global__ void __launch_bounds__(NT) k_narrow_write(Geo g, Params P, float ds_f, const int* ovI, const int* ovJ,
-                                                     const int* cnt, const int* off, const int* lst, const float* vb,
-                                                     const float* eb, const float* fb, const int* sub_cnt,
-                                                     const int* ov_pt_off, const int* ov_ee_off, NarrowOut out,
-                                                     const int* stage_off) {
-  __shared__ int wcnt[NT / 32];
-  const int u = blockIdx.x;
-  const int* sc = sub_cnt + 3 * u;
-  if (sc[0] + sc[1] + sc[2] == 0 || stage_off[u] >= 0) return;
-  const int* n = cnt + 6 * u;
-  const int* o = off + 6 * u;
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const unsigned below = (1u << lane) - 1u;
-  int run_pt = ov_pt_off[u], run_ee = ov_ee_off[u];
+// 5a'. The FP64 test of every staged candidate, a thread each: its distance type, or -1. Bound by
+// FP64 issue (189 k candidates of the pile, of which 181 k are pairs: 115 us; 185 us while warps
+// held both kinds and ran both tests).
+__global__ void __launch_bounds__(128) k_narrow_exact(Geo g, Params P, const int* ovI, const int* ovJ, const int* cnt,
+                                                      const int* off, const int* lst, StageOut so) {
+  if (!so.valid()) return;
+  const int np = so.total[0], ne = so.total[1], np32 = (np + 31) & ~31;  // whole warps of one kind
+  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < np32 + ne; k += gridDim.x * blockDim.x) {
+    if (k >= np && k < np32) continue;
+    const int t = k < np ? k : so.cap - ne + (k - np32);
+    const unsigned long long key = so.key[t];
+    const int u = so.ov[t], sub = (int)(key >> 60), i = (int)((key >> 30) & 0x3fffffffull), j = (int)(key & 0x3fffffffull);
+    const SubLists L = sub_lists(g, sub, ovI[u], ovJ[u], cnt + 6 * u, off + 6 * u, lst, nullptr, nullptr, nullptr);
+    so.ty[t] = (int8_t)(exact_pair(g, P, sub, L.offA + L.LA[i], L.offB + L.LB[j]) - 1);
+  }
+}
+
+// Ordered count and write of an overlap whose candidates did not fit the shared-memory sort:
+// the (i, j) space of each sub-problem is walked in row-major order (the order of the
+// reference's nested loops), a CTA's threads at a time; f(sub, hit, i, j, type, L) is called by
+// all threads for each step of the walk.
+template <typename F>
+__device__ __forceinline__ void narrow_walk(const Geo& g, const Params& P, float ds_f, int I, int J, const int* n,
+                                            const int* o, const int* lst, const float* vb, const float* eb,
+                                            const float* fb, F&& f) {
 #pragma unroll 1
   for (int sub = 0; sub < 3; ++sub) {
-    if (sc[sub] == 0) continue;
-    SubLists L = sub_lists(g, sub, ovI[u], ovJ[u], n, o, lst, vb, eb, fb);
-    const int need = sc[sub];
-    int done = 0;
+    SubLists L = sub_lists(g, sub, I, J, n, o, lst, vb, eb, fb);
     const long long tot = (long long)L.nA * L.nB;
 #pragma unroll 1
-    for (long long k0 = 0; k0 < tot && done < need; k0 += NT) {
-      long long k = k0 + threadIdx.x;
-      int f = 0, i = 0, j = 0;
+    for (long long k0 = 0; k0 < tot; k0 += blockDim.x) {
+      const long long k = k0 + threadIdx.x;
+      int ty = 0, i = 0, j = 0;
       if (k < tot) {
         i = (int)(k / L.nB);
         j = (int)(k - (long long)i * L.nB);
         float a[6];
         finflate(L.boxA + 6 * (L.offA + L.LA[i]), ds_f, a);
         if (f_hit(a, L.boxB + 6 * (L.offB + L.LB[j])))
-          f = exact_pair(g, P, sub, L.offA + L.LA[i], L.offB + L.LB[j]);
+          ty = exact_pair(g, P, sub, L.offA + L.LA[i], L.offB + L.LB[j]);
       }
-      unsigned m = __ballot_sync(0xffffffffu, f != 0);
-      if (lane == 0) wcnt[w] = __popc(m);
-      __syncthreads();
-      int pre = 0, total = 0;
-#pragma unroll
-      for (int q = 0; q < NT / 32; ++q) {
-        pre += (q < w) ? wcnt[q] : 0;
-        total += wcnt[q];
-      }
-      if (f) {
-        int idx = (sub < 2 ? run_pt : run_ee) + pre + __popc(m & below);
-        int* dst = sub < 2 ? out.pt : out.ee;
-        dst[4 * idx] = L.A; dst[4 * idx + 1] = L.LA[i]; dst[4 * idx + 2] = L.B; dst[4 * idx + 3] = L.LB[j];
-        (sub < 2 ? out.pt_ty : out.ee_ty)[idx] = (int8_t)(f - 1);
-        (sub < 2 ? out.pt_ov : out.ee_ov)[idx] = u;
-      }
-      if (sub < 2) run_pt += total;
-      else run_ee += total;
-      done += total;
-      __syncthreads();
+      f(sub, ty != 0, i, j, ty - 1, L);
     }
   }
 }
 
-__global__ void k_sub_totals(int nov, const int* sub_cnt, int* npt, int* nee) {
-  int u = blockIdx.x * blockDim.x + threadIdx.x;
-  if (u >= nov) return;
-  npt[u] = sub_cnt[3 * u] + sub_cnt[3 * u + 1];
-  nee[u] = sub_cnt[3 * u + 2];
+// 5b. Accepted pairs of every overlap: point-triangle and edge-edge.
+constexpr int NW = 128;  // threads of the tally and of the ordered writes
+__global__ void __launch_bounds__(NW) k_narrow_tally(Geo g, Params P, float ds_f, const int* ovI, const int* ovJ,
+                                                     const int* cnt, const int* off, const int* lst, const float* vb,
+                                                     const float* eb, const float* fb, StageOut so, int* npt, int* nee) {
+  __shared__ int s_pt, s_ee;
+  const int u = blockIdx.x;
+  const int4 sg = so.seg[u];
+  if ((sg.x >= 0 && sg.y + sg.w == 0) || !so.valid()) {
+    if (threadIdx.x == 0) npt[u] = nee[u] = 0;
+    return;
+  }
+  if (threadIdx.x == 0) s_pt = s_ee = 0;
+  __syncthreads();
+  int c[2] = {0, 0};
+  if (sg.x >= 0) {
+    for (int k = threadIdx.x; k < sg.y; k += NW) c[0] += so.ty[sg.x + k] >= 0;
+    for (int k = threadIdx.x; k < sg.w; k += NW) c[1] += so.ty[sg.z + k] >= 0;
+  } else {
+    narrow_walk(g, P, ds_f, ovI[u], ovJ[u], cnt + 6 * u, off + 6 * u, lst, vb, eb, fb,
+                [&](int sub, bool hit, int, int, int, const SubLists&) { (sub < 2 ? c[0] : c[1]) += hit; });
+  }
+#pragma unroll
+  for (int q = 16; q > 0; q >>= 1) {
+    c[0] += __shfl_xor_sync(0xffffffffu, c[0], q);
+    c[1] += __shfl_xor_sync(0xffffffffu, c[1], q);
+  }
+  if ((threadIdx.x & 31) == 0) {
+    atomicAdd(&s_pt, c[0]);
+    atomicAdd(&s_ee, c[1]);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    npt[u] = s_pt;
+    nee[u] = s_ee;
+  }
+}
+
+// 5c. Ordered write: the accepted candidates of each overlap in the order of their keys
+// (point-triangle ones first), or those of the walk.
+__global__ void __launch_bounds__(NW) k_narrow_write(Geo g, Params P, float ds_f, const int* ovI, const int* ovJ,
+                                                     const int* cnt, const int* off, const int* lst, const float* vb,
+                                                     const float* eb, const float* fb, StageOut so, const int* npt,
+                                                     const int* ov_pt_off, const int* ov_ee_off, NarrowOut out) {
+  __shared__ int wcnt[2][NW / 32];
+  const int u = blockIdx.x;
+  const int4 sg = so.seg[u];
+  const int nr = sg.y + sg.w;
+  if (sg.x >= 0 && nr == 0) return;
+  const int I = ovI[u], J = ovJ[u];
+  const int* n = cnt + 6 * u;
+  const int* o = off + 6 * u;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const unsigned below = (1u << lane) - 1u;
+  const int pt0 = ov_pt_off[u], ee0 = ov_ee_off[u], np = npt[u];
+  int done = 0, par = 0;  // accepted pairs written (both kinds)
+  auto put = [&](int sub, bool hit, int i, int j, int ty, const SubLists& L) {
+    const unsigned m = __ballot_sync(0xffffffffu, hit);
+    if (lane == 0) wcnt[par][w] = __popc(m);
+    __syncthreads();
+    int r = done + __popc(m & below), total = 0;
+#pragma unroll
+    for (int q = 0; q < NW / 32; ++q) {
+      r += (q < w) ? wcnt[par][q] : 0;
+      total += wcnt[par][q];
+    }
+    if (hit) {
+      const int idx = sub < 2 ? pt0 + r : ee0 + (r - np);
+      int* dst = sub < 2 ? out.pt : out.ee;
+      dst[4 * idx] = L.A; dst[4 * idx + 1] = L.LA[i]; dst[4 * idx + 2] = L.B; dst[4 * idx + 3] = L.LB[j];
+      (sub < 2 ? out.pt_ty : out.ee_ty)[idx] = (int8_t)ty;
+      (sub < 2 ? out.pt_ov : out.ee_ov)[idx] = u;
+    }
+    done += total;
+    par ^= 1;  // the counts of the step before are read while these are written
+  };
+  if (sg.x < 0) {
+    narrow_walk(g, P, ds_f, I, J, n, o, lst, vb, eb, fb, put);
+    return;
+  }
+  for (int k0 = 0; k0 < nr; k0 += NW) {
+    const int k = k0 + threadIdx.x;
+    const int p = k < sg.y ? sg.x + k : sg.z + (k - sg.y);
+    const unsigned long long key = k < nr ? so.key[p] : 0;
+    const int ty = k < nr ? so.ty[p] : -1;
+    const int sub = (int)(key >> 60);
+    const SubLists L = sub_lists(g, sub, I, J, n, o, lst, vb, eb, fb);
+    put(sub, ty >= 0, (int)((key >> 30) & 0x3fffffffull), (int)(key & 0x3fffffffull), ty, L);
+  }
 }
 
 // 6a. vertex-ground pairs: flags + per-CTA counts, then ordered write
@@ -1198,9 +1238,9 @@ static void narrow_smem_attr() {
   if (done_dev == dev) return;
 #define ABD_NARROW_ATTR(M, ST) \
   CK(cudaFuncSetAttribute(k_narrow_scan<M, ST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)narrow_smem(M, ST)))
-  ABD_NARROW_ATTR(0, 32);
-  ABD_NARROW_ATTR(0, 64);
-  ABD_NARROW_ATTR(0, 96);
+  ABD_NARROW_ATTR(0, 8);
+  ABD_NARROW_ATTR(0, 16);
+  ABD_NARROW_ATTR(0, 48);
   ABD_NARROW_ATTR(2, 24);
   ABD_NARROW_ATTR(2, 36);
   ABD_NARROW_ATTR(2, 64);
@@ -1218,11 +1258,8 @@ struct NarrowLaunch {
   const int* off;
   int* lst;
   const float *vb, *eb, *fb;
-  int* sub_cnt;
-  unsigned long long *toi_key, *stage_key;
-  int8_t* stage_ty;
-  int *stage_off, *stage_total;
-  int stage_cap;
+  unsigned long long* toi_key;
+  StageOut so;
   const int* order;
   ToiCand tc;
 };
@@ -1232,17 +1269,17 @@ static void launch_narrow(int mode, int variant, int nov, const NarrowLaunch& a,
   const int tag = mode == 2 ? K_NARROW_TOI : K_NARROW_SCAN;
 #define ABD_NARROW_LAUNCH(M, ST)                                                                                   \
   KLAUNCH(tag, s, k_narrow_scan<M, ST><<<nov, NT, narrow_smem(M, ST), s>>>(                                       \
-                      a.g, a.P, a.ds_f, a.ovI, a.ovJ, a.cnt, a.off, a.lst, a.vb, a.eb, a.fb, a.sub_cnt, a.toi_key, \
-                      a.stage_key, a.stage_ty, a.stage_off, a.stage_total, a.stage_cap, a.order, a.tc))
+                      a.g, a.P, a.ds_f, a.ovI, a.ovJ, a.cnt, a.off, a.lst, a.vb, a.eb, a.fb, a.toi_key, a.so,      \
+                      a.order, a.tc))
   const int st = kNarrowStep[mode == 2 ? 1 : 0][variant];
   if (mode == 2) {
     if (st == 24) ABD_NARROW_LAUNCH(2, 24);
     else if (st == 36) ABD_NARROW_LAUNCH(2, 36);
     else ABD_NARROW_LAUNCH(2, 64);
   } else {
-    if (st == 32) ABD_NARROW_LAUNCH(0, 32);
-    else if (st == 64) ABD_NARROW_LAUNCH(0, 64);
-    else ABD_NARROW_LAUNCH(0, 96);
+    if (st == 8) ABD_NARROW_LAUNCH(0, 8);
+    else if (st == 16) ABD_NARROW_LAUNCH(0, 16);
+    else ABD_NARROW_LAUNCH(0, 48);
   }
 #undef ABD_NARROW_LAUNCH
 }
@@ -1333,9 +1370,9 @@ void traj_floats(const Geo& g, CullScratch& cs, cudaStream_t s) {
 }
 
 // Narrow phase of a pair cull over binned (and refined, ordered) lists of nov overlaps:
-// classification with staging (grown and repeated when it overflows), per-overlap counts
-// and offsets, one host read of the totals (pt, ee, vg, staged, unstaged overlaps), then
-// the ordered write of the pairs into S.
+// candidates (grown and repeated when the staging overflows), their FP64 tests, per-overlap
+// counts and offsets, one host read of the totals (pt, ee, vg, staged of both kinds),
+// then the ordered write of the pairs into S.
 static void narrow_pairs(const Geo& g, const Params& P, float ds_f, int nov, const int* ovI, const int* ovJ,
                          CullScratch& cs, PairSet& S, int& npt, int& nee, cudaStream_t s) {
   int* d_tot = cs.tmp_int.p;
@@ -1343,28 +1380,33 @@ static void narrow_pairs(const Geo& g, const Params& P, float ds_f, int nov, con
   cs.blk_b.ensure(nov + 1);
   cs.blk_a_off.ensure(nov + 1);
   cs.blk_b_off.ensure(nov + 1);
-  cs.sub_cnt.ensure(3 * (size_t)nov + 3);
-  cs.stage_off.ensure(nov + 1);
-  if (cs.stage_key.cap < (1u << 16)) {
-    cs.stage_key.ensure(1u << 16);
-    cs.stage_ty.ensure(1u << 16);
-  }
+  cs.stage_seg.ensure(nov + 1);
+  // room for 32 candidates an overlap (piles and columns of spheres: 11 to 19), 64 k at least
+  size_t want = std::max({cs.stage_key.cap, (size_t)1 << 16, (size_t)32 * nov});
+  StageOut so{};
   for (int attempt = 0; attempt < 4; ++attempt) {
+    cs.stage_key.ensure(want);
+    cs.stage_ty.ensure(cs.stage_key.cap);
+    cs.stage_ov.ensure(cs.stage_key.cap);
+    so = StageOut{cs.stage_key.p, cs.stage_ov.p, cs.stage_ty.p, cs.stage_seg.p, d_tot + 6, (int)cs.stage_key.cap};
     narrow_smem_attr();
     NarrowLaunch a{g, P, ds_f, ovI, ovJ, cs.bin_cnt.p, cs.bin_off.p, cs.lst.p, cs.vbox.p, cs.ebox.p, cs.fbox.p,
-                   cs.sub_cnt.p, nullptr, cs.stage_key.p, cs.stage_ty.p, cs.stage_off.p, d_tot + 6,
-                   (int)cs.stage_key.cap, cs.order.p, ToiCand{}};
+                   nullptr, so, cs.order.p, ToiCand{}};
     narrow_phase(0, nov, a, cs, d_tot + 6, s);
+    KLAUNCH(K_NARROW_SCAN, s, k_narrow_exact<<<1216, 128, 0, s>>>(g, P, ovI, ovJ, cs.bin_cnt.p, cs.bin_off.p,
+                                                                  cs.lst.p, so));
     // per-overlap pair counts and their offsets, read together with the staged total
-    KLAUNCH(K_NARROW_WRITE, s, k_sub_totals<<<nblk(nov, 256), 256, 0, s>>>(nov, cs.sub_cnt.p, cs.blk_a.p, cs.blk_b.p));
+    KLAUNCH(K_NARROW_WRITE, s, k_narrow_tally<<<nov, NW, 0, s>>>(g, P, ds_f, ovI, ovJ, cs.bin_cnt.p, cs.bin_off.p,
+                                                                 cs.lst.p, cs.vbox.p, cs.ebox.p, cs.fbox.p, so,
+                                                                 cs.blk_a.p, cs.blk_b.p));
     scan_exclusive_int(cs.blk_a.p, cs.blk_a_off.p, nov, d_tot + 3, s, cs.vflag_cnt);
     scan_exclusive_int(cs.blk_b.p, cs.blk_b_off.p, nov, d_tot + 4, s, cs.vflag_cnt);
     CK(cudaMemcpyAsync(cs.h_small + 3, d_tot + 3, 5 * sizeof(int), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
-    if ((size_t)cs.h_small[6] <= cs.stage_key.cap) break;
-    // staging overflowed: grow to the reported total and classify again
-    cs.stage_key.ensure((size_t)cs.h_small[6] + (cs.h_small[6] >> 2) + 1024);
-    cs.stage_ty.ensure(cs.stage_key.cap);
+    const size_t staged = (size_t)cs.h_small[6] + cs.h_small[7];
+    if (staged <= cs.stage_key.cap) break;
+    // staging overflowed: grow to the reported total and repeat
+    want = staged + (staged >> 2) + 1024;
   }
   npt = cs.h_small[3];
   nee = cs.h_small[4];
@@ -1376,14 +1418,10 @@ static void narrow_pairs(const Geo& g, const Params& P, float ds_f, int nov, con
   S.ee_ty.ensure(nee + 1);
   S.ee_ov.ensure(nee + 1);
   NarrowOut no{S.pt.p, S.pt_ov.p, S.ee.p, S.ee_ov.p, S.pt_ty.p, S.ee_ty.p};
-  KLAUNCH(K_NARROW_WRITE, s, k_narrow_copy<<<nov, 128, 0, s>>>(nov, ovI, ovJ, cs.bin_off.p, cs.lst.p, cs.sub_cnt.p,
-                                                                cs.stage_key.p, cs.stage_ty.p, cs.stage_off.p,
-                                                                cs.blk_a_off.p, cs.blk_b_off.p, no));
-  if (cs.h_small[7] > 0)  // some overlap was not staged: the recomputing pass writes it
-    KLAUNCH(K_NARROW_WRITE, s, k_narrow_write<<<nov, NT, 0, s>>>(g, P, ds_f, ovI, ovJ, cs.bin_cnt.p, cs.bin_off.p,
-                                                                  cs.lst.p, cs.vbox.p, cs.ebox.p, cs.fbox.p,
-                                                                  cs.sub_cnt.p, cs.blk_a_off.p, cs.blk_b_off.p, no,
-                                                                  cs.stage_off.p));
+  if (npt + nee > 0)
+    KLAUNCH(K_NARROW_WRITE, s, k_narrow_write<<<nov, NW, 0, s>>>(g, P, ds_f, ovI, ovJ, cs.bin_cnt.p, cs.bin_off.p,
+                                                                 cs.lst.p, cs.vbox.p, cs.ebox.p, cs.fbox.p, so,
+                                                                 cs.blk_a.p, cs.blk_a_off.p, cs.blk_b_off.p, no));
 }
 
 void cull(const Geo& g_in, const Params& P, int vtn, double alpha, CullScratch& cs, PairSet& out, double* toi_p,
@@ -1414,8 +1452,8 @@ void cull(const Geo& g_in, const Params& P, int vtn, double alpha, CullScratch& 
   KLAUNCH(K_OV_COUNT, s, k_ov_count<<<nblk((long long)nb * 32, 256), 256, 0, s>>>(g, cs.bbox.p, cs.bbox_f.p, cs.cnt_all.p,
                                                                                   cs.cnt_up.p));
   cs.tmp_int.ensure(64);
-  int* d_tot = cs.tmp_int.p;  // [0] nnz, [1] nov, [2] list entries, [3] PT, [4] EE, [5] VG, [6] staged,
-                              // [7] overlaps left to the recomputing write pass
+  int* d_tot = cs.tmp_int.p;  // [0] nnz, [1] nov, [2] list entries, [3] PT, [4] EE, [5] VG, staged
+                              // PT and EE ([6], [7])
   scan_exclusive_int(cs.cnt_all.p, S.row_ptr.p, nb, d_tot, s, cs.vflag_cnt);
   scan_exclusive_int(cs.cnt_up.p, cs.up_ptr.p, nb, d_tot + 1, s, cs.vflag_cnt);
   // the vertex-ground pairs need only the positions: counted now, read with the overlaps
@@ -1501,7 +1539,7 @@ void cull(const Geo& g_in, const Params& P, int vtn, double alpha, CullScratch& 
       cs.toi_cand.ensure(kToiCand);
       cs.toi_n.ensure(2);
       NarrowLaunch a{g, P, ds_f, S.ovI.p, S.ovJ.p, cs.bin_cnt.p, cs.bin_off.p, cs.lst.p, cs.vbox.p, cs.ebox.p,
-                     cs.fbox.p, nullptr, cs.toi_key.p, nullptr, nullptr, nullptr, nullptr, 0, cs.order.p,
+                     cs.fbox.p, cs.toi_key.p, StageOut{}, cs.order.p,
                      ToiCand{cs.vend.p, cs.toi_cand.p, cs.toi_n.p, kToiCand}};
       narrow_phase(2, nov, a, cs, reinterpret_cast<int*>(cs.toi_n.p), s);
       KLAUNCH(K_NARROW_TOI, s, k_toi_list<<<1216, 128, 0, s>>>(g, a.tc, cs.toi_key.p));
