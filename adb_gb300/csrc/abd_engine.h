@@ -59,6 +59,7 @@ struct Geo {
   int ns;                               // scenes (independent sub-problems of a batch)
   const int* bscene;                    // nb: scene of each body
   const int *sc_beg, *sc_end;           // ns: body range of each scene
+  bool any_big, any_small;              // scenes of at least / below BIG_SCENE bodies
   const double* alpha_s;                // ns or null: per-scene step for positions at q + alpha dq
   const int* sc_act;                    // ns or null: scenes to process (culls, pair terms, energies);
                                         // the others get no pairs and identity blocks
@@ -69,6 +70,13 @@ struct Geo {
 
 __host__ __device__ inline bool scene_on(const Geo& g, int body) {
   return !g.sc_act || g.sc_act[g.bscene[body]] != 0;
+}
+
+// Bodies from which a scene keeps the forms of the pair terms whose rounding its truncated CG
+// amplifies (newton.cu).
+constexpr int BIG_SCENE = 512;
+__device__ inline bool big_scene(const Geo& g, int body) {
+  return g.scene_end[body] - g.scene_beg[body] >= BIG_SCENE;
 }
 
 // A culled pair set together with the overlap structure it was built on.

@@ -94,6 +94,7 @@ struct Engine {
   // line search (a single scene is the reference's ABD::implicit_euler)
   int ns = 1;
   DBuf<int> bscene, sc_beg, sc_end, sc_on, sc_iter, sc_search;
+  bool any_big = false, any_small = false;
   DBuf<double> sc_alpha, sc_factor;
   std::vector<int> h_sc_beg, h_sc_end;
   std::vector<int> iter, g_cnt, p_cnt;           // per scene (iter: cumulative, model/abd.h:53)
@@ -122,6 +123,7 @@ struct Engine {
     g.mass = mass.p; g.Ic = Ic.p; g.rest_box = rest_box.p;
     g.scene_beg = scene_beg.p; g.scene_end = scene_end.p;
     g.ns = ns; g.bscene = bscene.p; g.sc_beg = sc_beg.p; g.sc_end = sc_end.p; g.alpha_s = nullptr;
+    g.any_big = any_big; g.any_small = any_small;
     g.sc_act = nullptr;
     g.q = q.p; g.dq = dq.p; g.q0 = q0.p; g.dqdt = dqdt.p;
     g.X = X.p; g.Xq = Xq.p; g.X0 = X0.p; g.qa = qa.p;
@@ -301,6 +303,7 @@ struct Engine {
       b = e;
     }
     ns = (int)h_sc_beg.size();
+    for (int i = 0; i < ns; ++i) (h_sc_end[i] - h_sc_beg[i] >= abd::BIG_SCENE ? any_big : any_small) = true;
     iter.assign(ns, 0);
     g_cnt.assign(ns, 0);
     p_cnt.assign(ns, 0);

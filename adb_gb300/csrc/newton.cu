@@ -206,11 +206,10 @@ __global__ void __launch_bounds__(HESS_T) k_pair_hess(Geo g, Params P, int kind,
 // built entry by entry across the lanes and projected by the warp (jac9_project; a chain of
 // rotations, so it is bound by their latency: 256 columns of cubes and spheres 1154 -> 164 us a launch,
 // 333 bodies of the pile 436 -> 146 us).
-// Beside a launch of at least MOLL_HIDE pairs that hides them, up to MOLL_WAVE mollified pairs
-// keep the rotations one by one: the 1024-body pile gains 2% from the rounds, and with any other
-// rounding its CG, which stops at a residual, takes an iteration more or less and moves the
-// frame's velocities by 1e-9 (below 512 bodies by 2e-11).
-constexpr int MOLL_HIDE = 65536, MOLL_WAVE = 256;
+// Scenes of BIG_SCENE bodies or more (abd_engine.h) keep the rotations one by one: the 1024-body
+// pile gains 2% from the rounds, and with any other rounding its CG, which stops at a residual,
+// takes an iteration more or less and moves the frame's velocities by 1e-9 (below 512 bodies by
+// 2e-11). The choice is by scene, so that a scene of a batch gets the bits it gets alone.
 constexpr int MOLL_W = 2;  // warps (pairs) per CTA
 constexpr int MOLL_GRID = 608;  // CTAs at most (pairs are taken grid-stride)
 __global__ void __launch_bounds__(32 * MOLL_W) k_pair_moll(Geo g, Params P, int n, const int* tup,
@@ -276,8 +275,7 @@ __global__ void __launch_bounds__(32 * MOLL_W) k_pair_moll(Geo g, Params P, int 
         }
       } else {
         bool neg = false;
-        const int cur = !P.psd ? 0 : (nm <= MOLL_WAVE && n >= MOLL_HIDE ? jac9_project_serial(w9, neg)
-                                                                      : jac9_project(w9, neg));
+        const int cur = !P.psd ? 0 : (big_scene(g, Ab) ? jac9_project_serial(w9, neg) : jac9_project(w9, neg));
 #pragma unroll
         for (int k = 0; k < 2; ++k) {
           if (k == 1 && lane >= 13) continue;
@@ -347,7 +345,8 @@ __constant__ Sym12Table c_sym12 = Sym12Table();
 // Y_A's column 1 is zero for both kinds (body A holds vertex 0, and 1 for edge-edge) and
 // Y_B's column 0 is zero for edge-edge pairs: those terms are left out (KIND 0:
 // point-triangle, 1: edge-edge).
-// SPLIT: the six (r, s) slices of a pair by a thread each (blockIdx.y); else one after the other.
+// SPLIT: the six (r, s) slices of a pair by a thread each (blockIdx.y), for the pairs of scenes
+// below BIG_SCENE bodies; else one after the other, for those of the larger ones.
 template <int KIND, bool SPLIT>
 __global__ void __launch_bounds__(128) k_pair_chain(Geo g, int n, const int* tup, const int* pov,
                                                     const int* ovI, const double* R, double* C) {
@@ -357,7 +356,7 @@ __global__ void __launch_bounds__(128) k_pair_chain(Geo g, int n, const int* tup
   if (p >= n) return;
   int vid[4], na_, A, B;
   pair_vertices(g, kind, tup, p, vid, na_, A, B);
-  if (!scene_on(g, A)) return;
+  if (!scene_on(g, A) || big_scene(g, A) == SPLIT) return;
   const size_t N = n;
   const int I = ovI[pov[p]];
   const bool a_is_I = (A == I);
@@ -2029,21 +2028,22 @@ __global__ void k_copy(double* d, const double* s, int n) {
 
 }  // namespace
 
-// Chain rule of n pairs of a kind: slices by thread up to CHAIN_SPLIT pairs.
+// Chain rule of n pairs of a kind: slices by thread in scenes below BIG_SCENE bodies.
 // A pair's slices one after the other are a chain of 50-67 us; by thread 15 us (a stack's 96
 // pairs) to 43 us (12k). At 136k pairs the gain is 10% (309 -> 280 us) and the rounding of the
-// friction terms differs, which the large pile's truncated CG amplifies (see MOLL_HIDE).
-constexpr int CHAIN_SPLIT = 16384;
+// friction terms differs, which the large pile's truncated CG amplifies (see k_pair_moll).
 template <int KIND>
 static void launch_chain(const Geo& g, int n, const int* tup, const int* pov, const int* ovI, const double* R,
                          double* C, cudaStream_t s) {
   const int nb = nblk(n, 128);
-  if (n <= CHAIN_SPLIT)
+  if (g.any_small)
     KLAUNCH(K_PAIR_TERMS, s, k_pair_chain<KIND, true><<<dim3(nb, 6), 128, 0, s>>>(g, n, tup, pov, ovI, R, C));
-  else
+  if (g.any_big)
     KLAUNCH(K_PAIR_TERMS, s, k_pair_chain<KIND, false><<<nb, 128, 0, s>>>(g, n, tup, pov, ovI, R, C));
 }
 
+// Edge-edge pairs from which their kernels fill the chip (assemble).
+constexpr int WIDE_EE = 65536;
 void assemble(const Geo& g, const Params& P, PairSet& S, NewtonBufs& B, cudaStream_t s) {
   int nb = g.nb, npt = S.npt, nee = S.nee, nov = S.nov;
   B.pt_c.ensure((size_t)PAIRC * npt + 1);
@@ -2065,7 +2065,7 @@ void assemble(const Geo& g, const Params& P, PairSet& S, NewtonBufs& B, cudaStre
   // The two kinds share nothing before the overlap sums: point-triangle pairs run on a stream
   // of their own beside the edge-edge ones (a kernel of either is a chain of 50 to 170 us
   // however few its pairs: a chain's frame 4.75 -> 4.24 ms, a batch's 20.9 -> 18.4), and the few
-  // mollified pairs, one warp each, on a third. At MOLL_HIDE pairs the edge-edge kernels fill
+  // mollified pairs, one warp each, on a third. At WIDE_EE pairs the edge-edge kernels fill
   // the chip and the two get in each other's way (a Newton step of the pile 7.40 -> 7.64 ms).
   if (!B.side) {
     CK(cudaStreamCreateWithFlags(&B.side, cudaStreamNonBlocking));
@@ -2073,7 +2073,7 @@ void assemble(const Geo& g, const Params& P, PairSet& S, NewtonBufs& B, cudaStre
     for (cudaEvent_t* e : {&B.ev_fork, &B.ev_join, &B.ev_fork_pt, &B.ev_join_pt})
       CK(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
   }
-  const bool both = npt > 0 && nee > 0 && nee < MOLL_HIDE;
+  const bool both = npt > 0 && nee > 0 && nee < WIDE_EE;
   if (both) {
     CK(cudaEventRecord(B.ev_fork_pt, s));
     CK(cudaStreamWaitEvent(B.side_pt, B.ev_fork_pt, 0));
