@@ -296,9 +296,11 @@ struct NewtonBufs {
   int tri_nlev = 0, tri_width = 0;       // levels, bodies of the first (largest) one
   // adjoint: friction-frame Jacobians and contributions per pair, the exact system's
   // blocks, GMRES bases
-  DBuf<double> fj_pt, fj_ee, fc_pt, fc_ee, D_ex, ovr_ex, adj_V, adj_Z, adj_w, adj_t, adj_x;
+  DBuf<double> fj_pt, fj_ee, fc_pt, fc_ee, D_ex, ovr_ex, adj_V, adj_Z, adj_w, adj_x, adj_h;
+  DBuf<double2> vg_coef;
+  int n_pcg_scenes = 0, n_tri_scenes = 0;  // tri_classify of the last solve
   DBuf<int> has_ex;
-  double* h_dot = nullptr;               // pinned: one dot product
+  double* h_dot = nullptr;               // pinned: dot products
   int ngrp = 0;
   DBuf<double> sc_rz, sc_bb; // per-scene CG scalars
   DBuf<int> sc_conv, sc_iters, n_active;
@@ -332,6 +334,8 @@ struct SolveOpts {
   double refine_tol = 1e-8;
   int dense = 0;
   int tri = 0;  // block-tridiagonal scenes by block Cholesky (tri_solve)
+  bool same_system = false;  // the matrix, scenes and options of the call before on these buffers
+                             // (its rows, block inverses and classification stand)
 };
 // on (host, ns): the scenes solved (the others get dq = 0); sc_on is its device copy.
 int pcg_solve(const Geo& g, PairSet& S, NewtonBufs& nb, const SolveOpts& o, const int* sc_on,
@@ -364,20 +368,19 @@ void launch_copy_scene(const Geo& g, double* dst, const double* src, const int* 
 void launch_scale_scene(const Geo& g, double* v, const double* f, cudaStream_t st);
 // y = H x with the system assembled last on S (no synchronisation)
 void spmv(const Geo& g, const PairSet& S, NewtonBufs& nb, const double* x, double* y, cudaStream_t st);
-// y = H x with explicitly given blocks (saved copies of an assembly on S)
-void spmv_blocks(const Geo& g, const PairSet& S, const int* has, const double* ovr, const double* D, const double* x,
-                 double* y, cudaStream_t st);
 // ---------------- adjoint (adjoint.cu) ----------------
-// Per PT/EE pair of S: the Jacobian of its friction force through its tangent frame and
-// multiplier at the positions in g.X (reference positions g.X0), kept in B.fj_pt / fj_ee.
-void fric_frame_jacobians(const Geo& g, const Params& P, PairSet& S, NewtonBufs& B, cudaStream_t s);
-// out = (those Jacobians, in body coordinates)^T w, summed per body in a fixed order
-// (needs the overlap segments of the last assembly on S).
-void fric_frame_apply_t(const Geo& g, PairSet& S, NewtonBufs& B, const double* w, double* out, cudaStream_t s);
+// What the product below needs of the positions in g.X (reference positions g.X0): per PT/EE pair
+// of S the Jacobian of its friction force through its tangent frame and multiplier (B.fj_pt,
+// fj_ee), per vertex-ground pair the multiplier coupling (B.vg_coef, if vg_coupling).
+void adj_terms(const Geo& g, const Params& P, PairSet& S, NewtonBufs& B, bool vg_coupling, cudaStream_t s);
+// out = J^T z: the kept exact blocks (B.D_ex, ovr_ex, has_ex), the pairs' friction Jacobians and
+// the vertex-ground coupling (needs the overlap segments of the last assembly on S).
+void adj_apply(const Geo& g, PairSet& S, NewtonBufs& B, bool vg_coupling, const double* z, double* out,
+               cudaStream_t s);
+// V_{k+1} (n entries each) made orthonormal to V_0 .. V_k; h: k + 2 coefficients (synchronises)
+void orthogonalize(int n, int k, double* V, double* h, NewtonBufs& B, cudaStream_t s);
 double dev_dot(int n, const double* a, const double* b, NewtonBufs& B, cudaStream_t s);  // synchronises
 void dev_axpby(int n, double a, const double* x, double b, double* y, cudaStream_t s);   // y = a x + b y
-// out = C^T w for the ground-friction multiplier coupling of an adjoint system
-void vg_lag_adjoint(const Geo& g, const Params& P, const PairSet& S, const double* w, double* out, cudaStream_t st);
 void launch_q_update_scene(const Geo& g, double* q, const double* dq, const double* alpha, cudaStream_t st);
 void launch_frame_end(double* q, double* q0, double* dqdt, int n, double dt, cudaStream_t st);
 void launch_copy(double* dst, const double* src, int n, cudaStream_t st);

@@ -864,7 +864,7 @@ __global__ void __launch_bounds__(NT, MODE == 0 ? (STEP <= 8 ? 4 : STEP <= 16 ? 
   const float lim_f = __double2float_ru(P.dhat * (1.0 + 1e-4));
   int* n = cnt + 6 * u;
   const int* o = off + 6 * u;
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
   const unsigned below = (1u << lane) - 1u;
   if (threadIdx.x == 0) {
     rec_n = rec_np = 0;

@@ -178,7 +178,7 @@ struct Engine {
     nbufs.tri_Li.release(); nbufs.tri_W.release(); nbufs.tri_y.release();
     nbufs.fj_pt.release(); nbufs.fj_ee.release(); nbufs.fc_pt.release(); nbufs.fc_ee.release();
     nbufs.D_ex.release(); nbufs.ovr_ex.release(); nbufs.has_ex.release(); nbufs.adj_V.release();
-    nbufs.adj_Z.release(); nbufs.adj_w.release(); nbufs.adj_t.release(); nbufs.adj_x.release();
+    nbufs.adj_Z.release(); nbufs.adj_w.release(); nbufs.adj_h.release(); nbufs.vg_coef.release(); nbufs.adj_x.release();
     if (nbufs.h_dot) cudaFreeHost(nbufs.h_dot);
     if (nbufs.h_red) cudaFreeHost(nbufs.h_red);
     if (nbufs.h_int) cudaFreeHost(nbufs.h_int);
@@ -1062,8 +1062,8 @@ int abd_adjoint_frame(abd_handle* h, const double* q_t, const double* v_t, const
                          s));
       CK(cudaMemcpyAsync(B.has_ex.p, B.has.p, nov * sizeof(int), cudaMemcpyDeviceToDevice, s));
     }
-    abd::fric_frame_jacobians(g, Pe, S, B, s);
     const bool vg_coupling = e.P.mu > 0.0 && e.cfg.ground && e.cfg.vg_fric && S.nvg > 0;
+    abd::adj_terms(g, Pe, S, B, vg_coupling, s);
     // the preconditioner: the forward step's (projected, undamped) Newton matrix
     abd::Params Pp = e.P;
     Pp.psd = 1;
@@ -1081,29 +1081,20 @@ int abd_adjoint_frame(abd_handle* h, const double* q_t, const double* v_t, const
     B.adj_V.ensure((size_t)(m + 1) * n);
     B.adj_Z.ensure((size_t)m * n);
     B.adj_w.ensure(n);
-    B.adj_t.ensure(n);
     B.adj_x.ensure(n);
     double* V = B.adj_V.p;
     double* Z = B.adj_Z.p;
     double* wv = B.adj_w.p;
-    double* tv = B.adj_t.p;
     double* xv = B.adj_x.p;
     int st = ABD_OK;
     // out = J^T z
-    auto apply = [&](const double* z, double* out) {
-      abd::spmv_blocks(g, S, B.has_ex.p, B.ovr_ex.p, B.D_ex.p, z, out, s);
-      if (vg_coupling) {
-        abd::vg_lag_adjoint(g, Pe, S, z, tv, s);
-        abd::dev_axpby(n, 1.0, tv, 1.0, out, s);
-      }
-      abd::fric_frame_apply_t(g, S, B, z, tv, s);
-      abd::dev_axpby(n, 1.0, tv, 1.0, out, s);
-    };
+    auto apply = [&](const double* z, double* out) { abd::adj_apply(g, S, B, vg_coupling, z, out, s); };
     // z = P^-1 v by the PCG on the preconditioner's system
     auto precond = [&](const double* v, double* z) {
       CK(cudaMemcpyAsync(B.grad.p, v, n * sizeof(double), cudaMemcpyDeviceToDevice, s));
       int ps = 0;
       abd::pcg_solve(g, S, B, po, e.sc_on.p, all_on, e.dq.p, s, &ps, nullptr);
+      po.same_system = true;
       if (ps == ABD_ERR_NOT_SPD) st = ABD_ERR_NOT_SPD;
       CK(cudaMemcpyAsync(z, B.x.p, n * sizeof(double), cudaMemcpyDeviceToDevice, s));
     };
@@ -1113,7 +1104,7 @@ int abd_adjoint_frame(abd_handle* h, const double* q_t, const double* v_t, const
     const double tol = 1e-12 * bnorm;
     double beta = bnorm;
     bool converged = bnorm == 0.0;
-    std::vector<double> H((size_t)(m + 1) * m), cs(m), sn(m), gg(m + 1), y(m);
+    std::vector<double> H((size_t)(m + 1) * m), cs(m), sn(m), gg(m + 1), y(m), hk(m + 1);
     int total_its = 0;
     double last_res = bnorm;
     for (int rs = 0; rs < max_restarts && !converged && st == ABD_OK; ++rs) {
@@ -1134,17 +1125,11 @@ int abd_adjoint_frame(abd_handle* h, const double* q_t, const double* v_t, const
       for (; k < m; ++k) {
         double* vk = V + (size_t)k * n;
         double* zk = Z + (size_t)k * n;
-        double* vn = V + (size_t)(k + 1) * n;
         precond(vk, zk);
-        apply(zk, vn);
-        for (int i = 0; i <= k; ++i) {  // modified Gram-Schmidt
-          const double hik = abd::dev_dot(n, vn, V + (size_t)i * n, B, s);
-          H[(size_t)i * m + k] = hik;
-          abd::dev_axpby(n, -hik, V + (size_t)i * n, 1.0, vn, s);
-        }
-        const double hn = std::sqrt(abd::dev_dot(n, vn, vn, B, s));
-        H[(size_t)(k + 1) * m + k] = hn;
-        if (hn > 0.0) abd::dev_axpby(n, 0.0, vn, 1.0 / hn, vn, s);
+        apply(zk, V + (size_t)(k + 1) * n);
+        abd::orthogonalize(n, k, V, hk.data(), B, s);
+        for (int i = 0; i <= k + 1; ++i) H[(size_t)i * m + k] = hk[i];
+        const double hn = hk[k + 1];
         for (int i = 0; i < k; ++i) {  // the earlier rotations on the new column
           const double a0 = H[(size_t)i * m + k], a1 = H[(size_t)(i + 1) * m + k];
           H[(size_t)i * m + k] = cs[i] * a0 + sn[i] * a1;

@@ -1915,46 +1915,6 @@ __global__ void k_copy_scene(double* dst, const double* src, int n, const int* b
   if (i < n && on[bscene[i / 12]]) dst[i] = src[i];
 }
 
-// Transpose of the ground-friction multiplier coupling (adjoint systems): the lagged
-// multiplier lam(y) = -2 b'(d) (y + off) of each vertex-ground pair moves with the
-// vertex height at the solution, which adds C = (r_f / lam) (dlam/dy J_y)^T to the
-// Jacobian of the gradient. out = C^T w, one thread per body.
-__global__ void k_vg_lag_adj(Geo g, Params P, const int* vg, const int* vg_seg, const double* w, double* out) {
-  int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= g.nb) return;
-  double acc[4] = {0, 0, 0, 0};
-  const double* wb = w + 12 * b;
-  if (g.mass[b] > 0.0 && P.ground && P.vg_fric) {
-    BarrierP bp{P.dhat, P.kappa};
-    for (int kk = vg_seg[b]; kk < vg_seg[b + 1]; ++kk) {
-      int v = g.v_off[b] + vg[2 * kk + 1];
-      double _d = g.X[g.nv + v] + P.ground_offset;
-      double dd = _d * _d;
-      if (!(dd < P.dhat)) continue;
-      double b1 = barrier_b1(dd, bp), b2 = barrier_b2(dd, bp);
-      double lam = -b1 * 2 * _d;
-      if (lam == 0.0) continue;
-      double dlam = -2.0 * (2.0 * b2 * dd + b1);
-      double uk[2] = {g.X[v] - g.X0[v], g.X[2 * g.nv + v] - g.X0[2 * g.nv + v]};
-      double gs = 0.0, M[2][2];
-      friction_2x2(uk, lam, FrictionP{P.mu, P.epsv, P.max_uk}, gs, M);
-      double xt[4] = {1.0, g.rest[3 * v], g.rest[3 * v + 1], g.rest[3 * v + 2]};
-      double wx = 0.0, wz = 0.0;
-      for (int k = 0; k < 4; ++k) {
-        wx += xt[k] * wb[3 * k];
-        wz += xt[k] * wb[3 * k + 2];
-      }
-      double c = dlam * (gs / lam) * (uk[0] * wx + uk[1] * wz);
-      for (int k = 0; k < 4; ++k) acc[k] += xt[k] * c;
-    }
-  }
-  for (int k = 0; k < 4; ++k) {
-    out[12 * b + 3 * k] = 0.0;
-    out[12 * b + 3 * k + 1] = acc[k];
-    out[12 * b + 3 * k + 2] = 0.0;
-  }
-}
-
 // y = H x over the assembled block-sparse matrix (diagonal blocks D, off-diagonal blocks
 // in the per-overlap records), one thread per (body, row) slot.
 __global__ void k_spmv(int nb, const int* row_ptr, const int* col, const int* upidx, const int* has,
@@ -2172,10 +2132,12 @@ int pcg_solve(const Geo& g, PairSet& S, NewtonBufs& B, const SolveOpts& o, const
   B.sc_iters.ensure(ns);
   B.n_active.ensure(3);
   // solve setup (counted with the preconditioner): row-block copy of the system
-  KLAUNCH(K_BLOCK_INVERSE, s, k_pcg_rows<<<nblk((long long)nb * 32, 256), 256, 0, s>>>(nb, S.row_ptr.p, S.col.p,
-                                                                                        S.upidx.p, B.has.p, B.ovr.p,
-                                                                                        B.D.p, B.Hrow.p, B.rcol.p,
-                                                                                        B.rn.p, B.status.p + 2, B.slots.p, pcg1_words(B, nb)));
+  if (o.same_system)
+    CK(cudaMemsetAsync(B.slots.p, 0, pcg1_words(B, nb) * sizeof(unsigned long long), s));
+  else
+    KLAUNCH(K_BLOCK_INVERSE, s, k_pcg_rows<<<nblk((long long)nb * 32, 256), 256, 0, s>>>(
+                                    nb, S.row_ptr.p, S.col.p, S.upidx.p, B.has.p, B.ovr.p, B.D.p, B.Hrow.p, B.rcol.p,
+                                    B.rn.p, B.status.p + 2, B.slots.p, pcg1_words(B, nb)));
   auto block_inverse = [&]() {
     KLAUNCH(K_BLOCK_INVERSE, s, k_block_inverse<<<nblk(nb, BINV_W), 32 * BINV_W, 0, s>>>(nb, B.D.p, B.Dinv.p,
                                                                                           B.status.p));
@@ -2195,12 +2157,14 @@ int pcg_solve(const Geo& g, PairSet& S, NewtonBufs& B, const SolveOpts& o, const
   int n_pcg = 1, n_tri = 0;
   const int* pcg_mask = sc_on;
   if (o.tri) {
-    tri_classify(g, S, B, 1, sc_on, s, &n_pcg, &n_tri);
+    if (!o.same_system) tri_classify(g, S, B, 1, sc_on, s, &B.n_pcg_scenes, &B.n_tri_scenes);
+    n_pcg = B.n_pcg_scenes;
+    n_tri = B.n_tri_scenes;
     if (n_tri > 0) pcg_mask = B.pcg_on.p;
   }
   const bool run_pcg = n_tri == 0 || n_pcg > 0;
   // the preconditioner; the direct solve checks its own pivots
-  if (run_pcg) block_inverse();
+  if (run_pcg && !o.same_system) block_inverse();
   static int max_blocks = 0, max_blocks1 = 0;
   if (!max_blocks) {
     int dev, sms, per, per1;
@@ -2431,16 +2395,6 @@ void launch_copy_scene(const Geo& g, double* dst, const double* src, const int* 
 void spmv(const Geo& g, const PairSet& S, NewtonBufs& B, const double* x, double* y, cudaStream_t st) {
   KLAUNCH(K_PCG, st, k_spmv<<<nblk((long long)g.nb * 16, 256), 256, 0, st>>>(g.nb, S.row_ptr.p, S.col.p, S.upidx.p,
                                                                             B.has.p, B.ovr.p, B.D.p, x, y));
-}
-
-void spmv_blocks(const Geo& g, const PairSet& S, const int* has, const double* ovr, const double* D, const double* x,
-                 double* y, cudaStream_t st) {
-  KLAUNCH(K_PCG, st, k_spmv<<<nblk((long long)g.nb * 16, 256), 256, 0, st>>>(g.nb, S.row_ptr.p, S.col.p, S.upidx.p,
-                                                                            has, ovr, D, x, y));
-}
-
-void vg_lag_adjoint(const Geo& g, const Params& P, const PairSet& S, const double* w, double* out, cudaStream_t st) {
-  KLAUNCH(K_BODY_SYSTEM, st, k_vg_lag_adj<<<nblk(g.nb, 128), 128, 0, st>>>(g, P, S.vg.p, S.vg_seg.p, w, out));
 }
 
 void launch_scale_scene(const Geo& g, double* v, const double* f, cudaStream_t st) {
