@@ -462,8 +462,8 @@ constexpr int REC_CAP = 2048;  // candidates of one overlap kept in shared memor
 // less often; a shorter one leaves shared memory for more CTAs per SM. The result does not
 // depend on STEP (candidates are sorted by key before they are written, TOIs are
 // min-reduced), so the autotuner picks among these variants by time: pair cull (mode 0)
-// 16 / 8 / 48, CCD (mode 2) 24 / 36 / 64; the defaults are the middle ones (columns: 237 us
-// with 16 at 3 CTAs per SM, 212 us with 8 at 4; the pile 198 us with either).
+// 16 / 8 / 48, CCD (mode 2) 24 / 36 / 64; the defaults are the middle ones (with
+// a phase per sub-problem, columns: 237 us with 16 at 3 CTAs per SM, 212 us with 8 at 4).
 constexpr int kNarrowVariants = 3;
 constexpr int kNarrowStep[2][kNarrowVariants] = {{16, 8, 48}, {24, 36, 64}};
 constexpr int kNarrowDefault = 1;
@@ -849,47 +849,41 @@ __global__ void k_refine(Geo g, float ds, int nov, const int* ovI, const int* ov
   }
 }
 
-// Stages one chunk of each list's float boxes in shared memory (A side inflated by
-// sqrt(dhat), rounded outward, unless `traj`).
-// With sVA / sVB (pair cull) it also stages the vertex ids of the chunk's primitives:
-// A entry k at sVA[2k] (a point: its id; an edge: its two), B entry k at sVB[3k] (a face:
-// its three; an edge: its two), so the exact phase reads them from shared memory.
-__device__ __forceinline__ void stage(const Geo& g, int sub, const SubLists& L, int a0, int ca, int b0, int cb,
-                                      bool inflate_a, float ds_f, float* sA, float* sB, int* sVA, int* sVB) {
-  __syncthreads();
-  for (int k = threadIdx.x; k < ca; k += blockDim.x) {
-    const int pa = L.offA + L.LA[a0 + k];
-    const float* src = L.boxA + 6 * pa;
-    if (inflate_a) finflate(src, ds_f, sA + 6 * k);
-    else
+// One entry of a list into shared memory: the float box of A entry k (inflated by sqrt(dhat),
+// rounded outward, for the pair cull) or B entry k, and for the pair cull (v not null) the vertex
+// ids (A: a point's id or an edge's two at v[0 ..]; B: a face's three or an edge's two).
+__device__ __forceinline__ void stage_a(const Geo& g, int sub, const SubLists& L, int k, bool inflate, float ds_f,
+                                        float* s, int* v) {
+  const int pa = L.offA + L.LA[k];
+  const float* src = L.boxA + 6 * pa;
+  if (inflate) finflate(src, ds_f, s);
+  else
 #pragma unroll
-      for (int c = 0; c < 6; ++c) sA[6 * k + c] = src[c];
-    if (sVA) {
-      if (sub < 2) {
-        sVA[2 * k] = pa;
-      } else {
-        sVA[2 * k] = g.ev[2 * pa];
-        sVA[2 * k + 1] = g.ev[2 * pa + 1];
-      }
+    for (int c = 0; c < 6; ++c) s[c] = src[c];
+  if (v) {
+    if (sub < 2) {
+      v[0] = pa;
+    } else {
+      v[0] = g.ev[2 * pa];
+      v[1] = g.ev[2 * pa + 1];
     }
   }
-  for (int k = threadIdx.x; k < cb; k += blockDim.x) {
-    const int pb = L.offB + L.LB[b0 + k];
-    const float* src = L.boxB + 6 * pb;
+}
+__device__ __forceinline__ void stage_b(const Geo& g, int sub, const SubLists& L, int k, float* s, int* v) {
+  const int pb = L.offB + L.LB[k];
+  const float* src = L.boxB + 6 * pb;
 #pragma unroll
-    for (int c = 0; c < 6; ++c) sB[6 * k + c] = src[c];
-    if (sVB) {
-      if (sub < 2) {
-        sVB[3 * k] = g.fv[3 * pb];
-        sVB[3 * k + 1] = g.fv[3 * pb + 1];
-        sVB[3 * k + 2] = g.fv[3 * pb + 2];
-      } else {
-        sVB[3 * k] = g.ev[2 * pb];
-        sVB[3 * k + 1] = g.ev[2 * pb + 1];
-      }
+  for (int c = 0; c < 6; ++c) s[c] = src[c];
+  if (v) {
+    if (sub < 2) {
+      v[0] = g.fv[3 * pb];
+      v[1] = g.fv[3 * pb + 1];
+      v[2] = g.fv[3 * pb + 2];
+    } else {
+      v[0] = g.ev[2 * pb];
+      v[1] = g.ev[2 * pb + 1];
     }
   }
-  __syncthreads();
 }
 
 __device__ __forceinline__ bool f_hit(const float* a, const float* b) {
@@ -934,8 +928,8 @@ __global__ void __launch_bounds__(128) k_toi_list(Geo g, ToiCand tc, unsigned lo
 
 // 5a. Narrow phase, one CTA per overlap: pair cull (MODE 0) or trajectory (MODE 2).
 // For each sub-problem (v(I) x f(J), v(J) x f(I), e(I) x e(J)) the float boxes of both
-// lists are staged in shared memory. The work alternates between two phases so that the
-// FP64 work is spread evenly over the CTA:
+// lists are staged in shared memory, all three together while they fit. The work alternates
+// between two phases so that the tests are spread evenly over the CTA:
 //  - box phase: each thread keeps one A box in registers and walks its B boxes (a
 //    shared-memory broadcast per step), STEP candidates per thread, and appends the
 //    float-box hits to a shared queue (warp-aggregated);
@@ -947,8 +941,8 @@ __global__ void __launch_bounds__(128) k_toi_list(Geo g, ToiCand tc, unsigned lo
 // impact) instructions of 64 cycles a warp, which a CTA with a handful of candidates used to
 // pay for each sub-problem and box phase. MODE 0 keeps an overlap's candidates in shared
 // memory and writes them sorted, so that the accepted ones come out in order. One cull of a
-// batch of columns (7291 overlaps, 11 candidates each) 893 -> 280 us, of the pile (9871, 19
-// each) 583 -> 310 us, the FP64 kernel included.
+// batch of columns (7291 overlaps, 11 candidates each) 893 -> 238 us, of the pile (9871, 19
+// each) 583 -> 300 us, the FP64 kernel included.
 template <int MODE, int STEP>
 __global__ void __launch_bounds__(NT, MODE == 0 ? (STEP <= 8 ? 4 : STEP <= 16 ? 3 : 2) : (STEP <= 36 ? 4 : 2))
     k_narrow_scan(Geo g, Params P, float ds_f, const int* ovI, const int* ovJ, int* cnt, const int* off, int* lst,
@@ -963,100 +957,172 @@ __global__ void __launch_bounds__(NT, MODE == 0 ? (STEP <= 8 ? 4 : STEP <= 16 ? 
   int* sVB = MODE == 0 ? sVA + 2 * TILE : nullptr;                          // 3 * TILE (MODE 0)
   __shared__ int sq_n[2];
   __shared__ int rec_n, rec_np, rec_base[2];
+  __shared__ SubLists sL[3];
   const int u = order[blockIdx.x];
   const float lim_f = __double2float_ru(P.dhat * (1.0 + 1e-4));
-  int* n = cnt + 6 * u;
-  const int* o = off + 6 * u;
   const int lane = threadIdx.x & 31;
   const unsigned below = (1u << lane) - 1u;
+  if (threadIdx.x < 3) {
+    SubLists L = sub_lists(g, threadIdx.x, ovI[u], ovJ[u], cnt + 6 * u, off + 6 * u, lst, vb, eb, fb);  // refined
+    if (L.nA == 0 || L.nB == 0) L.nA = L.nB = 0;
+    sL[threadIdx.x] = L;
+  }
   if (threadIdx.x == 0) {
     rec_n = rec_np = 0;
     sq_n[0] = 0;
     sq_n[1] = 0;
   }
-  int par = 0;
+  __syncthreads();
+  // Box phase over rows of one staged chunk: thread t has the rows i = t mod ca (ca < NT) or
+  // t, t + NT, ... (ca >= NT) and the columns j = ph, ph + phases, ... with phases = NT / ca
+  // threads sharing a row.
+  struct Walk {
+    int ca, cb, rows, phases, ph, row0, ncol, nrow, max_items, ri, cj;
+  };
+  auto walk_of = [&](int ca, int cb) {
+    Walk w;
+    w.ca = ca;
+    w.cb = cb;
+    w.rows = ca < NT ? ca : NT;
+    w.phases = ca < NT ? NT / ca : 1;
+    w.ph = ca < NT ? threadIdx.x / ca : 0;
+    w.row0 = threadIdx.x % w.rows;
+    w.ncol = w.ph < w.phases ? (cb - w.ph + w.phases - 1) / w.phases : 0;
+    w.nrow = w.ncol > 0 ? (ca - w.row0 + w.rows - 1) / w.rows : 0;
+    w.max_items = (ca < NT ? 1 : (ca + NT - 1) / NT) * ((cb + w.phases - 1) / w.phases);
+    w.ri = w.cj = 0;
+    return w;
+  };
+  // its candidates: the hits to the queue (qa, qb: the chunk's first A and B entry in it)
+  auto boxes = [&](Walk& w, int items, const float* A, const float* B, float (&a)[6], int par, unsigned tag) {
 #pragma unroll 1
-  for (int sub = 0; sub < 3; ++sub) {
-    SubLists L = sub_lists(g, sub, ovI[u], ovJ[u], n, o, lst, vb, eb, fb);  // lists refined by k_refine
-    if (L.nA == 0 || L.nB == 0) continue;
-#pragma unroll 1
-    for (int a0 = 0; a0 < L.nA; a0 += TILE) {
-      const int ca = min(TILE, L.nA - a0);
-#pragma unroll 1
-      for (int b0 = 0; b0 < L.nB; b0 += TILE) {
-        const int cb = min(TILE, L.nB - b0);
-        stage(g, sub, L, a0, ca, b0, cb, MODE != 2, ds_f, sA, sB, sVA, sVB);
-        // thread t: rows i = t mod ca (ca < NT) or t, t + NT, ... (ca >= NT); columns
-        // j = ph, ph + phases, ... with phases = NT / ca threads sharing a row
-        const int rows = ca < NT ? ca : NT;
-        const int phases = ca < NT ? NT / ca : 1;
-        const int ph = ca < NT ? threadIdx.x / ca : 0;
-        const int row0 = threadIdx.x % rows;
-        const bool live = ph < phases;
-        const int ncol = live ? (cb - ph + phases - 1) / phases : 0;        // columns per row
-        const int nrow = (live && ncol > 0) ? (ca - row0 + rows - 1) / rows : 0;  // rows of this thread
-        const int max_items = (ca < NT ? 1 : (ca + NT - 1) / NT) * ((cb + phases - 1) / phases);
-        const int steps = (max_items + STEP - 1) / STEP;
-        int ri = 0, cj = 0;  // cursor: row index (of this thread's rows), column index
-        float a[6];
-        if (nrow > 0)
+    for (int it = 0; it < items; ++it) {
+      bool hit = false;
+      unsigned code = 0;
+      if (w.ri < w.nrow) {
+        const int i = w.row0 + w.ri * w.rows, j = w.ph + w.cj * w.phases;
+        hit = i < w.ca && j < w.cb && f_hit(a, B + 6 * j);
+        code = tag + (((unsigned)i << 15) | (unsigned)j);
+        if (++w.cj == w.ncol) {
+          w.cj = 0;
+          if (++w.ri < w.nrow)
 #pragma unroll
-          for (int c = 0; c < 6; ++c) a[c] = sA[6 * row0 + c];
+            for (int c = 0; c < 6; ++c) a[c] = A[6 * (w.row0 + w.ri * w.rows) + c];
+        }
+      }
+      const unsigned m = __ballot_sync(0xffffffffu, hit);
+      if (m) {
+        int base = 0;
+        if (lane == 0) base = atomicAdd(&sq_n[par], __popc(m));
+        base = __shfl_sync(0xffffffffu, base, 0);
+        const int pos = base + __popc(m & below);
+        if (hit && pos < NT * STEP) sq[pos] = code;
+      }
+    }
+  };
+  // test of a candidate: A entry i and B entry j of the lists, staged at (si, sj)
+  auto test = [&](int sub, const SubLists& L, int i, int j, int si, int sj) {
+    if (MODE == 2) {
+      const int pa = L.offA + L.LA[i], pb = L.offB + L.LB[j];
+      if (f_toi_miss(g, tc.ve, sub, pa, pb)) return;
+      const unsigned o = atomicAdd(tc.n, 1u);
+      if (o < tc.cap) tc.cand[o] = make_int2(sub < 2 ? pa : ~pa, pb);
+      else toi_one(g, sub, pa, pb, toi_key);
+    } else {
+      const int w0 = sVA[2 * si];
+      const int w1 = sub < 2 ? sVB[3 * sj] : sVA[2 * si + 1];
+      const int w2 = sub < 2 ? sVB[3 * sj + 1] : sVB[3 * sj];
+      const int w3 = sub < 2 ? sVB[3 * sj + 2] : sVB[3 * sj + 1];
+      if (f_reject_v(vb, sub, w0, w1, w2, w3, lim_f)) return;
+      const int slot = atomicAdd(&rec_n, 1);
+      if (slot < REC_CAP)
+        recK[slot] = ((unsigned long long)sub << 60) | ((unsigned long long)i << 30) | (unsigned long long)j;
+    }
+  };
+  const int a1 = sL[0].nA, a2 = a1 + sL[1].nA, a3 = a2 + sL[2].nA;
+  const int b1 = sL[0].nB, b2 = b1 + sL[1].nB, b3 = b2 + sL[2].nB;
+  // Short lists: the three sub-problems are staged together and share one box and one test
+  // phase, so the CTA waits once for the lists, the boxes and the vertices instead of three
+  // times. On the pile's trajectories 235 -> 151 us, on columns 207 -> 172 us (pair cull) and 132 -> 82 us.
+  bool general = a3 > TILE || b3 > TILE;
+  if (!general && a3 > 0) {
+    for (int k = threadIdx.x; k < a3; k += NT) {
+      const int sub = (k >= a1) + (k >= a2);
+      stage_a(g, sub, sL[sub], k - (sub == 0 ? 0 : (sub == 1 ? a1 : a2)), MODE != 2, ds_f, sA + 6 * k,
+              MODE == 0 ? sVA + 2 * k : nullptr);
+    }
+    for (int k = threadIdx.x; k < b3; k += NT) {
+      const int sub = (k >= b1) + (k >= b2);
+      stage_b(g, sub, sL[sub], k - (sub == 0 ? 0 : (sub == 1 ? b1 : b2)), sB + 6 * k,
+              MODE == 0 ? sVB + 3 * k : nullptr);
+    }
+    __syncthreads();
 #pragma unroll 1
-        for (int st = 0; st < steps; ++st) {
-          // box phase
-#pragma unroll 1
-          for (int it = 0, its = min(STEP, max_items - st * STEP); it < its; ++it) {
-            bool hit = false;
-            unsigned code = 0;
-            if (ri < nrow) {
-              int i = row0 + ri * rows, j = ph + cj * phases;
-              hit = i < ca && j < cb && f_hit(a, sB + 6 * j);
-              code = ((unsigned)i << 16) | (unsigned)j;
-              if (++cj == ncol) {
-                cj = 0;
-                if (++ri < nrow)
+    for (int sub = 0; sub < 3; ++sub) {
+      const int ca = sL[sub].nA, cb = sL[sub].nB;
+      if (ca == 0) continue;
+      const int qa = sub == 0 ? 0 : (sub == 1 ? a1 : a2), qb = sub == 0 ? 0 : (sub == 1 ? b1 : b2);
+      Walk w = walk_of(ca, cb);
+      float a[6];
+      if (w.nrow > 0)
 #pragma unroll
-                  for (int c = 0; c < 6; ++c) a[c] = sA[6 * (row0 + ri * rows) + c];
-              }
-            }
-            unsigned m = __ballot_sync(0xffffffffu, hit);
-            if (m) {
-              int base = 0;
-              if (lane == 0) base = atomicAdd(&sq_n[par], __popc(m));
-              base = __shfl_sync(0xffffffffu, base, 0);
-              if (hit) sq[base + __popc(m & below)] = code;
-            }
-          }
-          __syncthreads();
-          // test phase
-          const int nq = sq_n[par];
-          if (threadIdx.x == 0) sq_n[par ^ 1] = 0;
+        for (int c = 0; c < 6; ++c) a[c] = sA[6 * (qa + w.row0) + c];
+      boxes(w, w.max_items, sA + 6 * qa, sB + 6 * qb, a, 0,
+            ((unsigned)sub << 30) + ((unsigned)qa << 15) + (unsigned)qb);
+    }
+    __syncthreads();
+    const int nq = sq_n[0];
+    general = nq > NT * STEP;  // more hits than the queue holds
+    if (!general) {
 #pragma unroll 1
-          for (int k = threadIdx.x; k < nq; k += NT) {
-            unsigned code = sq[k];
-            int i = (int)(code >> 16), j = (int)(code & 0xffffu);
-            if (i >= ca || j >= cb) continue;
-            if (MODE == 2) {
-              const int pa = L.offA + L.LA[a0 + i], pb = L.offB + L.LB[b0 + j];
-              if (f_toi_miss(g, tc.ve, sub, pa, pb)) continue;
-              const unsigned o = atomicAdd(tc.n, 1u);
-              if (o < tc.cap) tc.cand[o] = make_int2(sub < 2 ? pa : ~pa, pb);
-              else toi_one(g, sub, pa, pb, toi_key);
-            } else {
-              const int w0 = sVA[2 * i];
-              const int w1 = sub < 2 ? sVB[3 * j] : sVA[2 * i + 1];
-              const int w2 = sub < 2 ? sVB[3 * j + 1] : sVB[3 * j];
-              const int w3 = sub < 2 ? sVB[3 * j + 2] : sVB[3 * j + 1];
-              if (f_reject_v(vb, sub, w0, w1, w2, w3, lim_f)) continue;
-              const int slot = atomicAdd(&rec_n, 1);
-              if (slot < REC_CAP)
-                recK[slot] = ((unsigned long long)sub << 60) | ((unsigned long long)(a0 + i) << 30) |
-                             (unsigned long long)(b0 + j);
-            }
-          }
-          par ^= 1;
+      for (int k = threadIdx.x; k < nq; k += NT) {
+        const unsigned code = sq[k];
+        const int sub = (int)(code >> 30), si = (int)(code >> 15 & 0x7fffu), sj = (int)(code & 0x7fffu);
+        test(sub, sL[sub], si - (sub == 0 ? 0 : (sub == 1 ? a1 : a2)), sj - (sub == 0 ? 0 : (sub == 1 ? b1 : b2)), si,
+             sj);
+      }
+    } else {
+      __syncthreads();
+      if (threadIdx.x == 0) sq_n[0] = 0;
+    }
+  }
+  if (general) {
+    int par = 0;
+#pragma unroll 1
+    for (int sub = 0; sub < 3; ++sub) {
+      const SubLists L = sL[sub];
+#pragma unroll 1
+      for (int a0 = 0; a0 < L.nA; a0 += TILE) {
+        const int ca = min(TILE, L.nA - a0);
+#pragma unroll 1
+        for (int b0 = 0; b0 < L.nB; b0 += TILE) {
+          const int cb = min(TILE, L.nB - b0);
           __syncthreads();
+          for (int k = threadIdx.x; k < ca; k += NT)
+            stage_a(g, sub, L, a0 + k, MODE != 2, ds_f, sA + 6 * k, MODE == 0 ? sVA + 2 * k : nullptr);
+          for (int k = threadIdx.x; k < cb; k += NT)
+            stage_b(g, sub, L, b0 + k, sB + 6 * k, MODE == 0 ? sVB + 3 * k : nullptr);
+          __syncthreads();
+          Walk w = walk_of(ca, cb);
+          float a[6];
+          if (w.nrow > 0)
+#pragma unroll
+            for (int c = 0; c < 6; ++c) a[c] = sA[6 * w.row0 + c];
+#pragma unroll 1
+          for (int st = 0; st < w.max_items; st += STEP) {
+            boxes(w, min(STEP, w.max_items - st), sA, sB, a, par, 0u);
+            __syncthreads();
+            const int nq = sq_n[par];
+            if (threadIdx.x == 0) sq_n[par ^ 1] = 0;
+#pragma unroll 1
+            for (int k = threadIdx.x; k < nq; k += NT) {
+              const unsigned code = sq[k];
+              const int i = (int)(code >> 15), j = (int)(code & 0x7fffu);
+              test(sub, L, a0 + i, b0 + j, i, j);
+            }
+            par ^= 1;
+            __syncthreads();
+          }
         }
       }
     }

@@ -33,3 +33,21 @@ def test_lists(gpu_lib, oracle_lib, pairs, lo, hi):
         assert n.max() > 2048 and n.min() < 200
     if pairs == 100:
         assert n[n < 1700].sum() > 65536
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("subdiv,shift", [(0, 0.3), (1, 0.01), (1, 0.2), (1, 0.9)])
+def test_short_lists(gpu_lib, oracle_lib, subdiv, shift):
+    """Lists that are staged together: of few box hits, and of more than the queue of hits holds."""
+    from adb_gb300.abd import ABD
+    sb, rng = S.SceneBuilder(), np.random.default_rng(4)
+    for k in range(12):
+        sb.add(S.icosphere_mesh(subdiv, 0.5), np.array([3.0 * (k // 2), 2.0, 0.0]) + (k % 2) * shift * np.array([0.8, 0.5, -0.33]),
+               S.rotation_zyx(*rng.uniform(-1e-2, 1e-2, 3)))
+    sc, cfg = sb.build(), S.workload_config("pile")
+    gpu, orc = ABD(sc, cfg), oracle_lib.OracleSim(sc, cfg)
+    dq = rng.normal(size=sc.q0.shape) * 0.01
+    for args in ((1, sc.q0), (2, sc.q0, dq)):
+        for a, b in zip(gpu.cull(*args), orc.cull(*args)):
+            assert a.shape == b.shape and np.array_equal(a, b)
+    assert gpu.cull(3, sc.q0, dq) == orc.cull(3, sc.q0, dq)
