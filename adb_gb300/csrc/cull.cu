@@ -324,10 +324,19 @@ __device__ __forceinline__ void tight_box(const Geo& g, int body, const float* v
 // stores the count (one pass instead of two when that capacity fits).
 enum { BIN_COUNT = 0, BIN_WRITE = 1, BIN_ONCE = 2 };
 
-// Capacity of list slot (overlap u, side, kind): the primitive count of that body.
-__global__ void k_bin_caps(Geo g, int nov, const int* ovI, const int* ovJ, int* cap) {
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= 6 * nov) return;
+// Capacity of list slot (overlap u, side, kind): the primitive count of that body (cap null: not
+// wanted), and the box of each body's vertex boxes (a warp a body).
+__global__ void k_bin_caps(Geo g, int nov, const int* ovI, const int* ovJ, const float* vb, const float* cl, int* cap,
+                           float* tight) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x, w = t >> 5, lane = threadIdx.x & 31;
+  if (w < g.nb) {
+    float o[6];
+    tight_box(g, w, vb, cl, o);
+    if (lane == 0)
+#pragma unroll
+      for (int c = 0; c < 6; ++c) tight[6 * w + c] = o[c];
+  }
+  if (!cap || t >= 6 * nov) return;
   int u = t / 6, side = (t / 3) & 1, kind = t % 3;
   int body = side ? ovJ[u] : ovI[u];
   const int* o = kind == 0 ? g.v_off : (kind == 1 ? g.e_off : g.f_off);
@@ -342,11 +351,11 @@ __global__ void k_bin_caps(Geo g, int nov, const int* ovI, const int* ovJ, int* 
 // lists also leave out what no box of the other body can hit: entries on the A side of their
 // sub-problem (vertices, and the first body's edges), inflated by ds, that miss the union of the
 // other body's vertex boxes, and entries on the B side that miss that union inflated (inflating
-// rounds monotonically, so this is the union of the inflated boxes). Now 66 us, and k_refine
-// 91 -> 26 us.
+// rounds monotonically, so this is the union of the inflated boxes); where neither body's box
+// meets the other's inflated one the lists are empty. Now 54 us, and k_refine 91 -> 27 us.
 __global__ void __launch_bounds__(256, 3) k_bin(Geo g, float ds, int nov, int pass, int traj, const int* ovI, const int* ovJ,
                                                 const double* ovcull, const float* ovcull_f, const float* vb,
-                                                const float* eb, const float* fb, BinClusters cl, int* cnt,
+                                                const float* eb, const float* fb, BinClusters cl, const float* tights, int* cnt,
                                                 const int* off, int* lst) {
   int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (warp >= 2 * nov) return;
@@ -365,8 +374,24 @@ __global__ void __launch_bounds__(256, 3) k_bin(Geo g, float ds, int nov, int pa
     ci[k + 3] = nextafterf(cf[k + 3], -INFINITY);
   }
   unsigned below = (1u << lane) - 1u;
-  float tight[6];
-  tight_box(g, side ? ovI[u] : ovJ[u], vb, cl.v, tight);
+  float tight[6];  // of the other body
+  {
+    float own[6], x[6];
+    const int other = side ? ovI[u] : ovJ[u];
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {
+      tight[k] = tights[6 * other + k];
+      own[k] = tights[6 * body + k];
+    }
+    finflate(own, ds, x);
+    bool meet = f_overlap(x, tight);
+    finflate(tight, ds, x);
+    meet = (meet || f_overlap(own, x)) && f_overlap(cf, own);
+    if (!meet) {
+      if (pass != BIN_WRITE && lane < 3) cnt[6 * u + 3 * side + lane] = 0;
+      return;
+    }
+  }
 #pragma unroll 1
   for (int kind = 0; kind < 3; ++kind) {
     const bool on_a = kind == 0 || (kind == 1 && side == 0);
@@ -899,18 +924,33 @@ __device__ __forceinline__ int work_bucket(const int* n) {
   long long c = (long long)n[0] * n[5] + (long long)n[3] * n[2] + (long long)n[1] * n[4];
   return c >= 16384 ? 0 : (c >= 2048 ? 1 : (c > 0 ? 2 : 3));
 }
-__global__ void k_order_count(int nov, const int* cnt, int* bc) {
-  int u = blockIdx.x * blockDim.x + threadIdx.x;
-  if (u < nov) atomicAdd(&bc[work_bucket(cnt + 6 * u)], 1);
+// Bucket b's overlaps at order[b * nov ...], bc[b] of them.
+__global__ void k_order(int nov, const int* cnt, int* bc, int* order) {
+  const int u = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
+  const int b = u < nov ? work_bucket(cnt + 6 * u) : NBUCKET - 1;
+#pragma unroll
+  for (int k = 0; k < NBUCKET - 1; ++k) {  // the empty ones are not taken
+    const unsigned m = __ballot_sync(0xffffffffu, b == k);
+    if (!m) continue;
+    int base = 0;
+    if (lane == 0) base = atomicAdd(&bc[k], __popc(m));
+    base = __shfl_sync(0xffffffffu, base, 0);
+    if (b == k) order[k * (size_t)nov + base + __popc(m & ((1u << lane) - 1u))] = u;
+  }
 }
-__global__ void k_order_place(int nov, const int* cnt, int* bc, int* order) {
-  int u = blockIdx.x * blockDim.x + threadIdx.x;
-  if (u >= nov) return;
-  int b = work_bucket(cnt + 6 * u);
-  int base = 0;
-  for (int k = 0; k < b; ++k) base += bc[k];
-  order[base + atomicAdd(&bc[NBUCKET + b], 1)] = u;
-}
+// The overlap of place i of the order, -1 past the last.
+struct Order {
+  const int *at, *bc;
+  int nov;
+  __device__ __forceinline__ int operator[](int i) const {
+    for (int k = 0; k < NBUCKET - 1; ++k) {
+      const int n = bc[k];
+      if (i < n) return at[k * (size_t)nov + i];
+      i -= n;
+    }
+    return -1;
+  }
+};
 
 // The FP64 test of one candidate into its scene's key.
 __device__ __noinline__ void toi_one(const Geo& g, int sub, int pa, int pb, unsigned long long* toi_key) {
@@ -947,7 +987,7 @@ template <int MODE, int STEP>
 __global__ void __launch_bounds__(NT, MODE == 0 ? (STEP <= 8 ? 4 : STEP <= 16 ? 3 : 2) : (STEP <= 36 ? 4 : 2))
     k_narrow_scan(Geo g, Params P, float ds_f, const int* ovI, const int* ovJ, int* cnt, const int* off, int* lst,
                   const float* vb, const float* eb, const float* fb, unsigned long long* toi_key, StageOut so,
-                  const int* order, ToiCand tc) {
+                  Order order, ToiCand tc) {
   extern __shared__ __align__(16) unsigned char smem_dyn[];
   unsigned long long* recK = reinterpret_cast<unsigned long long*>(smem_dyn);  // REC_CAP (MODE 0)
   float* sA = reinterpret_cast<float*>(smem_dyn + (MODE == 0 ? REC_CAP * sizeof(unsigned long long) : 0));
@@ -959,6 +999,7 @@ __global__ void __launch_bounds__(NT, MODE == 0 ? (STEP <= 8 ? 4 : STEP <= 16 ? 
   __shared__ int rec_n, rec_np, rec_base[2];
   __shared__ SubLists sL[3];
   const int u = order[blockIdx.x];
+  if (u < 0) return;  // no candidates: k_narrow_tally sees that from the lists
   const float lim_f = __double2float_ru(P.dhat * (1.0 + 1e-4));
   const int lane = threadIdx.x & 31;
   const unsigned below = (1u << lane) - 1u;
@@ -1239,9 +1280,13 @@ __global__ void __launch_bounds__(NW) k_narrow_tally(Geo g, Params P, float ds_f
                                                      const float* eb, const float* fb, StageOut so, int* npt, int* nee) {
   __shared__ int s_pt, s_ee;
   const int u = blockIdx.x;
-  const int4 sg = so.seg[u];
-  if ((sg.x >= 0 && sg.y + sg.w == 0) || !so.valid()) {
-    if (threadIdx.x == 0) npt[u] = nee[u] = 0;
+  const int4 sg = so.seg[u];  // not written where no list pair is left
+  const bool none = work_bucket(cnt + 6 * u) == NBUCKET - 1 || (sg.x >= 0 && sg.y + sg.w == 0);
+  if (none || !so.valid()) {
+    if (threadIdx.x == 0) {
+      npt[u] = nee[u] = 0;
+      if (none) so.seg[u] = make_int4(0, 0, 0, 0);
+    }
     return;
   }
   if (threadIdx.x == 0) s_pt = s_ee = 0;
@@ -1429,7 +1474,7 @@ struct NarrowLaunch {
   const float *vb, *eb, *fb;
   unsigned long long* toi_key;
   StageOut so;
-  const int* order;
+  Order order;
   ToiCand tc;
 };
 
@@ -1489,13 +1534,12 @@ static void narrow_phase(int mode, int nov, const NarrowLaunch& a, CullScratch& 
 }
 
 
-// Fills cs.order with the overlaps heaviest bucket first (k_order_count / k_order_place).
+// Fills cs.order with the overlaps that have work, heaviest bucket first.
 static void order_overlaps(int nov, CullScratch& cs, cudaStream_t s, int tag) {
-  cs.order.ensure(nov + 1);
-  cs.order_cnt.ensure(2 * NBUCKET);
-  CK(cudaMemsetAsync(cs.order_cnt.p, 0, 2 * NBUCKET * sizeof(int), s));
-  KLAUNCH(tag, s, k_order_count<<<nblk(nov, 256), 256, 0, s>>>(nov, cs.bin_cnt.p, cs.order_cnt.p));
-  KLAUNCH(tag, s, k_order_place<<<nblk(nov, 256), 256, 0, s>>>(nov, cs.bin_cnt.p, cs.order_cnt.p, cs.order.p));
+  cs.order.ensure((NBUCKET - 1) * (size_t)nov + 1);
+  cs.order_cnt.ensure(NBUCKET);
+  CK(cudaMemsetAsync(cs.order_cnt.p, 0, NBUCKET * sizeof(int), s));
+  KLAUNCH(tag, s, k_order<<<nblk(nov, 256), 256, 0, s>>>(nov, cs.bin_cnt.p, cs.order_cnt.p, cs.order.p));
 }
 
 float float_round_up(double d) {
@@ -1570,7 +1614,7 @@ static void narrow_pairs(const Geo& g, const Params& P, float ds_f, int nov, con
     so = StageOut{cs.stage_key.p, cs.stage_ov.p, cs.stage_ty.p, cs.stage_seg.p, d_tot + 6, (int)cs.stage_key.cap};
     narrow_smem_attr();
     NarrowLaunch a{g, P, ds_f, ovI, ovJ, cs.bin_cnt.p, cs.bin_off.p, cs.lst.p, cs.vbox.p, cs.ebox.p, cs.fbox.p,
-                   nullptr, so, cs.order.p, ToiCand{}};
+                   nullptr, so, Order{cs.order.p, cs.order_cnt.p, nov}, ToiCand{}};
     narrow_phase(0, nov, a, cs, d_tot + 6, s);
     KLAUNCH(K_NARROW_SCAN, s, k_narrow_exact<<<1216, 128, 0, s>>>(g, P, ovI, ovJ, cs.bin_cnt.p, cs.bin_off.p,
                                                                   cs.lst.p, so));
@@ -1669,12 +1713,13 @@ void cull(const Geo& g_in, const Params& P, int vtn, double alpha, CullScratch& 
     // list capacity = the primitive counts of both bodies of every overlap; when it fits
     // (at most 2^28 entries) one binning pass writes the lists in place
     bool once = 2ll * nov * g.max_prims < (1ll << 28);
-    if (once) {
-      KLAUNCH(K_BIN, s, k_bin_caps<<<nblk(6ll * nov, 256), 256, 0, s>>>(g, nov, S.ovI.p, S.ovJ.p, cs.bin_cnt.p));
-    } else {
+    cs.tight.ensure(6 * (size_t)g.nb);
+    KLAUNCH(K_BIN, s, k_bin_caps<<<nblk(std::max(6ll * nov, 32ll * g.nb), 256), 256, 0, s>>>(
+                          g, nov, S.ovI.p, S.ovJ.p, cs.vbox.p, cl.v, once ? cs.bin_cnt.p : nullptr, cs.tight.p));
+    if (!once) {
       KLAUNCH(K_BIN, s, k_bin<<<nblk((long long)nw * 32, 256), 256, 0, s>>>(g, ds_f, nov, BIN_COUNT, traj, S.ovI.p, S.ovJ.p,
                                                           cs.ovcull.p, cs.ovcull_f.p, cs.vbox.p, cs.ebox.p,
-                                                          cs.fbox.p, cl, cs.bin_cnt.p, nullptr, nullptr));
+                                                          cs.fbox.p, cl, cs.tight.p, cs.bin_cnt.p, nullptr, nullptr));
     }
     scan_exclusive_int(cs.bin_cnt.p, cs.bin_off.p, 6 * nov, d_tot + 2, s, cs.vflag_cnt);
     if (once) {
@@ -1688,7 +1733,7 @@ void cull(const Geo& g_in, const Params& P, int vtn, double alpha, CullScratch& 
     cs.lst.ensure((size_t)nlst + 1);
     KLAUNCH(K_BIN, s, k_bin<<<nblk((long long)nw * 32, 256), 256, 0, s>>>(g, ds_f, nov, once ? BIN_ONCE : BIN_WRITE, traj,
                                                         S.ovI.p, S.ovJ.p, cs.ovcull.p, cs.ovcull_f.p, cs.vbox.p,
-                                                        cs.ebox.p, cs.fbox.p, cl, cs.bin_cnt.p, cs.bin_off.p, cs.lst.p));
+                                                        cs.ebox.p, cs.fbox.p, cl, cs.tight.p, cs.bin_cnt.p, cs.bin_off.p, cs.lst.p));
   }
   if (traj) {
     const int nk = 2 * g.ns;
@@ -1719,7 +1764,7 @@ void cull(const Geo& g_in, const Params& P, int vtn, double alpha, CullScratch& 
       cs.toi_cand.ensure(kToiCand);
       cs.toi_n.ensure(2);
       NarrowLaunch a{g, P, ds_f, S.ovI.p, S.ovJ.p, cs.bin_cnt.p, cs.bin_off.p, cs.lst.p, cs.vbox.p, cs.ebox.p,
-                     cs.fbox.p, cs.toi_key.p, StageOut{}, cs.order.p,
+                     cs.fbox.p, cs.toi_key.p, StageOut{}, Order{cs.order.p, cs.order_cnt.p, nov},
                      ToiCand{cs.vend.p, cs.toi_cand.p, cs.toi_n.p, kToiCand}};
       narrow_phase(2, nov, a, cs, reinterpret_cast<int*>(cs.toi_n.p), s);
       KLAUNCH(K_NARROW_TOI, s, k_toi_list<<<1216, 128, 0, s>>>(g, a.tc, cs.toi_key.p));
