@@ -15,8 +15,8 @@
 // What bounds it: the dependent FP64 chain of one 12 x 12 factorization and the chain of
 // loads before it. In body order a chain of n links is n of them, one after the other on one
 // SM; by levels it is log2 n, at about twice the operations. Measured per solve, in body
-// order and by levels: 200 links in contact 2.49 -> 0.26 ms, 256 columns (8212 bodies in all)
-// 1.83 -> 0.62 ms, a stack of ten 0.117 -> 0.091 ms.
+// order and by levels: 200 links in contact 2.49 -> 0.17 ms, 256 columns (8212 bodies in all)
+// 1.83 -> 0.42 ms, a stack of ten 0.117 -> 0.069 ms.
 // Couplings that are absent (runs broken by missing contacts) are flagged and cost nothing.
 // Every sum runs in a fixed order, and a body's arithmetic depends only on its own scene and
 // its place there, so a scene gets the same solution in a batch as alone.
@@ -31,7 +31,7 @@ namespace cg = cooperative_groups;
 namespace abd {
 namespace {
 
-constexpr int TNT = 160;  // threads per body: 144 for the 12 x 12 entries, 12 for the right-hand side
+constexpr int TNT = 192;  // threads per body
 constexpr int TWARPS = TNT / 32;
 
 inline int nblk_t(long long n, int t) { return (int)((n + t - 1) / t); }
@@ -77,16 +77,16 @@ struct TriArgs {
   int* status;
 };
 
-// Pivot of a right-looking Cholesky: r = 1 / sqrt(a), L_kk = a r. A non-positive pivot
-// sets ABD_ERR_NOT_SPD and is replaced by 1e-300, as the block-Jacobi preconditioner does.
-__device__ __forceinline__ void tri_pivot(double a, double* r, double* lkk, int* status) {
+// Pivot of a right-looking Cholesky: r = 1 / sqrt(a), d = r^2. A non-positive pivot sets
+// ABD_ERR_NOT_SPD and is replaced by 1e-300, as the block-Jacobi preconditioner does.
+__device__ __forceinline__ void tri_pivot(double a, double* r, double* d, int* status) {
   if (!(a > 0)) {
     atomicExch(status, (int)ABD_ERR_NOT_SPD);
     a = 1e-300;
   }
   const double q = rsqrt(a);
   *r = q;
-  *lkk = a * q;
+  *d = q * q;
 }
 
 // acc += sum over r of P[r][i] Q[r], Q read with stride qs (a column of a 12 x 12 block: 12,
@@ -101,20 +101,28 @@ __device__ __forceinline__ double tri_dot_t(const double* P, int i, const double
 // each, then the back substitution from the last level to the first. A CTA eliminates one
 // body at a time.
 //
-// The 12 x 12 work of a body is spread over 156 threads (thread t < 144: entry (t / 12,
-// t % 12); 144..155: the right-hand side as a 13th column), because on this part a dependent
-// FP64 instruction of one warp waits ~64 cycles: the Cholesky factor is right-looking, one
-// barrier per column (the column scaled and the trailing triangle updated in the same
-// phase; the thread that updates the next pivot takes its reciprocal square root), and row
-// c of L^-1, which needs L's column c, is formed one phase later by the threads of columns
-// <= c, which the factorization no longer uses.
-__global__ void __launch_bounds__(TNT) k_tri_solve(TriArgs a) {
+// An FP64 instruction of a warp takes 64 cycles of its quarter of the SM however many lanes
+// are active, so the 12 x 12 work is laid out for few warp instructions: six warps, the
+// lower triangles packed. Warps 0-2: the 78 entries of the body's Schur complement and the
+// right-hand side, then the right-looking factor, an entry kept in its thread's register and
+// put in shared memory when its column is next (the thread that updates the next pivot takes
+// its reciprocal square root). Warps 3-5: the two coupling blocks, then L^-1, row c formed one
+// column behind the factor from the rows above (T holds I minus their contributions). Then
+// each warp forms two rows of L^-1 [U_lower U_upper b], a short and a long one. A batch of
+// columns (128 bodies in the deepest) 622 -> 418 us, a chain of 200 256 -> 174 us against
+// five warps with a thread per entry of the square.
+__global__ void __launch_bounds__(TNT, 5) k_tri_solve(TriArgs a) {
   cg::grid_group grid = cg::this_grid();
   __shared__ double sA[12][13], sL[12][13], sT[12][13], sLi[12][13], sU[2][12][13];
-  __shared__ double st[12], sR[12];
-  const int t = threadIdx.x;
-  const bool ent = t < 144, act = t < 156;
-  const int ei = ent ? t / 12 : (act ? t - 144 : 0), ej = ent ? t - 12 * (t / 12) : 12;
+  __shared__ double st[12], sR[12], sD[12];
+  const int t = threadIdx.x, w = t >> 5, lane = t & 31;
+  const bool fac = t < 96;               // else: couplings and L^-1
+  const int q = fac ? t : t - 96;        // entry (ei, ej) of a lower triangle; 78..89: rhs
+  int ei = 0;
+  while ((ei + 1) * (ei + 2) / 2 <= q) ++ei;
+  const int ej = q - ei * (ei + 1) / 2;
+  const bool ent = q < 78, rhs = fac && q >= 78 && q < 90;
+  const int ri = q - 78;                 // row of the right-hand side
   for (int l = 0; l < a.nlev; ++l) {
     const int h = 1 << l, hh = h >> 1;
     for (int it = a.lv_off[l] + blockIdx.x; it < a.lv_off[l + 1]; it += gridDim.x) {
@@ -137,99 +145,101 @@ __global__ void __launch_bounds__(TNT) k_tri_solve(TriArgs a) {
         cl = a.fl[k - hh] == 3;
         cr = k + hh < end && a.fl[k + hh] == 3;
       }
-      double v = 0.0, ul = 0.0, ur = 0.0;
-      if (ent) {
-        const double* Hd = a.Hrow + (size_t)base * 144;
-        v = 0.5 * (Hd[t] + Hd[12 * ej + ei]);
-        if (l == 0) {
-          if (cl) ul = a.Hrow[(size_t)cl * 144 + t];
-          if (cr) ur = a.Hrow[(size_t)cr * 144 + t];
-        } else {
-          if (cl) {
-            const double* Wm = a.W + (size_t)288 * (k - hh);
-            ul = -tri_dot_t(Wm + 144, ei, Wm + ej, 12, 0.0);
+      double v = 0.0, u[3] = {0.0, 0.0, 0.0};
+      if (fac) {
+        // the Schur complement: the bodies eliminated next to this one at the earlier levels
+        if (ent || rhs) {
+          const double* Hd = a.Hrow + (size_t)base * 144;
+          v = ent ? 0.5 * (Hd[12 * ei + ej] + Hd[12 * ej + ei]) : a.b[12 * k + ri];
+          const int i = ent ? ei : ri;
+          double accl = 0.0, accr = 0.0;
+          for (int m = 0; m < l; ++m) {
+            const int kl = k - (1 << m), kr = k + (1 << m);
+            if (a.fl[kl] & 2) {
+              const double* Wr = a.W + (size_t)288 * kl + 144;
+              accl = tri_dot_t(Wr, i, ent ? Wr + ej : a.y + 12 * kl, ent ? 12 : 1, accl);
+            }
+            if (kr < end && (a.fl[kr] & 1)) {
+              const double* Wl = a.W + (size_t)288 * kr;
+              accr = tri_dot_t(Wl, i, ent ? Wl + ej : a.y + 12 * kr, ent ? 12 : 1, accr);
+            }
           }
-          if (cr) {
-            const double* Wm = a.W + (size_t)288 * (k + hh);
-            ur = -tri_dot_t(Wm, ei, Wm + 144 + ej, 12, 0.0);
+          v -= accl + accr;
+        }
+      } else {
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+          const int e = q + 96 * j, side = e / 144, x = e - 144 * side;
+          const int c = side ? cr : cl;
+          if (!c) continue;
+          if (l == 0) {
+            u[j] = a.Hrow[(size_t)c * 144 + x];
+          } else {
+            const double* Wm = a.W + (size_t)288 * (side ? k + hh : k - hh);
+            u[j] = -tri_dot_t(Wm + (side ? 0 : 144), x / 12, Wm + (side ? 144 : 0) + x % 12, 12, 0.0);
           }
         }
-      } else if (act) {
-        v = a.b[12 * k + ei];
-      }
-      // the Schur complement: the bodies eliminated next to this one at the earlier levels
-      if (act) {
-        double accl = 0.0, accr = 0.0;
-        for (int m = 0; m < l; ++m) {
-          const int kl = k - (1 << m), kr = k + (1 << m);
-          if (a.fl[kl] & 2) {
-            const double* Wr = a.W + (size_t)288 * kl + 144;
-            accl = tri_dot_t(Wr, ei, ent ? Wr + ej : a.y + 12 * kl, ent ? 12 : 1, accl);
-          }
-          if (kr < end && (a.fl[kr] & 1)) {
-            const double* Wl = a.W + (size_t)288 * kr;
-            accr = tri_dot_t(Wl, ei, ent ? Wl + ej : a.y + 12 * kr, ent ? 12 : 1, accr);
-          }
-        }
-        v -= accl + accr;
       }
       __syncthreads();  // the previous body's shared blocks are no longer read
-      if (ent) {
-        sA[ei][ej] = v;
-        sT[ei][ej] = ei == ej ? 1.0 : 0.0;
-        sU[0][ei][ej] = ul;
-        sU[1][ei][ej] = ur;
-        if (t == 0) tri_pivot(v, &sR[0], &sL[0][0], a.status);
-      } else if (act) {
-        st[ei] = v;
+      if (fac) {
+        if (ent && ej == 0) sA[ei][0] = v;
+        if (rhs) st[ri] = v;
+        if (t == 0) tri_pivot(v, &sR[0], &sD[0], a.status);
+      } else {
+        if (ent) sT[ei][ej] = ei == ej ? 1.0 : 0.0;
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+          const int e = q + 96 * j, side = e / 144, x = e - 144 * side;
+          sU[side][x / 12][x % 12] = u[j];
+        }
+        v = ei == ej ? 1.0 : 0.0;  // this thread's entry of T
       }
       __syncthreads();
-      // S = L L^T column by column (threads of columns >= c); row c - 1 of L^-1 beside it
-      // (threads of columns <= c - 1). T holds I minus the finished rows' contributions.
       for (int c = 0; c <= 12; ++c) {
-        if (ent && c < 12 && ej >= c && ei >= ej) {
-          const double r = sR[c];
-          if (ej == c) {
-            if (ei > c) sL[ei][c] = sA[ei][c] * r;
-          } else {
-            const double w = sA[ei][ej] - (sA[ei][c] * r) * (sA[ej][c] * r);
-            sA[ei][ej] = w;
-            if (ei == ej && ej == c + 1) tri_pivot(w, &sR[c + 1], &sL[c + 1][c + 1], a.status);
+        if (ent && fac) {
+          if (c < 12 && ej >= c) {
+            if (ej == c) {
+              if (ei > c) sL[ei][c] = v * sR[c];
+            } else {
+              v -= (sA[ei][c] * sD[c]) * sA[ej][c];
+              if (ej == c + 1) sA[ei][ej] = v;
+              if (ei == c + 1 && ej == c + 1) tri_pivot(v, &sR[c + 1], &sD[c + 1], a.status);
+            }
           }
-        }
-        if (ent && c >= 1 && ej <= c - 1 && ei >= c - 1) {
+        } else if (ent && c >= 1 && ej < c && ei >= c - 1) {
           const int rw = c - 1;
           const double li = sT[rw][ej] * sR[rw];
-          if (ei == rw) sLi[rw][ej] = li;
-          else sT[ei][ej] -= sL[ei][rw] * li;
+          if (ei == rw) {
+            sLi[rw][ej] = li;
+            a.Li[(size_t)144 * k + 12 * rw + ej] = li;
+          } else {
+            v -= sL[ei][rw] * li;
+            if (ei == c) sT[ei][ej] = v;
+          }
         }
         __syncthreads();
       }
-      // y = L^-1 rhs, W = L^-1 U for both couplings (L^-1 lower triangular)
-      if (ent) {
-        a.Li[(size_t)144 * k + t] = ej <= ei ? sLi[ei][ej] : 0.0;
-        double wl = 0.0, wr = 0.0;
-        if (cl || cr)
-          for (int m = 0; m <= ei; ++m) {
-            const double li = sLi[ei][m];
-            wl += li * sU[0][m][ej];
-            wr += li * sU[1][m][ej];
-          }
-        if (cl) a.W[(size_t)288 * k + t] = wl;
-        if (cr) a.W[(size_t)288 * k + 144 + t] = wr;
-        if (t == 0) a.fl[k] = (cl ? 1 : 0) | (cr ? 2 : 0);
-      } else if (act) {
-        double w = 0.0;
-        for (int m = 0; m <= ei; ++m) w += sLi[ei][m] * st[m];
-        a.y[12 * k + ei] = w;
+      // y = L^-1 rhs, W = L^-1 U for both couplings (L^-1 lower triangular): rows w and 11 - w
+      if (lane < 25 && (lane == 24 || (lane < 12 ? cl : cr))) {
+        const int side = lane / 12, col = lane - 12 * side;  // lane 24: the right-hand side
+#pragma unroll
+        for (int z = 0; z < 2; ++z) {
+          const int row = z ? 11 - w : w;
+          double s = 0.0;
+          for (int m = 0; m <= row; ++m) s += sLi[row][m] * (lane == 24 ? st[m] : sU[side][m][col]);
+          if (lane == 24) a.y[12 * k + row] = s;
+          else a.W[(size_t)288 * k + 144 * side + 12 * row + col] = s;
+        }
       }
+      if (fac && ent && ei > ej) a.Li[(size_t)144 * k + 12 * ej + ei] = 0.0;
+      if (t == 0) a.fl[k] = (cl ? 1 : 0) | (cr ? 2 : 0);
     }
     grid.sync();
   }
   // back substitution, one warp per body: lanes 0..11 the rows' lower coupling, lanes
   // 16..27 the upper one, then x = L^-T v with the even terms on the low half, the odd ones
   // on the high half. Bodies of scenes that take no step get x = 0, dq = -0.
-  const int w = t >> 5, lane = t & 31, row = lane & 15, side = lane >> 4;
+  const int row = lane & 15, side = lane >> 4;
   const bool rl = row < 12;
   for (int l = a.nlev - 1; l >= 0; --l) {
     const int h = 1 << l;
