@@ -236,10 +236,10 @@ static __device__ __noinline__ void psd_project9(double (&S)[9][9]) { psd_projec
 // two. Each column's norm^2 = 1 + e with |e| ~ 1e-7 is normalised by the Taylor series
 // (1 + e)^(-1/2) = 1 - e/2 + 3e^2/8 - 5e^3/16 (remainder < 35 e^4 / 128). Returns false
 // (Q untouched) for a zero, non-finite or out-of-FP32-range matrix, or a column whose
-// norm is not within 1e-5 of 1; the caller then starts from the identity.
+// norm is not within 1e-5 of 1; the caller then starts from the identity. v: the FP32 estimate.
 template <int N>
-DEV bool jacobi_f32_start(const double (&S)[N][N], double (&Q)[N][N]) {
-  float a[N][N], v[N][N];
+DEV bool jacobi_f32_start(const double (&S)[N][N], double (&Q)[N][N], float (&v)[N][N]) {
+  float a[N][N];
   float mx = 0.f;
 #pragma unroll
   for (int i = 0; i < N; ++i)
@@ -342,14 +342,24 @@ DEV bool jacobi_f32_start(const double (&S)[N][N], double (&Q)[N][N]) {
 // a_pq = 0), and only the entries of one triangle. Where h^2 + a_pq^2 is below the
 // normal range the rotation takes t = a_pq / (|h| + r) by division instead. The
 // projection V max(L, 0) V^T is formed on the upper triangle and mirrored.
-template <int N>
+//
+// FIRST: the sweeps also end where a first-order correction does the rest. With off-diagonals E
+// left, the projection in this basis is max(L, 0) + E o K, K_ij = (max(l_i, 0) - max(l_j, 0)) /
+// (l_i - l_j) (1 for two positive eigenvalues, 0 for two negative ones), up to E^2 over the
+// smaller eigenvalues; the test keeps that below 1e-17 of the norm. After one sweep E is about
+// 1e-14 of the norm, so FP32 has the correction to 1e-20 of it, with the FP32 eigenvectors, and the
+// second FP64 sweep (ten rotations of a 5x5, a third of the projection) is not needed.
+template <int N, bool FIRST = false>
 DEV bool psd_project_small(double (&S)[N][N]) {
   double A[N][N], V[N][N];
+  float vf[N][N];
+  bool started = false, first = false;
 #pragma unroll
   for (int i = 0; i < N; ++i)
 #pragma unroll
     for (int j = 0; j < N; ++j) V[i][j] = (i == j) ? 1.0 : 0.0;
-  if (jacobi_f32_start<N>(S, V)) {
+  if (jacobi_f32_start<N>(S, V, vf)) {
+    started = true;
 #pragma unroll
     for (int q = 0; q < N; ++q) {
       double t[N];
@@ -383,6 +393,18 @@ DEV bool psd_project_small(double (&S)[N][N]) {
       for (int j = i + 1; j < N; ++j) off += A[i][j] * A[i][j];
     }
     if (off == 0.0 || 2 * off <= 1e-32 * (dg + 2 * off)) break;
+    if (FIRST && started && off <= 1e-22 * dg) {
+      double lo = fabs(A[0][0]), hi = lo;
+#pragma unroll
+      for (int i = 1; i < N; ++i) {
+        lo = fmin(lo, fabs(A[i][i]));
+        hi = fmax(hi, fabs(A[i][i]));
+      }
+      if (off <= 1e-17 * lo * hi) {
+        first = true;
+        break;
+      }
+    }
 #pragma unroll
     for (int p = 0; p < N - 1; ++p)
 #pragma unroll
@@ -438,13 +460,46 @@ DEV bool psd_project_small(double (&S)[N][N]) {
     neg |= lam[i] < 0.0;
   }
   if (!neg) return false;
+  float cor[N][N];  // FIRST: vf (E o K) vf^T
+  if (FIRST && first) {
+    float ek[N][N], lf[N];
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      lf[i] = __double2float_rn(lam[i]);
+      ek[i][i] = 0.f;
+    }
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+#pragma unroll
+      for (int j = i + 1; j < N; ++j) {
+        const float hi = fmaxf(lf[i], lf[j]), lo = fminf(lf[i], lf[j]);
+        const float k = lo >= 0.f ? 1.f : (hi > 0.f ? __fdividef(hi, hi - lo) : 0.f);
+        ek[i][j] = ek[j][i] = __double2float_rn(A[i][j]) * k;
+      }
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      float t[N];
+#pragma unroll
+      for (int l = 0; l < N; ++l) {
+        t[l] = 0.f;
+#pragma unroll
+        for (int k = 0; k < N; ++k) t[l] += vf[i][k] * ek[k][l];
+      }
+#pragma unroll
+      for (int j = i; j < N; ++j) {
+        cor[i][j] = 0.f;
+#pragma unroll
+        for (int l = 0; l < N; ++l) cor[i][j] += t[l] * vf[j][l];
+      }
+    }
+  }
 #pragma unroll
   for (int k = 0; k < N; ++k) lam[k] = lam[k] > 0.0 ? lam[k] : 0.0;
 #pragma unroll
   for (int i = 0; i < N; ++i)
 #pragma unroll
     for (int j = i; j < N; ++j) {
-      double acc = 0;
+      double acc = FIRST && first ? (double)cor[i][j] : 0.0;
 #pragma unroll
       for (int k = 0; k < N; ++k) acc += (V[i][k] * lam[k]) * V[j][k];
       S[i][j] = acc;
@@ -806,7 +861,7 @@ DEV double vertex_entry(int i, int j, int r, int s, F&& S) {
 // orthonormalised against c; at most 3 + m <= 5 columns), where
 //   S_r = [[2 b' |c|^2 I + 4 b'' |c|^2 w w^T, 0], [0, 0]] - b' Phi_r G^-1 Phi_r^T.
 // S_r is projected (analytically for m = 0) and written back in the 9-dim Q (x) I basis.
-template <int M, class Out>
+template <int M, bool FIRST, class Out>
 DEV void reduced_project(const Stencil& st, d3 w, const d3* W, const double (&Gi)[2][2], double B1, double B2,
                          bool psd, Out& S9) {
   constexpr int N = 3 + M;
@@ -901,7 +956,7 @@ DEV void reduced_project(const Stencil& st, d3 w, const d3* W, const double (&Gi
           for (int j = 0; j < 3; ++j) Sr[i][j] = lnp * (i == j ? 1.0 : 0.0) + (lwp - lnp) * whv[i] * whv[j];
       }
     } else {
-      psd_project_small<N>(Sr);
+      psd_project_small<N, FIRST>(Sr);
     }
   }
   // back to the 9-dim basis: column alpha of the reduced basis has Q-coordinates
@@ -935,6 +990,22 @@ DEV void reduced_project(const Stencil& st, d3 w, const d3* W, const double (&Gi
         for (int l2 = 0; l2 < M; ++l2) acc += aq[l][a] * Sr[3 + l][3 + l2] * aq[l2][b];
       be[a][b] = acc;
     }
+  }
+  if (FIRST && M > 0) {
+    // the same, the products of column (b, s) formed once for the rows
+#pragma unroll
+    for (int b = 0; b < 3; ++b)
+#pragma unroll
+      for (int s = 0; s < 3; ++s) {
+        double f[3], h[3];  // S9[3a+r][3b+s] = cq_a f_r + w_r h_a
+#pragma unroll
+        for (int r = 0; r < 3; ++r) f[r] = cq[b] * (r <= s ? Sr[r][s] : Sr[s][r]) + whv[s] * al[b][r];
+#pragma unroll
+        for (int a = 0; a <= b; ++a) h[a] = cq[b] * al[a][s] + whv[s] * be[a][b];
+#pragma unroll
+        for (int p = 0; p <= 3 * b + s; ++p) s9_put(S9, p, 3 * b + s, cq[p / 3] * f[p % 3] + whv[p % 3] * h[p / 3]);
+      }
+    return;
   }
 #pragma unroll
   for (int p = 0; p < 9; ++p)
@@ -1203,7 +1274,8 @@ DEV void pair_gradient(const Stencil& st, d3 w, const MollData& md, d3 gu, d3 gv
 
 // Reduced 9x9 Hessian S of a pair. Returns the vertex-space gradient g[4] (3-vectors).
 // kind 0: point-triangle, 1: edge-edge (mollified when the edges are near parallel).
-template <class Out>
+// FIRST: the projection ends with the first-order correction (psd_project_small).
+template <bool FIRST, class Out>
 DEV void pair_reduced(int kind, int ty, const d3* X, double d, const BarrierP& bp, double eps_x_param, bool psd,
                       Out& S, d3* g) {
   Stencil st;
@@ -1212,9 +1284,9 @@ DEV void pair_reduced(int kind, int ty, const d3* X, double d, const BarrierP& b
   MollData md;
   const bool mollified = pair_setup(kind, ty, X, d, bp, eps_x_param, st, w, W, Gi, md, gu, gv);
   if (!mollified) {
-    if (st.m == 0) reduced_project<0>(st, w, W, Gi, md.B1, md.B2, psd, S);
-    else if (st.m == 1) reduced_project<1>(st, w, W, Gi, md.B1, md.B2, psd, S);
-    else reduced_project<2>(st, w, W, Gi, md.B1, md.B2, psd, S);
+    if (st.m == 0) reduced_project<0, FIRST>(st, w, W, Gi, md.B1, md.B2, psd, S);
+    else if (st.m == 1) reduced_project<1, FIRST>(st, w, W, Gi, md.B1, md.B2, psd, S);
+    else reduced_project<2, FIRST>(st, w, W, Gi, md.B1, md.B2, psd, S);
 #pragma unroll
     for (int i = 0; i < 4; ++i) g[i] = fscl(md.B1 * 2 * st.c[i], w);
     return;

@@ -131,8 +131,12 @@ __device__ __forceinline__ int pair_class(const Geo& g, const Params& P, int kin
 // barrier's reduced Hessian and gradient, the lagged friction frame and the friction
 // terms, written to the pair's record. Threads take pairs in stencil-class order (perm).
 // One warp a CTA: a warp's FP64 instruction takes 64 cycles of its sub-partition (76 with all
-// four busy), so single warps spread over the SMs and end one by one.
+// four busy), so single warps spread over the SMs and end one by one. A warp's chain is what a
+// small set waits for: 164 us for a stack of ten, 147 us since the projection takes one
+// FP64 sweep (FIRST of psd_project_small); BIG: the pairs of scenes of BIG_SCENE bodies or more,
+// which keep two (see k_pair_moll).
 constexpr int HESS_T = 32;
+template <bool BIG>
 __global__ void __launch_bounds__(HESS_T) k_pair_hess(Geo g, Params P, int kind, int n, const int* tup,
                                                    const int8_t* tys, const int* perm, const int* n_moll, double* R,
                                                    double* lag) {
@@ -142,7 +146,7 @@ __global__ void __launch_bounds__(HESS_T) k_pair_hess(Geo g, Params P, int kind,
   if (p < 0) return;
   int vid[4], na, A, B;
   pair_vertices(g, kind, tup, p, vid, na, A, B);
-  if (!scene_on(g, A)) return;  // scene not iterating: its blocks are not used
+  if (!scene_on(g, A) || big_scene(g, A) != BIG) return;  // scene not iterating: its blocks are not used
   d3 X[4], X0[4];
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
@@ -170,7 +174,7 @@ __global__ void __launch_bounds__(HESS_T) k_pair_hess(Geo g, Params P, int kind,
     }
     lam = -barrier_b1(d, bp) * 2 * sqrt(d);
     S9Rec rec{R + REC_S * N + p, N};
-    pair_reduced(kind, ty, X, d, bp, P.eps_x, P.psd != 0, rec, gv);
+    pair_reduced<!BIG>(kind, ty, X, d, bp, P.eps_x, P.psd != 0, rec, gv);
     if (!(P.terms & TERM_BARRIER)) {
       for (int k = 0; k < 45; ++k) R[(REC_S + k) * N + p] = 0.0;
       for (int i = 0; i < 4; ++i) gv[i] = fd3(0, 0, 0);
@@ -271,7 +275,7 @@ __global__ void __launch_bounds__(32 * MOLL_W) k_pair_moll(Geo g, Params P, int 
         if (lane == 0) {
           S9Rec rec{R + REC_S * N + p, N};
           d3 gtmp[4];
-          pair_reduced(1, ty, X, d, bp, P.eps_x, P.psd != 0, rec, gtmp);
+          pair_reduced<false>(1, ty, X, d, bp, P.eps_x, P.psd != 0, rec, gtmp);
         }
       } else {
         bool neg = false;
@@ -2066,8 +2070,14 @@ void assemble(const Geo& g, const Params& P, PairSet& S, NewtonBufs& B, cudaStre
                                                                                   prec.p, S.ee_lag.p));
       CK(cudaEventRecord(B.ev_join, B.side));
     }
-    KLAUNCH(K_PAIR_TERMS, st, k_pair_hess<<<nblk(class_slots(n), HESS_T), HESS_T, 0, st>>>(
-                                  g, P, kind, n, tup, ty, perm.p, n_moll, prec.p, kind ? S.ee_lag.p : S.pt_lag.p));
+    double* lag = kind ? S.ee_lag.p : S.pt_lag.p;
+    const int nb_h = nblk(class_slots(n), HESS_T);
+    if (g.any_small)
+      KLAUNCH(K_PAIR_TERMS, st, k_pair_hess<false><<<nb_h, HESS_T, 0, st>>>(g, P, kind, n, tup, ty, perm.p, n_moll,
+                                                                            prec.p, lag));
+    if (g.any_big)
+      KLAUNCH(K_PAIR_TERMS, st, k_pair_hess<true><<<nb_h, HESS_T, 0, st>>>(g, P, kind, n, tup, ty, perm.p, n_moll,
+                                                                           prec.p, lag));
     if (kind) CK(cudaStreamWaitEvent(st, B.ev_join, 0));
     if (kind) launch_chain<1>(g, n, tup, S.ee_ov.p, S.ovI.p, prec.p, B.ee_c.p, st);
     else launch_chain<0>(g, n, tup, S.pt_ov.p, S.ovI.p, prec.p, B.pt_c.p, st);

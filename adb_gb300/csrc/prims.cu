@@ -100,9 +100,9 @@ __global__ void __launch_bounds__(HESS_BT) k_hess(HessArgs a) {
         s_moll[atomicAdd(&s_nm, 1)] = i;
       } else {
         S9Reg S;
-        if (m == 2) reduced_project<2>(st, w, W, Gi, md.B1, md.B2, a.psd != 0, S);
-        else if (m == 1) reduced_project<1>(st, w, W, Gi, md.B1, md.B2, a.psd != 0, S);
-        else reduced_project<0>(st, w, W, Gi, md.B1, md.B2, a.psd != 0, S);
+        if (m == 2) reduced_project<2, true>(st, w, W, Gi, md.B1, md.B2, a.psd != 0, S);
+        else if (m == 1) reduced_project<1, true>(st, w, W, Gi, md.B1, md.B2, a.psd != 0, S);
+        else reduced_project<0, true>(st, w, W, Gi, md.B1, md.B2, a.psd != 0, S);
         double* H = a.H + 144 * (size_t)i;
 #pragma unroll
         for (int e = 0; e < 144; ++e) {
@@ -139,9 +139,9 @@ __global__ void __launch_bounds__(HESS_BT) k_hess(HessArgs a) {
       smd[KIND ? warp : 0] = md;
       if (!moll) {  // compiled apart, the two tests could differ at the very edge
         double S[9][9];
-        if (st.m == 0) reduced_project<0>(st, w, W, Gi, md.B1, md.B2, a.psd != 0, S);
-        else if (st.m == 1) reduced_project<1>(st, w, W, Gi, md.B1, md.B2, a.psd != 0, S);
-        else reduced_project<2>(st, w, W, Gi, md.B1, md.B2, a.psd != 0, S);
+        if (st.m == 0) reduced_project<0, true>(st, w, W, Gi, md.B1, md.B2, a.psd != 0, S);
+        else if (st.m == 1) reduced_project<1, true>(st, w, W, Gi, md.B1, md.B2, a.psd != 0, S);
+        else reduced_project<2, true>(st, w, W, Gi, md.B1, md.B2, a.psd != 0, S);
         for (int e = 0; e < 81; ++e) w9.S[e / 9][e % 9] = S[e / 9][e % 9];
       }
     }
