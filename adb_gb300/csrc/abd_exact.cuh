@@ -152,16 +152,15 @@ HD double ll_dist(d3 a0, d3 a1, d3 b0, d3 b1) {
   double s = dot(sub(b0, a0), n);
   return XD(XM(s, s), sqn(n));
 }
+// The distance of a type: its vertices are selected first, so that a warp of mixed types runs
+// three formulas (two points, point and line, plane or two lines) instead of seven or nine.
+HD d3 vsel(bool c, d3 a, d3 b) { return mk(c ? a.x : b.x, c ? a.y : b.y, c ? a.z : b.z); }
 HD double pt_dist(d3 p, d3 t0, d3 t1, d3 t2, int ty) {
-  switch (ty) {
-    case P_T0: return pp_dist(p, t0);
-    case P_T1: return pp_dist(p, t1);
-    case P_T2: return pp_dist(p, t2);
-    case P_E0: return pl_dist(p, t0, t1);
-    case P_E1: return pl_dist(p, t1, t2);
-    case P_E2: return pl_dist(p, t2, t0);
-    default: return plane_dist(p, t0, t1, t2);
-  }
+  if ((unsigned)ty >= (unsigned)P_T) return plane_dist(p, t0, t1, t2);
+  const int k = ty < P_E0 ? ty : ty - P_E0;  // the nearest vertex, or the first of the nearest edge
+  const d3 q = vsel(k == 0, t0, vsel(k == 1, t1, t2));
+  if (ty < P_E0) return pp_dist(p, q);
+  return pl_dist(p, q, vsel(k == 0, t1, vsel(k == 1, t2, t0)));
 }
 
 HD int ee_parallel_type(d3 a0, d3 a1, d3 b0, d3 b1) {
@@ -220,17 +219,10 @@ HD int ee_type(d3 a0, d3 a1, d3 b0, d3 b1) {
 }
 
 HD double ee_dist(d3 a0, d3 a1, d3 b0, d3 b1, int ty) {
-  switch (ty) {
-    case EA0_EB0: return pp_dist(a0, b0);
-    case EA0_EB1: return pp_dist(a0, b1);
-    case EA1_EB0: return pp_dist(a1, b0);
-    case EA1_EB1: return pp_dist(a1, b1);
-    case EA_EB0: return pl_dist(b0, a0, a1);
-    case EA_EB1: return pl_dist(b1, a0, a1);
-    case EA0_EB: return pl_dist(a0, b0, b1);
-    case EA1_EB: return pl_dist(a1, b0, b1);
-    default: return ll_dist(a0, a1, b0, b1);
-  }
+  if ((unsigned)ty >= (unsigned)EA_EB) return ll_dist(a0, a1, b0, b1);
+  if (ty < EA_EB0) return pp_dist(vsel(ty & 2, a1, a0), vsel(ty & 1, b1, b0));
+  const bool ea = ty < EA0_EB, one = ty & 1;  // an end of b against a, or one of a against b
+  return pl_dist(vsel(ea, vsel(one, b1, b0), vsel(one, a1, a0)), vsel(ea, a0, b0), vsel(ea, a1, b1));
 }
 
 // ---------------------------------------------------------------------------------

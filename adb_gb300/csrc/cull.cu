@@ -1228,7 +1228,7 @@ __global__ void __launch_bounds__(NT, MODE == 0 ? (STEP <= 8 ? 4 : STEP <= 16 ? 
 }
 
 // 5a'. The FP64 test of every staged candidate, a thread each: its distance type, or -1. Bound by
-// FP64 issue (189 k candidates of the pile, of which 181 k are pairs: 115 us; 185 us while warps
+// FP64 issue (189 k candidates of the pile, of which 181 k are pairs: 90 us; 185 us while warps
 // held both kinds and ran both tests).
 __global__ void __launch_bounds__(128) k_narrow_exact(Geo g, Params P, const int* ovI, const int* ovJ, const int* cnt,
                                                       const int* off, const int* lst, StageOut so) {

@@ -1790,8 +1790,11 @@ __global__ void k_scene_chunks(Geo g, EnergyArgs a, const int* off, int* chunk_c
   chunk_cnt[s] = c > 0 ? (int)c : 1;
 }
 
-__global__ void __launch_bounds__(256) k_energy(Geo g, Params P, EnergyArgs a) {
-  __shared__ double sh[80];
+// A chunk's terms by a thread each, then summed as by 256 threads with two terms each (t, then
+// t + 256). Half as many threads with two terms took 48 us for a chain of 200, now 32 us (and 97, now
+// 72 us for 256 columns), with the distance formulas by selected vertices.
+__global__ void __launch_bounds__(ECHUNK, 2) k_energy(Geo g, Params P, EnergyArgs a) {
+  __shared__ double sh[80], upper[ECHUNK / 2];
   const int nchunk = a.chunk_off[a.ns];
   for (int c = blockIdx.x; c < nchunk; c += gridDim.x) {
     // scene of chunk c: last s with chunk_off[s] <= c
@@ -1819,8 +1822,8 @@ __global__ void __launch_bounds__(256) k_energy(Geo g, Params P, EnergyArgs a) {
     long long e0 = (long long)(c - a.chunk_off[s]) * ECHUNK;
     long long e1 = e0 + ECHUNK < total ? e0 + ECHUNK : total;
     double acc = 0.0;
-    for (long long e = e0 + threadIdx.x; e < e1; e += blockDim.x) {
-      long long i = e;
+    if (e0 + threadIdx.x < e1) {
+      long long i = e0 + threadIdx.x;
       int k = 0;
       while (i >= len[k]) {
         i -= len[k];
@@ -1828,10 +1831,20 @@ __global__ void __launch_bounds__(256) k_energy(Geo g, Params P, EnergyArgs a) {
       }
       acc += energy_term(g, P, a, k - 1, beg[k] + (int)i);
     }
-    double dummy = 0;
-    block_sum2(acc, dummy, sh);
-    if (threadIdx.x == 0) a.partial[c] = acc;
+    if (threadIdx.x >= ECHUNK / 2) upper[threadIdx.x - ECHUNK / 2] = acc;
     __syncthreads();
+    if (threadIdx.x < ECHUNK / 2) {
+      acc += upper[threadIdx.x];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+      if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = acc;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      double t = 0.0;
+      for (int w = 0; w < ECHUNK / 64; ++w) t += sh[w];
+      a.partial[c] = t;
+    }
   }
 }
 
@@ -2376,7 +2389,7 @@ void energy(const Geo& g, const Params& P, double alpha, PairSet& Snew, PairSet&
   const int G = 608;
   prof_work(K_ENERGY, (double)a.npt + a.nee + a.lpt + a.lee,
             136.0 * ((double)a.npt + a.nee + a.lpt + a.lee) + 96.0 * g.nb);
-  KLAUNCH(K_ENERGY, s, k_energy<<<G, 256, 0, s>>>(g, P, a));
+  KLAUNCH(K_ENERGY, s, k_energy<<<G, ECHUNK, 0, s>>>(g, P, a));
   KLAUNCH(K_ENERGY, s, k_scene_energy<<<nblk(32ll * ns, 128), 128, 0, s>>>(ns, B.e_chunk_off.p, B.red.p, B.e_out.p));
   CK(cudaMemcpyAsync(out, B.e_out.p, ns * sizeof(double), cudaMemcpyDeviceToHost, s));
   CK(cudaStreamSynchronize(s));
