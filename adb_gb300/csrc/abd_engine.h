@@ -201,7 +201,7 @@ void cull(const Geo& g, const Params& P, int vtn, double alpha, CullScratch& cs,
 
 // Float boxes of the vertices, edges and faces, rounded outward, of X or of the trajectory from
 // Xq to X (cs.vbox / ebox / fbox), and the float positions of the vertices at Xq and X (cs.vend).
-void prim_boxes(const Geo& g, bool traj, bool clusters, CullScratch& cs, cudaStream_t s);
+void prim_boxes(const Geo& g, bool traj, CullScratch& cs, cudaStream_t s);
 void traj_floats(const Geo& g, CullScratch& cs, cudaStream_t s);
 
 // Line-search cull at q + alpha dq (per-scene steps of g) that reuses the overlaps and the

@@ -30,6 +30,35 @@ namespace {
 
 __device__ __forceinline__ d3 ldX(const double* X, int nv, int v) { return mk(X[v], X[nv + v], X[2 * nv + v]); }
 
+struct fbox6 {
+  float lo[3], hi[3];
+};
+__device__ __forceinline__ void put_fbox(float* dst, const box& b) {
+  dst[0] = __double2float_rd(b.lo.x); dst[1] = __double2float_rd(b.lo.y); dst[2] = __double2float_rd(b.lo.z);
+  dst[3] = __double2float_ru(b.hi.x); dst[4] = __double2float_ru(b.hi.y); dst[5] = __double2float_ru(b.hi.z);
+}
+// Clusters: the unions of the boxes of 32 primitives in a row, which the binning tests before the
+// primitives (BinClusters; in memory order, so a cluster can hold the ends of two bodies). A
+// box without an order (NaN) adds nothing: it hits no box either.
+struct BinClusters {
+  float *v, *e, *f;  // null: not wanted
+};
+__device__ __forceinline__ int ford(float x) {  // order-preserving, its own inverse on the bits
+  const int i = __float_as_int(x);
+  return i >= 0 ? i : i ^ 0x7fffffff;
+}
+__device__ __forceinline__ void put_cluster(float* cl, int t, const float (&o)[6]) {  // whole warps
+  float mine = 0.f;
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int c = 0; c < 6; ++c) {
+    const int r = c < 3 ? __reduce_min_sync(0xffffffffu, ford(fminf(o[c], INFINITY)))
+                        : __reduce_max_sync(0xffffffffu, ford(fmaxf(o[c], -INFINITY)));
+    if (lane == c) mine = __int_as_float(r >= 0 ? r : r ^ 0x7fffffff);
+  }
+  if (lane < 6) cl[6 * (size_t)(t >> 5) + lane] = mine;
+}
+
 // ---------------------------------------------------------------------------------
 // 1. projection: which 0 -> X0 at q0; 1 -> X and Xq at q; 2 -> X at q + alpha dq;
 //    3 -> Xq at q only
@@ -43,22 +72,33 @@ __global__ void k_trial_state(Geo g, double alpha) {
   g.qa[i] = XA(g.q[i], XM(g.dq[i], a));
 }
 
-__global__ void k_project(Geo g, int which, double alpha) {
-  int v = blockIdx.x * blockDim.x + threadIdx.x;
-  if (v >= g.nv) return;
-  int b = g.vbody[v];
-  (void)alpha;
-  const double* qq = (which == 0) ? g.q0 + 12 * b : ((which == 2) ? g.qa + 12 * b : g.q + 12 * b);
-  d3 x = project(qq, g.rest[3 * v], g.rest[3 * v + 1], g.rest[3 * v + 2]);
-  double* dst = (which == 0) ? g.X0 : ((which == 3) ? g.Xq : g.X);
-  dst[v] = x.x;
-  dst[g.nv + v] = x.y;
-  dst[2 * g.nv + v] = x.z;
-  if (which == 1) {
-    g.Xq[v] = x.x;
-    g.Xq[g.nv + v] = x.y;
-    g.Xq[2 * g.nv + v] = x.z;
+// With vb the float boxes of the vertices (which 1, 2: at X; 3: of the path from Xq to X, already
+// there) and, with cl, of their clusters are written too: a kernel of their own read the positions
+// again (pile 26 + 16 us, now 33 us).
+__global__ void __launch_bounds__(256) k_project(Geo g, int which, float* vb, float* cl) {
+  const int v = blockIdx.x * blockDim.x + threadIdx.x;
+  if ((v & ~31) >= g.nv) return;
+  float o[6] = {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY};
+  if (v < g.nv) {
+    int b = g.vbody[v];
+    const double* qq = (which == 0) ? g.q0 + 12 * b : ((which == 2) ? g.qa + 12 * b : g.q + 12 * b);
+    d3 x = project(qq, g.rest[3 * v], g.rest[3 * v + 1], g.rest[3 * v + 2]);
+    double* dst = (which == 0) ? g.X0 : ((which == 3) ? g.Xq : g.X);
+    dst[v] = x.x;
+    dst[g.nv + v] = x.y;
+    dst[2 * g.nv + v] = x.z;
+    if (which == 1) {
+      g.Xq[v] = x.x;
+      g.Xq[g.nv + v] = x.y;
+      g.Xq[2 * g.nv + v] = x.z;
+    }
+    if (vb) {
+      put_fbox(o, which == 3 ? box2(ldX(g.X, g.nv, v), x) : box{x, x});
+#pragma unroll
+      for (int c = 0; c < 6; ++c) vb[6 * (size_t)v + c] = o[c];
+    }
   }
+  if (cl) put_cluster(cl, v, o);
 }
 
 // 2. body boxes
@@ -184,51 +224,17 @@ __global__ void k_ov_lower(int nnz, const int* row_ptr, const int* col, const in
 // ---------------------------------------------------------------------------------
 // Float prefilter boxes of every primitive (outward rounded). Trajectory mode spans the
 // positions at q (Xq) and at the target (X).
-struct fbox6 {
-  float lo[3], hi[3];
-};
-__device__ __forceinline__ void put_fbox(float* dst, const box& b) {
-  dst[0] = __double2float_rd(b.lo.x); dst[1] = __double2float_rd(b.lo.y); dst[2] = __double2float_rd(b.lo.z);
-  dst[3] = __double2float_ru(b.hi.x); dst[4] = __double2float_ru(b.hi.y); dst[5] = __double2float_ru(b.hi.z);
-}
 // Float boxes of the primitives (outward rounded). Vertices first, from their FP64
 // positions (at X, or the trajectory from Xq to X); edges and faces are then the float
 // unions of their vertices' boxes: rounding down (up) commutes with min (max), so
 // rd(min(a, b)) = min(rd a, rd b) and the result equals rounding the FP64 box, without
 // any FP64 min/max.
-//
-// Clusters: the unions of the boxes of 32 primitives in a row, which the binning tests before the
-// primitives (BinClusters; in memory order, so a cluster can hold the ends of two bodies). A
-// box without an order (NaN) adds nothing: it hits no box either.
-struct BinClusters {
-  float *v, *e, *f;  // null: not wanted
-};
-__device__ __forceinline__ int ford(float x) {  // order-preserving, its own inverse on the bits
-  const int i = __float_as_int(x);
-  return i >= 0 ? i : i ^ 0x7fffffff;
-}
-__device__ __forceinline__ void put_cluster(float* cl, int t, const float (&o)[6]) {  // whole warps
-  float mine = 0.f;
-  const int lane = threadIdx.x & 31;
-#pragma unroll
-  for (int c = 0; c < 6; ++c) {
-    const int r = c < 3 ? __reduce_min_sync(0xffffffffu, ford(fminf(o[c], INFINITY)))
-                        : __reduce_max_sync(0xffffffffu, ford(fmaxf(o[c], -INFINITY)));
-    if (lane == c) mine = __int_as_float(r >= 0 ? r : r ^ 0x7fffffff);
-  }
-  if (lane < 6) cl[6 * (size_t)(t >> 5) + lane] = mine;
-}
-__global__ void k_vert_boxes(Geo g, int traj, float* vb, float* cl) {
+__global__ void k_vert_boxes(Geo g, int traj, float* vb) {
   int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if ((t & ~31) >= g.nv) return;
-  float o[6] = {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY};
-  if (t < g.nv) {
-    d3 p = ldX(g.X, g.nv, t);
-    put_fbox(o, traj ? box2(p, ldX(g.Xq, g.nv, t)) : box{p, p});
-#pragma unroll
-    for (int c = 0; c < 6; ++c) vb[6 * t + c] = o[c];
-  }
-  if (cl) put_cluster(cl, t, o);
+  if (t >= g.nv) return;
+  d3 p = ldX(g.X, g.nv, t);
+  box b = traj ? box2(p, ldX(g.Xq, g.nv, t)) : box{p, p};
+  put_fbox(vb + 6 * t, b);
 }
 // Float positions (to nearest) of every vertex at q and at the target, for the FP32
 // certificates of the trajectories.
@@ -1555,15 +1561,20 @@ double key_to_double(unsigned long long k) {
   return d;
 }
 
+// launch_project, with the vertices' float boxes (and their clusters') when vb (and cl) are given
+static void project_boxes(const Geo& g, int which, double alpha, float* vb, float* cl, cudaStream_t s) {
+  if (which == 2 && g.nb > 0) KLAUNCH(K_PROJECT, s, k_trial_state<<<nblk(12ll * g.nb, 256), 256, 0, s>>>(g, alpha));
+  if (g.nv == 0) return;
+  KLAUNCH(K_PROJECT, s, k_project<<<nblk(g.nv, 256), 256, 0, s>>>(g, which, vb, cl));
+  prof_work(K_PROJECT, g.nv, 48.0 * g.nv);  // rest read + world write per vertex
+}
+
 }  // namespace
 
 int narrow_step_of(int mode, int variant) { return kNarrowStep[mode == 2 ? 1 : 0][variant]; }
 
 void launch_project(const Geo& g, int which, double alpha, cudaStream_t s) {
-  if (which == 2 && g.nb > 0) KLAUNCH(K_PROJECT, s, k_trial_state<<<nblk(12ll * g.nb, 256), 256, 0, s>>>(g, alpha));
-  if (g.nv == 0) return;
-  KLAUNCH(K_PROJECT, s, k_project<<<nblk(g.nv, 256), 256, 0, s>>>(g, which, alpha));
-  prof_work(K_PROJECT, g.nv, 48.0 * g.nv);  // rest read + world write per vertex
+  project_boxes(g, which, alpha, nullptr, nullptr, s);
 }
 
 static BinClusters bin_clusters(const Geo& g, CullScratch& cs) {
@@ -1572,19 +1583,23 @@ static BinClusters bin_clusters(const Geo& g, CullScratch& cs) {
   return {cs.cbox.p, cs.cbox.p + 6 * nv, cs.cbox.p + 6 * (nv + ne)};
 }
 
-// Float boxes of the primitives, and of their clusters when the lists are binned from them.
-void prim_boxes(const Geo& g, bool traj, bool clusters, CullScratch& cs, cudaStream_t s) {
+// Float boxes of the edges and faces from those of the vertices (in cs.vbox), and of their clusters
+// when the lists are binned from them.
+static void edge_face_boxes(const Geo& g, bool clusters, CullScratch& cs, cudaStream_t s) {
   BinClusters cl{};
   if (clusters) cl = bin_clusters(g, cs);
-  cs.vbox.ensure(6 * (size_t)g.nv + 6);
   cs.ebox.ensure(6 * (size_t)g.ne + 6);
   cs.fbox.ensure(6 * (size_t)g.nf + 6);
-  if (g.nv > 0)
-    KLAUNCH(K_PRIM_BOXES, s, k_vert_boxes<<<nblk(g.nv, 256), 256, 0, s>>>(g, traj ? 1 : 0, cs.vbox.p, cl.v));
   if (g.ne + g.nf > 0) {
     KLAUNCH(K_PRIM_BOXES, s, k_prim_boxes<<<nblk((long long)g.ne + g.nf + 31, 256), 256, 0, s>>>(
                                  g, cs.vbox.p, cs.ebox.p, cs.fbox.p, cl));
   }
+}
+
+void prim_boxes(const Geo& g, bool traj, CullScratch& cs, cudaStream_t s) {
+  cs.vbox.ensure(6 * (size_t)g.nv + 6);
+  if (g.nv > 0) KLAUNCH(K_PRIM_BOXES, s, k_vert_boxes<<<nblk(g.nv, 256), 256, 0, s>>>(g, traj ? 1 : 0, cs.vbox.p));
+  edge_face_boxes(g, false, cs, s);
 }
 
 void traj_floats(const Geo& g, CullScratch& cs, cudaStream_t s) {
@@ -1658,10 +1673,13 @@ void cull(const Geo& g_in, const Params& P, int vtn, double alpha, CullScratch& 
     CK(cudaMallocHost(&cs.h_ll, 8 * sizeof(long long)));
   }
   // 1. projection
-  if (vtn == 1) launch_project(g, 1, 0.0, s);
-  else {
-    launch_project(g, 2, alpha, s);
-    if (traj) launch_project(g, 3, 0.0, s);
+  cs.vbox.ensure(6 * (size_t)g.nv + 6);
+  float* vb_cl = bin_clusters(g, cs).v;
+  if (vtn == 1) {
+    project_boxes(g, 1, 0.0, cs.vbox.p, vb_cl, s);
+  } else {
+    project_boxes(g, 2, alpha, traj ? nullptr : cs.vbox.p, traj ? nullptr : vb_cl, s);
+    if (traj) project_boxes(g, 3, 0.0, cs.vbox.p, vb_cl, s);
   }
   // 2-3. body boxes and overlaps
   cs.bbox.ensure(6 * (size_t)nb);
@@ -1703,7 +1721,7 @@ void cull(const Geo& g_in, const Params& P, int vtn, double alpha, CullScratch& 
   }
   // 4. primitive boxes and binning
   const float ds_f = float_round_up(P.d_sqrt);
-  prim_boxes(g, traj, true, cs, s);
+  edge_face_boxes(g, true, cs, s);
   int nlst = 0;
   if (nov > 0) {
     cs.bin_cnt.ensure(6 * (size_t)nov + 6);
@@ -1806,7 +1824,8 @@ void cull_trial(const Geo& g_in, const Params& P, double alpha, CullScratch& cs,
                 cudaStream_t s) {
   Geo g = g_in;
   const int nb = g.nb, nov = H.nov, nnz = H.nnz;
-  launch_project(g, 2, alpha, s);
+  cs.vbox.ensure(6 * (size_t)g.nv + 6);
+  project_boxes(g, 2, alpha, cs.vbox.p, nullptr, s);
   vg_count(g, P, cs, s);
   PairSet& S = out;
   S.row_ptr.ensure(nb + 1);
@@ -1825,7 +1844,7 @@ void cull_trial(const Geo& g_in, const Params& P, double alpha, CullScratch& cs,
   }
   S.nnz = nnz;
   S.nov = nov;
-  prim_boxes(g, false, false, cs, s);
+  edge_face_boxes(g, false, cs, s);
   int npt = 0, nee = 0, nvg = 0;
   if (nov > 0) {
     narrow_pairs(g, P, float_round_up(P.d_sqrt), nov, S.ovI.p, S.ovJ.p, cs, S, npt, nee, s);
