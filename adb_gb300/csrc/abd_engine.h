@@ -113,7 +113,7 @@ struct CullScratch {
   DBuf<int> cnt_all, cnt_up, up_ptr, rowid;
   DBuf<double> ovcull;
   DBuf<float> ovcull_f;
-  DBuf<float> vbox, ebox, fbox, cbox, tight;  // boxes of vertices, edges, faces; of 32 in a row; of bodies
+  DBuf<float> vbox, ebox, fbox, cbox;  // boxes of vertices, edges, faces; of 32 in a row and of bodies
   DBuf<float> vend;                     // float positions of each vertex at q and at the target
   DBuf<int> order, order_cnt;           // narrow-phase processing order of the overlaps
   DBuf<int> bin_cnt, bin_off, lst;

@@ -42,6 +42,7 @@ __device__ __forceinline__ void put_fbox(float* dst, const box& b) {
 // box without an order (NaN) adds nothing: it hits no box either.
 struct BinClusters {
   float *v, *e, *f;  // null: not wanted
+  float* tight;      // the boxes of the bodies (k_bin_caps)
 };
 __device__ __forceinline__ int ford(float x) {  // order-preserving, its own inverse on the bits
   const int i = __float_as_int(x);
@@ -1579,8 +1580,8 @@ void launch_project(const Geo& g, int which, double alpha, cudaStream_t s) {
 
 static BinClusters bin_clusters(const Geo& g, CullScratch& cs) {
   const size_t nv = (g.nv + 31) / 32, ne = (g.ne + 31) / 32, nf = (g.nf + 31) / 32;
-  cs.cbox.ensure(6 * (nv + ne + nf) + 6);
-  return {cs.cbox.p, cs.cbox.p + 6 * nv, cs.cbox.p + 6 * (nv + ne)};
+  cs.cbox.ensure(6 * (nv + ne + nf + g.nb) + 6);
+  return {cs.cbox.p, cs.cbox.p + 6 * nv, cs.cbox.p + 6 * (nv + ne), cs.cbox.p + 6 * (nv + ne + nf)};
 }
 
 // Float boxes of the edges and faces from those of the vertices (in cs.vbox), and of their clusters
@@ -1619,8 +1620,9 @@ static void narrow_pairs(const Geo& g, const Params& P, float ds_f, int nov, con
   cs.blk_a_off.ensure(nov + 1);
   cs.blk_b_off.ensure(nov + 1);
   cs.stage_seg.ensure(nov + 1);
-  // room for 32 candidates an overlap (piles and columns of spheres: 11 to 19), 64 k at least
-  size_t want = std::max({cs.stage_key.cap, (size_t)1 << 16, (size_t)32 * nov});
+  // room for 32 candidates an overlap (piles and columns of spheres: 11 to 19), 64 k at least,
+  // 256 M entries at most before the count is known
+  size_t want = std::max({cs.stage_key.cap, (size_t)1 << 16, std::min((size_t)32 * nov, (size_t)1 << 28)});
   StageOut so{};
   for (int attempt = 0; attempt < 4; ++attempt) {
     cs.stage_key.ensure(want);
@@ -1731,13 +1733,12 @@ void cull(const Geo& g_in, const Params& P, int vtn, double alpha, CullScratch& 
     // list capacity = the primitive counts of both bodies of every overlap; when it fits
     // (at most 2^28 entries) one binning pass writes the lists in place
     bool once = 2ll * nov * g.max_prims < (1ll << 28);
-    cs.tight.ensure(6 * (size_t)g.nb);
     KLAUNCH(K_BIN, s, k_bin_caps<<<nblk(std::max(6ll * nov, 32ll * g.nb), 256), 256, 0, s>>>(
-                          g, nov, S.ovI.p, S.ovJ.p, cs.vbox.p, cl.v, once ? cs.bin_cnt.p : nullptr, cs.tight.p));
+                          g, nov, S.ovI.p, S.ovJ.p, cs.vbox.p, cl.v, once ? cs.bin_cnt.p : nullptr, cl.tight));
     if (!once) {
       KLAUNCH(K_BIN, s, k_bin<<<nblk((long long)nw * 32, 256), 256, 0, s>>>(g, ds_f, nov, BIN_COUNT, traj, S.ovI.p, S.ovJ.p,
                                                           cs.ovcull.p, cs.ovcull_f.p, cs.vbox.p, cs.ebox.p,
-                                                          cs.fbox.p, cl, cs.tight.p, cs.bin_cnt.p, nullptr, nullptr));
+                                                          cs.fbox.p, cl, cl.tight, cs.bin_cnt.p, nullptr, nullptr));
     }
     scan_exclusive_int(cs.bin_cnt.p, cs.bin_off.p, 6 * nov, d_tot + 2, s, cs.vflag_cnt);
     if (once) {
@@ -1751,7 +1752,7 @@ void cull(const Geo& g_in, const Params& P, int vtn, double alpha, CullScratch& 
     cs.lst.ensure((size_t)nlst + 1);
     KLAUNCH(K_BIN, s, k_bin<<<nblk((long long)nw * 32, 256), 256, 0, s>>>(g, ds_f, nov, once ? BIN_ONCE : BIN_WRITE, traj,
                                                         S.ovI.p, S.ovJ.p, cs.ovcull.p, cs.ovcull_f.p, cs.vbox.p,
-                                                        cs.ebox.p, cs.fbox.p, cl, cs.tight.p, cs.bin_cnt.p, cs.bin_off.p, cs.lst.p));
+                                                        cs.ebox.p, cs.fbox.p, cl, cl.tight, cs.bin_cnt.p, cs.bin_off.p, cs.lst.p));
   }
   if (traj) {
     const int nk = 2 * g.ns;

@@ -143,7 +143,7 @@ struct Engine {
       S.vg.release(); S.vg_seg.release(); S.pt_lag.release(); S.ee_lag.release(); S.vg_lam.release();
     }
     cs.bbox.release(); cs.bbox_f.release(); cs.cnt_all.release(); cs.cnt_up.release(); cs.up_ptr.release(); cs.rowid.release();
-    cs.ovcull.release(); cs.ovcull_f.release(); cs.vbox.release(); cs.ebox.release(); cs.fbox.release(); cs.cbox.release(); cs.tight.release();
+    cs.ovcull.release(); cs.ovcull_f.release(); cs.vbox.release(); cs.ebox.release(); cs.fbox.release(); cs.cbox.release();
     cs.order.release(); cs.order_cnt.release(); cs.vend.release(); cs.toi_cand.release(); cs.toi_n.release();
     shw.release();
     cs.bin_cnt.release(); cs.bin_off.release(); cs.lst.release(); cs.cand_cnt.release(); cs.cand_off.release();
