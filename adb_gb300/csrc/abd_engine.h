@@ -188,6 +188,9 @@ inline void prof_work(int tag, double units, double bytes) {
   } while (0)
 
 // ---------------- scan ----------------
+// two scans of n entries (totals wanted)
+void scan_exclusive_int2(const int* in0, int* out0, int* tot0, const int* in1, int* out1, int* tot1, int n,
+                         cudaStream_t s, DBuf<int>& tmp);
 void scan_exclusive_int(const int* in, int* out, int n, int* d_total, cudaStream_t s, DBuf<int>& tmp);
 void scan_exclusive_ll(const long long* in, long long* out, int n, long long* d_total, cudaStream_t s,
                        DBuf<long long>& tmp);

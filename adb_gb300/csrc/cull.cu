@@ -1639,8 +1639,8 @@ static void narrow_pairs(const Geo& g, const Params& P, float ds_f, int nov, con
     KLAUNCH(K_NARROW_WRITE, s, k_narrow_tally<<<nov, NW, 0, s>>>(g, P, ds_f, ovI, ovJ, cs.bin_cnt.p, cs.bin_off.p,
                                                                  cs.lst.p, cs.vbox.p, cs.ebox.p, cs.fbox.p, so,
                                                                  cs.blk_a.p, cs.blk_b.p));
-    scan_exclusive_int(cs.blk_a.p, cs.blk_a_off.p, nov, d_tot + 3, s, cs.vflag_cnt);
-    scan_exclusive_int(cs.blk_b.p, cs.blk_b_off.p, nov, d_tot + 4, s, cs.vflag_cnt);
+    scan_exclusive_int2(cs.blk_a.p, cs.blk_a_off.p, d_tot + 3, cs.blk_b.p, cs.blk_b_off.p, d_tot + 4, nov, s,
+                        cs.vflag_cnt);
     CK(cudaMemcpyAsync(cs.h_small + 3, d_tot + 3, 5 * sizeof(int), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
     const size_t staged = (size_t)cs.h_small[6] + cs.h_small[7];
@@ -1697,8 +1697,7 @@ void cull(const Geo& g_in, const Params& P, int vtn, double alpha, CullScratch& 
   cs.tmp_int.ensure(64);
   int* d_tot = cs.tmp_int.p;  // [0] nnz, [1] nov, [2] list entries, [3] PT, [4] EE, [5] VG, staged
                               // PT and EE ([6], [7])
-  scan_exclusive_int(cs.cnt_all.p, S.row_ptr.p, nb, d_tot, s, cs.vflag_cnt);
-  scan_exclusive_int(cs.cnt_up.p, cs.up_ptr.p, nb, d_tot + 1, s, cs.vflag_cnt);
+  scan_exclusive_int2(cs.cnt_all.p, S.row_ptr.p, d_tot, cs.cnt_up.p, cs.up_ptr.p, d_tot + 1, nb, s, cs.vflag_cnt);
   // the vertex-ground pairs need only the positions: counted now, read with the overlaps
   if (!traj) vg_count(g, P, cs, s);
   CK(cudaMemcpyAsync(cs.h_small, d_tot, 6 * sizeof(int), cudaMemcpyDeviceToHost, s));

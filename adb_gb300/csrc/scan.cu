@@ -88,7 +88,7 @@ constexpr int ONE_T = 1024;
 constexpr int ONE_ITEMS = 16;
 constexpr int SCAN_ONE = ONE_T * ONE_ITEMS;
 template <typename T>
-__global__ void __launch_bounds__(ONE_T) k_scan_one(const T* in, T* out, int n, T* grand) {
+__device__ __forceinline__ void scan_one(const T* in, T* out, int n, T* grand) {
   __shared__ T sh[32];
   const int base = threadIdx.x * ONE_ITEMS;
   T v[ONE_ITEMS];
@@ -128,6 +128,10 @@ __global__ void __launch_bounds__(ONE_T) k_scan_one(const T* in, T* out, int n, 
   }
   if (grand && threadIdx.x == 0) *grand = sh[31];
 }
+template <typename T>
+__global__ void __launch_bounds__(ONE_T) k_scan_one(const T* in, T* out, int n, T* grand) {
+  scan_one<T>(in, out, n, grand);
+}
 
 // Exclusive scan of in[0, n) into out; *grand (if not null) receives the total.
 template <typename T>
@@ -158,7 +162,47 @@ size_t scan_scratch(int n) {
   }
   return tot + 4;
 }
+// Two scans of n entries each, a CTA each (n up to SCAN_ONE).
+struct Scan2 {
+  const int* in[2];
+  int *out[2], *grand[2];
+};
+__global__ void __launch_bounds__(SCAN_T) k_scan_tile2(Scan2 a, int n) {
+  __shared__ int sh[32];
+  const int q = blockIdx.x, base = threadIdx.x * SCAN_ITEMS;
+  int v[SCAN_ITEMS], loc = 0;
+#pragma unroll
+  for (int k = 0; k < SCAN_ITEMS; ++k) {
+    v[k] = base + k < n ? a.in[q][base + k] : 0;
+    loc += v[k];
+  }
+  int total;
+  int pre = block_excl_scan<int>(loc, sh, total);
+#pragma unroll
+  for (int k = 0; k < SCAN_ITEMS; ++k) {
+    if (base + k < n) a.out[q][base + k] = pre;
+    pre += v[k];
+  }
+  if (threadIdx.x == 0) *a.grand[q] = total;
+}
+__global__ void __launch_bounds__(ONE_T) k_scan_one2(Scan2 a, int n) {
+  scan_one<int>(a.in[blockIdx.x], a.out[blockIdx.x], n, a.grand[blockIdx.x]);
+}
 }  // namespace
+
+// Up to 16384 entries the two share a launch: a scan of few entries is the 3 us of a launch (a stack's
+// step has some twenty of them less), one of ten thousand 8 us on one SM, now beside the other.
+void scan_exclusive_int2(const int* in0, int* out0, int* tot0, const int* in1, int* out1, int* tot1, int n,
+                         cudaStream_t s, DBuf<int>& tmp) {
+  if (n <= 0 || n > SCAN_ONE) {
+    scan_exclusive_int(in0, out0, n, tot0, s, tmp);
+    scan_exclusive_int(in1, out1, n, tot1, s, tmp);
+    return;
+  }
+  const Scan2 a{{in0, in1}, {out0, out1}, {tot0, tot1}};
+  if (n <= SCAN_TILE) KLAUNCH(K_SCAN, s, k_scan_tile2<<<2, SCAN_T, 0, s>>>(a, n));
+  else KLAUNCH(K_SCAN, s, k_scan_one2<<<2, ONE_T, 0, s>>>(a, n));
+}
 
 void scan_exclusive_int(const int* in, int* out, int n, int* d_total, cudaStream_t s, DBuf<int>& tmp) {
   tmp.ensure(scan_scratch<int>(n) + 8);

@@ -51,3 +51,20 @@ def test_short_lists(gpu_lib, oracle_lib, subdiv, shift):
         for a, b in zip(gpu.cull(*args), orc.cull(*args)):
             assert a.shape == b.shape and np.array_equal(a, b)
     assert gpu.cull(3, sc.q0, dq) == orc.cull(3, sc.q0, dq)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [1, 1023, 1024, 1025, 2047, 2048, 2049])
+def test_counts_of_many_overlaps(gpu_lib, oracle_lib, n):
+    """n overlaps of 2 n bodies: the scans of the counts by bodies and by overlaps around a tile."""
+    from adb_gb300.abd import ABD
+    sb, mesh = S.SceneBuilder(), S.cube_mesh()
+    for k in range(n):
+        at = np.array([3.0 * (k % 46), 2.0, 3.0 * (k // 46)])
+        sb.add(mesh, at)
+        sb.add(mesh, at + np.array([0.1 * (k % 7) / 7, 1.0 + 0.04 * (k % 3) / 3, 0.2]))
+    sc, cfg = sb.build(), S.workload_config("pile")
+    g, o = ABD(sc, cfg).cull(1, sc.q0), oracle_lib.OracleSim(sc, cfg).cull(1, sc.q0)
+    assert len(o[0]) + len(o[2]) > n
+    for a, b in zip(g, o):
+        assert a.shape == b.shape and np.array_equal(a, b)
