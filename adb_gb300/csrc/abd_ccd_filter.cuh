@@ -63,7 +63,7 @@ CFD bool f_no_root(f3 u0, f3 u1, f3 v0, f3 v1, f3 w0, f3 w1, float E, float m) {
 }
 
 // A vector along the step: its value half-way and a bound on its distance from that at any
-// time (half its change, plus its error E and the rounding of the mean).
+// time (half its change, plus its error E and the rounding of the mean, 2^-24 of it).
 struct f3m {
   f3 c;
   float len, dev;
@@ -72,7 +72,7 @@ CFD f3m f3m_of(f3 a0, f3 a1, float E) {
   f3m r;
   r.c = f3_mid(a0, a1);
   r.len = f3_len(r.c);
-  r.dev = 0.5f * f3_len(f3_sub(a1, a0)) + 1.3f * E;
+  r.dev = 0.5f * f3_len(f3_sub(a1, a0)) + E + 6.1e-8f * r.len;
   return r;
 }
 // Cross product of two such vectors: value half-way and a bound on its distance from that,
