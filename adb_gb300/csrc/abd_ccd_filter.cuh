@@ -140,14 +140,15 @@ CFD bool f_ee_miss(const f3* a0, const f3* a1, const f3* b0, const f3* b1) {
 
 // The verification of a root in FP32: 1 passes, 0 fails, -1 not certain (the FP64 test then
 // decides). The vectors at the root's time t are off by E (both ends'), by 2^-24 of t times
-// the change of the vector for each rounding of t, of the change and of their product, and by
-// 2^-24 of the vector for that of the sum; the slacks are those of the certificates.
+// the change of the vector (at most sqrt 3 times its largest coordinate, cheaper than its norm)
+// for each rounding of t, of the change and of their product, and by 2^-24 of the vector for
+// that of the sum; the slacks are those of the certificates.
 CFD f3m f3m_at(f3 a0, f3 a1, float t, float E) {
   const f3 d = f3_sub(a1, a0);
   f3m r;
   r.c = f3{a0.x + t * d.x, a0.y + t * d.y, a0.z + t * d.z};
   r.len = f3_len(r.c);
-  r.dev = E + 6.1e-8f * (3.f * t * f3_len(d) + r.len);
+  r.dev = E + 6.1e-8f * (5.2f * t * f3_maxabs(d) + r.len);
   return r;
 }
 CFD int f_pt_verify(f3 p0, f3 p1, const f3* t0, const f3* t1, float t) {
