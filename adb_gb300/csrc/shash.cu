@@ -130,12 +130,15 @@ __global__ void k_reg_cells(Geo g, ShGrid G, int kind, int n, int traj, int fix_
   if ((threadIdx.x & 31) == 0 && c) atomicAdd(total, c);
 }
 
-// The buckets of a cell range, each once (f(bucket)): cells 2^bits apart share a bucket, so
-// no axis takes more than 2^bits of them.
+// Cells l .. u of an axis that differ in their bucket: those 2^bits apart share one.
+__device__ __forceinline__ int cell_count(int l, int u, int bits) {
+  return (int)min((unsigned)u - (unsigned)l, (1u << bits) - 1u) + 1;
+}
+// The buckets of a cell range, each once (f(bucket)).
 template <typename F>
 __device__ __forceinline__ void for_buckets(const ShCells& r, int bits, F&& f) {
-  const int M = 1 << bits;
-  const int n0 = min(r.u[0] - r.l[0] + 1, M), n1 = min(r.u[1] - r.l[1] + 1, M), n2 = min(r.u[2] - r.l[2] + 1, M);
+  const int n0 = cell_count(r.l[0], r.u[0], bits), n1 = cell_count(r.l[1], r.u[1], bits),
+            n2 = cell_count(r.l[2], r.u[2], bits);
   for (int i = 0; i < n0; ++i)
     for (int j = 0; j < n1; ++j)
       for (int k = 0; k < n2; ++k) f(sh_hash(r.l[0] + i, r.l[1] + j, r.l[2] + k, bits));
@@ -250,12 +253,14 @@ __global__ void __launch_bounds__(128) k_sh_query(Geo g, ShQuery Q, int qbeg, in
     }
   }
   const ShCells r = Q.qcells[q];
-  const int M = 1 << Q.G.bits;
-  const int e0 = r.l[0] + min(r.u[0] - r.l[0], M - 1), e1 = r.l[1] + min(r.u[1] - r.l[1], M - 1),
-            e2 = r.l[2] + min(r.u[2] - r.l[2], M - 1);
-  for (int i = r.l[0]; i <= e0; ++i)
-    for (int j = r.l[1]; j <= e1; ++j)
-      for (int k = r.l[2]; k <= e2; ++k) {
+  // Cells are counted: a coordinate past 2^31 cells is in the last one an int holds, and a loop
+  // up to that cell would not end.
+  const int n0 = cell_count(r.l[0], r.u[0], Q.G.bits), n1 = cell_count(r.l[1], r.u[1], Q.G.bits),
+            n2 = cell_count(r.l[2], r.u[2], Q.G.bits);
+  for (int di = 0; di < n0; ++di)
+    for (int dj = 0; dj < n1; ++dj)
+      for (int dk = 0; dk < n2; ++dk) {
+        const int i = r.l[0] + di, j = r.l[1] + dj, k = r.l[2] + dk;
         const unsigned b = sh_hash(i, j, k, Q.G.bits);
         const int n = Q.cnt[b];
         if (n == 0) continue;  // an unused bucket has no segment
