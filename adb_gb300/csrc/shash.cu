@@ -123,7 +123,10 @@ __global__ void k_reg_cells(Geo g, ShGrid G, int kind, int n, int traj, int fix_
     sh_cells(lo, G, r.l);
     sh_cells(hi, G, r.u);
     cells[id] = r;
-    c = (unsigned long long)(r.u[0] - r.l[0] + 1) * (r.u[1] - r.l[1] + 1) * (r.u[2] - r.l[2] + 1);
+    // capped where it is too many anyway: the product of three counts can wrap around (2^22 by
+    // 2^21 by 2^21 cells would count as none, and the entries go past a list of no length)
+    c = 1;
+    for (int a = 0; a < 3; ++a) c = min(c * ((unsigned long long)((unsigned)r.u[a] - (unsigned)r.l[a]) + 1ull), 1ull << 31);
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);

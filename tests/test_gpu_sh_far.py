@@ -34,3 +34,21 @@ def test_far_body(gpu_lib, axes):
         out.append((sim.cull(1, sc.q0), sim.cull(3, sc.q0, dq)))
     assert len(out[0][0][0]) and out[0][1] < 1.0
     assert all(np.array_equal(a, b) for a, b in zip(out[0][0], out[1][0])) and out[0][1] == out[1][1]
+
+
+@pytest.mark.parametrize("cells", [(1 << 22, 1 << 21, 1 << 21), (1 << 11, 1 << 10, 1 << 10), (1 << 30, 1 << 30, 1)])
+def test_too_many_cells(gpu_lib, cells):
+    """Motions over more cells than a table can hold are refused, those whose number of cells is a
+    multiple of 2^64 (the first) among them."""
+    from adb_gb300._lib import AbdError
+    from adb_gb300.abd import ABD
+    sb = S.SceneBuilder()
+    sb.add(S.cube_mesh(), (32.0, 32.0, 32.0))
+    sb.add(S.cube_mesh(), (64.0 * 5 + 32.0, 32.0, 32.0))
+    sc = sb.build()
+    sim = ABD(sc, S.Config(iaabb=0, full_ccd=True, sh_min_xyz=0.0, sh_dx=64.0, ground=False))
+    dq = np.zeros_like(sc.q0)
+    dq[0, :3] = [64.0 * (n - 1) for n in cells]
+    with pytest.raises(AbdError, match="too many cell registrations"):
+        sim.cull(3, sc.q0, dq)
+    assert sim.cull(3, sc.q0, np.zeros_like(dq)) == 1.0
