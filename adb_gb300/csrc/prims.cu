@@ -3,12 +3,12 @@
 // ee_collision_time), evaluated on the GPU with the same device code as the step, and
 // the FP64 throughput probe used as the roofline denominator of FP64-bound kernels.
 #include <algorithm>
-#include <mutex>
 #include <vector>
 
 #include "abd_ccd_filter.cuh"
 #include "abd_engine.h"
 #include "abd_ipc.cuh"
+#include "batch_pool.h"
 
 namespace abd {
 namespace {
@@ -215,76 +215,15 @@ __global__ void k_fma64(double* out, int iters, double a, double b) {
   out[tid] = x0 + x1 + x2 + x3 + x4 + x5 + x6 + x7;
 }
 
-// Device buffers of finished batch calls, kept for the next ones: cudaMalloc and cudaFree cost a
-// call of few stencils more than its copies and its kernel (497 us a call of 300 edge pairs,
-// 332 us with the pool). At most POOL_BUFS of at most POOL_BYTES each; a buffer belongs to one
-// call at a time, which hands it back after its last synchronous copy (after an error it is
-// freed). All are freed when an allocation fails and when the library is unloaded.
-constexpr int POOL_BUFS = 4;
-constexpr size_t POOL_BYTES = (size_t)32 << 20;
-struct BatchPool {
-  struct Buf {
-    void* p;
-    size_t bytes;
-    int dev;
-  };
-  std::mutex m;
-  std::vector<Buf> idle;
-  Buf take(size_t bytes) {
-    int dev = 0;
-    CK(cudaGetDevice(&dev));
-    {
-      std::lock_guard<std::mutex> l(m);
-      int best = -1;
-      for (int i = 0; i < (int)idle.size(); ++i)
-        if (idle[i].dev == dev && idle[i].bytes >= bytes && (best < 0 || idle[i].bytes < idle[best].bytes)) best = i;
-      if (best >= 0) {
-        const Buf b = idle[best];
-        idle.erase(idle.begin() + best);
-        return b;
-      }
-    }
-    Buf b{nullptr, bytes, dev};
-    if (cudaMalloc(&b.p, bytes) != cudaSuccess) {
-      (void)cudaGetLastError();
-      trim();
-      CK(cudaMalloc(&b.p, bytes));
-    }
-    return b;
-  }
-  void give(const Buf& b, bool keep) {
-    Buf out = b;
-    if (keep && b.bytes <= POOL_BYTES) {
-      std::lock_guard<std::mutex> l(m);
-      if ((int)idle.size() < POOL_BUFS) {
-        idle.push_back(b);
-        return;
-      }
-      // the smallest one goes
-      for (Buf& i : idle)
-        if (i.bytes < out.bytes) std::swap(i, out);
-    }
-    cudaFree(out.p);
-  }
-  void trim() {
-    std::lock_guard<std::mutex> l(m);
-    for (Buf& b : idle) cudaFree(b.p);
-    idle.clear();
-  }
-  BatchPool() { idle.reserve(POOL_BUFS); }
-  ~BatchPool() { trim(); }
-};
-BatchPool g_pool;
-
 template <typename T>
 struct DevArr {
-  BatchPool::Buf b;
+  BatchBuf b;
   T* p;
   bool done = false;  // the call's work on it has ended
-  explicit DevArr(size_t n) : b(g_pool.take((n ? n : 1) * sizeof(T))), p(static_cast<T*>(b.p)) {}
+  explicit DevArr(size_t n) : b(batch_take((n ? n : 1) * sizeof(T))), p(static_cast<T*>(b.p)) {}
   DevArr(const DevArr&) = delete;
   DevArr& operator=(const DevArr&) = delete;
-  ~DevArr() { g_pool.give(b, done); }
+  ~DevArr() { batch_give(b, done); }
 };
 
 inline int nblk(long long n, int t) { return (int)((n + t - 1) / t); }
