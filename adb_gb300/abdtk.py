@@ -136,3 +136,8 @@ def ee_distance_batch(x):
     d = np.zeros(x.shape[0])
     L.check(L.lib().abd_ee_distance_batch(x.shape[0], L.dptr(x), L.iptr(t), L.dptr(d)), None, "ee_distance")
     return t, d
+
+
+def release_buffers():
+    """Frees the device buffers that finished batch calls leave for the next ones."""
+    L.check(L.lib().abd_release_buffers(), None, "release_buffers")

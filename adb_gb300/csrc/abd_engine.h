@@ -18,6 +18,10 @@ struct CudaError {
 void check(cudaError_t e, const char* where);  // throws CudaError
 #define CK(x) ::abd::check((x), #x)
 
+// Device memory; when there is none, the batch calls' kept buffers are given back first
+// (batch_pool.cpp).
+void* device_alloc(size_t bytes);
+
 // Grow-only device buffer (contents are not preserved on growth unless asked).
 template <typename T>
 struct DBuf {
@@ -27,8 +31,7 @@ struct DBuf {
     if (n <= cap) return;
     size_t nc = cap ? cap : 1024;
     while (nc < n) nc = nc + nc / 2 + 1;
-    T* np_ = nullptr;
-    CK(cudaMalloc(&np_, nc * sizeof(T)));
+    T* np_ = static_cast<T*>(device_alloc(nc * sizeof(T)));
     if (keep && p && keep_n) CK(cudaMemcpy(np_, p, keep_n * sizeof(T), cudaMemcpyDeviceToDevice));
     if (p) CK(cudaFree(p));
     p = np_;

@@ -62,6 +62,18 @@ Pool g_pool;
 
 }  // namespace
 
+void* device_alloc(size_t bytes) {
+  void* p = nullptr;
+  if (cudaMalloc(&p, bytes) != cudaSuccess) {
+    (void)cudaGetLastError();
+    batch_release();
+    CK(cudaMalloc(&p, bytes));
+  }
+  return p;
+}
+
+void batch_release() { g_pool.trim(); }
+
 BatchBuf batch_take(size_t bytes) {
   void* ctx = current_context();
   if (!ctx && cudaFree(nullptr) == cudaSuccess) ctx = current_context();  // a thread's first call
@@ -80,11 +92,7 @@ BatchBuf batch_take(size_t bytes) {
   }
   BatchBuf b;
   b.bytes = bytes;
-  if (cudaMalloc(&b.p, bytes) != cudaSuccess) {
-    (void)cudaGetLastError();
-    g_pool.trim();
-    CK(cudaMalloc(&b.p, bytes));
-  }
+  b.p = device_alloc(bytes);
   b.ctx = current_context();
   b.id = b.ctx ? buffer_id(b.p) : 0;
   return b;
@@ -108,3 +116,8 @@ void batch_give(const BatchBuf& b, bool keep) {
 }
 
 }  // namespace abd
+
+extern "C" int abd_release_buffers(void) {
+  abd::batch_release();
+  return ABD_OK;
+}

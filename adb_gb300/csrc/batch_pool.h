@@ -3,7 +3,8 @@
 // pairs, 332 us with the pool). At most POOL_BUFS of at most POOL_BYTES each: 32 MB are a batch of
 // 24 000 Hessians, whose call takes 1.1 to 1.7 ms, against 0.17 to 0.3 ms of allocation and release.
 // A buffer belongs to one call at a time, which hands it back after its last synchronous
-// copy (after an error it is freed).
+// copy (after an error it is freed). The kept ones are freed when any allocation of the library finds
+// the device full, on abd_release_buffers, and when the library is unloaded.
 //
 // A kept address is only as good as its allocation: after cudaDeviceReset, or in another
 // context of the same device, it may be nobody's or somebody else's (a reset gives the same
@@ -27,5 +28,6 @@ struct BatchBuf {
 };
 BatchBuf batch_take(size_t bytes);             // throws CudaError
 void batch_give(const BatchBuf& b, bool keep);  // keep: the work on it has ended
+void batch_release();                           // frees the kept buffers
 
 }  // namespace abd

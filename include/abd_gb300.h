@@ -244,6 +244,10 @@ int abd_ee_collision_time_batch(int n, const double* x, double* toi);
 int abd_pt_distance_batch(int n, const double* x, int* type, double* dist);
 int abd_ee_distance_batch(int n, const double* x, int* type, double* dist);
 
+/* Frees the device buffers that finished batch calls above leave for the next ones (at most four of
+ * 32 MB; also freed when an allocation of this library finds the device full). */
+int abd_release_buffers(void);
+
 /* Allocation-free minimum point-triangle time of impact. No counterpart in the
  * reference. For callers that cannot allocate device memory where they call it (inside
  * a CUDA-graph stream capture, or under a host framework whose pool allocator owns all

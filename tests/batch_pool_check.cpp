@@ -132,6 +132,21 @@ int main() {
     got = false;
   }
   expect(got, "a batch call gets the room of the kept buffers");
+  room = (size_t)1 << 30;
+  for (int i = 0; i < 4; ++i) many[i] = batch_take((i + 2) * MB);
+  for (int i = 0; i < 4; ++i) batch_give(many[i], true);
+  room = used + 4 * MB;
+  DBuf<char> handle;  // a simulation's buffer
+  try {
+    handle.ensure(10 * MB);
+  } catch (const CudaError&) {
+  }
+  expect(handle.p != nullptr, "a simulation gets the room of the kept buffers");
+  handle.release();
+  room = (size_t)1 << 30;
+  batch_give(batch_take(MB), true);
+  batch_release();
+  expect(used == 8 * MB, "a release leaves nothing kept");  // their eight
   expect(wrong_frees == 0, "nothing is freed twice");
   return bad != 0;
 }
