@@ -128,9 +128,8 @@ struct CullScratch {
   DBuf<int> vg_cnt;  // vertex-ground pairs per block of vertices
   DBuf<unsigned long long> stage_key;   // sorted candidates per overlap (sub, i, j)
   DBuf<int8_t> stage_ty;
-  DBuf<unsigned long long> toi_key;     // 2 per scene: pt/ee, ground
-  DBuf<int2> toi_cand;                  // trajectory candidates left to the FP64 test, and their number
-  DBuf<unsigned> toi_n;
+  DBuf<unsigned long long> toi_key;     // 2 per scene: pt/ee, ground; the number of candidates
+  DBuf<int2> toi_cand;                  // trajectory candidates left to the FP64 test
   DBuf<int> tmp_int;
   DBuf<long long> tmp_ll;
   // autotuned narrow-phase variants (index into the step table; -1 = not tuned yet) of the

@@ -744,7 +744,11 @@ struct ToiCand {
   unsigned* n;
   unsigned cap;
 };
-constexpr unsigned kToiCand = 1u << 21;  // 16 MB; a candidate past it is evaluated where it is found
+// Room for as many candidates as the overlaps' lists can have entries (two spheres of 3842
+// primitives each: 7684), 4096 at least and 16 MB at most; a candidate past it is evaluated
+// where it is found, and the list is then large enough for the next call. (16 MB for every handle
+// made one of ten cubes 21.8 MB instead of 2.9.)
+constexpr unsigned kToiCandMin = 1u << 12, kToiCandMax = 1u << 21;
 
 // Candidates of the pair cull left to the FP64 test, by overlap, each overlap's sorted by
 // (sub, i, j): the point-triangle ones from the front of the buffer, the edge-edge ones from its
@@ -1754,13 +1758,14 @@ void cull(const Geo& g_in, const Params& P, int vtn, double alpha, CullScratch& 
                                                         cs.ebox.p, cs.fbox.p, cl, cl.tight, cs.bin_cnt.p, cs.bin_off.p, cs.lst.p));
   }
   if (traj) {
-    const int nk = 2 * g.ns;
-    cs.toi_key.ensure(nk);
-    if (cs.h_toi_cap < nk) {
+    const int nk = 2 * g.ns;  // then the number of candidates, read with the keys
+    cs.toi_key.ensure(nk + 1);
+    if (cs.h_toi_cap < nk + 1) {
       if (cs.h_toi) CK(cudaFreeHost(cs.h_toi));
-      CK(cudaMallocHost(&cs.h_toi, nk * sizeof(unsigned long long)));
-      cs.h_toi_cap = nk;
+      CK(cudaMallocHost(&cs.h_toi, (nk + 1) * sizeof(unsigned long long)));
+      cs.h_toi_cap = nk + 1;
     }
+    unsigned cap = 0;
     double o = 1.0;
     unsigned long long b;
     memcpy(&b, &o, sizeof(b));
@@ -1779,19 +1784,24 @@ void cull(const Geo& g_in, const Params& P, int vtn, double alpha, CullScratch& 
       order_overlaps(nov, cs, s, K_NARROW_TOI);
       narrow_smem_attr();
       traj_floats(g, cs, s);  // allocates cs.vend: before its address is taken
-      cs.toi_cand.ensure(kToiCand);
-      cs.toi_n.ensure(2);
+      cs.toi_cand.ensure(std::min(std::max((unsigned)nlst, kToiCandMin), kToiCandMax));
+      cap = (unsigned)std::min(cs.toi_cand.cap, (size_t)kToiCandMax);
+      unsigned* d_n = reinterpret_cast<unsigned*>(cs.toi_key.p + nk);
       NarrowLaunch a{g, P, ds_f, S.ovI.p, S.ovJ.p, cs.bin_cnt.p, cs.bin_off.p, cs.lst.p, cs.vbox.p, cs.ebox.p,
                      cs.fbox.p, cs.toi_key.p, StageOut{}, Order{cs.order.p, cs.order_cnt.p, nov},
-                     ToiCand{cs.vend.p, cs.toi_cand.p, cs.toi_n.p, kToiCand}};
-      narrow_phase(2, nov, a, cs, reinterpret_cast<int*>(cs.toi_n.p), s);
+                     ToiCand{cs.vend.p, cs.toi_cand.p, d_n, cap}};
+      narrow_phase(2, nov, a, cs, reinterpret_cast<int*>(d_n), s);
       KLAUNCH(K_NARROW_TOI, s, k_toi_list<<<1216, 128, 0, s>>>(g, a.tc, cs.toi_key.p));
     }
     if (P.ground && g.nv) {
       KLAUNCH(K_VG_TOI, s, k_vg_toi<<<nblk(g.nv, 256), 256, 0, s>>>(g, P, cs.toi_key.p + 1));
     }
-    CK(cudaMemcpyAsync(cs.h_toi, cs.toi_key.p, nk * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
+    CK(cudaMemcpyAsync(cs.h_toi, cs.toi_key.p, (nk + 1) * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
+    if (nov > 0) {
+      const unsigned found = (unsigned)cs.h_toi[nk];
+      if (found > cap) cs.toi_cand.ensure(std::min(found, kToiCandMax));
+    }
     for (int sc = 0; sc < g.ns; ++sc) {
       if (toi_p) toi_p[sc] = key_to_double(cs.h_toi[2 * sc]);
       if (toi_g) toi_g[sc] = key_to_double(cs.h_toi[2 * sc + 1]);

@@ -144,7 +144,7 @@ struct Engine {
     }
     cs.bbox.release(); cs.bbox_f.release(); cs.cnt_all.release(); cs.cnt_up.release(); cs.up_ptr.release(); cs.rowid.release();
     cs.ovcull.release(); cs.ovcull_f.release(); cs.vbox.release(); cs.ebox.release(); cs.fbox.release(); cs.cbox.release();
-    cs.order.release(); cs.order_cnt.release(); cs.vend.release(); cs.toi_cand.release(); cs.toi_n.release();
+    cs.order.release(); cs.order_cnt.release(); cs.vend.release(); cs.toi_cand.release();
     shw.release();
     cs.bin_cnt.release(); cs.bin_off.release(); cs.lst.release(); cs.cand_cnt.release(); cs.cand_off.release();
     cs.flags.release(); cs.blk_a.release(); cs.blk_b.release(); cs.blk_a_off.release(); cs.blk_b_off.release();
