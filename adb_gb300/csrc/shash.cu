@@ -591,7 +591,9 @@ static void sh_register(const Geo& g, const ShParams& H, int kind, int n, int tr
   KLAUNCH(K_SH, s, k_bucket_fill<<<nblk(n, 256), 256, 0, s>>>(g, G, kind, n, T.cells.p, T.cur.p, T.ent.p));
 }
 
-constexpr size_t kCandList = 1u << 21;  // candidates kept at a time (16 MB)
+// Candidates kept at a time: 32 an edge or face, 16 k at least, 16 MB at most. The list grows to what
+// a run of queries leaves; past 16 MB the queries are taken in parts.
+constexpr size_t kCandMin = 1u << 14, kCandMax = 1u << 21;
 
 // Registers the primitives that the queries of `kind` run against, computes the queries' cells
 // and fills Q (list and counters included).
@@ -612,14 +614,15 @@ static void sh_prepare(const Geo& g, const ShParams& H, int kind, int traj, ShSc
   Q.vend = cs.vend.p;
   W.n.ensure(2);
   Q.n = W.n.p;
-  W.cand.ensure(kCandList);
+  W.cand.ensure(std::min(std::max((size_t)32 * std::max(g.ne, g.nf), kCandMin), kCandMax));  // once, for both kinds
   if (!W.h_n) CK(cudaMallocHost(&W.h_n, 2 * sizeof(unsigned long long)));
 }
 
 // Runs the query over all primitives of a kind, `eval` on each list and `done` on its two
 // counters (false: the same queries again). The queries are taken all at once unless they
-// leave more candidates than the list holds; then in runs of half as many, down to single
-// queries, for which the list grows (a query has at most as many as there are primitives).
+// leave more candidates than the largest list holds; then in runs of half as many, down to single
+// queries, for which the list grows further (a query has at most as many as there are
+// primitives).
 template <int KIND, bool TRAJ, typename Eval, typename Done>
 static void sh_run(const Geo& g, ShQuery& Q, ShScratch& W, cudaStream_t s, Eval&& eval, Done&& done) {
   const int nq = KIND ? g.ne : g.nf;
@@ -633,9 +636,10 @@ static void sh_run(const Geo& g, ShQuery& Q, ShScratch& W, cudaStream_t s, Eval&
     eval();
     CK(cudaMemcpyAsync(W.h_n, Q.n, 2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
-    if (W.h_n[0] > Q.cand_cap) {
-      if (m == 1) W.cand.ensure((size_t)W.h_n[0]);
-      step = std::max(1, m / 2);
+    const size_t found = (size_t)W.h_n[0];
+    if (found > Q.cand_cap) {
+      if (found <= kCandMax || m == 1) W.cand.ensure(found);
+      else step = std::max(1, m / 2);
       continue;
     }
     if (done()) q0 += m;

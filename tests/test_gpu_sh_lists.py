@@ -1,0 +1,54 @@
+"""The candidate list of the spatial-hash queries (shash.cu): sized by the scene, so that a handle of
+few bodies stays small; grown when a run leaves more; sets and bounds of the oracle either
+way, the first time and again."""
+import dataclasses
+
+import numpy as np
+import pytest
+
+from adb_gb300 import scene as S
+
+pytestmark = pytest.mark.gpu
+
+
+def test_memory_of_a_small_handle(gpu_lib):
+    torch = pytest.importorskip("torch")
+    from adb_gb300.abd import ABD
+    sc = S.cube_stack(10, gap=0.01, seed=1)
+    cfg = dataclasses.replace(S.workload_config("cubes"), iaabb=0, full_ccd=True)
+
+    def used():
+        torch.cuda.synchronize()
+        return -torch.cuda.mem_get_info()[0]
+
+    def handle():
+        sim = ABD(sc, cfg)
+        sim.cull(1, sc.q0)
+        sim.cull(3, sc.q0, cfg.dt * sc.dqdt)
+        return sim
+
+    keep = [handle()]
+    before = used()
+    keep += [handle() for _ in range(16)]
+    # the bucket table has 3 MB; the list alone was 16 MB
+    assert (used() - before) / 16 < 9 << 20
+
+
+def test_growth(gpu_lib, oracle_lib):
+    """480 x 480 edge pairs within reach where the list starts with 30720 entries."""
+    from adb_gb300.abd import ABD
+    sb = S.SceneBuilder()
+    for k in range(2):
+        sb.add(S.icosphere_mesh(2, 0.5), (1.01 * k, 3.0, 0.0))
+    sc = sb.build()
+    cfg = S.Config(dhat=4.0, iaabb=0, full_ccd=True, sh_dx=4.0, sh_bits=2, ground=False)
+    gpu, orc = ABD(sc, cfg), oracle_lib.OracleSim(sc, cfg)
+    want = orc.cull(1, sc.q0)
+    assert len(want[2]) > 1 << 17
+    dq = np.zeros_like(sc.q0)
+    dq[1, 0] = -0.5
+    bound = orc.cull(3, sc.q0, dq)
+    assert bound < 1.0
+    for _ in range(2):
+        assert all(np.array_equal(a, b) for a, b in zip(gpu.cull(1, sc.q0), want))
+        assert gpu.cull(3, sc.q0, dq) == bound
