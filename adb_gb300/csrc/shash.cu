@@ -622,7 +622,7 @@ static void sh_prepare(const Geo& g, const ShParams& H, int kind, int traj, ShSc
 // counters (false: the same queries again). The queries are taken all at once unless they
 // leave more candidates than the largest list holds; then in runs of half as many, down to single
 // queries, for which the list grows further (a query has at most as many as there are
-// primitives).
+// primitives), and of twice as many after a run that fills at most half of it.
 template <int KIND, bool TRAJ, typename Eval, typename Done>
 static void sh_run(const Geo& g, ShQuery& Q, ShScratch& W, cudaStream_t s, Eval&& eval, Done&& done) {
   const int nq = KIND ? g.ne : g.nf;
@@ -642,7 +642,11 @@ static void sh_run(const Geo& g, ShQuery& Q, ShScratch& W, cudaStream_t s, Eval&
       else step = std::max(1, m / 2);
       continue;
     }
-    if (done()) q0 += m;
+    if (done()) {
+      q0 += m;
+      // past a dense part of the scene the runs become longer again
+      if (2 * found <= Q.cand_cap) step = m <= nq / 2 ? 2 * m : nq;
+    }
   }
 }
 

@@ -52,3 +52,30 @@ def test_growth(gpu_lib, oracle_lib):
     for _ in range(2):
         assert all(np.array_equal(a, b) for a, b in zip(gpu.cull(1, sc.q0), want))
         assert gpu.cull(3, sc.q0, dq) == bound
+
+
+def test_runs_grow_again(gpu_lib):
+    """Two spheres whose 1920 x 1920 edge pairs are within reach, then many that reach nothing: only the
+    former are taken in short runs."""
+    from adb_gb300.abd import ABD
+    mesh = S.icosphere_mesh(3, 0.5)
+    cfg = S.Config(dhat=4.0, iaabb=2, sh_dx=4.0, sh_bits=3, ground=False)
+
+    def cull(others):
+        sb = S.SceneBuilder()
+        for k in range(2):
+            sb.add(mesh, (1.01 * k, 3.0, 0.0))
+        for k in range(others):
+            sb.add(mesh, (20.0 + 4.0 * k, 3.0, 0.0))
+        sc = sb.build()
+        sim = ABD(sc, cfg)
+        sim.cull(1, sc.q0)
+        sim.profile(True)
+        sets = sim.cull(1, sc.q0)
+        return sets, sum(v["launches"] for k, v in sim.kernel_times().items() if "hash" in k)
+
+    alone, few = cull(0)
+    sets, launches = cull(30)
+    assert few > 0 and all(np.array_equal(a, b) for a, b in zip(alone, sets))
+    # 57 600 edges past the pair: at most a doubling run each, of two launches, for log2(61440)
+    assert launches <= few + 2 * 20
