@@ -78,6 +78,7 @@ def lib():
         L.abd_get_counts.argtypes = [H, _I, _I, _I, _I]
         L.abd_get_iter.argtypes = [H]
         L.abd_set_iter.argtypes = [H, C.c_int]
+        L.abd_set_poll_limit.argtypes = [H, C.c_int]
         L.abd_set_friction.argtypes = [H, C.c_double]
         L.abd_get_friction.argtypes = [H, C.POINTER(C.c_double)]
         L.abd_adjoint_frame.argtypes = [H, _D, _D, _D, _D, _D, _D, C.POINTER(C.c_double)]
@@ -114,7 +115,7 @@ def lib():
 
 # Every symbol include/abd_gb300.h declares (checked by the CPU test suite).
 EXPORTED = ["abd_create", "abd_create_from_files", "abd_step", "abd_get_state", "abd_set_state", "abd_trace_save", "abd_trace_load", "abd_set_trace", "abd_get_trace", "abd_trace_files", "abd_run", "abd_get_counts",
-            "abd_get_iter", "abd_set_iter", "abd_get_scene_count", "abd_get_scene_stats", "abd_set_friction", "abd_get_friction", "abd_adjoint_frame", "abd_adjoint_stats", "abd_autotune_info", "abd_last_error", "abd_destroy", "abd_profile", "abd_kernel_times", "abd_kernel_work", "abd_cull", "abd_get_pairs",
+            "abd_get_iter", "abd_set_iter", "abd_get_scene_count", "abd_get_scene_stats", "abd_set_poll_limit", "abd_set_friction", "abd_get_friction", "abd_adjoint_frame", "abd_adjoint_stats", "abd_autotune_info", "abd_last_error", "abd_destroy", "abd_profile", "abd_kernel_times", "abd_kernel_work", "abd_cull", "abd_get_pairs",
             "abd_newton_system", "abd_newton_dq", "abd_energy", "abd_ipc_hess_pt_batch", "abd_ipc_hess_ee_batch",
             "abd_pt_collision_time_batch", "abd_ee_collision_time_batch", "abd_pt_distance_batch",
             "abd_ee_distance_batch", "abd_release_buffers", "abd_pt_min_toi_noalloc", "abd_noalloc_last_error", "abd_measure_fp64_gflops"]

@@ -153,6 +153,10 @@ class ABD:
     def iter(self, v: int):
         L.lib().abd_set_iter(self._h, int(v))
 
+    def set_poll_limit(self, polls: int):
+        """Polls after which the CG gives up waiting for another CTA (tests of that path)."""
+        L.check(L.lib().abd_set_poll_limit(self._h, int(polls)), self._h, "abd_set_poll_limit")
+
     def set_friction(self, mu: float):
         L.check(L.lib().abd_set_friction(self._h, float(mu)), self._h, "abd_set_friction")
 

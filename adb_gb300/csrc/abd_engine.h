@@ -291,6 +291,7 @@ struct NewtonBufs {
   DBuf<int> grp_body, grp_n, grp_scene, sc_gbeg, sc_gend;  // PCG body groups (pcg_groups)
   DBuf<int> sc_box;          // per scene: where the boxes of its groups begin (one group per CTA)
   size_t n_box = 0;          // values in all boxes
+  int polls = 1 << 21;       // polls of such a word (a second or two) before a solve gives up
   std::vector<int> h_sc_beg, h_sc_end;  // body range of each scene (host)
   DBuf<double> dense_A, dense_y;         // dense solve: one scene's matrix and right-hand side
   // block-tridiagonal direct solve: per-scene flags and counts, the bodies by elimination

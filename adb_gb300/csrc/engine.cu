@@ -947,6 +947,11 @@ int abd_energy(abd_handle* h, const double* q, const double* dq, double* terms, 
   });
 }
 
+int abd_set_poll_limit(abd_handle* h, int polls) {
+  if (!h || polls < 0) return ABD_ERR_INVALID;
+  h->e.nbufs.polls = polls;
+  return ABD_OK;
+}
 int abd_set_friction(abd_handle* h, double mu) {
   if (!h || !(mu >= 0.0)) return ABD_ERR_INVALID;
   h->e.P.mu = mu;

@@ -856,6 +856,7 @@ struct PcgArgs {
   unsigned long long* slots;            // k_pcg1: tagged words (pcg1_words), zero at its start
   const int* sc_box;                    // k_pcg1: scene -> its boxes
   double* pnb;                          // k_pcg1: directions of the row blocks past the registers
+  int polls;                            // k_pcg1: polls of a word before the solve gives up
 };
 
 // 64-bit words that cross between the CTAs of k_pcg1: two each for every row of z and for three
@@ -1302,7 +1303,6 @@ __global__ void __launch_bounds__(PCG_NT) k_pcg(PcgArgs a) {
 constexpr int PCG1_NC = 2;     // row blocks per part kept in registers
 constexpr int PCG1_G = 5;      // groups of a scene per lane of an exchange
 constexpr int PCG1_MAXGRP = 32 * PCG1_G;
-constexpr int PCG1_SPIN = 1 << 21;  // polls of a word (a second or two) before the solve gives up
 
 // A double as two 64-bit words (16-byte aligned), each with the iteration's number in its upper
 // half: a reader that finds the number in both has the value (64-bit accesses are single).
@@ -1324,14 +1324,14 @@ __device__ __forceinline__ bool tag_ok(const Tagged& r, unsigned tag) {
 }
 __device__ __forceinline__ double tag_val(const Tagged& r) { return __hiloint2double((int)(unsigned)r.hi, (int)(unsigned)r.lo); }
 // A warp reads N tagged values a lane (w[i] null: none) into v. False when they did not all
-// arrive within PCG1_SPIN polls.
+// arrive within that many polls.
 template <int N>
-__device__ __forceinline__ bool tag_gather(const Tagged* (&w)[N], unsigned tag, double (&v)[N]) {
+__device__ __forceinline__ bool tag_gather(const Tagged* (&w)[N], unsigned tag, double (&v)[N], int polls) {
   unsigned miss = 0;
 #pragma unroll
   for (int i = 0; i < N; ++i)
     if (w[i]) miss |= 1u << i;
-  for (int spin = 0; spin < PCG1_SPIN; ++spin) {
+  for (int spin = 0; spin < polls; ++spin) {
     Tagged r[N];
 #pragma unroll
     for (int i = 0; i < N; ++i)
@@ -1348,14 +1348,14 @@ __device__ __forceinline__ bool tag_gather(const Tagged* (&w)[N], unsigned tag, 
 }
 // The partials of a scene's n groups from this group's box: lane l groups l, l + 32, ...;
 // their sum is formed in the order of warp_scene_sum.
-__device__ __forceinline__ bool sum_gather(const Tagged* box, int n, unsigned tag, double (&v)[PCG1_G]) {
+__device__ __forceinline__ bool sum_gather(const Tagged* box, int n, unsigned tag, double (&v)[PCG1_G], int polls) {
   const Tagged* w[PCG1_G];
 #pragma unroll
   for (int i = 0; i < PCG1_G; ++i) {
     const int k = (int)(threadIdx.x & 31) + 32 * i;
     w[i] = k < n ? box + k : nullptr;
   }
-  return tag_gather<PCG1_G>(w, tag, v);
+  return tag_gather<PCG1_G>(w, tag, v, polls);
 }
 __device__ __forceinline__ double sum_form(const double (&v)[PCG1_G], int n) {
   double s = 0.0;
@@ -1442,7 +1442,7 @@ __global__ void __launch_bounds__(PCG_NT) k_pcg1(PcgArgs a) {
     bool late = false;  // told at the next common barrier: all threads leave at the same one
     for (int k = 0;; ++k) {
       sent_wait();
-      if (!tag_gather<PCG1_NC>(wz, (unsigned)k + 1u, zn) || late) s_abort = 1;
+      if (!tag_gather<PCG1_NC>(wz, (unsigned)k + 1u, zn, a.polls) || late) s_abort = 1;
       __syncthreads();  // beta, or the end
       if (s_flag || s_abort) break;
       const double beta = s_beta;
@@ -1462,7 +1462,7 @@ __global__ void __launch_bounds__(PCG_NT) k_pcg1(PcgArgs a) {
               // of this iteration are, its direction is kept in memory of this thread's own
               const Tagged* w = t_z + 12 * (size_t)a.rcol[pbase + j] + prow;
               Tagged r = tag_ld(w);
-              for (int spin = 0; !tag_ok(r, (unsigned)k + 1u) && spin < PCG1_SPIN; ++spin) r = tag_ld(w);
+              for (int spin = 0; !tag_ok(r, (unsigned)k + 1u) && !late && spin < a.polls; ++spin) r = tag_ld(w);
               late |= !tag_ok(r, (unsigned)k + 1u);
               double* pm = a.pnb + (size_t)(pbase + j) * 12 + prow;
               v = dir(tag_val(r), beta, *pm);
@@ -1551,9 +1551,12 @@ __global__ void __launch_bounds__(PCG_NT) k_pcg1(PcgArgs a) {
   }
   for (int k = 0;; ++k) {
     // ---- A_k: r.r (warp 0) and r.z (warp 1) of the scene ----
+    // one answer a warp: a product warp may be giving up while it is read, and a gather wants
+    // all lanes
+    const bool gone = __any_sync(0xffffffffu, s_abort != 0);
     double sl[PCG1_G];
-    if (warp == 0 && !s_abort) {
-      if (!sum_gather(my_box + ng, ng, (unsigned)k + 1u, sl)) s_abort = 1;
+    if (warp == 0 && !gone) {
+      if (!sum_gather(my_box + ng, ng, (unsigned)k + 1u, sl, a.polls)) s_abort = 1;
       const double rr = sum_form(sl, ng);
       if (lane == 0) {
         bool conv;
@@ -1568,11 +1571,11 @@ __global__ void __launch_bounds__(PCG_NT) k_pcg1(PcgArgs a) {
         if (owner && stop) {
           a.sc_iters[sc] = k;
           atomicMax(&a.out[1], k);
-          if (!conv) a.out[0] = ABD_ERR_PCG_NOCONV;
+          if (!conv) atomicMax(a.out, (int)ABD_ERR_PCG_NOCONV);
         }
       }
-    } else if (warp == 1 && !s_abort) {
-      if (!sum_gather(my_box + 2 * ng, ng, (unsigned)k + 1u, sl)) s_abort = 1;
+    } else if (warp == 1 && !gone) {
+      if (!sum_gather(my_box + 2 * ng, ng, (unsigned)k + 1u, sl, a.polls)) s_abort = 1;
       rz_prev = rz;
       rz = sum_form(sl, ng);
       if (lane == 0) s_beta = k == 0 ? 0.0 : rz / rz_prev;
@@ -1603,7 +1606,7 @@ __global__ void __launch_bounds__(PCG_NT) k_pcg1(PcgArgs a) {
       send(0, t, (unsigned)k + 1u, threadIdx.x, PCG1_ROWT);
     }
     if (warp == 1) {
-      if (!sum_gather(my_box, ng, (unsigned)k + 1u, sl)) s_abort = 1;
+      if (!sum_gather(my_box, ng, (unsigned)k + 1u, sl, a.polls)) s_abort = 1;
       const double pq = sum_form(sl, ng);
       if (lane == 0) s_alpha = rz / pq;
     }
@@ -1626,7 +1629,7 @@ __global__ void __launch_bounds__(PCG_NT) k_pcg1(PcgArgs a) {
     }
     publish_rr_rz(d0, d1, (unsigned)k + 2u);
   }
-  if (threadIdx.x == 0 && s_abort) a.out[0] = ABD_ERR_CUDA;
+  if (threadIdx.x == 0 && s_abort) atomicMax(a.out, (int)ABD_ERR_CUDA);  // above what other scenes report
   if (mine) {
     a.x[idx] = x_r;
     a.dq[idx] = -x_r;
@@ -2258,6 +2261,7 @@ int pcg_solve(const Geo& g, PairSet& S, NewtonBufs& B, const SolveOpts& o, const
   a.slots = B.slots.p;
   a.pnb = B.pnb.p;
   a.sc_box = B.sc_box.p;
+  a.polls = B.polls;
   void* args[] = {&a};
   const void* kern = one ? (void*)k_pcg1 : (void*)k_pcg;
   if (run_pcg) KLAUNCH(K_PCG, s, CK(cudaLaunchCooperativeKernel(kern, dim3(grid), dim3(PCG_NT), args, 0, s)));

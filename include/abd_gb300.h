@@ -165,6 +165,10 @@ int abd_get_counts(abd_handle* h, int* n_bodies, int* n_vertices, int* n_edges, 
  * abd_get_iter, of every scene for abd_set_iter. */
 int abd_get_iter(abd_handle* h);
 int abd_set_iter(abd_handle* h, int iter);
+/* Polls of a value of another CTA after which the handle's CG gives up with ABD_ERR_CUDA instead of
+ * waiting on (default 2^21, a second or two; results do not depend on it). The next call on the
+ * handle is as good as any. For tests of that path. */
+int abd_set_poll_limit(abd_handle* h, int polls);
 /* Friction coefficient of the handle (config "mu"), e.g. between differentiated rollouts. */
 int abd_set_friction(abd_handle* h, double mu);
 int abd_get_friction(abd_handle* h, double* mu);
