@@ -2156,7 +2156,8 @@ int pcg_solve(const Geo& g, PairSet& S, NewtonBufs& B, const SolveOpts& o, const
   int nb = g.nb, ns = g.ns;
   B.status.ensure(4);
   if (!B.h_int) CK(cudaMallocHost(&B.h_int, 16 * sizeof(int)));
-  CK(cudaMemsetAsync(B.status.p, 0, 4 * sizeof(int), s));
+  // status, iterations, kept blocks (those of the rows copied: they stand with the rows)
+  CK(cudaMemsetAsync(B.status.p, 0, (o.same_system ? 2 : 4) * sizeof(int), s));
   B.x.ensure(12 * (size_t)nb);
   B.r.ensure(12 * (size_t)nb);
   B.z.ensure(12 * (size_t)nb);
@@ -2318,7 +2319,7 @@ int pcg_solve(const Geo& g, PairSet& S, NewtonBufs& B, const SolveOpts& o, const
   if (*status == ABD_ERR_CUDA) throw CudaError{cudaErrorLaunchTimeout, "pcg: the sums of a group did not arrive"};
   // per iteration: the kept blocks once (1152 B each) and ~6 vector streams
   prof_work(K_PCG, B.h_int[1], B.h_int[1] * (1152.0 * B.h_int[2] + 6 * 96.0 * nb) + 1152.0 * nb);
-  prof_work(K_BLOCK_INVERSE, 1, 2 * 1152.0 * B.h_int[2]);
+  if (!o.same_system) prof_work(K_BLOCK_INVERSE, 1, 2 * 1152.0 * B.h_int[2]);
   return B.h_int[1];
 }
 
