@@ -120,8 +120,6 @@ struct CullScratch {
   DBuf<float> vend;                     // float positions of each vertex at q and at the target
   DBuf<int> order, order_cnt;           // narrow-phase processing order of the overlaps
   DBuf<int> bin_cnt, bin_off, lst;
-  DBuf<long long> cand_cnt, cand_off;
-  DBuf<uint8_t> flags;
   DBuf<int> blk_a, blk_b, blk_a_off, blk_b_off;
   DBuf<int> vflag_cnt, vflag_off, stage_ov;
   DBuf<int4> stage_seg;
@@ -131,14 +129,12 @@ struct CullScratch {
   DBuf<unsigned long long> toi_key;     // 2 per scene: pt/ee, ground; the number of candidates
   DBuf<int2> toi_cand;                  // trajectory candidates left to the FP64 test
   DBuf<int> tmp_int;
-  DBuf<long long> tmp_ll;
   // autotuned narrow-phase variants (index into the step table; -1 = not tuned yet) of the
   // pair cull [0] and the CCD [1], and the times measured when tuning
   int autotune = 1;
   int narrow_variant[2] = {-1, -1};
   float narrow_ms[2][3] = {{0, 0, 0}, {0, 0, 0}};
   int* h_small = nullptr;               // pinned host scratch
-  long long* h_ll = nullptr;
   unsigned long long* h_toi = nullptr;
   int h_toi_cap = 0;
 };
@@ -194,8 +190,6 @@ inline void prof_work(int tag, double units, double bytes) {
 void scan_exclusive_int2(const int* in0, int* out0, int* tot0, const int* in1, int* out1, int* tot1, int n,
                          cudaStream_t s, DBuf<int>& tmp);
 void scan_exclusive_int(const int* in, int* out, int n, int* d_total, cudaStream_t s, DBuf<int>& tmp);
-void scan_exclusive_ll(const long long* in, long long* out, int n, long long* d_total, cudaStream_t s,
-                       DBuf<long long>& tmp);
 
 // ---------------- culling (cull.cu) ----------------
 void launch_project(const Geo& g, int which, double alpha, cudaStream_t s);
@@ -204,9 +198,9 @@ void launch_project(const Geo& g, int which, double alpha, cudaStream_t s);
 void cull(const Geo& g, const Params& P, int vtn, double alpha, CullScratch& cs, PairSet& out, double* toi_p,
           double* toi_g, cudaStream_t s);
 
-// Float boxes of the vertices, edges and faces, rounded outward, of X or of the trajectory from
-// Xq to X (cs.vbox / ebox / fbox), and the float positions of the vertices at Xq and X (cs.vend).
-void prim_boxes(const Geo& g, bool traj, CullScratch& cs, cudaStream_t s);
+// Float boxes of the vertices, edges and faces at X, rounded outward (cs.vbox / ebox / fbox), and the
+// float positions of the vertices at Xq and X (cs.vend).
+void prim_boxes(const Geo& g, CullScratch& cs, cudaStream_t s);
 void traj_floats(const Geo& g, CullScratch& cs, cudaStream_t s);
 
 // Line-search cull at q + alpha dq (per-scene steps of g) that reuses the overlaps and the

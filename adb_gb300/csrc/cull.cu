@@ -223,19 +223,16 @@ __global__ void k_ov_lower(int nnz, const int* row_ptr, const int* col, const in
 }
 
 // ---------------------------------------------------------------------------------
-// Float prefilter boxes of every primitive (outward rounded). Trajectory mode spans the
-// positions at q (Xq) and at the target (X).
-// Float boxes of the primitives (outward rounded). Vertices first, from their FP64
-// positions (at X, or the trajectory from Xq to X); edges and faces are then the float
-// unions of their vertices' boxes: rounding down (up) commutes with min (max), so
-// rd(min(a, b)) = min(rd a, rd b) and the result equals rounding the FP64 box, without
-// any FP64 min/max.
-__global__ void k_vert_boxes(Geo g, int traj, float* vb) {
+// Float prefilter boxes of every primitive (outward rounded). Vertices first, from their FP64
+// positions (here at X; k_project writes those of the culls, at X or of the trajectory from
+// Xq to X); edges and faces are then the float unions of their vertices' boxes: rounding down
+// (up) commutes with min (max), so rd(min(a, b)) = min(rd a, rd b) and the result equals
+// rounding the FP64 box, without any FP64 min/max.
+__global__ void k_vert_boxes(Geo g, float* vb) {
   int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= g.nv) return;
   d3 p = ldX(g.X, g.nv, t);
-  box b = traj ? box2(p, ldX(g.Xq, g.nv, t)) : box{p, p};
-  put_fbox(vb + 6 * t, b);
+  put_fbox(vb + 6 * t, box{p, p});
 }
 // Float positions (to nearest) of every vertex at q and at the target, for the FP32
 // certificates of the trajectories.
@@ -1601,9 +1598,9 @@ static void edge_face_boxes(const Geo& g, bool clusters, CullScratch& cs, cudaSt
   }
 }
 
-void prim_boxes(const Geo& g, bool traj, CullScratch& cs, cudaStream_t s) {
+void prim_boxes(const Geo& g, CullScratch& cs, cudaStream_t s) {
   cs.vbox.ensure(6 * (size_t)g.nv + 6);
-  if (g.nv > 0) KLAUNCH(K_PRIM_BOXES, s, k_vert_boxes<<<nblk(g.nv, 256), 256, 0, s>>>(g, traj ? 1 : 0, cs.vbox.p));
+  if (g.nv > 0) KLAUNCH(K_PRIM_BOXES, s, k_vert_boxes<<<nblk(g.nv, 256), 256, 0, s>>>(g, cs.vbox.p));
   edge_face_boxes(g, false, cs, s);
 }
 
@@ -1676,7 +1673,6 @@ void cull(const Geo& g_in, const Params& P, int vtn, double alpha, CullScratch& 
   const int nb = g.nb;
   if (!cs.h_small) {
     CK(cudaMallocHost(&cs.h_small, 64 * sizeof(int)));
-    CK(cudaMallocHost(&cs.h_ll, 8 * sizeof(long long)));
   }
   // 1. projection
   cs.vbox.ensure(6 * (size_t)g.nv + 6);
@@ -1903,7 +1899,6 @@ void vg_write(const Geo& g, const Params& P, CullScratch& cs, PairSet& S, int nv
 void vg_pairs(const Geo& g, const Params& P, CullScratch& cs, PairSet& S, cudaStream_t s) {
   if (!cs.h_small) {
     CK(cudaMallocHost(&cs.h_small, 64 * sizeof(int)));
-    CK(cudaMallocHost(&cs.h_ll, 8 * sizeof(long long)));
   }
   vg_count(g, P, cs, s);
   CK(cudaMemcpyAsync(cs.h_small + 5, cs.tmp_int.p + 5, sizeof(int), cudaMemcpyDeviceToHost, s));

@@ -146,12 +146,11 @@ struct Engine {
     cs.ovcull.release(); cs.ovcull_f.release(); cs.vbox.release(); cs.ebox.release(); cs.fbox.release(); cs.cbox.release();
     cs.order.release(); cs.order_cnt.release(); cs.vend.release(); cs.toi_cand.release();
     shw.release();
-    cs.bin_cnt.release(); cs.bin_off.release(); cs.lst.release(); cs.cand_cnt.release(); cs.cand_off.release();
-    cs.flags.release(); cs.blk_a.release(); cs.blk_b.release(); cs.blk_a_off.release(); cs.blk_b_off.release();
+    cs.bin_cnt.release(); cs.bin_off.release(); cs.lst.release();
+    cs.blk_a.release(); cs.blk_b.release(); cs.blk_a_off.release(); cs.blk_b_off.release();
     cs.vflag_cnt.release(); cs.vflag_off.release(); cs.stage_seg.release(); cs.stage_ov.release(); cs.vg_cnt.release();
-    cs.stage_key.release(); cs.stage_ty.release(); cs.toi_key.release(); cs.tmp_int.release(); cs.tmp_ll.release();
+    cs.stage_key.release(); cs.stage_ty.release(); cs.toi_key.release(); cs.tmp_int.release();
     if (cs.h_small) cudaFreeHost(cs.h_small);
-    if (cs.h_ll) cudaFreeHost(cs.h_ll);
     if (cs.h_toi) cudaFreeHost(cs.h_toi);
     nbufs.pt_c.release(); nbufs.ee_c.release(); nbufs.pt_seg.release(); nbufs.ee_seg.release();
     nbufs.ovr.release(); nbufs.has.release(); nbufs.off_pos.release(); nbufs.off_keys.release();

@@ -210,11 +210,4 @@ void scan_exclusive_int(const int* in, int* out, int n, int* d_total, cudaStream
   if (d_total && n <= 0) CK(cudaMemsetAsync(d_total, 0, sizeof(int), s));
 }
 
-void scan_exclusive_ll(const long long* in, long long* out, int n, long long* d_total, cudaStream_t s,
-                       DBuf<long long>& tmp) {
-  tmp.ensure(scan_scratch<long long>(n) + 8);
-  scan_rec<long long>(in, out, n, s, tmp.p, tmp.cap, d_total);
-  if (d_total && n <= 0) CK(cudaMemsetAsync(d_total, 0, sizeof(long long), s));
-}
-
 }  // namespace abd

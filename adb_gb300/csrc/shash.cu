@@ -691,7 +691,7 @@ void sh_cull(const Geo& g, const Params& P, const ShParams& H, int vtn, double a
   Q.thr = P.dhat * (sf * sf);
   if (!W.h_int) CK(cudaMallocHost(&W.h_int, 8 * sizeof(int)));
   const bool do_pt = P.pt && g.nv && g.nf, do_ee = P.ee && g.ne;
-  if (do_pt || do_ee) prim_boxes(g, false, cs, s);
+  if (do_pt || do_ee) prim_boxes(g, cs, s);
   // PT: vertices registered, triangles query; EE: edges registered, edges of the higher body
   // query
   const int npt = do_pt ? sh_pairs<0>(g, H, Q, W, cs, W.pt_keys, s) : 0;
