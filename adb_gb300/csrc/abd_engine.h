@@ -234,7 +234,8 @@ struct ShCells {
 };
 struct ShTable {
   DBuf<ShCells> cells;       // cell ranges of the registered primitives
-  DBuf<int> cnt, beg, cur;   // per bucket: entries (0 where unused), segment, write position
+  DBuf<int> cnt, cur;        // per bucket: entries (0 where unused), write position (once filled, the
+                             // end of its segment)
   DBuf<int> used, ctl;       // buckets in use; [0] their number, [1] entries, [2..3] cells in all
   DBuf<int2> ent;            // (primitive, body) by bucket
   unsigned long long h_tot = 0;

@@ -159,13 +159,11 @@ __global__ void k_bucket_count(ShGrid G, int n, const ShCells* cells, int* cnt, 
     if (atomicAdd(&cnt[b], 1) == 0) used[atomicAdd(&ctl[0], 1)] = (int)b;
   });
 }
-__global__ void k_bucket_alloc(int* ctl, const int* used, const int* cnt, int* beg, int* cur) {
+__global__ void k_bucket_alloc(int* ctl, const int* used, const int* cnt, int* cur) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= ctl[0]) return;
   const int b = used[i];
-  const int o = atomicAdd(&ctl[1], cnt[b]);
-  beg[b] = o;
-  cur[b] = o;
+  cur[b] = atomicAdd(&ctl[1], cnt[b]);
 }
 __global__ void k_bucket_fill(Geo g, ShGrid G, int kind, int n, const ShCells* cells, int* cur, int2* ent) {
   const int id = blockIdx.x * blockDim.x + threadIdx.x;
@@ -177,7 +175,7 @@ __global__ void k_bucket_fill(Geo g, ShGrid G, int kind, int n, const ShCells* c
 struct ShQuery {
   ShGrid G;
   const ShCells *rcells, *qcells;   // of the registered and of the query primitives
-  const int *cnt, *beg;             // buckets
+  const int *cnt, *end;             // buckets: entries, end of the segment
   const int2* ent;                  // (primitive, body)
   double qd;     // query box growth (d_sqrt * safe_factor); 0 for trajectories
   float qd_f;    // the same, rounded up past every rounding of the FP64 distance
@@ -267,7 +265,7 @@ __global__ void __launch_bounds__(128) k_sh_query(Geo g, ShQuery Q, int qbeg, in
         const unsigned b = sh_hash(i, j, k, Q.G.bits);
         const int n = Q.cnt[b];
         if (n == 0) continue;  // an unused bucket has no segment
-        const int2* ent = Q.ent + Q.beg[b];
+        const int2* ent = Q.ent + (Q.end[b] - n);
         for (int t0 = 0; t0 < n; t0 += 32) {
           bool take = false;
           int id = 0;
@@ -549,7 +547,7 @@ ShGrid grid_of(const ShParams& H) { return ShGrid{H.min_xyz, H.dx, H.bits}; }
 }  // namespace
 
 void ShScratch::release() {
-  tab.cells.release(); tab.cnt.release(); tab.beg.release(); tab.cur.release(); tab.used.release(); tab.ctl.release();
+  tab.cells.release(); tab.cnt.release(); tab.cur.release(); tab.used.release(); tab.ctl.release();
   tab.ent.release(); qcells.release(); cand.release(); n.release(); scan_i.release(); flag.release(); pos.release();
   pt_keys.release(); ee_keys.release(); bp_all.release(); tkeys.release(); bp_pt.release(); bp_ee.release();
   if (h_int) cudaFreeHost(h_int);
@@ -568,7 +566,6 @@ static void sh_register(const Geo& g, const ShParams& H, int kind, int n, int tr
   T.ctl.ensure(4);
   if (T.cnt.cap < nbuckets) {
     T.cnt.ensure(nbuckets);
-    T.beg.ensure(nbuckets);
     T.cur.ensure(nbuckets);
     CK(cudaMemsetAsync(T.cnt.p, 0, T.cnt.cap * sizeof(int), s));
   } else {
@@ -587,7 +584,7 @@ static void sh_register(const Geo& g, const ShParams& H, int kind, int n, int tr
   T.ent.ensure((size_t)tot);
   KLAUNCH(K_SH, s, k_bucket_count<<<nblk(n, 256), 256, 0, s>>>(G, n, T.cells.p, T.cnt.p, T.used.p, T.ctl.p));
   const long long most = (long long)std::min((size_t)tot, nbuckets);
-  KLAUNCH(K_SH, s, k_bucket_alloc<<<nblk(most, 256), 256, 0, s>>>(T.ctl.p, T.used.p, T.cnt.p, T.beg.p, T.cur.p));
+  KLAUNCH(K_SH, s, k_bucket_alloc<<<nblk(most, 256), 256, 0, s>>>(T.ctl.p, T.used.p, T.cnt.p, T.cur.p));
   KLAUNCH(K_SH, s, k_bucket_fill<<<nblk(n, 256), 256, 0, s>>>(g, G, kind, n, T.cells.p, T.cur.p, T.ent.p));
 }
 
@@ -606,7 +603,7 @@ static void sh_prepare(const Geo& g, const ShParams& H, int kind, int traj, ShSc
   Q.rcells = W.tab.cells.p;
   Q.qcells = W.qcells.p;
   Q.cnt = W.tab.cnt.p;
-  Q.beg = W.tab.beg.p;
+  Q.end = W.tab.cur.p;  // once filled
   Q.ent = W.tab.ent.p;
   Q.vb = cs.vbox.p;
   Q.eb = cs.ebox.p;

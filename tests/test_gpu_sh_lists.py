@@ -30,7 +30,7 @@ def test_memory_of_a_small_handle(gpu_lib):
     keep = [handle()]
     before = used()
     keep += [handle() for _ in range(16)]
-    # the bucket table has 3 MB; the list alone was 16 MB
+    # the bucket table has 2 MB; the list alone was 16 MB
     assert (used() - before) / 16 < 9 << 20
 
 
@@ -79,3 +79,19 @@ def test_runs_grow_again(gpu_lib):
     assert few > 0 and all(np.array_equal(a, b) for a, b in zip(alone, sets))
     # 57 600 edges past the pair: at most a doubling run each, of two launches, for log2(61440)
     assert launches <= few + 2 * 20
+
+
+def test_memory_of_the_buckets(gpu_lib):
+    """2^24 buckets (xyz_bits 8) of 8 bytes."""
+    torch = pytest.importorskip("torch")
+    from adb_gb300.abd import ABD
+    sc = S.cube_stack(2, gap=0.01, seed=1)
+    cfg = dataclasses.replace(S.workload_config("cubes"), iaabb=0, sh_bits=8)
+    ABD(sc, cfg).cull(1, sc.q0)
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    sim = ABD(sc, cfg)
+    sim.cull(1, sc.q0)
+    torch.cuda.synchronize()
+    # two arrays, by the steps in which buffers grow 66 MB each (a third one would make 198)
+    assert before - torch.cuda.mem_get_info()[0] < 160 << 20
