@@ -76,7 +76,9 @@ __host__ __device__ inline bool scene_on(const Geo& g, int body) {
 }
 
 // Bodies from which a scene keeps the forms of the pair terms whose rounding its truncated CG
-// amplifies (newton.cu).
+// amplifies (newton.cu). Both forms are as accurate; what differs is how far other rounding moves a
+// frame whose CG stops at a residual: of ten parts of the pile, by up to 2.4e-11 of its velocities
+// at 500 bodies and fewer, by up to 2.8e-9 at 700 and more.
 constexpr int BIG_SCENE = 512;
 __device__ inline bool big_scene(const Geo& g, int body) {
   return g.scene_end[body] - g.scene_beg[body] >= BIG_SCENE;

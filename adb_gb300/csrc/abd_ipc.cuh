@@ -347,8 +347,9 @@ DEV bool jacobi_f32_start(const double (&S)[N][N], double (&Q)[N][N], float (&v)
 // left, the projection in this basis is max(L, 0) + E o K, K_ij = (max(l_i, 0) - max(l_j, 0)) /
 // (l_i - l_j) (1 for two positive eigenvalues, 0 for two negative ones), up to E^2 over the
 // smaller eigenvalues; the test keeps that below 1e-17 of the norm. After one sweep E is about
-// 1e-14 of the norm, so FP32 has the correction to 1e-20 of it, with the FP32 eigenvectors, and the
-// second FP64 sweep (ten rotations of a 5x5, a third of the projection) is not needed.
+// 1e-14 of the norm, so FP32 has the correction to 1e-20 of it (to 1e-45, the least FP32
+// number, in matrices below 1e-25), with the FP32 eigenvectors, and the second FP64 sweep (ten
+// rotations of a 5x5, a third of the projection) is not needed.
 template <int N, bool FIRST = false>
 DEV bool psd_project_small(double (&S)[N][N]) {
   double A[N][N], V[N][N];

@@ -491,8 +491,11 @@ constexpr int REC_CAP = 2048;  // candidates of one overlap kept in shared memor
 // less often; a shorter one leaves shared memory for more CTAs per SM. The result does not
 // depend on STEP (candidates are sorted by key before they are written, TOIs are
 // min-reduced), so the autotuner picks among these variants by time: pair cull (mode 0)
-// 16 / 8 / 48, CCD (mode 2) 24 / 36 / 64; the defaults are the middle ones (with
-// a phase per sub-problem, columns: 237 us with 16 at 3 CTAs per SM, 212 us with 8 at 4).
+// 16 / 8 / 48, CCD (mode 2) 24 / 36 / 64. No variant wins everywhere (medians of seven
+// handles, us): 1024 bodies of the pile 153 / 193 / 149 and 144 / 145 / 114, 64 of them
+// 31 / 29 / 28 and 22 / 17 / 17, 256 columns 195 / 156 / 230 and 78 / 68 / 112, a chain of 200
+// 25 / 24 / 24 and 24 / 19 / 20. The middle ones are the defaults: the best of the small scenes,
+// which are the ones that are not tuned, and within a third of the best elsewhere.
 constexpr int kNarrowVariants = 3;
 constexpr int kNarrowStep[2][kNarrowVariants] = {{16, 8, 48}, {24, 36, 64}};
 constexpr int kNarrowDefault = 1;

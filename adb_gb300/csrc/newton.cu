@@ -1298,7 +1298,7 @@ __global__ void __launch_bounds__(PCG_NT) k_pcg(PcgArgs a) {
 //    bodies hold some 28 blocks: 10 warps instead of 16 half empty ones). The product's warps
 //    wait for z while the row warps reduce the scalars;
 //  - r.r and r.z share their reduction steps.
-// 1024 bodies of the pile, 359 iterations: 4.38 -> 3.40 ms a solve (9.5 us an iteration: two
+// 1024 bodies of the pile, 359 iterations: 4.38 -> 3.08 ms a solve (8.6 us an iteration: two
 // exchanges of about 1.2 us, the product 1.5 us, the rest FP64 chains of the reductions).
 constexpr int PCG1_NC = 2;     // row blocks per part kept in registers
 constexpr int PCG1_G = 5;      // groups of a scene per lane of an exchange
